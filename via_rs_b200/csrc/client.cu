@@ -16,11 +16,12 @@
 //             to plaintext mod p (round(p * c / q4), c centred).
 //
 // The PRG stream of a query is sequential (rejection sampling): its SHAKE256
-// blocks are computed in parallel beforehand, one warp walks it 32 draws at a
-// time, and the inner products run one CTA per LWE.
+// blocks are computed in parallel beforehand, one CTA walks it an LWE's mask at
+// a time (walk_mask), and the inner products run one CTA per LWE.
 #include <cstring>
 #include <memory>
 #include <string>
+#include <type_traits>
 #include <vector>
 
 #include "gadget.cuh"
@@ -63,6 +64,57 @@ __global__ void k_client_blocks(const uint8_t* __restrict__ seeds, int seed_len,
   for (int l = 0; l < RATE_LANES; ++l) dst[l] = out[l];
 }
 
+__device__ __forceinline__ i64 error_value(int err_kind, i64 err_bound, u64 x) {
+  return err_kind == 0 ? (x == 0 ? 0 : (x == 1 ? 1 : -1)) : (i64)x - err_bound;
+}
+
+// One CTA per query: LWE by LWE, the mask by a parallel scan of its candidates
+// (walk_mask, all limbs' draws nb bytes) and then the error's draws by thread 0,
+// with the outputs of k_client_walk. Flag 2 where the scan could not decide.
+// Latency-bound, an LWE after another: the warp walk of k_client_walk took
+// 8184 us for 24 queries of 40 LWEs (paper preset).
+__global__ void __launch_bounds__(WALK_THREADS) k_client_walk_scan(const u64* __restrict__ blocks, int nblk,
+                                                                   int n_lwe, int n1, u64 lwe_len, WalkLimbs W,
+                                                                   Draw D, int err_kind, i64 err_bound,
+                                                                   u64* __restrict__ out, i64* __restrict__ errs,
+                                                                   int* __restrict__ flag) {
+  __shared__ WalkShared sh;
+  __shared__ u64 s_pos;
+  const size_t q = blockIdx.x;
+  const u64* words = blocks + q * nblk * RATE_LANES;
+  const u64 avail = (u64)nblk * SHAKE_RATE;
+  u64 pos = 0;
+  for (int j = 0; j < n_lwe; ++j) {
+    const long used = walk_mask(words, avail, pos, W, n1, out + (q * n_lwe + j) * lwe_len, sh);
+    if (used == WALK_UNDECIDED) {
+      if (threadIdx.x == 0) atomicMax(flag, 2);
+      return;
+    }
+    pos += (u64)used * W.nb;
+    if (threadIdx.x == 0) {
+      int attempt = 0;
+      u64 x = 0;
+      bool ok = false;
+      for (; attempt < 64 && !ok && pos + D.nbytes[2] <= avail; ++attempt) {
+        x = 0;
+        for (int b = 0; b < D.nbytes[2]; ++b, ++pos)
+          x |= (u64)((words[pos >> 3] >> (8 * (pos & 7))) & 0xFF) << (8 * b);
+        x &= D.mask[2];
+        ok = x < D.bound[2];
+      }
+      if (!ok) atomicMax(flag, 2);  // the stream's end or 64 rejections: the general walk decides
+      errs[q * n_lwe + j] = error_value(err_kind, err_bound, x);
+      s_pos = ok ? pos : ~(u64)0;
+    }
+    __syncthreads();
+    pos = s_pos;
+    __syncthreads();
+    if (pos == ~(u64)0) return;
+  }
+}
+
+// The general walk, for limbs whose draws take different numbers of bytes and
+// for streams the scan leaves undecided.
 // One warp per query walks its stream through uniform_below (prg.rs), writing
 // every LWE's mask ([nl][n1], limb-major) into `out` and its error sample
 // (centred) into errs[q][lwe]. err_kind 0: ternary (draw r in [0,3): 0, 1,
@@ -138,7 +190,7 @@ __global__ void k_client_walk(const u64* __restrict__ blocks, const uint8_t* __r
       if (which < 2) {
         out[((size_t)q * n_lwe + j) * lwe_len + (size_t)l * n1 + k] = x;
       } else {
-        errs[(size_t)q * n_lwe + j] = err_kind == 0 ? (x == 0 ? 0 : (x == 1 ? 1 : -1)) : (i64)x - err_bound;
+        errs[(size_t)q * n_lwe + j] = error_value(err_kind, err_bound, x);
       }
     }
     if (rej) {
@@ -165,19 +217,23 @@ __global__ void __launch_bounds__(256) k_client_body(u64* __restrict__ out, cons
                                                      int n1, int nl, u64 lwe_len, DevMod m0, DevMod m1) {
   const long lw = blockIdx.x;  // q * n_lwe + j
   u64* lwe = out + (size_t)lw * lwe_len;
-  __shared__ u64 part[2][256][2];
+  __shared__ u64 part[2][8];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   for (int l = 0; l < nl; ++l) {
+    const DevMod& m = l ? m1 : m0;
     Acc128 acc{0, 0};
     for (int i = threadIdx.x; i < n1; i += blockDim.x) mac128(acc, lwe[(size_t)l * n1 + i], sk1[(size_t)l * n1 + i]);
-    part[l][threadIdx.x][0] = acc.lo;
-    part[l][threadIdx.x][1] = acc.hi;
+    u64 r = reduce128(acc.hi, acc.lo, m);
+#pragma unroll
+    for (int d = 16; d; d >>= 1) r = addmod(r, __shfl_xor_sync(0xffffffffu, r, d), m.q);
+    if (lane == 0) part[l][warp] = r;
   }
   __syncthreads();
   if (threadIdx.x < nl) {
     const int l = threadIdx.x;
     const DevMod& m = l ? m1 : m0;
     u64 r = 0;
-    for (int t = 0; t < (int)blockDim.x; ++t) r = addmod(r, reduce128(part[l][t][1], part[l][t][0], m), m.q);
+    for (int t = 0; t < 8; ++t) r = addmod(r, part[l][t], m.q);
     const i64 e = errs[lw];
     const u64 ev = e >= 0 ? reduce64((u64)e, m) : (m.q - reduce64((u64)(-e), m)) % m.q;
     r = addmod(addmod(r, ev, m.q), msgs[(size_t)lw * nl + l], m.q);
@@ -185,25 +241,42 @@ __global__ void __launch_bounds__(256) k_client_body(u64* __restrict__ out, cons
   }
 }
 
-// One CTA per answer, n2 threads: decrypt_asymmetric and decode.
+// One CTA per answer, n2 threads: decrypt_asymmetric and decode. NARROW (mask and
+// key words below 2^32, n2 of their products below 2^64): the negacyclic product's sums are plain
+// 64-bit multiply-adds of 32-bit words. Latency-bound: 24 answers of degree 512
+// took 51 us with 128-bit sums.
+template <bool NARROW>
 __global__ void k_client_recover(const u64* __restrict__ masks, const u64* __restrict__ bodies,
                                  const u64* __restrict__ sk2, int n2, DevMod m3, u64 q4, u64 p,
                                  u64* __restrict__ out) {
   extern __shared__ u64 sh[];
-  u64* a = sh;
-  u64* s = sh + n2;
+  typedef typename std::conditional<NARROW, u32, u64>::type word;
+  word* a = reinterpret_cast<word*>(sh);
+  word* s = a + n2;
   const long c = blockIdx.x;
   for (int i = threadIdx.x; i < n2; i += blockDim.x) {
-    a[i] = masks[(size_t)c * n2 + i];
-    s[i] = sk2[i];
+    a[i] = (word)masks[(size_t)c * n2 + i];
+    s[i] = (word)sk2[i];
   }
   __syncthreads();
   const u64 q3 = m3.q;
   for (int t = threadIdx.x; t < n2; t += blockDim.x) {
-    Acc128 pos{0, 0}, neg{0, 0};
-    for (int i = 0; i <= t; ++i) mac128(pos, a[i], s[t - i]);
-    for (int i = t + 1; i < n2; ++i) mac128(neg, a[i], s[n2 + t - i]);
-    const u64 prod = submod(reduce128(pos.hi, pos.lo, m3), reduce128(neg.hi, neg.lo, m3), q3);
+    u64 prod;
+    if constexpr (NARROW) {
+      u64 pos = 0, neg = 0;
+#pragma unroll 8
+      for (int i = 0; i < n2; ++i) {
+        const u64 x = (u64)a[i] * s[(t - i) & (n2 - 1)];
+        pos += i <= t ? x : 0;
+        neg += i <= t ? 0 : x;
+      }
+      prod = submod(reduce64(pos, m3), reduce64(neg, m3), q3);
+    } else {
+      Acc128 pos{0, 0}, neg{0, 0};
+      for (int i = 0; i <= t; ++i) mac128(pos, a[i], s[t - i]);
+      for (int i = t + 1; i < n2; ++i) mac128(neg, a[i], s[n2 + t - i]);
+      prod = submod(reduce128(pos.hi, pos.lo, m3), reduce128(neg.hi, neg.lo, m3), q3);
+    }
     // round(prod * q4 / q3) mod q4 (prod in [0, q3)).
     const u128 v = ((u128)prod * q4 + q3 / 2) / q3;
     const u64 sw = (u64)(v % q4);
@@ -247,6 +320,7 @@ struct Client {
   int device = 0;
   cudaStream_t stream = nullptr;
   DevBuf sk1, sk2;
+  u64 sk2_top = 0;  // the or of sk2's words, plus one
   int err_kind = 0;
   i64 err_bound = 1;
   ~Client() {
@@ -309,10 +383,10 @@ void make_queries(via_client* c, const uint64_t* indices, uint64_t count, const 
       }
   }
   const Draw D = make_draw(p, c->err_kind == 0 ? 3 : (u64)(2 * c->err_bound + 1));
-  // Every draw accepted, plus 2% and two blocks for rejections (more are made on the fly).
-  const u64 per_lwe = (u64)n1 * (D.nbytes[0] + (nl == 2 ? D.nbytes[1] : 0)) + D.nbytes[2];
-  const u64 need = per_lwe * n_lwe;
-  const int nblk = (int)((need + need / 50) / SHAKE_RATE + 2);
+  // Blocks for every draw and its expected rejections (more are made on the fly).
+  double need = walk_bytes((double)n_lwe, D.bound[2], D.nbytes[2]);
+  for (int l = 0; l < nl; ++l) need += walk_bytes((double)n1 * n_lwe, D.bound[l], D.nbytes[l]);
+  const int nblk = (int)((need + WALK_V * 8) / SHAKE_RATE + 2);
   DevBuf d_seeds(((size_t)count * seed_len + 7) / 8), d_blocks((size_t)count * nblk * RATE_LANES),
       d_errs((size_t)count * n_lwe), d_msgs(msgs.size()), d_flag(1);
   VIA_CUDA(cudaMemsetAsync(d_flag.p, 0, 8, st));
@@ -322,17 +396,28 @@ void make_queries(via_client* c, const uint64_t* indices, uint64_t count, const 
   k_client_blocks<<<(unsigned)((nb + 127) / 128), 128, 0, st>>>(reinterpret_cast<const uint8_t*>(d_seeds.p),
                                                                 (int)seed_len, (int)count, nblk, d_blocks.p);
   VIA_LAUNCHED();
-  k_client_walk<<<(unsigned)((count + 3) / 4), 128, 0, st>>>(
-      d_blocks.p, reinterpret_cast<const uint8_t*>(d_seeds.p), (int)seed_len, (int)count, nblk, n_lwe, n1, nl, ll, D,
-      c->err_kind, c->err_bound, d_out, reinterpret_cast<i64*>(d_errs.p), reinterpret_cast<int*>(d_flag.p));
-  VIA_LAUNCHED();
   const DevMod m0 = make_devmod(p.q1_0), m1 = make_devmod(p.q1_1 ? p.q1_1 : p.q1_0);
-  k_client_body<<<(unsigned)(count * n_lwe), 256, 0, st>>>(d_out, c->sk1.p, reinterpret_cast<const i64*>(d_errs.p),
-                                                           d_msgs.p, n1, nl, ll, m0, m1);
-  VIA_LAUNCHED();
   int flag = 0;
-  VIA_CUDA(cudaMemcpyAsync(&flag, d_flag.p, sizeof(int), cudaMemcpyDeviceToHost, st));
-  VIA_CUDA(cudaStreamSynchronize(st));  // the temporaries are freed on return
+  int* d_f = reinterpret_cast<int*>(d_flag.p);
+  i64* errs = reinterpret_cast<i64*>(d_errs.p);
+  bool scan = nl == 1 || D.nbytes[0] == D.nbytes[1];
+  for (;; scan = false) {
+    if (scan)
+      k_client_walk_scan<<<(unsigned)count, WALK_THREADS, 0, st>>>(
+          d_blocks.p, nblk, n_lwe, n1, ll, WalkLimbs{{D.bound[0], D.bound[1]}, {D.mask[0], D.mask[1]}, D.nbytes[0], nl}, D,
+          c->err_kind, c->err_bound, d_out, errs, d_f);
+    else
+      k_client_walk<<<(unsigned)((count + 3) / 4), 128, 0, st>>>(
+          d_blocks.p, reinterpret_cast<const uint8_t*>(d_seeds.p), (int)seed_len, (int)count, nblk, n_lwe, n1, nl, ll,
+          D, c->err_kind, c->err_bound, d_out, errs, d_f);
+    VIA_LAUNCHED();
+    k_client_body<<<(unsigned)(count * n_lwe), 256, 0, st>>>(d_out, c->sk1.p, errs, d_msgs.p, n1, nl, ll, m0, m1);
+    VIA_LAUNCHED();
+    VIA_CUDA(cudaMemcpyAsync(&flag, d_flag.p, sizeof(int), cudaMemcpyDeviceToHost, st));
+    VIA_CUDA(cudaStreamSynchronize(st));  // the temporaries are freed on return
+    if (flag != 2) break;
+    VIA_CUDA(cudaMemsetAsync(d_flag.p, 0, 8, st));
+  }
   if (flag) throw ApiErr(VIA_ERR_INVALID_PRG_SEED, "client query: a PRG stream rejected 64 draws in a row");
 }
 
@@ -364,6 +449,8 @@ via_status via_client_create(const via_params* params, const uint64_t* sk1, cons
     const int nl = params->q1_1 ? 2 : 1;
     c->sk1.alloc((size_t)nl * params->n1);
     c->sk2.alloc(params->n2);
+    for (u32 i = 0; i < params->n2; ++i) c->sk2_top |= sk2[i];
+    c->sk2_top += 1;
     VIA_CUDA(cudaMemcpy(c->sk1.p, sk1, c->sk1.n * 8, cudaMemcpyHostToDevice));
     VIA_CUDA(cudaMemcpy(c->sk2.p, sk2, c->sk2.n * 8, cudaMemcpyHostToDevice));
     *out = c.release();
@@ -405,8 +492,18 @@ via_status via_client_recover(via_client* c, const uint64_t* masks, const uint64
     VIA_CUDA(cudaMemcpyAsync(dm.p, masks, len * 8, cudaMemcpyHostToDevice, c->stream));
     VIA_CUDA(cudaMemcpyAsync(db.p, bodies, len * 8, cudaMemcpyHostToDevice, c->stream));
     const int threads = (int)std::min<u64>(p.n2, 1024);
-    k_client_recover<<<(unsigned)count, threads, 2 * p.n2 * 8, c->stream>>>(dm.p, db.p, c->sk2.p, (int)p.n2,
-                                                                            make_devmod(p.q3), p.q4, p.p, dout.p);
+    // The caller's residues are held to 32 bits here, not to q3: any value that
+    // does not fit takes the 128-bit sums.
+    u64 top = p.q3;
+    for (size_t i = 0; i < len; ++i) top |= masks[i];
+    const bool narrow = (top >> 32) == 0 && c->sk2_top <= ((u64)1 << 32) &&
+                        (u128)top * c->sk2_top * p.n2 < ((u128)1 << 64);
+    if (narrow)
+      k_client_recover<true><<<(unsigned)count, threads, 2 * p.n2 * 4, c->stream>>>(
+          dm.p, db.p, c->sk2.p, (int)p.n2, make_devmod(p.q3), p.q4, p.p, dout.p);
+    else
+      k_client_recover<false><<<(unsigned)count, threads, 2 * p.n2 * 8, c->stream>>>(
+          dm.p, db.p, c->sk2.p, (int)p.n2, make_devmod(p.q3), p.q4, p.p, dout.p);
     VIA_LAUNCHED();
     VIA_CUDA(cudaMemcpyAsync(out, dout.p, len * 8, cudaMemcpyDeviceToHost, c->stream));
     VIA_CUDA(cudaStreamSynchronize(c->stream));

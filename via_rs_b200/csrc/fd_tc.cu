@@ -623,7 +623,14 @@ Tiling tiling(int nq, const FdTile& tile, bool packed4) {
     T.N = fd_round_up((2 * nq + T.n_ct - 1) / T.n_ct, cap == 24 ? 8 : 16);
     T.Np = fd_round_up(FD_LIMBS * T.N, 16);
     T.stages = tile.stages ? tile.stages : 3;
-    T.order = tile.order;
+    // The default tile (all fields zero) walks one or two c-tiles slot-major and
+    // three or more tile-major. Measured (paper preset): 64 queries, three tiles:
+    // 43.0 ms slot-major, 14.2 ms tile-major at 256 x 4096; 27.3 and 20.3 ms at
+    // 16 x 4096. 32 queries, two tiles: 7.3 ms slot-major, above 10.4 ms
+    // tile-major at 256 x 4096. The SMs of three or more tiles drift apart and
+    // miss each other's planes in L2; two stay together and share them.
+    const bool builtin = !tile.n_max && !tile.stages && !tile.order;
+    T.order = builtin ? (T.n_ct >= 3 ? 1 : 0) : tile.order;
     // Limb k's MMA writes columns [k N, k N + Np); the epilogue reads [0, 9 N).
     acc_cols = std::max(9 * T.N, 4 * T.N + T.Np);
   }

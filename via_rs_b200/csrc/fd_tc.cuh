@@ -49,7 +49,9 @@ constexpr int FD_CHUNK_P4 = 4 * FD_PLANE + FD_PACK4;   // 34816 bytes
 //  order  : 0 walks units slot-major (the c-tiles of one slot run on
 //           neighbouring SMs at the same time and share the slot's planes in
 //           L2); 1 walks them tile-major (one c-tile over every slot, then the next).
-// Zero fields take the built-in default (48 columns, 3 stages; 4 for one query).
+// Zero fields take the built-in default (48 columns, 3 stages; 4 for one query);
+// with all fields zero the order is the default's too: slot-major up to two
+// c-tiles, tile-major from three on.
 struct FdTile {
   int n_max = 0, stages = 0, order = 0;
 };

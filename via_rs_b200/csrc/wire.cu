@@ -12,8 +12,8 @@
 // per limb, limb 0 first (prim/sampling/prg.rs:108-206). The PRG's byte stream
 // is counter-mode, block b = SHAKE256(seed || le64(b))[0..136), so every block
 // is one Keccak-f[1600] permutation and the device computes all blocks of all
-// packets in parallel; one thread per packet then walks its stream through the
-// rejection sampler (an accepted draw consumes ceil(bitlen(q) / 8) bytes).
+// packets in parallel; one CTA per packet then takes its mask from the stream
+// (walk_mask; an accepted draw consumes ceil(bitlen(q) / 8) bytes).
 #include <cstring>
 #include <string>
 #include <vector>
@@ -44,11 +44,33 @@ struct Sampler {
   int nbytes[2];
 };
 
-// One thread per compressed packet: uniform_below over the packet's stream,
-// writing the mask polynomial of LWE lwe[pkt] ([nl][n1] limb-major) of `query`.
-// Blocks beyond the precomputed nblk (a run of rejections) are computed here.
+// The mask and the body of one compressed packet per CTA: LWE lwe[pkt] of `query`
+// ([nl][n1] limb-major, then nl body residues). err: 2 where walk_mask could not
+// decide. Latency-bound: a chunk of 4096 candidates is one pass of the paper
+// preset's mask, four of the secure preset's. Against one thread walking each
+// stream (k_prg_masks): 3412 us before, see WALK figures below, for 42 packets
+// of the paper preset.
+__global__ void __launch_bounds__(WALK_THREADS) k_prg_masks_scan(const u64* __restrict__ blocks,
+                                                                 const u64* __restrict__ bodies,
+                                                                 const int* __restrict__ lwe, int nblk, int n1,
+                                                                 u64 lwe_len, WalkLimbs W, u64* __restrict__ query,
+                                                                 int* __restrict__ err) {
+  __shared__ WalkShared sh;
+  const int pkt = blockIdx.x;
+  u64* out = query + (size_t)lwe[pkt] * lwe_len;
+  if (threadIdx.x < W.nl) out[(size_t)W.nl * n1 + threadIdx.x] = bodies[(size_t)pkt * W.nl + threadIdx.x];
+  const u64 avail = (u64)nblk * SHAKE_RATE;
+  const long used = walk_mask(blocks + (size_t)pkt * nblk * RATE_LANES, avail, 0, W, n1, out, sh);
+  if (used == WALK_UNDECIDED && threadIdx.x == 0) atomicMax(err, 2);
+}
+
+// The general walk, for limbs whose draws take different numbers of bytes and
+// for streams walk_mask leaves undecided. One thread per compressed packet:
+// uniform_below over the packet's stream, writing the mask polynomial of LWE
+// lwe[pkt] ([nl][n1] limb-major) and its body. Blocks beyond the precomputed
+// nblk (a run of rejections) are computed here.
 __global__ void k_prg_masks(const u64* __restrict__ blocks, const uint8_t* __restrict__ seeds,
-                            const int* __restrict__ lwe, int npkt, int nblk, int n1, int nl, u64 lwe_len, Sampler S,
+                            const u64* __restrict__ bodies, const int* __restrict__ lwe, int npkt, int nblk, int n1, int nl, u64 lwe_len, Sampler S,
                             u64* __restrict__ query, int* __restrict__ err) {
   const int pkt = blockIdx.x * blockDim.x + threadIdx.x;
   if (pkt >= npkt) return;
@@ -72,6 +94,7 @@ __global__ void k_prg_masks(const u64* __restrict__ blocks, const uint8_t* __res
     return (unsigned)((lane >> (8 * (o % 8))) & 0xFF);
   };
   u64* out = query + (size_t)lwe[pkt] * lwe_len;
+  for (int l = 0; l < nl; ++l) out[(size_t)nl * n1 + l] = bodies[(size_t)pkt * nl + l];
   for (int k = 0; k < n1; ++k)
     for (int l = 0; l < nl; ++l) {
       // q >= 2^(bits-1) accepts at least half of the draws, so 64 rejections in
@@ -104,33 +127,38 @@ u64 rd64(const uint8_t* p) {
   return v;
 }
 
-// Parses the packets into `query` (host, flat layout); compressed packets
-// leave their mask to the device and are listed in seeds / lwes.
-void parse_wire(const via_params& p, const uint8_t* wire, u64 len, u64* query, std::vector<uint8_t>& seeds,
-                std::vector<int>& lwes) {
+// A parsed wire query. Compressed packets leave their LWE to the device and are
+// listed in seeds / bodies / lwes; `flat` (the flat layout) is made when an
+// uncompressed packet comes.
+struct WireQuery {
+  std::vector<u64> flat, bodies;
+  std::vector<uint8_t> seeds;
+  std::vector<int> lwes;
+};
+
+void parse_wire(const via_params& p, const uint8_t* wire, u64 len, WireQuery& Q) {
   const u64 n_lwe = query_lwes(p), ll = lwe_len(p), nl = p.q1_1 ? 2 : 1;
   u64 off = 0;
   for (u64 w = 0; w < n_lwe; ++w) {
     if (off >= len) throw ApiErr(VIA_ERR_BUFFER_TOO_SHORT, "wire query: " + std::to_string(w) + " of " +
                                                                std::to_string(n_lwe) + " LWE packets present");
     const uint8_t tag = wire[off];
-    u64* dst = query + w * ll;
     if (tag == 0x00) {
       if (len - off < 9) throw ApiErr(VIA_ERR_BUFFER_TOO_SHORT, "wire query: truncated packet header");
       const u64 count = rd64(wire + off + 1);
       if (count != ll) throw ApiErr(VIA_ERR_DIM_MISMATCH, "wire query: uncompressed LWE length mismatch");
       if ((len - off - 9) / 8 < count) throw ApiErr(VIA_ERR_BUFFER_TOO_SHORT, "wire query: truncated LWE");
-      for (u64 i = 0; i < count; ++i) dst[i] = rd64(wire + off + 9 + 8 * i);
+      Q.flat.resize(n_lwe * ll);
+      std::memcpy(Q.flat.data() + w * ll, wire + off + 9, count * 8);  // little-endian words
       off += 9 + 8 * count;
     } else if (tag == 0x01) {
       if (len - off < 1 + SEED_LEN + 8) throw ApiErr(VIA_ERR_BUFFER_TOO_SHORT, "wire query: truncated packet header");
       const u64 count = rd64(wire + off + 1 + SEED_LEN);
       if (count != nl) throw ApiErr(VIA_ERR_DIM_MISMATCH, "wire query: compressed body length mismatch");
       if ((len - off - 1 - SEED_LEN - 8) / 8 < count) throw ApiErr(VIA_ERR_BUFFER_TOO_SHORT, "wire query: truncated body");
-      seeds.insert(seeds.end(), wire + off + 1, wire + off + 1 + SEED_LEN);
-      lwes.push_back((int)w);
-      std::memset(dst, 0, (size_t)ll * 8);
-      for (u64 i = 0; i < count; ++i) dst[nl * p.n1 + i] = rd64(wire + off + 1 + SEED_LEN + 8 + 8 * i);
+      Q.seeds.insert(Q.seeds.end(), wire + off + 1, wire + off + 1 + SEED_LEN);
+      Q.lwes.push_back((int)w);
+      for (u64 i = 0; i < count; ++i) Q.bodies.push_back(rd64(wire + off + 1 + SEED_LEN + 8 + 8 * i));
       off += 1 + SEED_LEN + 8 + 8 * count;
     } else {
       throw ApiErr(VIA_ERR_UNKNOWN_FORMAT_TAG, "wire query: unknown format tag " + std::to_string(tag));
@@ -155,39 +183,55 @@ Sampler make_sampler(const via_params& p) {
 // Decodes a wire query into the device buffer d_query (flat layout).
 void decode_to_device(Server& s, const uint8_t* wire, u64 len, u64* d_query, cudaStream_t st) {
   const via_params& p = s.prm;
-  const u64 n_lwe = query_lwes(p), ll = lwe_len(p);
+  const u64 ll = lwe_len(p);
   const int nl = p.q1_1 ? 2 : 1;
-  std::vector<u64> host(n_lwe * ll);
-  std::vector<uint8_t> seeds;
-  std::vector<int> lwes;
-  parse_wire(p, wire, len, host.data(), seeds, lwes);
-  VIA_CUDA(cudaMemcpyAsync(d_query, host.data(), host.size() * 8, cudaMemcpyHostToDevice, st));
-  const int npkt = (int)lwes.size();
-  if (npkt) {
-    const Sampler S = make_sampler(p);
-    const int nbytes = std::max(S.nbytes[0], S.nbytes[1]);
-    // Every draw accepted: n1 * nl draws; 1% and 2 blocks of margin for rejections
-    // (more are generated on the fly).
-    const u64 need = (u64)p.n1 * nl * nbytes;
-    const int nblk = (int)((need + need / 100) / SHAKE_RATE + 2);
-    DevBuf d_seeds((seeds.size() + 7) / 8), d_lwes((lwes.size() + 1) / 2), d_blocks((size_t)npkt * nblk * RATE_LANES),
-        d_err(1);
-    VIA_CUDA(cudaMemsetAsync(d_err.p, 0, 8, st));
-    VIA_CUDA(cudaMemcpyAsync(d_seeds.p, seeds.data(), seeds.size(), cudaMemcpyHostToDevice, st));
-    VIA_CUDA(cudaMemcpyAsync(d_lwes.p, lwes.data(), lwes.size() * sizeof(int), cudaMemcpyHostToDevice, st));
-    const long nb = (long)npkt * nblk;
-    k_prg_blocks<<<(unsigned)((nb + 127) / 128), 128, 0, st>>>(reinterpret_cast<const uint8_t*>(d_seeds.p), npkt, nblk,
-                                                               d_blocks.p);
-    VIA_LAUNCHED();
-    k_prg_masks<<<(unsigned)((npkt + 63) / 64), 64, 0, st>>>(d_blocks.p, reinterpret_cast<const uint8_t*>(d_seeds.p),
-                                                            reinterpret_cast<const int*>(d_lwes.p), npkt, nblk, p.n1, nl,
-                                                            ll, S, d_query, reinterpret_cast<int*>(d_err.p));
-    VIA_LAUNCHED();
-    int err = 0;
-    VIA_CUDA(cudaMemcpyAsync(&err, d_err.p, sizeof(int), cudaMemcpyDeviceToHost, st));
-    VIA_CUDA(cudaStreamSynchronize(st));  // the temporaries are freed on return
-    if (err) throw ApiErr(VIA_ERR_INVALID_PRG_SEED, "wire query: a PRG seed's stream rejected 64 draws in a row");
+  WireQuery Q;
+  parse_wire(p, wire, len, Q);
+  if (!Q.flat.empty())
+    VIA_CUDA(cudaMemcpyAsync(d_query, Q.flat.data(), Q.flat.size() * 8, cudaMemcpyHostToDevice, st));
+  const int npkt = (int)Q.lwes.size();
+  if (npkt == 0) {
+    VIA_CUDA(cudaStreamSynchronize(st));  // Q is freed on return
+    return;
   }
+  const Sampler S = make_sampler(p);
+  WalkLimbs W{{S.q[0], S.q[1]}, {S.mask[0], S.mask[1]}, S.nbytes[0], nl};
+  const bool scan = nl == 1 || S.nbytes[0] == S.nbytes[1];
+  double need = 0;
+  for (int l = 0; l < nl; ++l) need += walk_bytes((double)p.n1, S.q[l], S.nbytes[l]);
+  // A whole number of the scan's thread loads past the last draw, as well.
+  const int nblk = (int)((need + WALK_V * 8) / SHAKE_RATE + 2);
+  // One upload and one allocation: bodies, seeds, LWE numbers, error word, then the blocks.
+  const size_t w_seeds = Q.bodies.size(), w_lwes = w_seeds + Q.seeds.size() / 8, w_err = w_lwes + (npkt + 1) / 2;
+  std::vector<u64> head(w_err + 1, 0);
+  std::memcpy(head.data(), Q.bodies.data(), Q.bodies.size() * 8);
+  std::memcpy(head.data() + w_seeds, Q.seeds.data(), Q.seeds.size());
+  std::memcpy(head.data() + w_lwes, Q.lwes.data(), Q.lwes.size() * sizeof(int));
+  DevBuf d(head.size() + (size_t)npkt * nblk * RATE_LANES);
+  VIA_CUDA(cudaMemcpyAsync(d.p, head.data(), head.size() * 8, cudaMemcpyHostToDevice, st));
+  const uint8_t* seeds = reinterpret_cast<const uint8_t*>(d.p + w_seeds);
+  const int* lwes = reinterpret_cast<const int*>(d.p + w_lwes);
+  int* d_err = reinterpret_cast<int*>(d.p + w_err);
+  u64* blocks = d.p + head.size();
+  const long nb = (long)npkt * nblk;
+  k_prg_blocks<<<(unsigned)((nb + 127) / 128), 128, 0, st>>>(seeds, npkt, nblk, blocks);
+  VIA_LAUNCHED();
+  int err = 2;
+  if (scan) {
+    k_prg_masks_scan<<<npkt, WALK_THREADS, 0, st>>>(blocks, d.p, lwes, nblk, p.n1, ll, W, d_query, d_err);
+    VIA_LAUNCHED();
+    VIA_CUDA(cudaMemcpyAsync(&err, d_err, sizeof(int), cudaMemcpyDeviceToHost, st));
+    VIA_CUDA(cudaStreamSynchronize(st));  // the temporaries are freed on return
+  }
+  if (err == 2) {
+    VIA_CUDA(cudaMemsetAsync(d_err, 0, 8, st));
+    k_prg_masks<<<(unsigned)((npkt + 63) / 64), 64, 0, st>>>(blocks, seeds, d.p, lwes, npkt, nblk, p.n1, nl, ll, S,
+                                                            d_query, d_err);
+    VIA_LAUNCHED();
+    VIA_CUDA(cudaMemcpyAsync(&err, d_err, sizeof(int), cudaMemcpyDeviceToHost, st));
+    VIA_CUDA(cudaStreamSynchronize(st));
+  }
+  if (err) throw ApiErr(VIA_ERR_INVALID_PRG_SEED, "wire query: a PRG seed's stream rejected 64 draws in a row");
 }
 
 template <class F>
