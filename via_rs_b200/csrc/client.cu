@@ -320,6 +320,7 @@ struct Client {
   int device = 0;
   cudaStream_t stream = nullptr;
   DevBuf sk1, sk2;
+  KeptScratch scratch;
   u64 sk2_top = 0;  // the or of sk2's words, plus one
   int err_kind = 0;
   i64 err_bound = 1;
@@ -387,36 +388,42 @@ void make_queries(via_client* c, const uint64_t* indices, uint64_t count, const 
   double need = walk_bytes((double)n_lwe, D.bound[2], D.nbytes[2]);
   for (int l = 0; l < nl; ++l) need += walk_bytes((double)n1 * n_lwe, D.bound[l], D.nbytes[l]);
   const int nblk = (int)((need + WALK_V * 8) / SHAKE_RATE + 2);
-  DevBuf d_seeds(((size_t)count * seed_len + 7) / 8), d_blocks((size_t)count * nblk * RATE_LANES),
-      d_errs((size_t)count * n_lwe), d_msgs(msgs.size()), d_flag(1);
-  VIA_CUDA(cudaMemsetAsync(d_flag.p, 0, 8, st));
-  VIA_CUDA(cudaMemcpyAsync(d_seeds.p, seeds, (size_t)count * seed_len, cudaMemcpyHostToDevice, st));
-  VIA_CUDA(cudaMemcpyAsync(d_msgs.p, msgs.data(), msgs.size() * 8, cudaMemcpyHostToDevice, st));
+  // One upload (seeds, messages, flag), then the error samples and the blocks.
+  const size_t w_msgs = ((size_t)count * seed_len + 7) / 8, w_flag = w_msgs + msgs.size(), w_errs = w_flag + 1,
+               w_blocks = w_errs + (size_t)count * n_lwe;
+  std::vector<u64> head(w_errs, 0);
+  std::memcpy(head.data(), seeds, (size_t)count * seed_len);
+  std::memcpy(head.data() + w_msgs, msgs.data(), msgs.size() * 8);
+  ScratchLease tmp(c->scratch, w_blocks + (size_t)count * nblk * RATE_LANES);
+  VIA_CUDA(cudaMemcpyAsync(tmp.p, head.data(), head.size() * 8, cudaMemcpyHostToDevice, st));
+  const uint8_t* d_seeds = reinterpret_cast<const uint8_t*>(tmp.p);
+  const u64* d_msgs = tmp.p + w_msgs;
+  int* d_f = reinterpret_cast<int*>(tmp.p + w_flag);
+  i64* errs = reinterpret_cast<i64*>(tmp.p + w_errs);
+  u64* d_blocks = tmp.p + w_blocks;
   const long nb = (long)count * nblk;
-  k_client_blocks<<<(unsigned)((nb + 127) / 128), 128, 0, st>>>(reinterpret_cast<const uint8_t*>(d_seeds.p),
-                                                                (int)seed_len, (int)count, nblk, d_blocks.p);
+  k_client_blocks<<<(unsigned)((nb + 127) / 128), 128, 0, st>>>(d_seeds, (int)seed_len, (int)count, nblk,
+                                                                d_blocks);
   VIA_LAUNCHED();
   const DevMod m0 = make_devmod(p.q1_0), m1 = make_devmod(p.q1_1 ? p.q1_1 : p.q1_0);
   int flag = 0;
-  int* d_f = reinterpret_cast<int*>(d_flag.p);
-  i64* errs = reinterpret_cast<i64*>(d_errs.p);
   bool scan = nl == 1 || D.nbytes[0] == D.nbytes[1];
   for (;; scan = false) {
     if (scan)
       k_client_walk_scan<<<(unsigned)count, WALK_THREADS, 0, st>>>(
-          d_blocks.p, nblk, n_lwe, n1, ll, WalkLimbs{{D.bound[0], D.bound[1]}, {D.mask[0], D.mask[1]}, D.nbytes[0], nl}, D,
+          d_blocks, nblk, n_lwe, n1, ll, WalkLimbs{{D.bound[0], D.bound[1]}, {D.mask[0], D.mask[1]}, D.nbytes[0], nl}, D,
           c->err_kind, c->err_bound, d_out, errs, d_f);
     else
       k_client_walk<<<(unsigned)((count + 3) / 4), 128, 0, st>>>(
-          d_blocks.p, reinterpret_cast<const uint8_t*>(d_seeds.p), (int)seed_len, (int)count, nblk, n_lwe, n1, nl, ll,
+          d_blocks, d_seeds, (int)seed_len, (int)count, nblk, n_lwe, n1, nl, ll,
           D, c->err_kind, c->err_bound, d_out, errs, d_f);
     VIA_LAUNCHED();
-    k_client_body<<<(unsigned)(count * n_lwe), 256, 0, st>>>(d_out, c->sk1.p, errs, d_msgs.p, n1, nl, ll, m0, m1);
+    k_client_body<<<(unsigned)(count * n_lwe), 256, 0, st>>>(d_out, c->sk1.p, errs, d_msgs, n1, nl, ll, m0, m1);
     VIA_LAUNCHED();
-    VIA_CUDA(cudaMemcpyAsync(&flag, d_flag.p, sizeof(int), cudaMemcpyDeviceToHost, st));
+    VIA_CUDA(cudaMemcpyAsync(&flag, d_f, sizeof(int), cudaMemcpyDeviceToHost, st));
     VIA_CUDA(cudaStreamSynchronize(st));  // the temporaries are freed on return
     if (flag != 2) break;
-    VIA_CUDA(cudaMemsetAsync(d_flag.p, 0, 8, st));
+    VIA_CUDA(cudaMemsetAsync(d_f, 0, 8, st));
   }
   if (flag) throw ApiErr(VIA_ERR_INVALID_PRG_SEED, "client query: a PRG stream rejected 64 draws in a row");
 }
@@ -488,9 +495,10 @@ via_status via_client_recover(via_client* c, const uint64_t* masks, const uint64
       throw ApiErr(VIA_ERR_INVALID_ARGUMENT, "null argument or count outside 1..2^20");
     const via_params& p = c->prm;
     const size_t len = (size_t)count * p.n2;
-    DevBuf dm(len), db(len), dout(len);
-    VIA_CUDA(cudaMemcpyAsync(dm.p, masks, len * 8, cudaMemcpyHostToDevice, c->stream));
-    VIA_CUDA(cudaMemcpyAsync(db.p, bodies, len * 8, cudaMemcpyHostToDevice, c->stream));
+    ScratchLease d(c->scratch, 3 * len);
+    u64 *dm = d.p, *db = dm + len, *dout = db + len;
+    VIA_CUDA(cudaMemcpyAsync(dm, masks, len * 8, cudaMemcpyHostToDevice, c->stream));
+    VIA_CUDA(cudaMemcpyAsync(db, bodies, len * 8, cudaMemcpyHostToDevice, c->stream));
     const int threads = (int)std::min<u64>(p.n2, 1024);
     // The caller's residues are held to 32 bits here, not to q3: any value that
     // does not fit takes the 128-bit sums.
@@ -500,12 +508,12 @@ via_status via_client_recover(via_client* c, const uint64_t* masks, const uint64
                         (u128)top * c->sk2_top * p.n2 < ((u128)1 << 64);
     if (narrow)
       k_client_recover<true><<<(unsigned)count, threads, 2 * p.n2 * 4, c->stream>>>(
-          dm.p, db.p, c->sk2.p, (int)p.n2, make_devmod(p.q3), p.q4, p.p, dout.p);
+          dm, db, c->sk2.p, (int)p.n2, make_devmod(p.q3), p.q4, p.p, dout);
     else
       k_client_recover<false><<<(unsigned)count, threads, 2 * p.n2 * 8, c->stream>>>(
-          dm.p, db.p, c->sk2.p, (int)p.n2, make_devmod(p.q3), p.q4, p.p, dout.p);
+          dm, db, c->sk2.p, (int)p.n2, make_devmod(p.q3), p.q4, p.p, dout);
     VIA_LAUNCHED();
-    VIA_CUDA(cudaMemcpyAsync(out, dout.p, len * 8, cudaMemcpyDeviceToHost, c->stream));
+    VIA_CUDA(cudaMemcpyAsync(out, dout, len * 8, cudaMemcpyDeviceToHost, c->stream));
     VIA_CUDA(cudaStreamSynchronize(c->stream));
   });
 }

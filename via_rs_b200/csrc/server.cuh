@@ -39,6 +39,34 @@ struct DevBuf {
   DevBuf& operator=(const DevBuf&) = delete;
 };
 
+// Device scratch an object keeps between the calls that end with a stream
+// synchronize (cudaMalloc and cudaFree cost 0.1 to several ms a call, and the
+// free waits for the whole device). One call at a time leases it; calls that
+// overlap from other threads allocate their own. A call above KEEP words gives
+// its memory back at once.
+struct KeptScratch {
+  static constexpr size_t KEEP = (size_t)32 << 20;  // 256 MiB
+  std::mutex mu;
+  DevBuf buf;
+};
+class ScratchLease {
+ public:
+  ScratchLease(KeptScratch& k, size_t count) : lock_(k.mu, std::try_to_lock) {
+    if (lock_.owns_lock() && count <= KeptScratch::KEEP) {
+      if (k.buf.n < count) k.buf.alloc(count);
+      p = k.buf.p;
+    } else {
+      own_.alloc(count);
+      p = own_.p;
+    }
+  }
+  u64* p = nullptr;
+
+ private:
+  std::unique_lock<std::mutex> lock_;
+  DevBuf own_;
+};
+
 struct Workspace;  // per-query scratch (pipeline.cu)
 struct WorkspaceDeleter {
   void operator()(Workspace* w) const;
@@ -70,6 +98,7 @@ struct Server {
   std::vector<size_t> repack_off;
   std::unique_ptr<Workspace, WorkspaceDeleter> ws;
   std::mutex mu;  // one in-flight answer per handle (the workspace is shared)
+  KeptScratch wire_scratch;  // wire ingest (wire.cu)
   int plan_gen = 0;  // bumped when the scan tiles change; captured graphs of older plans are dropped
   // Guards fd.tuned and plan_gen: the autotuner holds it exclusively, service
   // workers (which do not take `mu`) hold it shared while they enqueue a batch.

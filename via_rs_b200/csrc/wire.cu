@@ -201,13 +201,13 @@ void decode_to_device(Server& s, const uint8_t* wire, u64 len, u64* d_query, cud
   for (int l = 0; l < nl; ++l) need += walk_bytes((double)p.n1, S.q[l], S.nbytes[l]);
   // A whole number of the scan's thread loads past the last draw, as well.
   const int nblk = (int)((need + WALK_V * 8) / SHAKE_RATE + 2);
-  // One upload and one allocation: bodies, seeds, LWE numbers, error word, then the blocks.
+  // One upload and one scratch: bodies, seeds, LWE numbers, error word, then the blocks.
   const size_t w_seeds = Q.bodies.size(), w_lwes = w_seeds + Q.seeds.size() / 8, w_err = w_lwes + (npkt + 1) / 2;
   std::vector<u64> head(w_err + 1, 0);
   std::memcpy(head.data(), Q.bodies.data(), Q.bodies.size() * 8);
   std::memcpy(head.data() + w_seeds, Q.seeds.data(), Q.seeds.size());
   std::memcpy(head.data() + w_lwes, Q.lwes.data(), Q.lwes.size() * sizeof(int));
-  DevBuf d(head.size() + (size_t)npkt * nblk * RATE_LANES);
+  ScratchLease d(s.wire_scratch, head.size() + (size_t)npkt * nblk * RATE_LANES);
   VIA_CUDA(cudaMemcpyAsync(d.p, head.data(), head.size() * 8, cudaMemcpyHostToDevice, st));
   const uint8_t* seeds = reinterpret_cast<const uint8_t*>(d.p + w_seeds);
   const int* lwes = reinterpret_cast<const int*>(d.p + w_lwes);
