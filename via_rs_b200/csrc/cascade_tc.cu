@@ -1,0 +1,591 @@
+// Exact integer GEMMs of the cascade's first steps (cascade_tc.cuh).
+#include "cascade_tc.cuh"
+
+#include <algorithm>
+
+#include "tc.cuh"
+
+namespace via {
+namespace {
+
+constexpr int CT_EPI = 16;  // epilogue warps: four per TMEM lane quadrant, four coefficients each
+constexpr int CT_THREADS = 64 + 32 * CT_EPI;
+constexpr int CT_ACC = 3;   // accumulator sets of CT_N TMEM columns
+constexpr int CT_STAGE_A = CT_M * CT_KC, CT_STAGE_B = CT_N * CT_KC, CT_STAGE = CT_STAGE_A + CT_STAGE_B;
+constexpr int CT_STAGES = 7;
+constexpr int CT_SMEM = CT_STAGES * CT_STAGE + 256;
+static_assert(CT_SMEM <= 227 * 1024, "shared memory per block");
+
+struct CtParams {
+  CtStep st;
+  CtDigits D;
+  const uint8_t* a;   // digits of this step
+  const uint8_t* b;   // key planes of this step
+  const double* c;    // column constants of this step
+  uint8_t* out;       // next GEMM step's digits, or null
+  int8_t* dig8;       // signed digits [lwe][half][L][2 n] when this is the last GEMM step
+  u64* bsk;           // this step's region of the body accumulators
+  long bsk_stride;    // residues per (lwe, limb)
+  int* err;
+  long nlwe;
+  size_t a_tile, out_tile;  // bytes per 128-LWE tile
+  int mtiles, out_kp, out_half;
+};
+
+__device__ __forceinline__ double ct_u52(u64 x) {  // exact for x < 2^52
+  return __dadd_rn(__longlong_as_double((long long)(x | 0x4330000000000000ull)), -4503599627370496.0);
+}
+
+// The fixed-point fractions f[piece] (32 bits, rounded up by less than 3 ulp) of
+// the three base-T pieces of round(c S / Q) + o (S - 1) / (B - 1) mod S, most
+// significant piece first, for c / Q = y0 / q0 + y1 / q1 mod 1, |y_l| <= 0.5625 q_l.
+__device__ __forceinline__ void ct_pieces(double y0, double y1, const CtDigits& D, u32 (&f)[3]) {
+  int p[3];
+#pragma unroll
+  for (int i = 0; i < 3; ++i) {
+    // T y = qt q + r exactly, |r| <= 0.5625 q (fp_mulmod with its quotient kept);
+    // the quotient's low word is read off the rounding sum.
+    const double h0 = __dmul_rn(D.T, y0), h1 = __dmul_rn(D.T, y1);
+    const double l0 = __fma_rn(D.T, y0, -h0), l1 = __fma_rn(D.T, y1, -h1);
+    const double u0 = __fma_rn(h0, D.qinv[0], FP_ROUND), u1 = __fma_rn(h1, D.qinv[1], FP_ROUND);
+    p[i] = __double2loint(u0) + __double2loint(u1);
+    y0 = __dadd_rn(__fma_rn(-__dadd_rn(u0, -FP_ROUND), D.q[0], h0), l0);
+    y1 = __dadd_rn(__fma_rn(-__dadd_rn(u1, -FP_ROUND), D.q[1], h1), l1);
+  }
+  // Rounding: the remainder y0 / q0 + y1 / q1 to the nearest integer (no ties: Q is odd).
+  const double s = __fma_rn(y0, D.qinv[0], __dmul_rn(y1, D.qinv[1]));
+  const double us = __dadd_rn(s, FP_ROUND);
+  int rnd = __double2loint(us);
+  if (fabs(__dadd_rn(s, -__dadd_rn(us, -FP_ROUND))) > 0.5 - 1e-12) {  // too near to tell in doubles
+    const i128 num = (i128)(i64)y0 * (i128)D.qi[1] + (i128)(i64)y1 * (i128)D.qi[0];
+    const i128 Q = (i128)D.qi[0] * D.qi[1];
+    rnd = 2 * num > Q ? 1 : (2 * num < -Q ? -1 : 0);
+  }
+  // Pieces lie in (-1.2 T, 1.2 T); with off (below 3 T, at least 2 T) they are
+  // nonnegative and below 4.3 T < 2^29, where umulhi(x, M) >> sh = floor(x / T).
+  u32 carry = 2;
+#pragma unroll
+  for (int i = 2; i >= 0; --i) {
+    const u32 x = (u32)p[i] + (i == 2 ? (u32)rnd : 0u) + D.off + carry - 2;
+    carry = __umulhi(x, D.M) >> D.sh;
+    const u32 u = x - carry * D.Ti;
+    const u64 m = (u64)u * D.M;
+    f[i] = (u32)(m >> D.sh) + 1;
+  }
+}
+
+// The next base-B digit of a fraction, most significant first.
+__device__ __forceinline__ u32 ct_digit(u32& f, u32 base) {
+  const u64 m = (u64)f * base;
+  f = (u32)m;
+  return (u32)(m >> 32);
+}
+
+// Signed bytes of four unsigned digits w below 256: w - o.
+__device__ __forceinline__ u32 ct_signed(u32 w, u32 o) { return (w + (128 - o) * 0x01010101u) ^ 0x80808080u; }
+
+// First step's digits from the query: K position j kp + which L + s of LWE w holds
+// digit s of mask which * half + j. Thread = (8-LWE group, j, LWE of the group).
+__global__ void __launch_bounds__(256) k_ct_digits(const u64* __restrict__ q, long nlwe, long lwe_len, int n1,
+                                                   CtStep st, CtDigits D, size_t tile, uint8_t* __restrict__ out) {
+  const long gid = (long)blockIdx.x * blockDim.x + threadIdx.x;
+  const int l8 = (int)(gid & 7);
+  const int j = (int)((gid >> 3) % st.half);
+  const long grp = (gid >> 3) / st.half;
+  const long w = grp * 8 + l8;
+  if (w >= nlwe) return;
+  constexpr int KP = (2 * CT_L + 15) / 16 * 16;
+  u32 word[KP / 4];
+#pragma unroll
+  for (int i = 0; i < KP / 4; ++i) word[i] = 0;
+#pragma unroll
+  for (int which = 0; which < 2; ++which) {
+    const u64* src = q + w * lwe_len + j + which * st.half;
+    u64 a0 = src[0], a1 = src[n1];
+    if (a0 >= (1ull << 47)) a0 %= D.qi[0];  // as the integer path: any 64-bit input word
+    if (a1 >= (1ull << 47)) a1 %= D.qi[1];
+    u32 f[3];
+    ct_pieces(fp_mulmod(ct_u52(a0), D.yscale[0], D.q[0], D.qinv[0]),
+              fp_mulmod(ct_u52(a1), D.yscale[1], D.q[1], D.qinv[1]), D, f);
+#pragma unroll
+    for (int s = 0; s < CT_L; ++s) {
+      const int at = which * CT_L + s;
+      word[at / 4] |= ct_digit(f[s / CT_LP], D.base) << (8 * (at % 4));
+    }
+  }
+  const long mt = w / CT_M;
+  const long left = nlwe - mt * CT_M;
+  const int ng = (int)(((left < CT_M ? left : CT_M) + 7) / 8);
+  uint8_t* o = out + mt * tile + ((size_t)j * (KP / 16) * ng + (w % CT_M) / 8) * 128 + (w & 7) * 16;
+#pragma unroll
+  for (int b = 0; b < KP / 16; ++b)
+    *reinterpret_cast<uint4*>(o + (size_t)b * ng * 128) =
+        make_uint4(word[4 * b], word[4 * b + 1], word[4 * b + 2], word[4 * b + 3]);
+}
+
+// One step. Persistent CTAs walk the (unit, LWE tile) items, tiles fastest, so the CTAs
+// that run together share a unit's key planes in L2. Warp 0 copies the (digit, key) chunks
+// into a ring of shared-memory stages, warp 1 issues the MMAs into one of three TMEM
+// accumulator sets, sixteen epilogue warps fold the previous one.
+//
+// Bounds: at n <= 16 the epilogue (128 x 16 coefficients, 64 FP64 and about 100 integer
+// instructions each) is longer than the MMAs (18 n of 80 cycles each, 36 n K bytes); from
+// n = 64 on the MMAs and the key planes' L2 traffic (160 bytes a K byte) are.
+__global__ void __launch_bounds__(CT_THREADS, 1) k_ct_step(const __grid_constant__ CtParams P) {
+  extern __shared__ __align__(1024) uint8_t smem[];
+  u64* full = reinterpret_cast<u64*>(smem + CT_STAGES * CT_STAGE);
+  u64* empty = full + CT_STAGES;
+  u64* acc_full = empty + CT_STAGES;
+  u64* acc_empty = acc_full + CT_ACC;
+  u64* drain = acc_empty + CT_ACC;
+  u32* tmem_slot = reinterpret_cast<u32*>(drain + 1);
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < CT_STAGES; ++s) {
+      mbar_init(full + s, 1);
+      mbar_init(empty + s, 1);
+    }
+    for (int a = 0; a < CT_ACC; ++a) {
+      mbar_init(acc_full + a, 1);
+      mbar_init(acc_empty + a, CT_EPI * 32);
+    }
+    mbar_init(drain, 1);
+    *abort_flag = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (warp == 1) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_addr(tmem_slot)),
+                 "r"(512u)
+                 : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const u32 tmem = *tmem_slot;
+  const CtStep& S = P.st;
+  const int items = 2 * S.units * P.mtiles;
+  const int upj = S.n >= 8 ? 2 * S.n / CT_ROWS : 1;  // units per output mask (n >= 8)
+
+  if (warp == 0) {
+    if (lane == 0) {
+      int s = 0;
+      u32 ph = 0, armed = 0, armed_par = 0;
+      bool ok = true;
+      for (int it = blockIdx.x; ok && it < items; it += gridDim.x) {
+        const int unit = it / P.mtiles, mt = it % P.mtiles;
+        const int mu = unit % S.units;
+        const long left = P.nlwe - (long)mt * CT_M;
+        const u32 ng = (u32)((min(left, (long)CT_M) + 7) / 8);
+        const size_t k0 = (size_t)(S.n >= 8 ? mu / upj : mu * S.G) * S.kp;  // first K byte
+        const uint8_t* asrc = P.a + mt * P.a_tile + k0 / 16 * ng * 128;
+        const uint8_t* bsrc = P.b + (size_t)unit * S.chunks * CT_STAGE_B;
+        const u32 abytes = CT_KC / 16 * ng * 128;
+        for (int kc = 0; kc < S.chunks; ++kc) {
+          if (!mbar_wait(empty + s, ph ^ 1, abort_flag)) {
+            ok = false;
+            break;
+          }
+          uint8_t* dst = smem + s * CT_STAGE;
+          mbar_expect_tx(full + s, abytes + CT_STAGE_B);
+          bulk_g2s(dst, asrc + (size_t)kc * abytes, abytes, full + s);
+          bulk_g2s(dst + CT_STAGE_A, bsrc + (size_t)kc * CT_STAGE_B, CT_STAGE_B, full + s);
+          armed |= 1u << s;
+          armed_par = (armed_par & ~(1u << s)) | (ph << s);
+          if (++s == CT_STAGES) {
+            s = 0;
+            ph ^= 1;
+          }
+        }
+      }
+      if (!ok) {
+        atomicOr(P.err, 16);
+        *abort_flag = 1;
+      }
+      // Every copy started here lands before the CTA can exit.
+      for (int k = 0; k < CT_STAGES; ++k)
+        if ((armed >> k) & 1)
+          if (!mbar_wait(full + k, (armed_par >> k) & 1, abort_flag, false)) atomicOr(P.err, 16);
+    }
+  } else if (warp == 1) {
+    if (lane == 0) {
+      int s = 0, a = 0;
+      u32 ph = 0, aph = 0;
+      bool ok = true;
+      const u32 idesc = idesc_i8(CT_N, false);
+      constexpr u32 lbo_b = CT_N / 8 * 128;
+      for (int it = blockIdx.x; ok && it < items; it += gridDim.x) {
+        const long left = P.nlwe - (long)(it % P.mtiles) * CT_M;
+        // Tiles of fewer than 128 LWEs: rows past the last 8-LWE group read what
+        // follows in the stage; their accumulator lanes are never used.
+        const u32 lbo_a = (u32)((min(left, (long)CT_M) + 7) / 8) * 128;
+        if (!mbar_wait(acc_empty + a, aph ^ 1, abort_flag)) {
+          ok = false;
+          break;
+        }
+        tc_fence_after();
+        const u32 dacc = tmem + (u32)(a * CT_N);
+        for (int kc = 0; kc < S.chunks; ++kc) {
+          if (!mbar_wait(full + s, ph, abort_flag)) {
+            ok = false;
+            break;
+          }
+          tc_fence_after();
+          const u32 sa = smem_addr(smem + s * CT_STAGE), sb = sa + CT_STAGE_A;
+#pragma unroll
+          for (int ks = 0; ks < CT_KC / 32; ++ks)
+            mma_i8(dacc, smem_desc(sa + ks * 2 * lbo_a, lbo_a, 128), smem_desc(sb + ks * 2 * lbo_b, lbo_b, 128), idesc,
+                   kc == 0 && ks == 0 ? 0u : 1u);
+          mma_commit(empty + s);
+          if (++s == CT_STAGES) {
+            s = 0;
+            ph ^= 1;
+          }
+        }
+        if (!ok) break;
+        mma_commit(acc_full + a);
+        if (++a == CT_ACC) {
+          a = 0;
+          aph ^= 1;
+        }
+      }
+      if (!ok) {
+        atomicOr(P.err, 32);
+        *abort_flag = 1;
+      }
+      mma_commit(drain);
+      if (!mbar_wait(drain, 0, abort_flag, false)) atomicOr(P.err, 32);
+    }
+  } else {
+    const int quad = warp & 3, part = (warp - 2) >> 2;
+    const int m = quad * 32 + lane;  // LWE of the tile
+    const int n_out = 2 * S.n;
+    int a = 0;
+    u32 aph = 0;
+    bool ok = true;
+    for (int it = blockIdx.x; ok && it < items; it += gridDim.x) {
+      const int unit = it / P.mtiles, mt = it % P.mtiles;
+      const int mu = unit % S.units;
+      const long w = (long)mt * CT_M + m;
+      if (!__all_sync(0xffffffffu, mbar_wait(acc_full + a, aph, abort_flag))) {
+        ok = false;
+        break;
+      }
+      tc_fence_after();
+      const bool quad_live = (long)mt * CT_M + quad * 32 < P.nlwe;  // warp-uniform
+      u32 v[2][5][4];
+      if (quad_live) {
+        const u32 tb = tmem + (u32)(a * CT_N) + ((u32)(quad * 32) << 16) + part * 4;
+#pragma unroll
+        for (int l = 0; l < 2; ++l)
+#pragma unroll
+          for (int k = 0; k < 5; ++k) tmem_ld4(tb + (u32)((l * 5 + k) * CT_ROWS), v[l][k]);
+        tmem_wait_ld();
+#pragma unroll
+        for (int l = 0; l < 2; ++l)
+#pragma unroll
+          for (int k = 0; k < 5; ++k) pin(v[l][k]);
+      }
+      tc_fence_before();
+      mbar_arrive(acc_empty + a);
+      if (++a == CT_ACC) {
+        a = 0;
+        aph ^= 1;
+      }
+      if (!quad_live || w >= P.nlwe) continue;
+      // Fold: five byte sums (below 2^31) less the digit offset's constant, mod q_l,
+      // |y| <= q / 2 + 1.
+      double y[2][4];
+#pragma unroll
+      for (int l = 0; l < 2; ++l) {
+        const double q = P.D.q[l], qinv = P.D.qinv[l];
+        const double* cc = P.c + ((size_t)unit * 2 + l) * CT_ROWS + part * 4;
+#pragma unroll
+        for (int r = 0; r < 4; ++r) {
+          const u64 lo = (u64)v[l][0][r] + ((u64)v[l][1][r] << 8) + ((u64)v[l][2][r] << 16);
+          const u64 hi = (u64)v[l][3][r] + ((u64)v[l][4][r] << 8);
+          const double x = __dadd_rn(__dadd_rn(ct_u52(lo), fp_mulmod(ct_u52(hi), P.D.c24[l], q, qinv)), -__ldg(cc + r));
+          y[l][r] = __fma_rn(-__dadd_rn(__fma_rn(x, qinv, FP_ROUND), -FP_ROUND), q, x);
+        }
+      }
+      // Rows part * 4 .. + 3 of the unit: output mask jj, coefficients yy .. (n >= 2),
+      // or masks jj, jj + 1 of two coefficients each (n = 1).
+      const int r0 = part * 4;
+      const int jj = S.n >= 8 ? mu / upj : mu * S.G + r0 / n_out;
+      const int yy = S.n >= 8 ? (mu % upj) * CT_ROWS + r0 : r0 % n_out;
+      if (unit >= S.units) {  // body sums, canonical, added over the output masks
+#pragma unroll
+        for (int l = 0; l < 2; ++l) {
+          unsigned long long* o = reinterpret_cast<unsigned long long*>(P.bsk + (w * 2 + l) * P.bsk_stride) + yy;
+          u64 b[4];
+#pragma unroll
+          for (int r = 0; r < 4; ++r) b[r] = __double2ull_rn(fp_canonical(y[l][r], P.D.q[l], P.D.qinv[l]));
+          if (S.n == 1) {
+            atomicAdd(o, b[0] + b[2]);
+            atomicAdd(o + 1, b[1] + b[3]);
+          } else {
+#pragma unroll
+            for (int r = 0; r < 4; ++r) atomicAdd(o + r, b[r]);
+          }
+        }
+        continue;
+      }
+      u32 f[4][3];
+#pragma unroll
+      for (int r = 0; r < 4; ++r) ct_pieces(y[0][r], y[1][r], P.D, f[r]);
+      if (P.out) {
+        const int which = jj / P.out_half, j2 = jj % P.out_half;
+        const long left = P.nlwe - (long)mt * CT_M;
+        const size_t ngb = (size_t)((min(left, (long)CT_M) + 7) / 8) * 128;
+        uint8_t* base = P.out + mt * P.out_tile + (m / 8) * 128 + (m & 7) * 16;
+        int pos = j2 * P.out_kp + which * CT_L * n_out + yy;
+#pragma unroll
+        for (int i = 0; i < 3; ++i)
+#pragma unroll
+          for (int k = 0; k < CT_LP; ++k, pos += n_out) {
+            u32 d = 0;
+#pragma unroll
+            for (int r = 0; r < 4; ++r) d |= ct_digit(f[r][i], P.D.base) << (8 * r);
+            uint8_t* o = base + (size_t)(pos >> 4) * ngb + (pos & 15);
+            if (S.n == 1) {
+              *reinterpret_cast<uint16_t*>(o) = (uint16_t)d;
+              const int p2 = pos + P.out_kp;
+              *reinterpret_cast<uint16_t*>(base + (size_t)(p2 >> 4) * ngb + (p2 & 15)) = (uint16_t)(d >> 16);
+            } else {
+              *reinterpret_cast<u32*>(o) = d;
+            }
+          }
+      } else {
+        int8_t* o = P.dig8 + ((w * S.half + jj) * CT_L) * (long)n_out + yy;
+#pragma unroll
+        for (int i = 0; i < 3; ++i)
+#pragma unroll
+          for (int k = 0; k < CT_LP; ++k, o += n_out) {
+            u32 d = 0;
+#pragma unroll
+            for (int r = 0; r < 4; ++r) d |= ct_digit(f[r][i], P.D.base) << (8 * r);
+            d = ct_signed(d, P.D.o);
+            if (S.n == 1) {
+              *reinterpret_cast<uint16_t*>(o) = (uint16_t)d;
+              *reinterpret_cast<uint16_t*>(o + CT_L * n_out) = (uint16_t)(d >> 16);
+            } else {
+              *reinterpret_cast<u32*>(o) = d;
+            }
+          }
+      }
+    }
+    if (!ok) {
+      atomicOr(P.err, 64);
+      *abort_flag = 1;
+    }
+  }
+  tc_fence_before();
+  __syncthreads();
+  if (warp == 1) {
+    tc_fence_after();
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512u) : "memory");
+  }
+}
+
+// Key planes of one step: thread = (unit, 16 K bytes, limb, row), five 16-byte core-matrix
+// rows each. key: the step's coefficient-form samples [R][L][2][2][n_out]. Mask entries
+// are -K (Q / q_l)^-1 mod q_l, body entries K.
+__global__ void k_ct_planes(const u64* __restrict__ key, CtStep st, DevRing R, u64 inv0, u64 inv1,
+                            uint8_t* __restrict__ planes) {
+  const long gid = (long)blockIdx.x * blockDim.x + threadIdx.x;
+  const int k16s = st.chunks * (CT_KC / 16);
+  if (gid >= (long)2 * st.units * k16s * 32) return;
+  const int r = (int)(gid & 15), l = (int)((gid >> 4) & 1);
+  const int k16 = (int)((gid >> 5) % k16s), unit = (int)((gid >> 5) / k16s);
+  const int mb = unit >= st.units, mu = unit - mb * st.units;
+  const int n_out = 2 * st.n, L = CT_L;
+  const int upj = st.n >= 8 ? n_out / CT_ROWS : 1;
+  const int g_row = st.n >= 8 ? 0 : r / n_out;
+  const int j = st.n >= 8 ? mu / upj : mu * st.G + g_row;
+  const int y = st.n >= 8 ? (mu % upj) * CT_ROWS + r : r % n_out;
+  const DevMod& m = R.m[l];
+  const u64 inv = l ? inv1 : inv0;
+  u32 word[5][4];
+#pragma unroll
+  for (int k = 0; k < 5; ++k) word[k][0] = word[k][1] = word[k][2] = word[k][3] = 0;
+#pragma unroll
+  for (int x = 0; x < 16; ++x) {
+    const int kk = k16 * 16 + x;
+    const int g = kk / st.kp, e = kk % st.kp;
+    if (g != g_row || e >= 2 * L * st.n) continue;
+    const int which = e / (L * st.n), s = (e / st.n) % L, c = e % st.n;
+    int at = y - 2 * c;
+    const bool wrap = at < 0;
+    if (wrap) at += n_out;
+    u64 v = key[((((long)(j + which * st.half) * L + s) * 2 + mb) * 2 + l) * n_out + at];
+    v = reduce64(v, m);
+    if (mb == 0) v = mulmod(v, inv, m);
+    if (wrap != (mb == 0)) v = negmod(v, m.q);
+#pragma unroll
+    for (int k = 0; k < 5; ++k) word[k][x >> 2] |= (u32)((v >> (8 * k)) & 0xFF) << (8 * (x & 3));
+  }
+  const int kc = k16 / (CT_KC / 16), kb = k16 % (CT_KC / 16);
+  uint8_t* base = planes + ((size_t)unit * st.chunks + kc) * CT_STAGE_B + (size_t)kb * (CT_N / 8) * 128;
+#pragma unroll
+  for (int k = 0; k < 5; ++k) {
+    const int row = (l * 5 + k) * CT_ROWS + r;
+    *reinterpret_cast<uint4*>(base + (row / 8) * 128 + (row % 8) * 16) =
+        make_uint4(word[k][0], word[k][1], word[k][2], word[k][3]);
+  }
+}
+
+// Column constants o * (sum of the column's key entries) mod q_l, one warp per (unit, limb,
+// row): read back from the planes.
+__global__ void k_ct_consts(const uint8_t* __restrict__ planes, CtStep st, DevRing R, u32 o, double* __restrict__ out) {
+  const long gid = ((long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  const int lane = threadIdx.x & 31;
+  if (gid >= (long)2 * st.units * 32) return;
+  const int r = (int)(gid & 15), l = (int)((gid >> 4) & 1), unit = (int)(gid >> 5);
+  u64 sum[5] = {0, 0, 0, 0, 0};
+  for (int k16 = lane; k16 < st.chunks * (CT_KC / 16); k16 += 32) {
+    const uint8_t* base = planes + ((size_t)unit * st.chunks + k16 / (CT_KC / 16)) * CT_STAGE_B +
+                          (size_t)(k16 % (CT_KC / 16)) * (CT_N / 8) * 128;
+#pragma unroll
+    for (int k = 0; k < 5; ++k) {
+      const int row = (l * 5 + k) * CT_ROWS + r;
+      const uint4 v = *reinterpret_cast<const uint4*>(base + (row / 8) * 128 + (row % 8) * 16);
+      const u32 w[4] = {v.x, v.y, v.z, v.w};
+      for (int i = 0; i < 4; ++i)
+        for (int b = 0; b < 4; ++b) sum[k] += (w[i] >> (8 * b)) & 0xFF;
+    }
+  }
+#pragma unroll
+  for (int k = 0; k < 5; ++k)
+    for (int d = 16; d; d >>= 1) sum[k] += __shfl_xor_sync(0xffffffffu, sum[k], d);
+  if (lane == 0) {
+    const DevMod& m = R.m[l];
+    u64 acc = 0;
+    for (int k = 4; k >= 0; --k) acc = reduce64((acc << 8) + reduce64(sum[k], m), m);
+    out[((size_t)unit * 2 + l) * CT_ROWS + r] = (double)mulmod(acc, o, m);
+  }
+}
+
+CtDigits make_digits(const via_params& p, const DevRing& R) {
+  CtDigits D{};
+  for (int l = 0; l < 2; ++l) {
+    const u64 q = R.m[l].q;
+    D.qi[l] = q;
+    D.q[l] = (double)q;
+    D.qinv[l] = 1.0 / (double)q;
+    D.c24[l] = (double)(((u64)1 << 24) % q);
+    D.yscale[l] = (double)h_inv(R.m[1 - l].q % q, q);
+  }
+  u64 T = 1;
+  for (int i = 0; i < CT_LP; ++i) T *= p.ck_base;
+  D.T = (double)T;
+  D.Ti = (u32)T;
+  D.base = (u32)p.ck_base;
+  D.o = (u32)(p.ck_base - 1 - p.ck_base / 2);
+  int sh = 0;
+  while (((u64)1 << (sh + 1)) < T) ++sh;  // 2^sh < T <= 2^(sh + 1)
+  D.sh = sh;
+  D.M = (u32)((((u128)1 << (32 + sh)) + T - 1) / T);
+  D.off = (u32)(D.o * ((T - 1) / (p.ck_base - 1)) + 2 * T);
+  return D;
+}
+
+}  // namespace
+
+// Two-prime NTT rings of degree 256 .. 4096, primes of 26 to 40 bits (five bytes; a quotient of
+// T y / q fits the low word), gadgets of 18 digits with B^6 < 2^26 (a piece's arithmetic
+// fits 32 bits).
+bool ct_supported(const via_params& p, const DevRing& R) {
+  if (!R.ntt || R.nl != 2 || p.n1 < 256 || p.l_ck != CT_L || p.ck_base < 3) return false;
+  u64 T = 1;
+  for (int i = 0; i < CT_LP; ++i) T *= p.ck_base;
+  if (p.ck_base > 255 || T >= (1ull << 26)) return false;
+  for (int l = 0; l < 2; ++l)
+    if (R.m[l].q >= (1ull << 40) || R.m[l].q < (1ull << 26)) return false;
+  return true;
+}
+
+int ct_steps(const via_params&) { return 7; }  // input degrees 1 .. 64
+
+void ct_prepare_device() {
+  VIA_CUDA(cudaFuncSetAttribute(k_ct_step, cudaFuncAttributeMaxDynamicSharedMemorySize, CT_SMEM));
+}
+
+void ct_prepare(Server& s) {
+  const via_params& p = s.prm;
+  if (!ct_supported(p, s.r1) || !s.cascade_eval.p || !s.fd_err.p) return;
+  const int K = ct_steps(p), n1 = (int)p.n1;
+  size_t bytes = 0, consts = 0;
+  std::vector<CtStep> steps;
+  for (int k = 0; k < K; ++k) {
+    CtStep st = ct_step(n1, 1 << k);
+    st.b_off = bytes;
+    st.c_off = consts;
+    bytes += (size_t)2 * st.units * st.chunks * CT_STAGE_B;
+    consts += (size_t)2 * st.units * 2 * CT_ROWS;
+    steps.push_back(st);
+  }
+  ct_prepare_device();
+  s.ct_planes.alloc(bytes / 8);
+  s.ct_consts.alloc(consts);
+  const CtDigits D = make_digits(p, s.r1);
+  const u64 step_len = (u64)2 * n1 * CT_L * 2 * 2;
+  const u64 inv0 = (u64)D.yscale[0], inv1 = (u64)D.yscale[1];
+  for (int k = 0; k < K; ++k) {
+    const CtStep& st = steps[k];
+    uint8_t* planes = reinterpret_cast<uint8_t*>(s.ct_planes.p) + st.b_off;
+    const long threads = (long)2 * st.units * st.chunks * (CT_KC / 16) * 32;
+    k_ct_planes<<<(unsigned)((threads + 255) / 256), 256, 0, s.stream>>>(s.cascade_eval.p + k * step_len, st, s.r1, inv0,
+                                                                        inv1, planes);
+    VIA_LAUNCHED();
+    const long warps = (long)2 * st.units * 32;
+    k_ct_consts<<<(unsigned)((warps * 32 + 255) / 256), 256, 0, s.stream>>>(
+        planes, st, s.r1, D.o, reinterpret_cast<double*>(s.ct_consts.p) + st.c_off);
+    VIA_LAUNCHED();
+  }
+  s.ct_steps = K;
+}
+
+void ct_run(Server& s, const u64* d_query, long nlwe, uint8_t* da, uint8_t* db, int8_t* dig8, u64* bsk,
+            cudaStream_t st) {
+  const via_params& p = s.prm;
+  const int n1 = (int)p.n1;
+  const CtDigits D = make_digits(p, s.r1);
+  const int mtiles = (int)((nlwe + CT_M - 1) / CT_M);
+  CtStep cur = ct_step(n1, 1);
+  const long threads = (nlwe + 7) / 8 * 8 * cur.half;
+  k_ct_digits<<<(unsigned)((threads + 255) / 256), 256, 0, st>>>(d_query, nlwe, (long)lwe_len(p), n1, cur, D,
+                                                                (size_t)CT_M * cur.half * cur.kp, da);
+  VIA_LAUNCHED();
+  size_t b_off = 0, c_off = 0;
+  for (int k = 0; k < s.ct_steps; ++k) {
+    const CtStep nxt = ct_step(n1, 2 << k);
+    const bool last = k + 1 == s.ct_steps;
+    CtParams P{};
+    P.st = cur;
+    P.D = D;
+    P.a = da;
+    P.b = reinterpret_cast<const uint8_t*>(s.ct_planes.p) + b_off;
+    P.c = reinterpret_cast<const double*>(s.ct_consts.p) + c_off;
+    P.out = last ? nullptr : db;
+    P.dig8 = dig8;
+    P.bsk = bsk + (2L << k) - 2;
+    P.bsk_stride = 2L * n1;
+    P.err = reinterpret_cast<int*>(s.fd_err.p);
+    P.nlwe = nlwe;
+    P.a_tile = (size_t)CT_M * cur.half * cur.kp;
+    P.out_tile = (size_t)CT_M * nxt.half * nxt.kp;
+    P.mtiles = mtiles;
+    P.out_kp = nxt.kp;
+    P.out_half = nxt.half;
+    const int items = 2 * cur.units * mtiles;
+    k_ct_step<<<std::min(items, s.fd.grid), CT_THREADS, CT_SMEM, st>>>(P);
+    VIA_LAUNCHED();
+    b_off += (size_t)2 * cur.units * cur.chunks * CT_STAGE_B;
+    c_off += (size_t)2 * cur.units * 2 * CT_ROWS;
+    std::swap(da, db);
+    cur = nxt;
+  }
+}
+
+}  // namespace via

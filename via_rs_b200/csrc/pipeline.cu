@@ -19,6 +19,7 @@
 #include <cmath>
 #include <cstring>
 
+#include "cascade_tc.cuh"
 #include "first_dim.cuh"
 #include "gadget.cuh"
 #include "ntt_fp.cuh"
@@ -555,12 +556,13 @@ __global__ void __launch_bounds__(256, 2) k_cascade_mac_fp(const double* __restr
 
 // The cascade's final body in the eval domain, [lwe][nl][n1] (n1 = 2^K). Step k
 // (output degree 2^(k+1)) maps body to embed_at(body, 0) - bsum_k, and the eval
-// form of embed_at repeats every slot, so
+// form of embed_at repeats every slot, so the steps from k0 on give
 //   body[t] = b - sum_k bsum_k[t >> (K - 1 - k)]
-// with b the LWE body (the degree-1 body, [lwe][nl]) and bsum_k the step's
-// accumulated sums, bsk[(lwe nl + l) * 2 n1 + 2^(k+1) - 2 + slot].
-__global__ void k_cascade_body_final(const u64* __restrict__ b0, const u64* __restrict__ bsk, int K, int nl,
-                                     long nlwe, DevRing Rg, u64* __restrict__ body) {
+// with b the LWE body (the degree-1 body, b0[lwe * b0_stride + l]) and bsum_k the step's
+// accumulated sums, bsk[(lwe nl + l) * 2 n1 + 2^(k+1) - 2 + slot]. The steps before
+// k0 (the GEMM steps) leave their sums in coefficient form (k_pack_rlwe).
+__global__ void k_cascade_body_final(const u64* __restrict__ b0, long b0_stride, const u64* __restrict__ bsk, int k0,
+                                     int K, int nl, long nlwe, DevRing Rg, u64* __restrict__ body) {
   const int n1 = 1 << K;
   const long gid = (long)blockIdx.x * blockDim.x + threadIdx.x;
   if (gid >= nlwe * nl * n1) return;
@@ -569,8 +571,8 @@ __global__ void k_cascade_body_final(const u64* __restrict__ b0, const u64* __re
   const DevMod& m = Rg.m[l];
   const u64* sk = bsk + ll * 2 * n1;
   u64 acc = 0;
-  for (int k = 0; k < K; ++k) acc = addmod(acc, reduce64(sk[(2 << k) - 2 + (t >> (K - 1 - k))], m), m.q);
-  body[gid] = submod(b0[ll], acc, m.q);
+  for (int k = k0; k < K; ++k) acc = addmod(acc, reduce64(sk[(2 << k) - 2 + (t >> (K - 1 - k))], m), m.q);
+  body[gid] = submod(b0[ll / nl * b0_stride + l], acc, m.q);
 }
 
 // body_out[lwe] = embed_at(body_in[lwe], N_out, 0) - bsum[lwe] (coefficient form).
@@ -588,15 +590,23 @@ __global__ void k_cascade_body(const u64* __restrict__ body_in, const u64* __res
   body_out[w * per + rem] = submod(e, bsum[w * per + rem], q);
 }
 
-// Assemble cascade outputs into RLWEs [lwe][2][nl][n1].
-__global__ void k_pack_rlwe(const u64* masks, const u64* body, long nlwe, int n1, int nl, u64* out) {
+// Assemble cascade outputs into RLWEs [lwe][2][nl][n1]. The first k0 steps' body sums
+// are in coefficient form: step k's coefficient c sits at coefficient c n1 / 2^(k+1).
+__global__ void k_pack_rlwe(const u64* masks, const u64* body, const u64* __restrict__ bsk, int k0, int K, long nlwe,
+                            int n1, int nl, DevRing Rg, u64* out) {
   long per = (long)nl * n1;
   long gid = (long)blockIdx.x * blockDim.x + threadIdx.x;
   if (gid >= nlwe * per) return;
   long w = gid / per;
   int rem = (int)(gid % per);
   out[(2 * w) * per + rem] = masks[w * per + rem];
-  out[(2 * w + 1) * per + rem] = body[w * per + rem];
+  u64 b = body[w * per + rem];
+  const int l = rem / n1, i = rem % n1;
+  for (int k = k0 - 1; k >= 0 && (i & ((1 << (K - 1 - k)) - 1)) == 0; --k) {
+    const DevMod& m = Rg.m[l];
+    b = submod(b, reduce64(bsk[(w * nl + l) * 2 * n1 + (2 << k) - 2 + (i >> (K - 1 - k))], m), m.q);
+  }
+  out[(2 * w + 1) * per + rem] = b;
 }
 
 // rlwe_to_rgsw assembly (prim/gates/convert.rs:162-178): for bit b, level i:
@@ -770,7 +780,9 @@ static size_t workspace_build(Server& s, int bmax, Workspace* w, bool count_only
   A(w->c_body_b, nlwe * n1 * nl);
   // NTT rings transform the cascade digits at the input degree (half of the
   // embedded degree); the other rings use the embedded digits and the P buffer.
-  A(w->c_digits, nlwe * (s.r1.ntt ? 1 : 2) * n1 * Lck * nl);
+  // The GEMM steps' two digit buffers lie in the same memory.
+  const long tc_words = s.ct_steps ? 2 * (long)(ct_digit_bytes((int)n1) / 8) * ((nlwe + 7) / 8 * 8) : 0;
+  A(w->c_digits, std::max(nlwe * (s.r1.ntt ? 1 : 2) * n1 * Lck * nl, tc_words));
   A(w->c_P, s.r1.ntt ? 0 : nlwe * 2 * n1 * 2 * nl);
   A(w->c_bsum, 2 * nlwe * n1 * nl);
   A(w->c_dig8, p.ck_base <= 255 && s.r1.ntt ? (nlwe * n1 * Lck + 7) / 8 : 0);
@@ -890,7 +902,17 @@ static void mod_switch(const DevRing& S, const u64* in, const DevRing& D, u64* o
 // first being LWE lwe0 of the workspace (LWE-indexed buffers are used from that
 // LWE's region on), forming the RGSWs of `nbits` query bits starting at bit
 // bit0 -> rgsw_q1 [bit][2L][2][nl][n1] (coefficient form). Disjoint (lwe0,
-// nlwe) ranges may run concurrently on different streams.
+// nlwe) ranges may run concurrently on different streams. Servers with GEMM
+// steps (cascade_tc.cuh) have run those for every LWE (cascade_gemm): the
+// cascade continues from their digits and body sums.
+static void cascade_gemm(Server& s, Workspace& w, const u64* d_query, long nlwe, cudaStream_t st) {
+  const long n1 = s.prm.n1;
+  uint8_t* da = reinterpret_cast<uint8_t*>(w.c_digits.p);
+  uint8_t* db = da + ct_digit_bytes((int)n1) * ((nlwe + 7) / 8 * 8);
+  VIA_CUDA(cudaMemsetAsync(w.c_bsum.p, 0, (size_t)nlwe * 2 * n1 * s.r1.nl * 8, st));
+  ct_run(s, d_query, nlwe, da, db, reinterpret_cast<int8_t*>(w.c_dig8.p), w.c_bsum.p, st);
+}
+
 static void query_decomp_range(Server& s, Workspace& w, const u64* d_query, long lwe0, long nlwe, long bit0,
                                long nbits, cudaStream_t st) {
   const via_params& p = s.prm;
@@ -908,20 +930,26 @@ static void query_decomp_range(Server& s, Workspace& w, const u64* d_query, long
   u64* rlwe = w.c_rlwe.p + lwe0 * 2 * lwe_n;
   // Bases up to 255: digits as bytes, lifted and transformed by the 8-bit NTT.
   int8_t* dig8 = w.c_dig8.p ? reinterpret_cast<int8_t*>(w.c_dig8.p) + lwe0 * (long)n1 * L : nullptr;
-  k_lwe_to_mlwe<<<blocks(nlwe * nl * (n1 + 1)), 256, 0, st>>>(d_query + lwe0 * (long)lwe_len(p), n1, nl, nlwe, mi, bi);
-  VIA_LAUNCHED();
-  if (R.ntt) VIA_CUDA(cudaMemsetAsync(bsk, 0, (size_t)nlwe * 2 * lwe_n * 8, st));
+  const int k0 = s.ct_steps;  // steps already run as GEMMs
+  const u64* query = d_query + lwe0 * (long)lwe_len(p);
+  if (!k0) {
+    k_lwe_to_mlwe<<<blocks(nlwe * nl * (n1 + 1)), 256, 0, st>>>(query, n1, nl, nlwe, mi, bi);
+    VIA_LAUNCHED();
+    if (R.ntt) VIA_CUDA(cudaMemsetAsync(bsk, 0, (size_t)nlwe * 2 * lwe_n * 8, st));
+  }
   const u64 step_len = (u64)2 * n1 * L * 2 * nl;
-  int k = 0;
-  for (int n_in = 1; n_in < n1; n_in <<= 1, ++k) {
+  int k = k0;
+  for (int n_in = 1 << k0; n_in < n1; n_in <<= 1, ++k) {
     const int n_out = 2 * n_in, rank_in = n1 / n_in;
     const long polys = nlwe * rank_in;
     if (R.ntt) {
       // Digits at the input degree; see k_cascade_mac for the repeated slots.
       const bool fp_mac = dig8 && s.cascade_eval_d.p;
       if (dig8 && (n_in > 1 || fp_mac)) {
-        k_decompose_i8<<<blocks(polys * n_in, 128), 128, 0, st>>>(mi, n_in, polys, R, w.g_ck, dig8);
-        VIA_LAUNCHED();
+        if (k != k0 || k0 == 0) {  // the last GEMM step left its successor's digits in dig8
+          k_decompose_i8<<<blocks(polys * n_in, 128), 128, 0, st>>>(mi, n_in, polys, R, w.g_ck, dig8);
+          VIA_LAUNCHED();
+        }
         if (n_in == 1)
           ;  // degree 1: the MAC reads the digits themselves
         else if (fp_mac)
@@ -968,12 +996,13 @@ static void query_decomp_range(Server& s, Workspace& w, const u64* d_query, long
     std::swap(bi, bo);
   }
   if (R.ntt) {  // the cascade's body, from the LWE bodies in bi and every step's sums
-    k_cascade_body_final<<<blocks(nlwe * nl * n1), 256, 0, st>>>(bi, bsk, k, nl, nlwe, R, bo);
+    k_cascade_body_final<<<blocks(nlwe * nl * n1), 256, 0, st>>>(k0 ? query + (long)nl * n1 : bi,
+                                                                 k0 ? (long)lwe_len(p) : nl, bsk, k0, k, nl, nlwe, R, bo);
     VIA_LAUNCHED();
     from_eval(R, bo, n1, nlwe * nl, st);
     std::swap(bi, bo);
   }
-  k_pack_rlwe<<<blocks(nlwe * nl * n1), 256, 0, st>>>(mi, bi, nlwe, n1, nl, rlwe);
+  k_pack_rlwe<<<blocks(nlwe * nl * n1), 256, 0, st>>>(mi, bi, bsk, k0, k, nlwe, n1, nl, R, rlwe);
   VIA_LAUNCHED();
   // RLWE -> RGSW with the conversion key (prim/gates/convert.rs:162-178); the
   // final rank-1 masks are already contiguous [lwe][nl][n1] in `mi`.
@@ -1330,7 +1359,8 @@ void answer_device_stages(Server& s, Workspace& w, const u64* d_query, int nq, u
   }
   u64* const rgsw_b1 = w.rgsw_q1.p + B * nd * rgsw1;  // the CMux / CRot bits' group
   u64* const rgsw_b2 = w.rgsw_q2.p + B * nd * rgsw2;
-  // Answers that run to the end expand the CMux / CRot bits (their cascades,
+  if (s.ct_steps) cascade_gemm(s, w, qsrc, nlwe_all, st);
+  // Answers that run to the end expand the CMux / CRot bits (the rest of their cascades,
   // RGSWs and q1 -> q2 switch) on the side stream while the DMux tree and the
   // database scan run on `st`; `st` waits for them before the CMux tree. The
   // two groups' LWEs, buffer regions and scratch are disjoint.

@@ -5,6 +5,7 @@
 #include <mutex>
 #include <string>
 
+#include "cascade_tc.cuh"
 #include "first_dim.cuh"
 #include "server.cuh"
 
@@ -77,7 +78,7 @@ static void check_device_flags(Server& s, cudaStream_t st) {
   VIA_CUDA(cudaMemcpyAsync(&flag, s.fd_err.p, sizeof(int), cudaMemcpyDeviceToHost, st));
   VIA_CUDA(cudaStreamSynchronize(st));
   if (flag)
-    throw ApiError(VIA_ERR_TIMEOUT, "FirstDim scan: a bounded device wait ran out (flag " + std::to_string(flag) + ")");
+    throw ApiError(VIA_ERR_TIMEOUT, "a bounded device wait ran out in the scan or the cascade (flag " + std::to_string(flag) + ")");
 }
 
 int ilog2(u64 v) { return v <= 1 ? 0 : 63 - __builtin_clzll(v); }
@@ -223,6 +224,7 @@ static void load_keys(Server& s, const via_public_keys* keys) {
   VIA_CUDA(cudaMemcpyAsync(s.conv_eval.p, keys->conv_key, s.conv_eval.n * 8, cudaMemcpyHostToDevice, s.stream));
   VIA_CUDA(cudaMemcpyAsync(s.rsk_eval.p, keys->rsk, s.rsk_eval.n * 8, cudaMemcpyHostToDevice, s.stream));
   derive_repack_keys(s);  // VIA-B: from the coefficient-form cascade key, before it is transformed
+  ct_prepare(s);          // the GEMM steps' key planes, likewise
   transform_keys(s);
 }
 
