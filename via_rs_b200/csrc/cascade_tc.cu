@@ -24,8 +24,7 @@ struct CtParams {
   const double* c;    // column constants of this step
   uint8_t* out;       // next GEMM step's digits, or null
   int8_t* dig8;       // signed digits [lwe][half][L][2 n] when this is the last GEMM step
-  u64* bsk;           // this step's region of the body accumulators
-  long bsk_stride;    // residues per (lwe, limb)
+  u64* body;          // this step's body accumulators [2 n][2][nlwe]
   int* err;
   long nlwe;
   size_t a_tile, out_tile;  // bytes per 128-LWE tile
@@ -34,6 +33,14 @@ struct CtParams {
 
 __device__ __forceinline__ double ct_u52(u64 x) {  // exact for x < 2^52
   return __dadd_rn(__longlong_as_double((long long)(x | 0x4330000000000000ull)), -4503599627370496.0);
+}
+
+// First output mask of a unit. Mask units of n >= 8 run over the coefficient blocks of
+// one output mask, body units over the output masks of one coefficient block.
+__host__ __device__ __forceinline__ int ct_first_mask(const CtStep& S, int unit) {
+  const int mu = unit < S.units ? unit : unit - S.units;
+  if (S.n < 8) return mu * S.G;
+  return unit < S.units ? mu / (2 * S.n / CT_ROWS) : mu % S.half;
 }
 
 // The fixed-point fractions f[piece] (32 bits, rounded up by less than 3 ulp) of
@@ -165,7 +172,7 @@ __global__ void __launch_bounds__(CT_THREADS, 1) k_ct_step(const __grid_constant
   tc_fence_after();
   const u32 tmem = *tmem_slot;
   const CtStep& S = P.st;
-  const int items = 2 * S.units * P.mtiles;
+  const int items = S.items() * P.mtiles;
   const int upj = S.n >= 8 ? 2 * S.n / CT_ROWS : 1;  // units per output mask (n >= 8)
 
   if (warp == 0) {
@@ -174,15 +181,16 @@ __global__ void __launch_bounds__(CT_THREADS, 1) k_ct_step(const __grid_constant
       u32 ph = 0, armed = 0, armed_par = 0;
       bool ok = true;
       for (int it = blockIdx.x; ok && it < items; it += gridDim.x) {
-        const int unit = it / P.mtiles, mt = it % P.mtiles;
-        const int mu = unit % S.units;
+        const int item = it / P.mtiles, mt = it % P.mtiles;
+        const int len = item < S.units ? 1 : S.chain;
+        const int unit0 = item < S.units ? item : S.units + (item - S.units) * S.chain;
         const long left = P.nlwe - (long)mt * CT_M;
         const u32 ng = (u32)((min(left, (long)CT_M) + 7) / 8);
-        const size_t k0 = (size_t)(S.n >= 8 ? mu / upj : mu * S.G) * S.kp;  // first K byte
-        const uint8_t* asrc = P.a + mt * P.a_tile + k0 / 16 * ng * 128;
-        const uint8_t* bsrc = P.b + (size_t)unit * S.chunks * CT_STAGE_B;
         const u32 abytes = CT_KC / 16 * ng * 128;
-        for (int kc = 0; kc < S.chunks; ++kc) {
+        const uint8_t* asrc = nullptr;
+        const uint8_t* bsrc = P.b + (size_t)unit0 * S.chunks * CT_STAGE_B;
+        for (int i = 0, kc = 0; i < len * S.chunks; ++i) {
+          if (kc == 0) asrc = P.a + mt * P.a_tile + (size_t)ct_first_mask(S, unit0 + i / S.chunks) * S.kp / 16 * ng * 128;
           if (!mbar_wait(empty + s, ph ^ 1, abort_flag)) {
             ok = false;
             break;
@@ -190,7 +198,8 @@ __global__ void __launch_bounds__(CT_THREADS, 1) k_ct_step(const __grid_constant
           uint8_t* dst = smem + s * CT_STAGE;
           mbar_expect_tx(full + s, abytes + CT_STAGE_B);
           bulk_g2s(dst, asrc + (size_t)kc * abytes, abytes, full + s);
-          bulk_g2s(dst + CT_STAGE_A, bsrc + (size_t)kc * CT_STAGE_B, CT_STAGE_B, full + s);
+          bulk_g2s(dst + CT_STAGE_A, bsrc + (size_t)i * CT_STAGE_B, CT_STAGE_B, full + s);
+          if (++kc == S.chunks) kc = 0;
           armed |= 1u << s;
           armed_par = (armed_par & ~(1u << s)) | (ph << s);
           if (++s == CT_STAGES) {
@@ -226,7 +235,8 @@ __global__ void __launch_bounds__(CT_THREADS, 1) k_ct_step(const __grid_constant
         }
         tc_fence_after();
         const u32 dacc = tmem + (u32)(a * CT_N);
-        for (int kc = 0; kc < S.chunks; ++kc) {
+        const int nk = (it / P.mtiles < S.units ? 1 : S.chain) * S.chunks;
+        for (int kc = 0; kc < nk; ++kc) {
           if (!mbar_wait(full + s, ph, abort_flag)) {
             ok = false;
             break;
@@ -265,8 +275,7 @@ __global__ void __launch_bounds__(CT_THREADS, 1) k_ct_step(const __grid_constant
     u32 aph = 0;
     bool ok = true;
     for (int it = blockIdx.x; ok && it < items; it += gridDim.x) {
-      const int unit = it / P.mtiles, mt = it % P.mtiles;
-      const int mu = unit % S.units;
+      const int item = it / P.mtiles, mt = it % P.mtiles;
       const long w = (long)mt * CT_M + m;
       if (!__all_sync(0xffffffffu, mbar_wait(acc_full + a, aph, abort_flag))) {
         ok = false;
@@ -300,7 +309,7 @@ __global__ void __launch_bounds__(CT_THREADS, 1) k_ct_step(const __grid_constant
 #pragma unroll
       for (int l = 0; l < 2; ++l) {
         const double q = P.D.q[l], qinv = P.D.qinv[l];
-        const double* cc = P.c + ((size_t)unit * 2 + l) * CT_ROWS + part * 4;
+        const double* cc = P.c + ((size_t)item * 2 + l) * CT_ROWS + part * 4;
 #pragma unroll
         for (int r = 0; r < 4; ++r) {
           const u64 lo = (u64)v[l][0][r] + ((u64)v[l][1][r] << 8) + ((u64)v[l][2][r] << 16);
@@ -309,51 +318,57 @@ __global__ void __launch_bounds__(CT_THREADS, 1) k_ct_step(const __grid_constant
           y[l][r] = __fma_rn(-__dadd_rn(__fma_rn(x, qinv, FP_ROUND), -FP_ROUND), q, x);
         }
       }
-      // Rows part * 4 .. + 3 of the unit: output mask jj, coefficients yy .. (n >= 2),
-      // or masks jj, jj + 1 of two coefficients each (n = 1).
       const int r0 = part * 4;
-      const int jj = S.n >= 8 ? mu / upj : mu * S.G + r0 / n_out;
-      const int yy = S.n >= 8 ? (mu % upj) * CT_ROWS + r0 : r0 % n_out;
-      if (unit >= S.units) {  // body sums, canonical, added over the output masks
+      if (item >= S.units) {  // body sums, canonical, added over the items of the same coefficients
+        const int yy = S.n >= 8 ? (item - S.units) * S.chain / S.half * CT_ROWS + r0 : r0 % n_out;
+        unsigned long long* o = reinterpret_cast<unsigned long long*>(P.body) + (size_t)yy * 2 * P.nlwe + w;
 #pragma unroll
         for (int l = 0; l < 2; ++l) {
-          unsigned long long* o = reinterpret_cast<unsigned long long*>(P.bsk + (w * 2 + l) * P.bsk_stride) + yy;
           u64 b[4];
 #pragma unroll
           for (int r = 0; r < 4; ++r) b[r] = __double2ull_rn(fp_canonical(y[l][r], P.D.q[l], P.D.qinv[l]));
           if (S.n == 1) {
-            atomicAdd(o, b[0] + b[2]);
-            atomicAdd(o + 1, b[1] + b[3]);
-          } else {
-#pragma unroll
-            for (int r = 0; r < 4; ++r) atomicAdd(o + r, b[r]);
+            b[0] += b[2];
+            b[1] += b[3];
           }
+#pragma unroll
+          for (int r = 0; r < 4; ++r)
+            if (S.n > 1 || r < 2) atomicAdd(o + (size_t)(2 * r + l) * P.nlwe, b[r]);
         }
         continue;
       }
+      // Rows part * 4 .. + 3 of the unit: output mask jj, coefficients yy .. (n >= 2),
+      // or masks jj, jj + 1 of two coefficients each (n = 1).
+      const int jj = S.n >= 8 ? item / upj : item * S.G + r0 / n_out;
+      const int yy = S.n >= 8 ? (item % upj) * CT_ROWS + r0 : r0 % n_out;
       u32 f[4][3];
 #pragma unroll
       for (int r = 0; r < 4; ++r) ct_pieces(y[0][r], y[1][r], P.D, f[r]);
       if (P.out) {
         const int which = jj / P.out_half, j2 = jj % P.out_half;
         const long left = P.nlwe - (long)mt * CT_M;
-        const size_t ngb = (size_t)((min(left, (long)CT_M) + 7) / 8) * 128;
+        const u32 ngb = (u32)((min(left, (long)CT_M) + 7) / 8) * 128;
         uint8_t* base = P.out + mt * P.out_tile + (m / 8) * 128 + (m & 7) * 16;
-        int pos = j2 * P.out_kp + which * CT_L * n_out + yy;
+        u32 pos = (u32)(j2 * P.out_kp + which * CT_L * n_out + yy);
+        uint8_t* o = base + (size_t)(pos >> 4) * ngb + (pos & 15);  // n >= 8: s steps by whole 16-byte rows
+        const u32 step = (u32)(n_out >> 4) * ngb;
 #pragma unroll
         for (int i = 0; i < 3; ++i)
 #pragma unroll
-          for (int k = 0; k < CT_LP; ++k, pos += n_out) {
-            u32 d = 0;
-#pragma unroll
-            for (int r = 0; r < 4; ++r) d |= ct_digit(f[r][i], P.D.base) << (8 * r);
-            uint8_t* o = base + (size_t)(pos >> 4) * ngb + (pos & 15);
-            if (S.n == 1) {
-              *reinterpret_cast<uint16_t*>(o) = (uint16_t)d;
-              const int p2 = pos + P.out_kp;
-              *reinterpret_cast<uint16_t*>(base + (size_t)(p2 >> 4) * ngb + (p2 & 15)) = (uint16_t)(d >> 16);
-            } else {
+          for (int k = 0; k < CT_LP; ++k) {
+            const u32 d = ct_digit(f[0][i], P.D.base) | ct_digit(f[1][i], P.D.base) << 8 |
+                          ct_digit(f[2][i], P.D.base) << 16 | ct_digit(f[3][i], P.D.base) << 24;
+            if (S.n >= 8) {
               *reinterpret_cast<u32*>(o) = d;
+              o += step;
+            } else if (S.n > 1) {
+              *reinterpret_cast<u32*>(base + ((pos >> 4) * ngb + (pos & 15))) = d;
+              pos += n_out;
+            } else {
+              *reinterpret_cast<uint16_t*>(base + ((pos >> 4) * ngb + (pos & 15))) = (uint16_t)d;
+              const u32 p2 = pos + P.out_kp;
+              *reinterpret_cast<uint16_t*>(base + ((p2 >> 4) * ngb + (p2 & 15))) = (uint16_t)(d >> 16);
+              pos += n_out;
             }
           }
       } else {
@@ -400,10 +415,9 @@ __global__ void k_ct_planes(const u64* __restrict__ key, CtStep st, DevRing R, u
   const int k16 = (int)((gid >> 5) % k16s), unit = (int)((gid >> 5) / k16s);
   const int mb = unit >= st.units, mu = unit - mb * st.units;
   const int n_out = 2 * st.n, L = CT_L;
-  const int upj = st.n >= 8 ? n_out / CT_ROWS : 1;
   const int g_row = st.n >= 8 ? 0 : r / n_out;
-  const int j = st.n >= 8 ? mu / upj : mu * st.G + g_row;
-  const int y = st.n >= 8 ? (mu % upj) * CT_ROWS + r : r % n_out;
+  const int j = ct_first_mask(st, unit) + g_row;
+  const int y = st.n >= 8 ? (mb ? mu / st.half : mu % (n_out / CT_ROWS)) * CT_ROWS + r : r % n_out;
   const DevMod& m = R.m[l];
   const u64 inv = l ? inv1 : inv0;
   u32 word[5][4];
@@ -435,16 +449,18 @@ __global__ void k_ct_planes(const u64* __restrict__ key, CtStep st, DevRing R, u
   }
 }
 
-// Column constants o * (sum of the column's key entries) mod q_l, one warp per (unit, limb,
-// row): read back from the planes.
+// Column constants o * (sum of the item's key entries of the column) mod q_l, one warp per
+// (item, limb, row): read back from the planes.
 __global__ void k_ct_consts(const uint8_t* __restrict__ planes, CtStep st, DevRing R, u32 o, double* __restrict__ out) {
   const long gid = ((long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
-  if (gid >= (long)2 * st.units * 32) return;
-  const int r = (int)(gid & 15), l = (int)((gid >> 4) & 1), unit = (int)(gid >> 5);
+  if (gid >= (long)st.items() * 32) return;
+  const int r = (int)(gid & 15), l = (int)((gid >> 4) & 1), item = (int)(gid >> 5);
+  const int unit0 = item < st.units ? item : st.units + (item - st.units) * st.chain;
+  const int len = item < st.units ? 1 : st.chain;
   u64 sum[5] = {0, 0, 0, 0, 0};
-  for (int k16 = lane; k16 < st.chunks * (CT_KC / 16); k16 += 32) {
-    const uint8_t* base = planes + ((size_t)unit * st.chunks + k16 / (CT_KC / 16)) * CT_STAGE_B +
+  for (int k16 = lane; k16 < len * st.chunks * (CT_KC / 16); k16 += 32) {
+    const uint8_t* base = planes + ((size_t)unit0 * st.chunks + k16 / (CT_KC / 16)) * CT_STAGE_B +
                           (size_t)(k16 % (CT_KC / 16)) * (CT_N / 8) * 128;
 #pragma unroll
     for (int k = 0; k < 5; ++k) {
@@ -462,7 +478,7 @@ __global__ void k_ct_consts(const uint8_t* __restrict__ planes, CtStep st, DevRi
     const DevMod& m = R.m[l];
     u64 acc = 0;
     for (int k = 4; k >= 0; --k) acc = reduce64((acc << 8) + reduce64(sum[k], m), m);
-    out[((size_t)unit * 2 + l) * CT_ROWS + r] = (double)mulmod(acc, o, m);
+    out[((size_t)item * 2 + l) * CT_ROWS + r] = (double)mulmod(acc, o, m);
   }
 }
 
@@ -522,7 +538,7 @@ void ct_prepare(Server& s) {
     st.b_off = bytes;
     st.c_off = consts;
     bytes += (size_t)2 * st.units * st.chunks * CT_STAGE_B;
-    consts += (size_t)2 * st.units * 2 * CT_ROWS;
+    consts += (size_t)st.items() * 2 * CT_ROWS;
     steps.push_back(st);
   }
   ct_prepare_device();
@@ -538,7 +554,7 @@ void ct_prepare(Server& s) {
     k_ct_planes<<<(unsigned)((threads + 255) / 256), 256, 0, s.stream>>>(s.cascade_eval.p + k * step_len, st, s.r1, inv0,
                                                                         inv1, planes);
     VIA_LAUNCHED();
-    const long warps = (long)2 * st.units * 32;
+    const long warps = (long)st.items() * 32;
     k_ct_consts<<<(unsigned)((warps * 32 + 255) / 256), 256, 0, s.stream>>>(
         planes, st, s.r1, D.o, reinterpret_cast<double*>(s.ct_consts.p) + st.c_off);
     VIA_LAUNCHED();
@@ -546,7 +562,7 @@ void ct_prepare(Server& s) {
   s.ct_steps = K;
 }
 
-void ct_run(Server& s, const u64* d_query, long nlwe, uint8_t* da, uint8_t* db, int8_t* dig8, u64* bsk,
+void ct_run(Server& s, const u64* d_query, long nlwe, uint8_t* da, uint8_t* db, int8_t* dig8, u64* body,
             cudaStream_t st) {
   const via_params& p = s.prm;
   const int n1 = (int)p.n1;
@@ -569,8 +585,7 @@ void ct_run(Server& s, const u64* d_query, long nlwe, uint8_t* da, uint8_t* db, 
     P.c = reinterpret_cast<const double*>(s.ct_consts.p) + c_off;
     P.out = last ? nullptr : db;
     P.dig8 = dig8;
-    P.bsk = bsk + (2L << k) - 2;
-    P.bsk_stride = 2L * n1;
+    P.body = body + ((2L << k) - 2) * 2 * nlwe;
     P.err = reinterpret_cast<int*>(s.fd_err.p);
     P.nlwe = nlwe;
     P.a_tile = (size_t)CT_M * cur.half * cur.kp;
@@ -578,11 +593,11 @@ void ct_run(Server& s, const u64* d_query, long nlwe, uint8_t* da, uint8_t* db, 
     P.mtiles = mtiles;
     P.out_kp = nxt.kp;
     P.out_half = nxt.half;
-    const int items = 2 * cur.units * mtiles;
+    const int items = cur.items() * mtiles;
     k_ct_step<<<std::min(items, s.fd.grid), CT_THREADS, CT_SMEM, st>>>(P);
     VIA_LAUNCHED();
     b_off += (size_t)2 * cur.units * cur.chunks * CT_STAGE_B;
-    c_off += (size_t)2 * cur.units * 2 * CT_ROWS;
+    c_off += (size_t)cur.items() * 2 * CT_ROWS;
     std::swap(da, db);
     cur = nxt;
   }

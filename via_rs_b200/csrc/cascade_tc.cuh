@@ -39,8 +39,10 @@ struct CtStep {
   int G;          // output masks per unit (units of n < 8 hold several)
   int chunks;     // pipeline stages per unit
   int units;      // mask units; as many body units follow
+  int chain;      // body units summed in one accumulator: body items are units / chain
   size_t b_off;   // byte offset of its units in the key planes
-  size_t c_off;   // its column constants: [unit][2][16] doubles
+  size_t c_off;   // its column constants: [item][2][16] doubles
+  __host__ __device__ int items() const { return units + units / chain; }
 };
 
 inline CtStep ct_step(int n1, int n) {
@@ -51,6 +53,10 @@ inline CtStep ct_step(int n1, int n) {
   s.G = n < 8 ? 8 / n : 1;
   s.chunks = (s.G * s.kp + CT_KC - 1) / CT_KC;
   s.units = n1 / CT_ROWS;
+  // Body sums run over every output mask, so units of the same coefficients chain in
+  // one accumulator: fewer epilogues and atomics, and with 128 mask units one item per SM
+  // for a single tile. Longer chains of the larger steps would outlast a mask item.
+  s.chain = n >= 128 ? 1 : (128 / n < 8 ? 128 / n : 8);
   return s;
 }
 
@@ -85,9 +91,12 @@ void ct_prepare(Server& s);
 void ct_prepare_device();
 // Runs the leading ct.steps steps for nlwe LWEs of d_query ([lwe][nl (n1 + 1)]): leaves the
 // next step's signed digits in dig8 ([lwe][rank][L][degree]) and adds every step's body
-// sums (coefficient form) to bsk ([lwe][nl][2 n1], zeroed by the caller). da and db are
+// sums (coefficient form) to body[((2 n - 2 + y) * 2 + limb) * nlwe + lwe] (n the step's
+// input degree, y < 2 n; ct_body_words(steps) words per LWE, zeroed by the caller), so that
+// the lanes of a warp, which are LWEs, add to consecutive words. da and db are
 // digit buffers of ct_digit_bytes(n1) bytes per LWE, LWEs rounded up to 8.
-void ct_run(Server& s, const u64* d_query, long nlwe, uint8_t* da, uint8_t* db, int8_t* dig8, u64* bsk,
+void ct_run(Server& s, const u64* d_query, long nlwe, uint8_t* da, uint8_t* db, int8_t* dig8, u64* body,
             cudaStream_t st);
+inline size_t ct_body_words(int steps) { return (((size_t)2 << steps) - 2) * 2; }
 
 }  // namespace via

@@ -591,9 +591,11 @@ __global__ void k_cascade_body(const u64* __restrict__ body_in, const u64* __res
 }
 
 // Assemble cascade outputs into RLWEs [lwe][2][nl][n1]. The first k0 steps' body sums
-// are in coefficient form: step k's coefficient c sits at coefficient c n1 / 2^(k+1).
-__global__ void k_pack_rlwe(const u64* masks, const u64* body, const u64* __restrict__ bsk, int k0, int K, long nlwe,
-                            int n1, int nl, DevRing Rg, u64* out) {
+// are in coefficient form (cascade_tc.cuh: gemm[((2^(k+1) - 2 + c) * 2 + l) * stride + lwe],
+// pointing at the first of these LWEs): step k's coefficient c sits at coefficient
+// c n1 / 2^(k+1).
+__global__ void k_pack_rlwe(const u64* masks, const u64* body, const u64* __restrict__ gemm, long stride, int k0, int K,
+                            long nlwe, int n1, int nl, DevRing Rg, u64* out) {
   long per = (long)nl * n1;
   long gid = (long)blockIdx.x * blockDim.x + threadIdx.x;
   if (gid >= nlwe * per) return;
@@ -604,7 +606,7 @@ __global__ void k_pack_rlwe(const u64* masks, const u64* body, const u64* __rest
   const int l = rem / n1, i = rem % n1;
   for (int k = k0 - 1; k >= 0 && (i & ((1 << (K - 1 - k)) - 1)) == 0; --k) {
     const DevMod& m = Rg.m[l];
-    b = submod(b, reduce64(bsk[(w * nl + l) * 2 * n1 + (2 << k) - 2 + (i >> (K - 1 - k))], m), m.q);
+    b = submod(b, reduce64(gemm[(long)(((2 << k) - 2 + (i >> (K - 1 - k))) * 2 + l) * stride + w], m), m.q);
   }
   out[(2 * w + 1) * per + rem] = b;
 }
@@ -701,6 +703,7 @@ struct Workspace {
   int bmax = 1;              // queries the buffers are sized for
   // Cascade.
   DevBuf c_masks_a, c_masks_b, c_body_a, c_body_b, c_digits, c_P, c_bsum, c_rlwe;
+  DevBuf c_gemm_body;  // body sums of the GEMM steps (cascade_tc.cuh)
   DevBuf c_dig8;   // 8-bit cascade / conversion-key digits [lwe][n1 * L_CK] bytes (base <= 255)
   // RLWE -> RGSW.
   // RGSWs grouped by use: the DMux bits of every query ([q][nd]), then the
@@ -785,6 +788,7 @@ static size_t workspace_build(Server& s, int bmax, Workspace* w, bool count_only
   A(w->c_digits, std::max(nlwe * (s.r1.ntt ? 1 : 2) * n1 * Lck * nl, tc_words));
   A(w->c_P, s.r1.ntt ? 0 : nlwe * 2 * n1 * 2 * nl);
   A(w->c_bsum, 2 * nlwe * n1 * nl);
+  A(w->c_gemm_body, s.ct_steps ? (long)ct_body_words(s.ct_steps) * nlwe : 0);
   A(w->c_dig8, p.ck_base <= 255 && s.r1.ntt ? (nlwe * n1 * Lck + 7) / 8 : 0);
   A(w->c_rlwe, nlwe * 2 * n1 * nl);
   A(w->g_digits, nlwe * Lck * nl * n1);
@@ -899,7 +903,7 @@ static void mod_switch(const DevRing& S, const u64* in, const DevRing& D, u64* o
 }
 
 // Step 1: QueryDecomp (query_decomp.rs:39-95) of `nlwe` consecutive LWEs, the
-// first being LWE lwe0 of the workspace (LWE-indexed buffers are used from that
+// first being LWE lwe0 of the nlwe_all in the workspace (LWE-indexed buffers are used from that
 // LWE's region on), forming the RGSWs of `nbits` query bits starting at bit
 // bit0 -> rgsw_q1 [bit][2L][2][nl][n1] (coefficient form). Disjoint (lwe0,
 // nlwe) ranges may run concurrently on different streams. Servers with GEMM
@@ -907,14 +911,15 @@ static void mod_switch(const DevRing& S, const u64* in, const DevRing& D, u64* o
 // cascade continues from their digits and body sums.
 static void cascade_gemm(Server& s, Workspace& w, const u64* d_query, long nlwe, cudaStream_t st) {
   const long n1 = s.prm.n1;
+  u64* body = w.c_gemm_body.p;
   uint8_t* da = reinterpret_cast<uint8_t*>(w.c_digits.p);
   uint8_t* db = da + ct_digit_bytes((int)n1) * ((nlwe + 7) / 8 * 8);
-  VIA_CUDA(cudaMemsetAsync(w.c_bsum.p, 0, (size_t)nlwe * 2 * n1 * s.r1.nl * 8, st));
-  ct_run(s, d_query, nlwe, da, db, reinterpret_cast<int8_t*>(w.c_dig8.p), w.c_bsum.p, st);
+  VIA_CUDA(cudaMemsetAsync(body, 0, ct_body_words(s.ct_steps) * nlwe * 8, st));
+  ct_run(s, d_query, nlwe, da, db, reinterpret_cast<int8_t*>(w.c_dig8.p), body, st);
 }
 
-static void query_decomp_range(Server& s, Workspace& w, const u64* d_query, long lwe0, long nlwe, long bit0,
-                               long nbits, cudaStream_t st) {
+static void query_decomp_range(Server& s, Workspace& w, const u64* d_query, long nlwe_all, long lwe0, long nlwe,
+                               long bit0, long nbits, cudaStream_t st) {
   const via_params& p = s.prm;
   const DevRing& R = s.r1;
   const int n1 = p.n1, nl = R.nl, L = p.l_ck;
@@ -935,8 +940,8 @@ static void query_decomp_range(Server& s, Workspace& w, const u64* d_query, long
   if (!k0) {
     k_lwe_to_mlwe<<<blocks(nlwe * nl * (n1 + 1)), 256, 0, st>>>(query, n1, nl, nlwe, mi, bi);
     VIA_LAUNCHED();
-    if (R.ntt) VIA_CUDA(cudaMemsetAsync(bsk, 0, (size_t)nlwe * 2 * lwe_n * 8, st));
   }
+  if (R.ntt) VIA_CUDA(cudaMemsetAsync(bsk, 0, (size_t)nlwe * 2 * lwe_n * 8, st));
   const u64 step_len = (u64)2 * n1 * L * 2 * nl;
   int k = k0;
   for (int n_in = 1 << k0; n_in < n1; n_in <<= 1, ++k) {
@@ -1002,7 +1007,8 @@ static void query_decomp_range(Server& s, Workspace& w, const u64* d_query, long
     from_eval(R, bo, n1, nlwe * nl, st);
     std::swap(bi, bo);
   }
-  k_pack_rlwe<<<blocks(nlwe * nl * n1), 256, 0, st>>>(mi, bi, bsk, k0, k, nlwe, n1, nl, R, rlwe);
+  k_pack_rlwe<<<blocks(nlwe * nl * n1), 256, 0, st>>>(mi, bi, w.c_gemm_body.p + lwe0, nlwe_all, k0, k, nlwe, n1, nl, R,
+                                                      rlwe);
   VIA_LAUNCHED();
   // RLWE -> RGSW with the conversion key (prim/gates/convert.rs:162-178); the
   // final rank-1 masks are already contiguous [lwe][nl][n1] in `mi`.
@@ -1368,14 +1374,14 @@ void answer_device_stages(Server& s, Workspace& w, const u64* d_query, int nq, u
   if (split) {
     VIA_CUDA(cudaEventRecord(w.ev_fork, st));
     VIA_CUDA(cudaStreamWaitEvent(w.side, w.ev_fork, 0));
-    query_decomp_range(s, w, qsrc, B * lwe_a, nlwe_all - B * lwe_a, B * nd, B * nb, w.side);
+    query_decomp_range(s, w, qsrc, nlwe_all, B * lwe_a, nlwe_all - B * lwe_a, B * nd, B * nb, w.side);
     mod_switch(s.r1, rgsw_b1, s.r2, rgsw_b2, B * nb * 2 * L * 2, n1, w.side);
     to_eval(s.r2, rgsw_b2, n1, B * nb * 2 * L * 2, w.side);
     VIA_CUDA(cudaEventRecord(w.ev_join, w.side));
-    query_decomp_range(s, w, qsrc, 0, B * lwe_a, 0, B * nd, st);
+    query_decomp_range(s, w, qsrc, nlwe_all, 0, B * lwe_a, 0, B * nd, st);
     to_eval(s.r1, w.rgsw_q1.p, n1, B * nd * 2 * L * 2 * nl, st);
   } else {
-    query_decomp_range(s, w, qsrc, 0, nlwe_all, 0, B * w.nbits, st);
+    query_decomp_range(s, w, qsrc, nlwe_all, 0, nlwe_all, 0, B * w.nbits, st);
     if (stop_stage == 1) return copy_out(w.c_rlwe.p, (size_t)w.nlwe * 2 * nl * n1);
     if (stop_stage == 2) return copy_out(w.rgsw_q1.p, (size_t)w.nbits * rgsw1);  // one query: bit order
 
