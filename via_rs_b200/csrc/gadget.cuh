@@ -153,6 +153,10 @@ struct Gadget {
   int c32;
   Div64 dc32;     // B^c32
   u32 bmagic;     // floor((2^32 - 1) / B)
+  // Splits in double precision (gadget_fp.cuh), where S < 2^47 and the limbs are odd:
+  bool fp;        // allowed
+  double dS, dB, dBinv;
+  double ys[2];   // two limbs: (Q / q_l)^-1 mod q_l
 };
 
 inline Gadget make_gadget(u64 base, int L, u128 Q, u64 q0 = 0, u64 q1 = 0) {
@@ -213,6 +217,14 @@ inline Gadget make_gadget(u64 base, int L, u128 Q, u64 q0 = 0, u64 q1 = 0) {
   g.c32 = c32;
   g.dc32 = make_div64(b32);
   g.bmagic = (u32)(0xFFFFFFFFull / base);
+  g.dS = dS;
+  g.dB = (double)base;
+  g.dBinv = 1.0 / (double)base;
+  g.fp = S < ((u128)1 << 47) && (u64)Q % 2 == 1 && (g.small || (g.mode == 1 && q0 < (1ull << 44) && q1 < (1ull << 44)));
+  if (g.fp && g.mode == 1) {
+    g.ys[0] = (double)h_inv(q1 % q0, q0);
+    g.ys[1] = (double)h_inv(q0 % q1, q1);
+  }
   return g;
 }
 

@@ -97,6 +97,26 @@ NttTableHost make_ntt_table(u64 q, int nmax) {
     h.dev.ninv_sh[l] = (u64)(((u128)ninv << 64) / q);
     h.dev.ninv_d[l] = (double)ninv;
   }
+  if (nmax >= 8) {
+    // psi[k] = psi^bitrev(k) is a prefix table: psi[1..7] serve every degree from 8 up.
+    const u64 w1 = host[1], w2 = host[2], w3 = host[3];
+    double* d = h.dev.d8;
+    auto neg = [&](u64 x) { return -(double)x; };
+    d[0] = (double)w1;
+    d[1] = (double)w2;
+    d[2] = (double)h_mulmod(w1, w2, q);
+    d[3] = (double)w3;
+    d[4] = (double)h_mulmod(w1, w3, q);
+    for (int i = 0; i < 4; ++i) {
+      const u64 w = host[4 + i], v = i < 2 ? w2 : w3;
+      const u64 a = h_mulmod(w, w1, q), b = h_mulmod(w, v, q), c = h_mulmod(a, v, q);
+      double* k = d + 5 + 4 * i;
+      k[0] = (double)w;                                  // x1
+      k[1] = i < 2 ? (double)a : neg(a);                 // x5: +- w1
+      k[2] = i % 2 ? neg(b) : (double)b;                 // x3: +- v
+      k[3] = (i < 2) == (i % 2 == 0) ? (double)c : neg(c);  // x7: the product of both signs
+    }
+  }
   h.valid = true;
   return h;
 }
@@ -211,111 +231,107 @@ __global__ void __launch_bounds__(ntt_cta<LOGN>()) k_ntt_reg_i8(const int8_t* __
 
 // ---------------------------------------------------------------------------
 // The register-resident transforms in double precision (ntt_fp.cuh), for primes
-// below 2^44: the same layouts and phases as ntt_phases, exact integer
-// arithmetic on doubles. Inputs are residues below 2^47 (larger values are
-// reduced first); outputs:
-//  * forward: canonical residues, or (LAZY) nonnegative residues below
-//    (1.125 LOGN + 3) q <= (1 + 2 LOGN) q, the integer kernel's lazy bound;
-//    forward values stay within |input| + 0.5625 LOGN q of zero;
-//  * inverse: canonical residues. Inverse values at most double per stage; for
-//    q above 2^35 every phase boundary first reduces them to within q/2, so a
-//    phase of three stages ends below 4 q and every product stays exact.
-// I8: the input is a polynomial of signed 8-bit digits.
+// below 2^44: exact integer arithmetic on doubles. Inputs are residues below 2^47
+// (larger values are reduced first); outputs:
+//  * forward: canonical residues, or (LAZY) nonnegative residues below 2 q;
+//  * inverse: canonical residues;
+//  * of digits (k_ntt_fp_i8): the signed doubles themselves (DOUT), within
+//    (1016 + 0.5625 LOGN) q of zero, or nonnegative residues below 2 q.
+//
+// Issue-bound on the FP64 pipe: 8 operations a butterfly, 11 * 4 of them for a thread's eight
+// elements at n = 2048. Every thread moves its consecutive elements by 32-byte accesses
+// where the caller's buffer is aligned to them.
 // ---------------------------------------------------------------------------
-// DOUT: the (forward, lazy) outputs are stored as the signed doubles themselves.
-template <int LOGN, bool INV, int P, bool LAZY, bool I8, bool DOUT = false>
-__device__ __forceinline__ void ntt_fp_phases(double (&e)[8], int tid, const NttTable& T, u64* g, double* sm,
-                                              int sbase, bool active, const int8_t* gin) {
-  using Ph = NttPhaseFp<LOGN, INV, P>;
-  using Ix = NttPhase<LOGN, INV, P>;
-  constexpr int NPH = (LOGN + 2) / 3;
-  const double q = T.qd, qinv = T.qinv;
-  if constexpr (P == 0) {
-    if constexpr (I8) {
-#pragma unroll
-      for (int v = 0; v < 8; ++v) e[v] = active ? (double)gin[Ix::index(v, tid)] : 0.0;
-    } else {
-#pragma unroll
-      for (int v = 0; v < 8; ++v) {
-        u64 x = active ? g[Ix::index(v, tid)] : 0;
-        if (x >= (1ull << 47)) x %= T.q;
-        e[v] = __ull2double_rn(x);
-      }
-    }
-  } else {
-    __syncthreads();
-#pragma unroll
-    for (int v = 0; v < 8; ++v) e[v] = sm[swz(sbase + Ix::index(v, tid))];
-    if (INV && q > 34359738368.0) {  // q > 2^35: restart the inverse's growth at q/2
-#pragma unroll
-      for (int v = 0; v < 8; ++v)
-        e[v] = __fma_rn(-__dadd_rn(__fma_rn(e[v], qinv, FP_ROUND), -FP_ROUND), q, e[v]);
-    }
-  }
-  Ph::run(e, tid, T);
-  if constexpr (P == NPH - 1) {
-    if constexpr (INV) {
-#pragma unroll
-      for (int v = 0; v < 8; ++v) e[v] = fp_canonical(fp_mulmod(e[v], T.ninv_d[LOGN], q, qinv), q, qinv);
-    } else if constexpr (DOUT) {
-      if (active) {
-        double* gd = reinterpret_cast<double*>(g);
-#pragma unroll
-        for (int v = 0; v < 8; ++v) gd[Ix::index(v, tid)] = e[v];
-      }
-      return;
-    } else if constexpr (LAZY) {
-      constexpr int OFF = (9 * LOGN + 15) / 16 + 1;  // ceil(0.5625 LOGN) + 1
-      const double off = (double)OFF * q;
-#pragma unroll
-      for (int v = 0; v < 8; ++v) e[v] = __dadd_rn(e[v], off);
-    } else {
-#pragma unroll
-      for (int v = 0; v < 8; ++v) e[v] = fp_canonical(e[v], q, qinv);
-    }
-    if (active) {
-#pragma unroll
-      for (int v = 0; v < 8; ++v) g[Ix::index(v, tid)] = __double2ull_rn(e[v]);
-    }
-  } else {
-    __syncthreads();
-#pragma unroll
-    for (int v = 0; v < 8; ++v) sm[swz(sbase + Ix::index(v, tid))] = e[v];
-    ntt_fp_phases<LOGN, INV, P + 1, LAZY, false, DOUT>(e, tid, T, g, sm, sbase, active, nullptr);
-  }
-}
-
 template <int LOGN, bool INV, bool LAZY = false>
 __global__ void __launch_bounds__(ntt_cta<LOGN>()) k_ntt_fp(u64* __restrict__ data, int nl, long segments,
-                                                            NttTable t0, NttTable t1) {
+                                                            const __grid_constant__ NttTable t0,
+                                                            const __grid_constant__ NttTable t1) {
   constexpr int n = 1 << LOGN;
   constexpr int TPS = n / 8;
   constexpr int SPC = ntt_cta<LOGN>() / TPS;
+  using L0 = NttPhase<LOGN, false, 0>;
   __shared__ double sm[ntt_cta<LOGN>() * 8];
   const int seg_local = threadIdx.x / TPS;
   const int tid = threadIdx.x % TPS;
   const long seg = (long)blockIdx.x * SPC + seg_local;
   const bool active = seg < segments;
   const NttTable& T = (nl == 2 && (seg & 1)) ? t1 : t0;
+  const double q = T.qd, qinv = T.qinv;
+  u64* g = data + seg * n;
+  const bool wide = (reinterpret_cast<uintptr_t>(data) & 31) == 0;
+  u64 x[8];
+#pragma unroll
+  for (int v = 0; v < 8; ++v) x[v] = 0;
+  if (active) {
+    if (!INV) {
+#pragma unroll
+      for (int v = 0; v < 8; ++v) x[v] = g[L0::index(v, tid)];
+    } else if (wide) {
+      ld8(g + 8 * tid, x);
+    } else {
+#pragma unroll
+      for (int v = 0; v < 8; ++v) x[v] = g[8 * tid + v];
+    }
+  }
   double e[8];
-  ntt_fp_phases<LOGN, INV, 0, LAZY, false>(e, tid, T, data + seg * n, sm, seg_local * n, active, nullptr);
+#pragma unroll
+  for (int v = 0; v < 8; ++v) {
+    if (x[v] >= (1ull << 47)) x[v] %= T.q;
+    e[v] = fp_from_u64(x[v]);
+  }
+  if constexpr (!INV) {
+    fp_forward<LOGN>(e, tid, T, sm, seg_local * n);
+  } else {
+    fp_inverse<LOGN>(e, tid, T, sm, seg_local * n);
+#pragma unroll
+    for (int v = 0; v < 8; ++v) e[v] = fp_mulmod(e[v], T.ninv_d[LOGN], q, qinv);
+  }
+#pragma unroll
+  for (int v = 0; v < 8; ++v) {
+    if constexpr (LAZY)
+      x[v] = fp_to_u64(__dadd_rn(fp_reduce(e[v], q, qinv), q));
+    else
+      x[v] = fp_to_u64(fp_canonical(e[v], q, qinv));
+  }
+  if (!active) return;
+  if (INV) {
+#pragma unroll
+    for (int v = 0; v < 8; ++v) g[L0::index(v, tid)] = x[v];
+  } else if (wide) {
+    st8(g + 8 * tid, x);
+  } else {
+#pragma unroll
+    for (int v = 0; v < 8; ++v) g[8 * tid + v] = x[v];
+  }
 }
 
+// `out` is the library's own buffer (32-byte aligned).
 template <int LOGN, bool DOUT = false>
 __global__ void __launch_bounds__(ntt_cta<LOGN>()) k_ntt_fp_i8(const int8_t* __restrict__ din, u64* __restrict__ out,
-                                                               int nl, long segments, NttTable t0, NttTable t1) {
+                                                               int nl, long segments,
+                                                               const __grid_constant__ NttTable t0,
+                                                               const __grid_constant__ NttTable t1) {
   constexpr int n = 1 << LOGN;
   constexpr int TPS = n / 8;
   constexpr int SPC = ntt_cta<LOGN>() / TPS;
+  using L0 = NttPhase<LOGN, false, 0>;
   __shared__ double sm[ntt_cta<LOGN>() * 8];
   const int seg_local = threadIdx.x / TPS;
   const int tid = threadIdx.x % TPS;
   const long seg = (long)blockIdx.x * SPC + seg_local;
   const bool active = seg < segments;
   const NttTable& T = (nl == 2 && (seg & 1)) ? t1 : t0;
+  const int8_t* gin = din + (active ? seg / nl : 0) * n;
   double e[8];
-  ntt_fp_phases<LOGN, false, 0, true, true, DOUT>(e, tid, T, out + seg * n, sm, seg_local * n, active,
-                                                  din + (active ? seg / nl : 0) * n);
+#pragma unroll
+  for (int v = 0; v < 8; ++v) e[v] = active ? (double)gin[L0::index(v, tid)] : 0.0;
+  fp_forward_digits<LOGN>(e, tid, T, sm, seg_local * n, T.qd <= FP_DIGIT_Q);
+  if (!active) return;
+  u64 x[8];
+#pragma unroll
+  for (int v = 0; v < 8; ++v)
+    x[v] = DOUT ? (u64)__double_as_longlong(e[v]) : fp_to_u64(__dadd_rn(fp_reduce(e[v], T.qd, T.qinv), T.qd));
+  st8(out + seg * n + 8 * tid, x);
 }
 
 // n = 2 and 4 on 8-bit digits, double outputs: one thread per segment.

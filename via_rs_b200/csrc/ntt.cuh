@@ -30,6 +30,11 @@ struct NttTable {
   const double* ipsi_d;
   double qd, qinv;  // q and a rounded 1 / q
   double ninv_d[NTT_MAX_LOGN + 1];
+  // Products of psi[1..7] for the dense first phase on digits (fp_digit_phase), with
+  // w_k = psi[k]: w1; w2, w1 w2; w3, w1 w3; then for w = w4, w5, w6, w7 the four of
+  // {w, w w1, w v, w w1 v} (v = w2 for the first two, w3 for the others) with the signs of
+  // the sub-block.
+  double d8[21];
 };
 
 // Host owner of the device tables of one prime.
@@ -132,55 +137,6 @@ __device__ __forceinline__ u64 ntt_canonical(u64 x, const NttTable& T) {
   return mul_shoup(x, T.ninv[0], T.ninv_sh[0], T.q);
 }
 
-// Forward transform of a segment whose residues a thread already holds in the
-// phase-0 layout (NttPhase<LOGN,false,0>::index); leaves them (exact) in the
-// layout of the last phase. `ssm` is an n-residue shared-memory exchange area
-// of one segment, addressed through swz().
-// With LAZY the outputs stay below (1 + 2 LOGN) q instead of being reduced,
-// for callers that reduce a sum of products once at the end.
-template <int LOGN, int P = 0, bool LAZY = false>
-__device__ __forceinline__ void ntt_forward_regs(u64 (&e)[8], int tid, const NttTable& T, u64* ssm) {
-  using Ph = NttPhase<LOGN, false, P>;
-  constexpr int NPH = (LOGN + 2) / 3;
-  Ph::run(e, tid, T);
-  if constexpr (P + 1 < NPH) {
-    using Nx = NttPhase<LOGN, false, P + 1>;
-    __syncthreads();
-#pragma unroll
-    for (int v = 0; v < 8; ++v) ssm[swz(Ph::index(v, tid))] = e[v];
-    __syncthreads();
-#pragma unroll
-    for (int v = 0; v < 8; ++v) e[v] = ssm[swz(Nx::index(v, tid))];
-    ntt_forward_regs<LOGN, P + 1, LAZY>(e, tid, T, ssm);
-  } else if constexpr (!LAZY) {
-#pragma unroll
-    for (int v = 0; v < 8; ++v) e[v] = ntt_canonical(e[v], T);
-  }
-}
-
-// Inverse transform (Gentleman-Sande, then the n^-1 scaling) of a segment whose
-// eval-form residues a thread holds in the layout NttPhase<LOGN,true,0>::index;
-// leaves the coefficients in the layout of the last inverse phase.
-template <int LOGN, int P = 0>
-__device__ __forceinline__ void ntt_inverse_regs(u64 (&e)[8], int tid, const NttTable& T, u64* ssm) {
-  using Ph = NttPhase<LOGN, true, P>;
-  constexpr int NPH = (LOGN + 2) / 3;
-  Ph::run(e, tid, T);
-  if constexpr (P + 1 < NPH) {
-    using Nx = NttPhase<LOGN, true, P + 1>;
-    __syncthreads();
-#pragma unroll
-    for (int v = 0; v < 8; ++v) ssm[swz(Ph::index(v, tid))] = e[v];
-    __syncthreads();
-#pragma unroll
-    for (int v = 0; v < 8; ++v) e[v] = ssm[swz(Nx::index(v, tid))];
-    ntt_inverse_regs<LOGN, P + 1>(e, tid, T, ssm);
-  } else {
-#pragma unroll
-    for (int v = 0; v < 8; ++v) e[v] = mul_shoup(e[v], T.ninv[LOGN], T.ninv_sh[LOGN], T.q);
-  }
-}
-
 // Builds tables for q (prime, 2*nmax | q-1). Returns valid=false otherwise.
 NttTableHost make_ntt_table(u64 q, int nmax);
 void free_ntt_table(NttTableHost& t);
@@ -200,8 +156,8 @@ void ntt_forward_lazy(u64* data, int n, int nl, long segments, const NttTable& t
 // polynomial s / nl) reads din + (s / nl) * n and writes out + s * n.
 void ntt_forward_i8_lazy(const int8_t* din, u64* out, int n, int nl, long segments, const NttTable& t0,
                          const NttTable& t1, cudaStream_t st);
-// The same with signed double outputs (within 0.5625 log2(n) q + 127 of zero,
-// exact integers), for the double-precision multiply-accumulates; primes below 2^44.
+// The same with signed double outputs (exact integers below 2^48), for the
+// double-precision multiply-accumulates; primes below 2^44, `out` 32-byte aligned.
 void ntt_forward_i8_fp(const int8_t* din, double* out, int n, int nl, long segments, const NttTable& t0,
                        const NttTable& t1, cudaStream_t st);
 // Whether the double-precision transforms serve these primes (both below 2^44).

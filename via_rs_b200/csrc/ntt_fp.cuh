@@ -15,11 +15,11 @@
 // itself exact. Explicit _rn intrinsics keep the compiler from contracting or
 // reassociating any step.
 //
-// Bounds (q < 2^36, n <= 4096): forward butterflies (a, c) -> (a + t, a - t),
-// t = fp_mulmod(c, w), grow by at most 0.5625 q per stage; inverse butterflies
-// (a, c) -> (a + c, fp_mulmod(a - c, w)) at most double per stage, so inputs
-// below q stay below 2^12 q < 2^48 after twelve stages. The inverse ends with
-// an fp_mulmod by n^-1.
+// Bounds: forward butterflies (a, c) -> (a + t, a - t), t = fp_mulmod(c, w), grow by at
+// most 0.5625 q per stage; inverse butterflies (a, c) -> (a + c, fp_mulmod(a - c, w)) at
+// most double per stage, so inputs below q of a prime below 2^36 stay below 2^12 q < 2^48
+// after twelve stages. Larger primes bring the values back within q / 2 on the way
+// (fp_inverse). The inverse ends with an fp_mulmod by n^-1.
 #pragma once
 #include "ntt.cuh"
 
@@ -43,98 +43,208 @@ __device__ __forceinline__ double fp_canonical(double x, double q, double qinv) 
   return r;
 }
 
-// One phase of the transform: the butterflies of NttPhase<LOGN, INV, P> on
-// doubles, with the same sub-block layout (NttPhase::index).
-template <int LOGN, bool INV, int P>
-struct NttPhaseFp {
-  using Ix = NttPhase<LOGN, INV, P>;
-  static constexpr int n = Ix::n, S0 = Ix::S0, R = Ix::R, NSUB = Ix::NSUB, STRIDE = Ix::STRIDE;
+// Integers below 2^52 to and from doubles, exactly, without the conversion unit: the
+// double 2^52 + x has the bit pattern 0x4330000000000000 | x.
+__device__ __forceinline__ double fp_from_u64(u64 x) {
+  return __dadd_rn(__longlong_as_double((long long)(x | 0x4330000000000000ull)), -4503599627370496.0);
+}
+__device__ __forceinline__ u64 fp_to_u64(double x) {
+  return (u64)__double_as_longlong(__dadd_rn(x, 4503599627370496.0)) & 0xFFFFFFFFFFFFFull;
+}
+// x brought back within q / 2 + 1 (|x| < 2^53).
+__device__ __forceinline__ double fp_reduce(double x, double q, double qinv) {
+  return __fma_rn(-__dadd_rn(__fma_rn(x, qinv, FP_ROUND), -FP_ROUND), q, x);
+}
 
-  __device__ __forceinline__ static void run(double (&e)[8], int tid, const NttTable& T) {
+// Eight consecutive words of a thread, as two 32-byte accesses.
+__device__ __forceinline__ void ld8(const u64* p, u64 (&x)[8]) {
+#pragma unroll
+  for (int h = 0; h < 2; ++h)
+    asm volatile("ld.global.v4.u64 {%0, %1, %2, %3}, [%4];"
+                 : "=l"(x[4 * h]), "=l"(x[4 * h + 1]), "=l"(x[4 * h + 2]), "=l"(x[4 * h + 3])
+                 : "l"(p + 4 * h));
+}
+__device__ __forceinline__ void ld8_nc(const u64* p, u64 (&x)[8]) {
+#pragma unroll
+  for (int h = 0; h < 2; ++h)
+    asm("ld.global.nc.v4.u64 {%0, %1, %2, %3}, [%4];"
+        : "=l"(x[4 * h]), "=l"(x[4 * h + 1]), "=l"(x[4 * h + 2]), "=l"(x[4 * h + 3])
+        : "l"(p + 4 * h));
+}
+__device__ __forceinline__ void st8(u64* p, const u64 (&x)[8]) {
+#pragma unroll
+  for (int h = 0; h < 2; ++h)
+    asm volatile("st.global.v4.u64 [%0], {%1, %2, %3, %4};" ::"l"(p + 4 * h), "l"(x[4 * h]), "l"(x[4 * h + 1]),
+                 "l"(x[4 * h + 2]), "l"(x[4 * h + 3])
+                 : "memory");
+}
+
+// One phase (up to three butterfly stages) on doubles, with the forward layouts of
+// NttPhase<LOGN, false, P>. Phase P works within aligned blocks of SPAN elements. The
+// inverse undoes the forward phases last to first in the same layouts: it starts on
+// eight consecutive elements a thread and ends in the layout the forward starts in.
+//
+// 32 threads hold the same aligned 256 elements in every layout with SPAN <= 256, so an
+// exchange between two such layouts stays within a warp (fp_sync); at n = 2048 one
+// exchange of three needs the whole CTA.
+template <int LOGN, int P>
+struct FpPhase {
+  using Ix = NttPhase<LOGN, false, P>;
+  static constexpr int n = Ix::n, S0 = Ix::S0, R = Ix::R, NSUB = Ix::NSUB, STRIDE = Ix::STRIDE, SPAN = n >> S0;
+
+  // Twiddles of level lvl: consecutive, aligned to their number.
+  __device__ __forceinline__ static void twiddles(const double* t, int at, int count, double (&w)[4]) {
+    if (count == 1) {
+      w[0] = __ldg(t + at);
+    } else {
+#pragma unroll
+      for (int j = 0; j < 4; j += 2)
+        if (j < count) {
+          const double2 v = __ldg(reinterpret_cast<const double2*>(t + at + j));
+          w[j] = v.x;
+          w[j + 1] = v.y;
+        }
+    }
+  }
+
+  __device__ __forceinline__ static void forward(double (&e)[8], int tid, const NttTable& T) {
     const double q = T.qd, qinv = T.qinv;
 #pragma unroll
     for (int sub = 0; sub < NSUB; ++sub) {
-      const int u = tid * NSUB + sub;
-      const int b0 = u / STRIDE;
+      const int b0 = (tid * NSUB + sub) / STRIDE;
 #pragma unroll
       for (int lvl = 0; lvl < R; ++lvl) {
-        const int hk = INV ? (1 << lvl) : (1 << (R - 1 - lvl));
-        const int len = STRIDE * hk;
-        const int m = n / (2 * len);
-        const int tw0 = m + (INV ? (b0 << (R - 1 - lvl)) : (b0 << lvl));
+        const int hk = 1 << (R - 1 - lvl);
         double w[4];
-        const int ntw = INV ? (1 << (R - 1 - lvl)) : (1 << lvl);
-#pragma unroll
-        for (int j = 0; j < 4; ++j)
-          if (j < ntw) w[j] = __ldg((INV ? T.ipsi_d : T.psi_d) + tw0 + j);
+        twiddles(T.psi_d, n / (2 * STRIDE * hk) + (b0 << lvl), 1 << lvl, w);
 #pragma unroll
         for (int k = 0; k < (1 << R); ++k) {
           if (k & hk) continue;
-          const int j = INV ? (k >> (lvl + 1)) : (k >> (R - lvl));
           double& a = e[sub * (1 << R) + k];
           double& c = e[sub * (1 << R) + k + hk];
-          if (!INV) {
-            const double t = fp_mulmod(c, w[j], q, qinv);
-            const double av = a;
-            a = __dadd_rn(av, t);
-            c = __dadd_rn(av, -t);
-          } else {
-            const double av = a, cv = c;
-            a = __dadd_rn(av, cv);
-            c = fp_mulmod(__dadd_rn(av, -cv), w[j], q, qinv);
-          }
+          const double t = fp_mulmod(c, w[k >> (R - lvl)], q, qinv), av = a;
+          a = __dadd_rn(av, t);
+          c = __dadd_rn(av, -t);
+        }
+      }
+    }
+  }
+
+  __device__ __forceinline__ static void inverse(double (&e)[8], int tid, const NttTable& T) {
+    const double q = T.qd, qinv = T.qinv;
+#pragma unroll
+    for (int sub = 0; sub < NSUB; ++sub) {
+      const int b0 = (tid * NSUB + sub) / STRIDE;
+#pragma unroll
+      for (int lvl = R - 1; lvl >= 0; --lvl) {
+        const int hk = 1 << (R - 1 - lvl);
+        double w[4];
+        twiddles(T.ipsi_d, n / (2 * STRIDE * hk) + (b0 << lvl), 1 << lvl, w);
+#pragma unroll
+        for (int k = 0; k < (1 << R); ++k) {
+          if (k & hk) continue;
+          double& a = e[sub * (1 << R) + k];
+          double& c = e[sub * (1 << R) + k + hk];
+          const double av = a, cv = c;
+          a = __dadd_rn(av, cv);
+          c = fp_mulmod(__dadd_rn(av, -cv), w[k >> (R - lvl)], q, qinv);
         }
       }
     }
   }
 };
 
-// Forward transform of a segment held in the phase-0 layout; leaves it in the
-// layout of the last phase, as signed residues below |input| + 0.5625 LOGN q.
-template <int LOGN, int P = 0>
-__device__ __forceinline__ void ntt_forward_fp(double (&e)[8], int tid, const NttTable& T, double* ssm) {
-  using Ph = NttPhaseFp<LOGN, false, P>;
-  constexpr int NPH = (LOGN + 2) / 3;
-  Ph::run(e, tid, T);
-  if constexpr (P + 1 < NPH) {
-    using Nx = NttPhase<LOGN, false, P + 1>;
-    __syncthreads();
+// The first three forward stages on small integers (digits): the eight outputs are sums
+// of the inputs times products of the seven twiddles, 34 exact multiply-adds instead of
+// twelve butterflies of eight operations. Sums stay below 8 |e| q: 2^48 for |e| <= 127 and
+// q <= 2^38.
+constexpr double FP_DIGIT_Q = 274877906944.0;  // 2^38
+__device__ __forceinline__ void fp_digit_phase(double (&e)[8], const NttTable& T) {
+  const double* c = T.d8;
+  const double s = __fma_rn(c[0], e[4], e[0]), d = __fma_rn(-c[0], e[4], e[0]);
+  const double t = __fma_rn(c[2], e[6], __dmul_rn(c[1], e[2])), u = __fma_rn(-c[4], e[6], __dmul_rn(c[3], e[2]));
+  const double ev[4] = {__dadd_rn(s, t), __dadd_rn(s, -t), __dadd_rn(d, u), __dadd_rn(d, -u)};
+  const double x1 = e[1], x5 = e[5], x3 = e[3], x7 = e[7];
 #pragma unroll
-    for (int v = 0; v < 8; ++v) ssm[swz(Ph::Ix::index(v, tid))] = e[v];
-    __syncthreads();
-#pragma unroll
-    for (int v = 0; v < 8; ++v) e[v] = ssm[swz(Nx::index(v, tid))];
-    ntt_forward_fp<LOGN, P + 1>(e, tid, T, ssm);
+  for (int i = 0; i < 4; ++i) {
+    const double* k = c + 5 + 4 * i;
+    const double o = __fma_rn(k[3], x7, __fma_rn(k[2], x3, __fma_rn(k[1], x5, __dmul_rn(k[0], x1))));
+    e[2 * i] = __dadd_rn(ev[i], o);
+    e[2 * i + 1] = __dadd_rn(ev[i], -o);
   }
 }
 
-// Inverse transform (then the n^-1 scaling) of a segment held in the layout
-// NttPhase<LOGN, true, 0>::index, inputs below 4 q in magnitude; leaves signed
-// coefficients, |x| <= 0.5625 q, in the layout of the last inverse phase. With
-// REDUCE (needed for q above 2^35) every phase boundary first brings the values
-// back within q/2, so a phase of three stages stays below 32 q.
-template <int LOGN, int P = 0, bool REDUCE = false>
-__device__ __forceinline__ void ntt_inverse_fp(double (&e)[8], int tid, const NttTable& T, double* ssm) {
-  using Ph = NttPhaseFp<LOGN, true, P>;
+template <int SPAN>
+__device__ __forceinline__ void fp_sync() {
+  if constexpr (SPAN <= 256)
+    __syncwarp();
+  else
+    __syncthreads();
+}
+
+// Forward transform of a segment held in the phase-0 layout (tid + k n / 8); leaves it as
+// eight consecutive elements a thread, signed residues below |input| + 0.5625 LOGN q.
+// Phases before P have run. `ssm`: the exchange area (addressed through swz from `sbase`).
+// On entry no other warp may still read it.
+template <int LOGN, int P = 0>
+__device__ __forceinline__ void fp_forward(double (&e)[8], int tid, const NttTable& T, double* ssm, int sbase = 0) {
   constexpr int NPH = (LOGN + 2) / 3;
-  Ph::run(e, tid, T);
-  if constexpr (P + 1 < NPH) {
-    using Nx = NttPhase<LOGN, true, P + 1>;
-    __syncthreads();
+  if constexpr (P > 0) {
+    using Pv = FpPhase<LOGN, P - 1>;
+    using Ph = FpPhase<LOGN, P>;
+    if constexpr (P > 1) fp_sync<Pv::SPAN>();  // the previous exchange's reads
 #pragma unroll
-    for (int v = 0; v < 8; ++v) ssm[swz(Ph::Ix::index(v, tid))] = e[v];
-    __syncthreads();
+    for (int v = 0; v < 8; ++v) ssm[swz(sbase + Pv::Ix::index(v, tid))] = e[v];
+    fp_sync<Pv::SPAN>();
 #pragma unroll
-    for (int v = 0; v < 8; ++v) e[v] = ssm[swz(Nx::index(v, tid))];
-    if constexpr (REDUCE) {
+    for (int v = 0; v < 8; ++v) e[v] = ssm[swz(sbase + Ph::Ix::index(v, tid))];
+  }
+  FpPhase<LOGN, P>::forward(e, tid, T);
+  if constexpr (P + 1 < NPH) fp_forward<LOGN, P + 1>(e, tid, T, ssm, sbase);
+}
+
+// The phases after the first.
+template <int LOGN>
+__device__ __forceinline__ void fp_forward_rest(double (&e)[8], int tid, const NttTable& T, double* ssm, int sbase) {
+  fp_forward<LOGN, 1>(e, tid, T, ssm, sbase);
+}
+
+// The same from digits, with the dense first phase where the caller finds its sums below
+// 2^48 (uniform in the CTA).
+template <int LOGN>
+__device__ __forceinline__ void fp_forward_digits(double (&e)[8], int tid, const NttTable& T, double* ssm, int sbase,
+                                                  bool dense) {
+  if (dense)
+    fp_digit_phase(e, T);
+  else
+    FpPhase<LOGN, 0>::forward(e, tid, T);
+  if constexpr (LOGN > 3) fp_forward_rest<LOGN>(e, tid, T, ssm, sbase);
+}
+
+// Inverse transform, without the n^-1 scaling, of a segment held as eight consecutive
+// elements a thread, inputs below 4 q in magnitude; leaves signed values in the phase-0
+// layout: below 2^12 q for q <= 2^35 (inputs below q), else below 2^6 q, 2^48 in any case.
+// Primes above 2^35 return to q / 2 after the second phase (six stages at most between
+// reductions: 2 * 4 q * 2^5 < 2^48 for q < 2^40), above 2^40 after every phase. On
+// entry no other warp may still read the exchange area.
+template <int LOGN, int P = (LOGN + 2) / 3 - 1>
+__device__ __forceinline__ void fp_inverse(double (&e)[8], int tid, const NttTable& T, double* ssm, int sbase = 0) {
+  constexpr int LAST = (LOGN + 2) / 3 - 1;
+  FpPhase<LOGN, P>::inverse(e, tid, T);
+  if constexpr (P > 0) {
+    using Ph = FpPhase<LOGN, P>;
+    using Nx = FpPhase<LOGN, P - 1>;
+    if (T.qd > 34359738368.0 && (P == LAST - 1 || T.qd > 1099511627776.0)) {
 #pragma unroll
-      for (int v = 0; v < 8; ++v)
-        e[v] = __fma_rn(-__dadd_rn(__fma_rn(e[v], T.qinv, FP_ROUND), -FP_ROUND), T.qd, e[v]);
+      for (int v = 0; v < 8; ++v) e[v] = fp_reduce(e[v], T.qd, T.qinv);
     }
-    ntt_inverse_fp<LOGN, P + 1, REDUCE>(e, tid, T, ssm);
-  } else {
+    if constexpr (P < LAST) fp_sync<Ph::SPAN>();  // the previous exchange's reads
 #pragma unroll
-    for (int v = 0; v < 8; ++v) e[v] = fp_mulmod(e[v], T.ninv_d[LOGN], T.qd, T.qinv);
+    for (int v = 0; v < 8; ++v) ssm[swz(sbase + Ph::Ix::index(v, tid))] = e[v];
+    fp_sync<Nx::SPAN>();
+#pragma unroll
+    for (int v = 0; v < 8; ++v) e[v] = ssm[swz(sbase + Nx::Ix::index(v, tid))];
+    fp_inverse<LOGN, P - 1>(e, tid, T, ssm, sbase);
   }
 }
 

@@ -22,7 +22,7 @@
 #include "cascade_tc.cuh"
 #include "first_dim.cuh"
 #include "gadget.cuh"
-#include "ntt_fp.cuh"
+#include "gadget_fp.cuh"
 #include "server.cuh"
 
 namespace via {
@@ -46,6 +46,18 @@ __global__ void k_decompose(const u64* __restrict__ in, int n_in, int stride, lo
   const long step = (long)nl * n_out;
   // Digit k goes to sample slot L - 1 - k.
   u64* o = out + p * (long)g.L * step + (long)(g.L - 1) * step + (long)i * stride;
+  if (g.fp && R.ntt && stride == 1 && a0 < R.m[0].q && a1 < R.m[1].q) {
+    double v = nl == 2 ? fp_scaled2(fp_from_u64(a0), fp_from_u64(a1), g, R)
+                       : fp_scaled(fp_reduce(fp_from_u64(a0), (double)R.m[0].q, R.t[0].qinv), g.dS, R.t[0].qinv);
+    for (int k = 0; k < g.L; ++k, o -= step) {
+      const double d = fp_next_digit(v, g);
+      for (int l = 0; l < nl; ++l) {
+        const double q = (double)R.m[l].q;
+        o[(long)l * n_out] = fp_to_u64(d < 0.0 ? __dadd_rn(d, q) : d);
+      }
+    }
+    return;
+  }
   for_each_digit(gadget_scaled(a0, a1, R, g), g, [&](int, i64 d) {
     for (int l = 0; l < nl; ++l) {
       u64* ol = o + (long)l * n_out;
@@ -208,24 +220,23 @@ __global__ void k_dmux_combine(u64* out, const u64* in, const u64* ext, long cou
 // rlev.rs:193-222), in double precision (ntt_fp.cuh). CTA (o, l) computes limb l
 // of ext[o] = bit (x) in[o] and writes out[2o] = in[o] - ext, out[2o+1] = ext:
 // the gadget digits (L = 2) of the mask and body coefficients (both limbs read,
-// one CRT scaling per coefficient, digits kept in shared memory), forward
-// transforms of the four digit polynomials at prime l, products with the RGSW
-// samples (each within 0.5625 q; digit k of input half h with sample
-// h L + L - 1 - k), and inverse transforms of the two sums (below 2.25 q).
-// Buffers: [ct][2][nl][n], RGSW [2L][2][nl][n] eval at q1; nl = 2 primes below 2^44.
+// one CRT scaling per coefficient), forward transforms of the four digit
+// polynomials at prime l, products with the RGSW samples (each within 0.5625 q;
+// digit k of input half h with sample h L + L - 1 - k), and inverse transforms of
+// the two sums. Buffers: [ct][2][nl][n], RGSW [2L][2][nl][n] eval at q1; nl = 2
+// primes below 2^44. FP64-issue and latency bound: the levels of 256 to 1024 products
+// of 64 queries took 728 us together with eight barriers a transform and 64-bit
+// integer digit splits, 307 us with one barrier and splits on doubles.
 template <int LOGN>
 __global__ void __launch_bounds__((1 << LOGN) / 8, 2) k_dmux_fp(u64* __restrict__ out, const u64* __restrict__ in,
-                                                                  KeySel ks, DevRing R, Gadget g) {
+                                                                  KeySel ks, const __grid_constant__ DevRing R,
+                                                                  const __grid_constant__ Gadget g) {
   constexpr int n = 1 << LOGN;
   constexpr int L = 2;
   constexpr int nl = 2;
-  using Fw0 = NttPhase<LOGN, false, 0>;
-  using FwL = NttPhase<LOGN, false, (LOGN + 2) / 3 - 1>;
-  using In0 = NttPhase<LOGN, true, 0>;
-  using InL = NttPhase<LOGN, true, (LOGN + 2) / 3 - 1>;
-  static_assert(In0::STRIDE == 1 && In0::R == 3 && FwL::STRIDE == 1, "contiguous end layouts");
-  __shared__ double ssm[n];
-  __shared__ int dgs[L][n];  // one half's digits; each thread reads back only its own slots
+  using L0 = NttPhase<LOGN, false, 0>;
+  __shared__ double ssm[2][n];  // alternate between transforms: one CTA barrier each
+  int buf = 0;
   const int tid = threadIdx.x;
   const long o = blockIdx.x;
   const int l = blockIdx.y;
@@ -236,51 +247,48 @@ __global__ void __launch_bounds__((1 << LOGN) / 8, 2) k_dmux_fp(u64* __restrict_
   double am[8], ab[8];
 #pragma unroll
   for (int v = 0; v < 8; ++v) am[v] = ab[v] = 0.0;
+#pragma unroll 1
   for (int h = 0; h < 2; ++h) {  // 0: mask digits (neg_s_m rows), 1: body digits (m rows)
+    double val[8];
 #pragma unroll
     for (int v = 0; v < 8; ++v) {
-      const int x = Fw0::index(v, tid);
-      const u64 a0 = ct[(long)h * nl * n + x], a1 = ct[(long)h * nl * n + n + x];
-      for_each_digit(gadget_scaled(a0, a1, R, g), g, [&](int k, i64 d) { dgs[k][x] = (int)d; });
+      const u64* c = ct + (long)h * nl * n + L0::index(v, tid);
+      val[v] = fp_scaled2(fp_from_u64(c[0]), fp_from_u64(c[n]), g, R);
     }
 #pragma unroll 1
     for (int k = 0; k < L; ++k) {
       double e[8];
 #pragma unroll
-      for (int v = 0; v < 8; ++v) e[v] = (double)dgs[k][Fw0::index(v, tid)];
-      ntt_forward_fp<LOGN>(e, tid, T, ssm);
+      for (int v = 0; v < 8; ++v) e[v] = fp_next_digit(val[v], g);
+      fp_forward<LOGN>(e, tid, T, ssm[buf]);
+      buf ^= 1;
       const int smp = h * L + L - 1 - k;
-      const ulonglong2* Km = reinterpret_cast<const ulonglong2*>(K + ((long)(2 * smp) * nl + l) * n + 8 * tid);
-      const ulonglong2* Kb = reinterpret_cast<const ulonglong2*>(K + ((long)(2 * smp + 1) * nl + l) * n + 8 * tid);
+      u64 key[8];
+      ld8_nc(K + ((long)(2 * smp) * nl + l) * n + 8 * tid, key);
 #pragma unroll
-      for (int c = 0; c < 4; ++c) {
-        const ulonglong2 km = __ldg(Km + c), kb = __ldg(Kb + c);
-        am[2 * c] = __dadd_rn(am[2 * c], fp_mulmod(e[2 * c], __ull2double_rn(km.x), q, qinv));
-        am[2 * c + 1] = __dadd_rn(am[2 * c + 1], fp_mulmod(e[2 * c + 1], __ull2double_rn(km.y), q, qinv));
-        ab[2 * c] = __dadd_rn(ab[2 * c], fp_mulmod(e[2 * c], __ull2double_rn(kb.x), q, qinv));
-        ab[2 * c + 1] = __dadd_rn(ab[2 * c + 1], fp_mulmod(e[2 * c + 1], __ull2double_rn(kb.y), q, qinv));
-      }
+      for (int v = 0; v < 8; ++v) am[v] = __dadd_rn(am[v], fp_mulmod(e[v], fp_from_u64(key[v]), q, qinv));
+      ld8_nc(K + ((long)(2 * smp + 1) * nl + l) * n + 8 * tid, key);
+#pragma unroll
+      for (int v = 0; v < 8; ++v) ab[v] = __dadd_rn(ab[v], fp_mulmod(e[v], fp_from_u64(key[v]), q, qinv));
     }
   }
   const u64 qi = R.m[l].q;
   u64* o0 = out + (2 * o) * 2 * nl * n;
   u64* o1 = o0 + 2 * nl * n;
-  ntt_inverse_fp<LOGN, 0, true>(am, tid, T, ssm);
+#pragma unroll 1
+  for (int part = 0; part < 2; ++part) {  // ext mask, ext body
 #pragma unroll
-  for (int v = 0; v < 8; ++v) {  // ext mask
-    const long at = (long)l * n + InL::index(v, tid);
-    const u64 ext = __double2ull_rn(fp_canonical(am[v], q, qinv));
-    o0[at] = submod(ct[at], ext, qi);
-    o1[at] = ext;
-  }
-  __syncthreads();  // the body's transform reuses the exchange area
-  ntt_inverse_fp<LOGN, 0, true>(ab, tid, T, ssm);
+    for (int v = 0; v < 8; ++v) am[v] = fp_reduce(am[v], q, qinv);
+    fp_inverse<LOGN>(am, tid, T, ssm[buf]);
+    buf ^= 1;
 #pragma unroll
-  for (int v = 0; v < 8; ++v) {  // ext body
-    const long at = (long)(nl + l) * n + InL::index(v, tid);
-    const u64 ext = __double2ull_rn(fp_canonical(ab[v], q, qinv));
-    o0[at] = submod(ct[at], ext, qi);
-    o1[at] = ext;
+    for (int v = 0; v < 8; ++v) {
+      const long at = (long)(part * nl + l) * n + L0::index(v, tid);
+      const u64 ext = fp_to_u64(fp_canonical(fp_mulmod(am[v], T.ninv_d[LOGN], q, qinv), q, qinv));
+      o0[at] = submod(ct[at], ext, qi);
+      o1[at] = ext;
+      am[v] = ab[v];
+    }
   }
 }
 
@@ -293,11 +301,9 @@ __global__ void __launch_bounds__((1 << LOGN) / 8, 2) k_dmux_fp(u64* __restrict_
 enum { INTT_STORE = 0, INTT_DMUX = 1, INTT_ADD = 2 };
 template <int LOGN, int MODE>
 __global__ void __launch_bounds__((1 << LOGN) / 8) k_intt_fp_epi(const u64* __restrict__ ext, const u64* base,
-                                                                 u64* out, DevRing R) {
+                                                                 u64* out, const __grid_constant__ DevRing R) {
   constexpr int n = 1 << LOGN;
-  using In0 = NttPhase<LOGN, true, 0>;
-  using InL = NttPhase<LOGN, true, (LOGN + 2) / 3 - 1>;
-  static_assert(In0::STRIDE == 1 && In0::R == 3, "contiguous first inverse layout");
+  using L0 = NttPhase<LOGN, false, 0>;
   __shared__ double ssm[n];
   const int tid = threadIdx.x;
   const int nl = R.nl;
@@ -305,28 +311,25 @@ __global__ void __launch_bounds__((1 << LOGN) / 8) k_intt_fp_epi(const u64* __re
   const int l = (int)(seg % nl);
   const NttTable& T = R.t[l];
   const double q = T.qd, qinv = T.qinv;
+  u64 x[8];
+  ld8(ext + seg * n + 8 * tid, x);
   double e[8];
-  const ulonglong2* src = reinterpret_cast<const ulonglong2*>(ext + seg * n + 8 * tid);
 #pragma unroll
-  for (int c = 0; c < 4; ++c) {
-    const ulonglong2 x = src[c];
-    e[2 * c] = __ull2double_rn(x.x);
-    e[2 * c + 1] = __ull2double_rn(x.y);
-  }
-  ntt_inverse_fp<LOGN, 0, true>(e, tid, T, ssm);
+  for (int v = 0; v < 8; ++v) e[v] = fp_from_u64(x[v]);
+  fp_inverse<LOGN>(e, tid, T, ssm);
   const u64 qi = R.m[l].q;
   const long per = 2L * nl * n, j = seg / (2 * nl), at0 = (seg % (2 * nl)) * n;
 #pragma unroll
   for (int v = 0; v < 8; ++v) {
-    const int x = InL::index(v, tid);
-    const u64 val = __double2ull_rn(fp_canonical(e[v], q, qinv));
+    const int c = L0::index(v, tid);
+    const u64 val = fp_to_u64(fp_canonical(fp_mulmod(e[v], T.ninv_d[LOGN], q, qinv), q, qinv));
     if constexpr (MODE == INTT_STORE) {
-      out[seg * n + x] = val;
+      out[seg * n + c] = val;
     } else if constexpr (MODE == INTT_DMUX) {
-      out[(2 * j) * per + at0 + x] = submod(base[j * per + at0 + x], val, qi);
-      out[(2 * j + 1) * per + at0 + x] = val;
+      out[(2 * j) * per + at0 + c] = submod(base[j * per + at0 + c], val, qi);
+      out[(2 * j + 1) * per + at0 + c] = val;
     } else {
-      out[seg * n + x] = addmod(base[seg * n + x], val, qi);
+      out[seg * n + c] = addmod(base[seg * n + c], val, qi);
     }
   }
 }
@@ -354,7 +357,7 @@ static bool R_fp_small(const DevRing& R) {
 }
 
 static bool dmux_fp_ok(const DevRing& R, const Gadget& g) {
-  return R.ntt && R.nl == 2 && g.L == 2 && ntt_fp_ok(R.t[0], R.t[1]) && R.n == 2048;
+  return R.ntt && R.nl == 2 && g.L == 2 && g.fp && ntt_fp_ok(R.t[0], R.t[1]) && R.n == 2048;
 }
 
 // Modulus switch (prim/switching/kernels/mod_switch.rs:59-61):
@@ -497,7 +500,7 @@ __global__ void __launch_bounds__(256) k_cascade_mac(const u64* __restrict__ D, 
 }
 
 // k_cascade_mac in double precision (ntt_fp.cuh): D holds the digits' signed
-// double transforms (ntt_forward_i8_fp, within 7 q of zero), keys the cascade
+// double transforms (ntt_forward_i8_fp, below 2^48), keys the cascade
 // key as exact doubles (below q). Every product is reduced to within 0.5625 q,
 // so a mask's 2 L products stay below 1.125 L q; the body partial is brought
 // back within q/2 after each output mask's 2 L products. Outputs as k_cascade_mac.
@@ -1048,92 +1051,88 @@ static void external_products(const DevRing& R, const Gadget& g, KeySel rgsw, co
 //   RGSW samples (mask digits with neg_s_m, body digits with m, digit k with
 //   sample L-1-k) -> out[o] = in[2o] + ext, eval form throughout.
 // cur: [count*2][2][n]; nxt: [count][2][n]; the RGSW of CMux o ([2L][2][n],
-// eval) is picked by `ks`. The digits never leave registers. Every transform
-// and RGSW product is exact integer arithmetic on doubles (ntt_fp.cuh: FMA
-// two-products and a floating-point quotient estimate). For single primes
-// q < 2^35 and small gadgets: differences of canonical residues are
-// below q; the inverse leaves coefficients within 0.5625 q, made canonical for
-// the digit split; digits below B/2 transform to values below 7 q; each product
-// with an RGSW sample (below q) is reduced to within 0.5625 q, so the 2L
-// products and the input residue sum to less than (1 + 1.125 L) q before the
-// final reduction.
+// eval) is picked by `ks`. The digits never leave registers. Every transform,
+// digit split and RGSW product is exact integer arithmetic on doubles (ntt_fp.cuh:
+// FMA two-products and a floating-point quotient estimate; gadget_fp.cuh). For
+// single primes q < 2^35 and small gadgets: differences of canonical residues are
+// below q; the n^-1 product leaves coefficients within 0.5625 q, which the split
+// takes as they are; each product with an RGSW sample (below q) is reduced to
+// within 0.5625 q, so the 2L products and the input residue sum to less than
+// (1 + 1.125 L) q before the final reduction.
+//
+// FP64-issue bound (about 3000 operations a thread, 2 CTAs of 8 warps an SM). At n = 2048
+// the first exchange of a forward transform and the last of an inverse cross warps, the
+// other two stay within one, and the inverse ends in the layout the forward starts in:
+// 6 CTA barriers a CMux where 40 were. With the digit split and the conversions on doubles
+// and the dense first phase: 8191 CMuxes of a five-query batch 624 -> 410 us.
 template <int LOGN>
 __global__ void __launch_bounds__((1 << LOGN) / 8, LOGN >= 12 ? 1 : 2) k_cmux_fp(const u64* __restrict__ cur,
                                                                                 u64* __restrict__ nxt, KeySel ks,
-                                                                                DevRing R, Gadget g) {
+                                                                                const __grid_constant__ DevRing R,
+                                                                                const __grid_constant__ Gadget g) {
   constexpr int n = 1 << LOGN;
-  using In0 = NttPhase<LOGN, true, 0>;
-  using InL = NttPhase<LOGN, true, (LOGN + 2) / 3 - 1>;
-  using Fw0 = NttPhase<LOGN, false, 0>;
-  using FwL = NttPhase<LOGN, false, (LOGN + 2) / 3 - 1>;
-  static_assert(In0::STRIDE == 1 && In0::R == 3 && FwL::STRIDE == 1, "contiguous end layouts");
-  __shared__ double ssm[n];
+  // Transforms alternate between two exchange areas, so each needs one CTA barrier
+  // (fp_forward, fp_inverse); at n = 4096 one area (32 KB) and a barrier before each.
+  constexpr int NB = LOGN >= 12 ? 1 : 2;
+  __shared__ double ssm[NB][n];
+  int buf = 0;
+  auto area = [&]() -> double* {
+    if constexpr (NB == 1) {
+      __syncthreads();
+      return ssm[0];
+    } else {
+      return ssm[buf ^= 1];
+    }
+  };
   const int tid = threadIdx.x;
   const long o = blockIdx.x;
   const NttTable& T = R.t[0];
   const double q = T.qd, qinv = T.qinv;
   const u64* a = cur + (2 * o) * 2 * n;
-  const u64* b = a + 2 * n;
   const u64* K = ks.base + ((o / ks.div) % ks.mod) * ks.stride;
   const int L = g.L;
+  const bool dense = 4.0 * g.dB * q < 281474976710656.0;  // |digit| <= B / 2: fp_digit_phase's sums below 2^48
   double am[8], ab[8];
 #pragma unroll
   for (int v = 0; v < 8; ++v) am[v] = ab[v] = 0.0;
+#pragma unroll 1
   for (int p = 0; p < 2; ++p) {  // 0: mask digits (neg_s_m rows), 1: body digits (m rows)
-    double e[8];
+    double val[8];
     {
-      const ulonglong2* bv = reinterpret_cast<const ulonglong2*>(b + p * n + 8 * tid);
-      const ulonglong2* av = reinterpret_cast<const ulonglong2*>(a + p * n + 8 * tid);
+      u64 x[8], y[8];
+      ld8(a + 2 * n + p * n + 8 * tid, x);
+      ld8(a + p * n + 8 * tid, y);
 #pragma unroll
-      for (int h = 0; h < 4; ++h) {
-        const ulonglong2 x = bv[h], y = av[h];
-        e[2 * h] = __dadd_rn(__ull2double_rn(x.x), -__ull2double_rn(y.x));
-        e[2 * h + 1] = __dadd_rn(__ull2double_rn(x.y), -__ull2double_rn(y.y));
-      }
+      for (int v = 0; v < 8; ++v) val[v] = __dadd_rn(fp_from_u64(x[v]), -fp_from_u64(y[v]));
     }
-    ntt_inverse_fp<LOGN>(e, tid, T, ssm);
-    __syncthreads();
+    fp_inverse<LOGN>(val, tid, T, area());
 #pragma unroll
-    for (int v = 0; v < 8; ++v) ssm[swz(InL::index(v, tid))] = e[v];
-    __syncthreads();
-    u32 dcur[8];  // scaled coefficients, below B^L < 2^32
-#pragma unroll
-    for (int v = 0; v < 8; ++v) {
-      double c = ssm[swz(Fw0::index(v, tid))];
-      if (c < 0.0) c = __dadd_rn(c, q);
-      dcur[v] = (u32)gadget_scaled_small((u64)__double2ull_rn(c), g);
-    }
+    for (int v = 0; v < 8; ++v) val[v] = fp_scaled(fp_mulmod(val[v], T.ninv_d[LOGN], q, qinv), g.dS, qinv);
+#pragma unroll 1
     for (int k = 0; k < L; ++k) {
+      double e[8];
 #pragma unroll
-      for (int v = 0; v < 8; ++v) e[v] = __ll2double_rn(gadget_next_digit32(dcur[v], g));
-      ntt_forward_fp<LOGN>(e, tid, T, ssm);
-      const ulonglong2* Km = reinterpret_cast<const ulonglong2*>(K + (long)(2 * (p * L + L - 1 - k)) * n + 8 * tid);
-      const ulonglong2* Kb = Km + n / 2;
+      for (int v = 0; v < 8; ++v) e[v] = fp_next_digit(val[v], g);
+      fp_forward_digits<LOGN>(e, tid, T, area(), 0, dense);
+      const u64* Km = K + (long)(2 * (p * L + L - 1 - k)) * n + 8 * tid;
+      u64 key[8];
+      ld8_nc(Km, key);
 #pragma unroll
-      for (int h = 0; h < 4; ++h) {
-        const ulonglong2 km = __ldg(Km + h), kb = __ldg(Kb + h);
-        am[2 * h] = __dadd_rn(am[2 * h], fp_mulmod(e[2 * h], __ull2double_rn(km.x), q, qinv));
-        am[2 * h + 1] = __dadd_rn(am[2 * h + 1], fp_mulmod(e[2 * h + 1], __ull2double_rn(km.y), q, qinv));
-        ab[2 * h] = __dadd_rn(ab[2 * h], fp_mulmod(e[2 * h], __ull2double_rn(kb.x), q, qinv));
-        ab[2 * h + 1] = __dadd_rn(ab[2 * h + 1], fp_mulmod(e[2 * h + 1], __ull2double_rn(kb.y), q, qinv));
-      }
+      for (int v = 0; v < 8; ++v) am[v] = __dadd_rn(am[v], fp_mulmod(e[v], fp_from_u64(key[v]), q, qinv));
+      ld8_nc(Km + n, key);
+#pragma unroll
+      for (int v = 0; v < 8; ++v) ab[v] = __dadd_rn(ab[v], fp_mulmod(e[v], fp_from_u64(key[v]), q, qinv));
     }
   }
-  ulonglong2* outm = reinterpret_cast<ulonglong2*>(nxt + o * 2 * n + 8 * tid);
-  ulonglong2* outb = outm + n / 2;
-  const ulonglong2* am_in = reinterpret_cast<const ulonglong2*>(a + 8 * tid);
-  const ulonglong2* ab_in = am_in + n / 2;
+  u64 x[8];
+  ld8(a + 8 * tid, x);
 #pragma unroll
-  for (int h = 0; h < 4; ++h) {
-    const ulonglong2 xm = am_in[h], xb = ab_in[h];
-    ulonglong2 ym, yb;
-    ym.x = __double2ull_rn(fp_canonical(__dadd_rn(__ull2double_rn(xm.x), am[2 * h]), q, qinv));
-    ym.y = __double2ull_rn(fp_canonical(__dadd_rn(__ull2double_rn(xm.y), am[2 * h + 1]), q, qinv));
-    yb.x = __double2ull_rn(fp_canonical(__dadd_rn(__ull2double_rn(xb.x), ab[2 * h]), q, qinv));
-    yb.y = __double2ull_rn(fp_canonical(__dadd_rn(__ull2double_rn(xb.y), ab[2 * h + 1]), q, qinv));
-    outm[h] = ym;
-    outb[h] = yb;
-  }
+  for (int v = 0; v < 8; ++v) x[v] = fp_to_u64(fp_canonical(__dadd_rn(fp_from_u64(x[v]), am[v]), q, qinv));
+  st8(nxt + o * 2 * n + 8 * tid, x);
+  ld8(a + n + 8 * tid, x);
+#pragma unroll
+  for (int v = 0; v < 8; ++v) x[v] = fp_to_u64(fp_canonical(__dadd_rn(fp_from_u64(x[v]), ab[v]), q, qinv));
+  st8(nxt + o * 2 * n + n + 8 * tid, x);
 }
 
 // The CMux of k_cmux_fp split over a cluster of four CTAs, for tree levels
@@ -1151,13 +1150,12 @@ __global__ void __launch_bounds__((1 << LOGN) / 8, LOGN >= 12 ? 1 : 2) k_cmux_fp
 // and 1 add the four partials to in[2o] and reduce once.
 template <int LOGN>
 __global__ void __cluster_dims__(4, 1, 1) __launch_bounds__((1 << LOGN) / 8, 2)
-    k_cmux_cluster_fp(const u64* __restrict__ cur, u64* __restrict__ nxt, KeySel ks, DevRing R, Gadget g) {
+    k_cmux_cluster_fp(const u64* __restrict__ cur, u64* __restrict__ nxt, KeySel ks, const __grid_constant__ DevRing R,
+                      const __grid_constant__ Gadget g) {
   namespace cg = cooperative_groups;
   constexpr int n = 1 << LOGN;
-  using InL = NttPhase<LOGN, true, (LOGN + 2) / 3 - 1>;
-  using Fw0 = NttPhase<LOGN, false, 0>;
-  __shared__ double ssm[n];    // transform exchanges, then the mask partial
-  __shared__ double pbody[n];  // the body partial
+  __shared__ double ssm[n];    // the inverse's exchanges, then the mask partial
+  __shared__ double pbody[n];  // the forward's exchanges, then the body partial
   cg::cluster_group cluster = cg::this_cluster();
   const int r = (int)cluster.block_rank();
   const int p = r & 1, k = r >> 1;
@@ -1166,46 +1164,35 @@ __global__ void __cluster_dims__(4, 1, 1) __launch_bounds__((1 << LOGN) / 8, 2)
   const NttTable& T = R.t[0];
   const double q = T.qd, qinv = T.qinv;
   const u64* a = cur + (2 * o) * 2 * n;
-  const u64* b = a + 2 * n;
   const u64* K = ks.base + ((o / ks.div) % ks.mod) * ks.stride;
+  const bool dense = 4.0 * g.dB * q < 281474976710656.0;
   double e[8];
   {
-    const ulonglong2* bv = reinterpret_cast<const ulonglong2*>(b + p * n + 8 * tid);
-    const ulonglong2* av = reinterpret_cast<const ulonglong2*>(a + p * n + 8 * tid);
+    u64 x[8], y[8];
+    ld8(a + 2 * n + p * n + 8 * tid, x);
+    ld8(a + p * n + 8 * tid, y);
 #pragma unroll
-    for (int h = 0; h < 4; ++h) {
-      const ulonglong2 x = bv[h], y = av[h];
-      e[2 * h] = __dadd_rn(__ull2double_rn(x.x), -__ull2double_rn(y.x));
-      e[2 * h + 1] = __dadd_rn(__ull2double_rn(x.y), -__ull2double_rn(y.y));
-    }
+    for (int v = 0; v < 8; ++v) e[v] = __dadd_rn(fp_from_u64(x[v]), -fp_from_u64(y[v]));
   }
-  ntt_inverse_fp<LOGN>(e, tid, T, ssm);
-  __syncthreads();
-#pragma unroll
-  for (int v = 0; v < 8; ++v) ssm[swz(InL::index(v, tid))] = e[v];
-  __syncthreads();
+  fp_inverse<LOGN>(e, tid, T, ssm);
 #pragma unroll
   for (int v = 0; v < 8; ++v) {
-    double c = ssm[swz(Fw0::index(v, tid))];
-    if (c < 0.0) c = __dadd_rn(c, q);
-    u32 sc = (u32)gadget_scaled_small((u64)__double2ull_rn(c), g);
-    i64 d = gadget_next_digit32(sc, g);
-    if (k) d = gadget_next_digit32(sc, g);
-    e[v] = __ll2double_rn(d);
+    double val = fp_scaled(fp_mulmod(e[v], T.ninv_d[LOGN], q, qinv), g.dS, qinv);
+    e[v] = fp_next_digit(val, g);
+    if (k) e[v] = fp_next_digit(val, g);
   }
-  ntt_forward_fp<LOGN>(e, tid, T, ssm);
+  fp_forward_digits<LOGN>(e, tid, T, pbody, 0, dense);
   const int smp = p * 2 + 1 - k;  // sample L - 1 - k of half p (L = 2)
-  const ulonglong2* Km = reinterpret_cast<const ulonglong2*>(K + (long)(2 * smp) * n + 8 * tid);
-  const ulonglong2* Kb = Km + n / 2;
-  __syncthreads();  // every thread is done with the transform's exchanges in ssm
+  u64 km[8], kb[8];
+  ld8_nc(K + (long)(2 * smp) * n + 8 * tid, km);
+  ld8_nc(K + (long)(2 * smp + 1) * n + 8 * tid, kb);
+  // The warp's lanes are done with their part of pbody; every thread left ssm before the
+  // forward transform's CTA barrier.
+  __syncwarp();
 #pragma unroll
-  for (int h = 0; h < 4; ++h) {
-    const ulonglong2 km = __ldg(Km + h), kb = __ldg(Kb + h);
-    const int s0 = 8 * tid + 2 * h;
-    ssm[s0] = fp_mulmod(e[2 * h], __ull2double_rn(km.x), q, qinv);
-    ssm[s0 + 1] = fp_mulmod(e[2 * h + 1], __ull2double_rn(km.y), q, qinv);
-    pbody[s0] = fp_mulmod(e[2 * h], __ull2double_rn(kb.x), q, qinv);
-    pbody[s0 + 1] = fp_mulmod(e[2 * h + 1], __ull2double_rn(kb.y), q, qinv);
+  for (int v = 0; v < 8; ++v) {
+    ssm[8 * tid + v] = fp_mulmod(e[v], fp_from_u64(km[v]), q, qinv);
+    pbody[8 * tid + v] = fp_mulmod(e[v], fp_from_u64(kb[v]), q, qinv);
   }
   cluster.sync();
   if (r < 2) {  // rank 0: the output mask, rank 1: the output body
