@@ -31,10 +31,6 @@ struct CtParams {
   int mtiles, out_kp, out_half;
 };
 
-__device__ __forceinline__ double ct_u52(u64 x) {  // exact for x < 2^52
-  return __dadd_rn(__longlong_as_double((long long)(x | 0x4330000000000000ull)), -4503599627370496.0);
-}
-
 // First output mask of a unit. Mask units of n >= 8 run over the coefficient blocks of
 // one output mask, body units over the output masks of one coefficient block.
 __host__ __device__ __forceinline__ int ct_first_mask(const CtStep& S, int unit) {
@@ -112,8 +108,8 @@ __global__ void __launch_bounds__(256) k_ct_digits(const u64* __restrict__ q, lo
     if (a0 >= (1ull << 47)) a0 %= D.qi[0];  // as the integer path: any 64-bit input word
     if (a1 >= (1ull << 47)) a1 %= D.qi[1];
     u32 f[3];
-    ct_pieces(fp_mulmod(ct_u52(a0), D.yscale[0], D.q[0], D.qinv[0]),
-              fp_mulmod(ct_u52(a1), D.yscale[1], D.q[1], D.qinv[1]), D, f);
+    ct_pieces(fp_mulmod(fp_from_u64(a0), D.yscale[0], D.q[0], D.qinv[0]),
+              fp_mulmod(fp_from_u64(a1), D.yscale[1], D.q[1], D.qinv[1]), D, f);
 #pragma unroll
     for (int s = 0; s < CT_L; ++s) {
       const int at = which * CT_L + s;
@@ -314,7 +310,7 @@ __global__ void __launch_bounds__(CT_THREADS, 1) k_ct_step(const __grid_constant
         for (int r = 0; r < 4; ++r) {
           const u64 lo = (u64)v[l][0][r] + ((u64)v[l][1][r] << 8) + ((u64)v[l][2][r] << 16);
           const u64 hi = (u64)v[l][3][r] + ((u64)v[l][4][r] << 8);
-          const double x = __dadd_rn(__dadd_rn(ct_u52(lo), fp_mulmod(ct_u52(hi), P.D.c24[l], q, qinv)), -__ldg(cc + r));
+          const double x = __dadd_rn(__dadd_rn(fp_from_u64(lo), fp_mulmod(fp_from_u64(hi), P.D.c24[l], q, qinv)), -__ldg(cc + r));
           y[l][r] = __fma_rn(-__dadd_rn(__fma_rn(x, qinv, FP_ROUND), -FP_ROUND), q, x);
         }
       }

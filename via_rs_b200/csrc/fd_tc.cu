@@ -44,6 +44,7 @@ struct KParams {
   int n, J, n_jt, n_kc, n_ct, N, Np, nq;
   int stages, grouped, acc_stride, nacc, tmem_cols, order;
   int packed4, chunk, stage_bytes, sel_off, unp_off;  // chunk layout (FD_CHUNK or FD_CHUNK_P4) and stage offsets
+  int tiled;  // output layout: 0 [query][J][2][n], 1 fd_scan's tiled columns
   unsigned fault_ns;  // test hook: > 0 makes the epilogue's first wait run out after this long
   double qd, qinv, c24, c48;  // q2, its rounded inverse, 2^24 and 2^48 mod q2, as doubles
 };
@@ -70,15 +71,6 @@ __device__ __forceinline__ void unit_coords(const KParams& P, int u, int& t, int
   }
 }
 
-// Integers below 2^52 to and from doubles, exactly: the double 2^52 + x has the
-// bit pattern 0x4330000000000000 | x.
-__device__ __forceinline__ double u52_to_double(u64 x) {
-  return __dadd_rn(__longlong_as_double((long long)(x | 0x4330000000000000ull)), -4503599627370496.0);
-}
-__device__ __forceinline__ u64 double_to_u52(double x) {
-  return (u64)__double_as_longlong(__dadd_rn(x, 4503599627370496.0)) & 0xFFFFFFFFFFFFFull;
-}
-
 // sum_g v_g 2^{8g} mod q for nine group sums v_g < 2^31 and q < 2^40, on the
 // FP64 pipe: with lo, m1, m2 the sums of groups 0-2, 3-5 and 6-8 at their own
 // scale (each below 2^31 (1 + 2^8 + 2^16) < 2^48), the value is
@@ -89,10 +81,10 @@ __device__ __forceinline__ u64 fold9(const u32 (&v)[9], const KParams& P) {
   const u64 lo = (u64)v[0] + ((u64)v[1] << 8) + ((u64)v[2] << 16);
   const u64 m1 = (u64)v[3] + ((u64)v[4] << 8) + ((u64)v[5] << 16);
   const u64 m2 = (u64)v[6] + ((u64)v[7] << 8) + ((u64)v[8] << 16);
-  const double r1 = fp_mulmod(u52_to_double(m1), P.c24, P.qd, P.qinv);
-  const double r2 = fp_mulmod(u52_to_double(m2), P.c48, P.qd, P.qinv);
-  const double s = __dadd_rn(__dadd_rn(u52_to_double(lo), r1), r2);
-  return double_to_u52(fp_canonical(s, P.qd, P.qinv));
+  const double r1 = fp_mulmod(fp_from_u64(m1), P.c24, P.qd, P.qinv);
+  const double r2 = fp_mulmod(fp_from_u64(m2), P.c48, P.qd, P.qinv);
+  const double s = __dadd_rn(__dadd_rn(fp_from_u64(lo), r1), r2);
+  return fp_to_u64(fp_canonical(s, P.qd, P.qinv));
 }
 
 template <int EPI>
@@ -318,7 +310,8 @@ __global__ void __launch_bounds__(fd_threads(EPI), 1) k_fd_tc(KParams P) {
           // folding and stores of that chunk.
           constexpr int CW = EPI >= 16 ? 4 : 8, STEP = (EPI / 4) * CW;
           const size_t qs = (size_t)2 * P.J * P.n;  // between queries
-          u64* orow = P.out + (size_t)j * 2 * P.n + t;
+          u64* orow = P.tiled ? P.out + ((size_t)jt * P.n + t) * P.nq * 2 * FD_MT + 2 * row
+                              : P.out + (size_t)j * 2 * P.n + t;
           for (int c0 = part * CW; c0 < P.N; c0 += STEP) {
             u32 v[9][CW];
 #pragma unroll
@@ -330,6 +323,23 @@ __global__ void __launch_bounds__(fd_threads(EPI), 1) k_fd_tc(KParams P) {
               tc_fence_before();
               mbar_arrive(acc_empty + a);
               released = true;
+            }
+            if (P.tiled) {  // a query's mask and body together: 512 consecutive bytes a warp
+#pragma unroll
+              for (int x = 0; x < CW; x += 2) {
+                const int cg = ct * P.N + c0 + x;
+                if (cg < 2 * P.nq) {
+                  u32 w0[9], w1[9];
+#pragma unroll
+                  for (int g = 0; g < 9; ++g) {
+                    w0[g] = v[g][x];
+                    w1[g] = v[g][x + 1];
+                  }
+                  *reinterpret_cast<ulonglong2*>(orow + (size_t)(cg >> 1) * 2 * FD_MT) =
+                      make_ulonglong2(fold9(w0, P), fold9(w1, P));
+                }
+              }
+              continue;
             }
 #pragma unroll
             for (int x = 0; x < CW; ++x) {
@@ -361,7 +371,10 @@ __global__ void __launch_bounds__(fd_threads(EPI), 1) k_fd_tc(KParams P) {
           u32 w[9];
 #pragma unroll
           for (int g = 0; g < 9; ++g) w[g] = part ? w1[g] : w0[g];
-          if (jok) P.out[((size_t)j * 2 + part) * P.n + t] = fold9(w, P);
+          if (P.tiled)
+            P.out[((size_t)jt * P.n + t) * 2 * FD_MT + 2 * row + part] = fold9(w, P);
+          else if (jok)
+            P.out[((size_t)j * 2 + part) * P.n + t] = fold9(w, P);
         }
         if (!released) {
           tc_fence_before();
@@ -490,8 +503,12 @@ struct Tiling {
   size_t smem;
 };
 
-// packed4: stages hold FD_CHUNK_P4 bytes of planes, then the expanded top plane.
-Tiling tiling(int nq, const FdTile& tile, bool packed4) {
+// Shared memory the default ring may take (the opt-in maximum of sm_100).
+constexpr int SMEM_OPTIN = 227 * 1024;
+
+// packed4: stages hold FD_CHUNK_P4 bytes of planes, then the expanded top plane. `tiled`
+// only decides the defaults.
+Tiling tiling(int nq, const FdTile& tile, bool packed4, bool tiled) {
   Tiling T{};
   int acc_cols;
   if (nq == 1) {
@@ -510,15 +527,19 @@ Tiling tiling(int nq, const FdTile& tile, bool packed4) {
     // rows, so that two accumulator sets (up to 224 columns each) fit in TMEM.
     T.N = fd_round_up((2 * nq + T.n_ct - 1) / T.n_ct, cap == 24 ? 8 : 16);
     T.Np = fd_round_up(FD_LIMBS * T.N, 16);
-    T.stages = tile.stages ? tile.stages : 3;
-    // The default tile (all fields zero) walks one or two c-tiles slot-major and
-    // three or more tile-major. Measured (paper preset): 64 queries, three tiles:
-    // 43.0 ms slot-major, 14.2 ms tile-major at 256 x 4096; 27.3 and 20.3 ms at
-    // 16 x 4096. 32 queries, two tiles: 7.3 ms slot-major, above 10.4 ms
-    // tile-major at 256 x 4096. The SMs of three or more tiles drift apart and
-    // miss each other's planes in L2; two stay together and share them.
+    // Defaults. Tiled outputs: slot-major (the c-tiles of a slot share its planes in L2) and
+    // four stages where they fit; answers differ by 4% at most over all tiles (3 queries at
+    // 256 x 4096: 3.48 ms with four stages, 3.63 with three; 64: 41.5 to 43.0 ms). Outputs of
+    // [query][J][2][n] only meet in L2 while the SMs walk the slots together: three stages, and
+    // tile-major from three c-tiles on (64 queries at 256 x 4096: 43.0 ms slot-major,
+    // 14.2 to 33 ms tile-major; 32 queries, two c-tiles: 7.3 ms slot-major, above
+    // 10.4 ms tile-major).
     const bool builtin = !tile.n_max && !tile.stages && !tile.order;
-    T.order = builtin ? (T.n_ct >= 3 ? 1 : 0) : tile.order;
+    const auto smem = [&](int stages) {
+      return (size_t)stages * (fd_stage_planes(packed4) + (size_t)T.Np * FD_KC) + ZERO_TILE + 256;
+    };
+    T.stages = tile.stages ? tile.stages : (tiled && smem(4) <= SMEM_OPTIN ? 4 : 3);
+    T.order = builtin ? (!tiled && T.n_ct >= 3 ? 1 : 0) : tile.order;
     // Limb k's MMA writes columns [k N, k N + Np); the epilogue reads [0, 9 N).
     acc_cols = std::max(9 * T.N, 4 * T.N + T.Np);
   }
@@ -543,25 +564,26 @@ size_t fd_planes_bytes(int I, int J, int n, bool packed4) {
 
 bool fd_supported(int I, int n, u64 q) { return I >= 1 && I <= 4096 && n >= 1 && q < (1ull << 40); }
 
-bool fd_tile_valid(const FdPlan& p, int nq, const FdTile& t) {
+bool fd_tile_valid(const FdPlan& p, int nq, const FdTile& t, bool tiled) {
   if (nq < 1) return false;
   if (t.n_max != 0 && t.n_max != 16 && t.n_max != 24 && t.n_max != 32 && t.n_max != 48) return false;
   if (t.stages != 0 && (t.stages < 2 || t.stages > 6)) return false;
   if (t.order != 0 && t.order != 1) return false;
   if (nq == 1 && (t.n_max != 0 || t.order != 0)) return false;
-  const Tiling T = tiling(nq, t, p.packed4);
+  const Tiling T = tiling(nq, t, p.packed4, tiled);
   const size_t limit = p.smem_max > 0 ? (size_t)p.smem_max : (size_t)SMEM_DEFAULT;
   return T.Np <= 256 && T.nacc * T.acc_stride <= 512 && T.smem <= limit;
 }
 
-FdTile fd_tile_for(const FdPlan& p, int nq) {
+FdTile fd_tile_for(const FdPlan& p, int nq, bool tiled) {
   const FdTile* below = nullptr;
   for (const auto& e : p.tuned) {
     if ((e.first == 1) != (nq == 1)) continue;  // one-query and batch tiles do not mix
-    if (e.first >= nq) return fd_tile_valid(p, nq, e.second) ? e.second : FdTile{};
+    if (e.second.tiled_only && !tiled) continue;
+    if (e.first >= nq) return fd_tile_valid(p, nq, e.second, tiled) ? e.second : FdTile{};
     below = &e.second;
   }
-  return below && fd_tile_valid(p, nq, *below) ? *below : FdTile{};
+  return below && fd_tile_valid(p, nq, *below, tiled) ? *below : FdTile{};
 }
 
 void fd_set_tile(FdPlan& p, int nq, const FdTile& t) {
@@ -575,14 +597,14 @@ void fd_set_tile(FdPlan& p, int nq, const FdTile& t) {
             [](const std::pair<int, FdTile>& a, const std::pair<int, FdTile>& b) { return a.first < b.first; });
 }
 
-std::vector<FdTile> fd_tile_candidates(const FdPlan& p, int nq) {
+std::vector<FdTile> fd_tile_candidates(const FdPlan& p, int nq, bool tiled) {
   std::vector<FdTile> out;
   out.push_back(FdTile{});  // the default first
   auto add = [&](FdTile t) {
-    const Tiling a = tiling(nq, t, p.packed4);
-    if (!fd_tile_valid(p, nq, t)) return;
+    const Tiling a = tiling(nq, t, p.packed4, tiled);
+    if (!fd_tile_valid(p, nq, t, tiled)) return;
     for (const FdTile& o : out) {  // skip tiles that launch the same kernel configuration
-      const Tiling b = tiling(nq, o, p.packed4);
+      const Tiling b = tiling(nq, o, p.packed4, tiled);
       if (a.N == b.N && a.n_ct == b.n_ct && a.stages == b.stages && a.order == b.order) return;
     }
     out.push_back(t);
@@ -607,8 +629,8 @@ void fd_rows_to_planes(const u64* stage, int i0, const FdPlan& p, uint8_t* plane
 size_t fd_sel_bytes(const FdPlan& p, int nq) {
   // Every candidate's split selection: n * n_ct * Np * I_pad bytes.
   size_t bytes = 0;
-  for (const FdTile& t : fd_tile_candidates(p, nq)) {
-    const Tiling T = tiling(nq, t, p.packed4);
+  for (const FdTile& t : fd_tile_candidates(p, nq, false)) {
+    const Tiling T = tiling(nq, t, p.packed4, false);
     bytes = std::max(bytes, (size_t)p.n * T.n_ct * (size_t)T.Np * p.I_pad);
   }
   return bytes;
@@ -625,10 +647,10 @@ int fd_prepare_device() {
 }
 
 void fd_scan(const FdPlan& p, const u64* sel_eval, u64* out_eval, int nq, uint8_t* scratch, cudaStream_t st,
-             const FdTile* force) {
-  const FdTile tile = force ? *force : fd_tile_for(p, nq);
-  if (force && !fd_tile_valid(p, nq, tile)) throw CudaError(100, "scan tile not valid for this batch");
-  const Tiling T = tiling(nq, tile, p.packed4);
+             const FdTile* force, bool tiled) {
+  const FdTile tile = force ? *force : fd_tile_for(p, nq, tiled);
+  if (force && !fd_tile_valid(p, nq, tile, tiled)) throw CudaError(100, "scan tile not valid for this batch");
+  const Tiling T = tiling(nq, tile, p.packed4, tiled);
   const int n_k16 = p.I_pad / 16, n_kc = p.I_pad / FD_KC;
   const int pad = T.grouped ? T.Np - FD_LIMBS * T.N : 0;
   const long total = (long)p.n * T.n_ct * (T.N + pad) * n_k16;
@@ -659,6 +681,7 @@ void fd_scan(const FdPlan& p, const u64* sel_eval, u64* out_eval, int nq, uint8_
   K.stage_bytes = fd_stage_planes(p.packed4) + T.Np * FD_KC;
   K.sel_off = fd_stage_planes(p.packed4);
   K.unp_off = FD_CHUNK_P4;
+  K.tiled = tiled ? 1 : 0;
   K.fault_ns = p.fault_wait_ns;
   K.qd = (double)p.m.q;
   K.qinv = 1.0 / K.qd;
@@ -674,16 +697,16 @@ void fd_scan(const FdPlan& p, const u64* sel_eval, u64* out_eval, int nq, uint8_
 }
 
 std::vector<FdTuneResult> fd_measure_tiles(const FdPlan& p, int nq, const u64* sel_eval, u64* out_eval,
-                                           uint8_t* scratch, cudaStream_t st, int reps) {
+                                           uint8_t* scratch, cudaStream_t st, int reps, bool tiled) {
   std::vector<FdTuneResult> out;
   cudaEvent_t e0, e1;
   VIA_CUDA(cudaEventCreate(&e0));
   VIA_CUDA(cudaEventCreate(&e1));
   try {
-    for (const FdTile& t : fd_tile_candidates(p, nq)) {
-      fd_scan(p, sel_eval, out_eval, nq, scratch, st, &t);  // warm-up
+    for (const FdTile& t : fd_tile_candidates(p, nq, tiled)) {
+      fd_scan(p, sel_eval, out_eval, nq, scratch, st, &t, tiled);  // warm-up
       VIA_CUDA(cudaEventRecord(e0, st));
-      for (int r = 0; r < reps; ++r) fd_scan(p, sel_eval, out_eval, nq, scratch, st, &t);
+      for (int r = 0; r < reps; ++r) fd_scan(p, sel_eval, out_eval, nq, scratch, st, &t, tiled);
       VIA_CUDA(cudaEventRecord(e1, st));
       VIA_CUDA(cudaEventSynchronize(e1));
       float ms = 0.f;

@@ -49,11 +49,13 @@ constexpr int FD_CHUNK_P4 = 4 * FD_PLANE + FD_PACK4;   // 34816 bytes
 //  order  : 0 walks units slot-major (the c-tiles of one slot run on
 //           neighbouring SMs at the same time and share the slot's planes in
 //           L2); 1 walks them tile-major (one c-tile over every slot, then the next).
-// Zero fields take the built-in default (48 columns, 3 stages; 4 for one query);
-// with all fields zero the order is the default's too: slot-major up to two
-// c-tiles, tile-major from three on.
+// Zero fields take the built-in default (48 columns; 3 or 4 stages; with all fields zero
+// the order is the default's too, see tiling()).
+//  tiled_only : measured with tiled outputs (fd_scan); scans that write the other layout
+//           do not take it, since their speed hangs on other things.
 struct FdTile {
   int n_max = 0, stages = 0, order = 0;
+  int tiled_only = 0;
 };
 
 struct FdPlan {
@@ -82,10 +84,10 @@ inline bool fd_packable(u64 q) { return q < (1ull << 34); }
 bool fd_supported(int I, int n, u64 q);
 
 // The tile a scan of nq queries runs with (tuned entry or default).
-FdTile fd_tile_for(const FdPlan& p, int nq);
+FdTile fd_tile_for(const FdPlan& p, int nq, bool tiled);
 // Every tile the autotuner tries for nq queries (all valid on this device).
-std::vector<FdTile> fd_tile_candidates(const FdPlan& p, int nq);
-bool fd_tile_valid(const FdPlan& p, int nq, const FdTile& t);
+std::vector<FdTile> fd_tile_candidates(const FdPlan& p, int nq, bool tiled);
+bool fd_tile_valid(const FdPlan& p, int nq, const FdTile& t, bool tiled = false);
 // Records `t` as the tile for batches of nq (replacing an entry for nq).
 void fd_set_tile(FdPlan& p, int nq, const FdTile& t);
 
@@ -98,7 +100,7 @@ struct FdTuneResult {
 // and `reps` timed scans each, with CUDA events on `st`. Returns the
 // measurements in candidate order; the first entry is the default tile.
 std::vector<FdTuneResult> fd_measure_tiles(const FdPlan& p, int nq, const u64* sel_eval, u64* out_eval,
-                                           uint8_t* scratch, cudaStream_t st, int reps);
+                                           uint8_t* scratch, cudaStream_t st, int reps, bool tiled);
 
 // Converts rows [i0, i0 + 16) of an eval-form database held as u64 [16][J][n]
 // (`stage`, rows beyond I ignored) into the byte planes.
@@ -116,7 +118,13 @@ size_t fd_sel_bytes(const FdPlan& p, int nq);
 // out_eval[b][j] = sum_i sel_eval[b][i] (.) db[i][j] for mask and body:
 // sel_eval [nq][I][2][n], out_eval [nq][J][2][n], eval form mod q2. `force`
 // overrides the tuned tile (it must be valid for nq).
+//
+// `tiled` changes the output to columns grouped by MMA tile, [J_pad / 128][n][nq][128][2]
+// (the 128 columns j of a tile, mask and body of each), for a consumer that gathers the
+// slots itself. An SM works on one slot t at a time, so [..][n] outputs are 8-byte writes
+// 32 KB apart that only meet in L2 while the SMs stay together: at 64 queries and
+// 256 x 4096 the scan took between 15 and 54 ms from one tile and run to the next.
 void fd_scan(const FdPlan& p, const u64* sel_eval, u64* out_eval, int nq, uint8_t* scratch, cudaStream_t st,
-             const FdTile* force = nullptr);
+             const FdTile* force = nullptr, bool tiled = false);
 
 }  // namespace via

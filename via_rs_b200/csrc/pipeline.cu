@@ -745,10 +745,11 @@ void WorkspaceDeleter::operator()(Workspace* w) const { delete w; }
 void workspace_destroy(Server& s) { s.ws.reset(); }
 uint8_t* workspace_sel_bytes(Server& s) { return reinterpret_cast<uint8_t*>(s.ws->sel_bytes.p); }
 
-void first_dim_queries(Server& s, const u64* sel_eval, u64* out_eval, int nq, uint8_t* scratch, cudaStream_t st) {
+void first_dim_queries(Server& s, const u64* sel_eval, u64* out_eval, int nq, uint8_t* scratch, cudaStream_t st,
+                       bool tiled) {
   const via_params& p = s.prm;
   if (s.tensor_fd()) {
-    fd_scan(s.fd, sel_eval, out_eval, nq, scratch, st);
+    fd_scan(s.fd, sel_eval, out_eval, nq, scratch, st, nullptr, tiled);
     return;
   }
   for (int q = 0; q < nq; ++q)
@@ -756,14 +757,26 @@ void first_dim_queries(Server& s, const u64* sel_eval, u64* out_eval, int nq, ui
                          (int)p.num_rows, (int)p.num_cols, (int)p.n1, s.r2.m[0], st);
 }
 
+static bool cmux_fused_ok(const DevRing& R, const Gadget& g);
+
+// Levels of at most this many CMuxes run on four-CTA clusters (cmux_fused).
+constexpr long CMUX_CLUSTER_MAX = 64;
+
+// Whether the scan of nq queries writes tiled columns, which the CMux tree's first level
+// gathers: answers with the fused CMux and a first level of single-CTA CMuxes.
+bool cmux_takes_tiles(Server& s, long nq) {
+  const via_params& p = s.prm;
+  return s.tensor_fd() && p.num_cols >= 2 && nq * (long)p.num_cols / 2 > CMUX_CLUSTER_MAX &&
+         cmux_fused_ok(s.r2, make_gadget(p.b_cmux, (int)p.l_query, s.r2));
+}
+
 // Times every candidate scan tile for nq queries on the handle's workspace
 // buffers (the workspace must hold batches of nq).
 std::vector<FdTuneResult> workspace_measure_tiles(Server& s, Workspace& w, int nq, int reps) {
   if (w.bmax < nq) throw CudaError(100, "workspace smaller than the batch to tune");
-  return fd_measure_tiles(s.fd, nq, w.sel.p, w.fd_out.p, reinterpret_cast<uint8_t*>(w.sel_bytes.p), s.stream, reps);
+  return fd_measure_tiles(s.fd, nq, w.sel.p, w.fd_out.p, reinterpret_cast<uint8_t*>(w.sel_bytes.p), s.stream, reps,
+                          cmux_takes_tiles(s, nq));
 }
-
-static bool cmux_fused_ok(const DevRing& R, const Gadget& g);
 
 // Allocates a workspace for batches of up to bmax queries, or (count_only)
 // returns the bytes it would take.
@@ -808,7 +821,7 @@ static size_t workspace_build(Server& s, int bmax, Workspace* w, bool count_only
     for (int nq = 1; nq <= B; ++nq) bytes = std::max(bytes, fd_sel_bytes(s.fd, nq));
     A(w->sel_bytes, (bytes + 7) / 8);
   }
-  A(w->fd_out, B * J * 2 * n1);
+  A(w->fd_out, B * (s.tensor_fd() ? (long)s.fd.J_pad : J) * 2 * n1);  // tiled columns come in whole tiles
   const bool fused = cmux_fused_ok(s.r2, make_gadget(p.b_cmux, (int)p.l_query, s.r2));
   A(w->cm_diff, fused ? 0 : B * std::max(1L, J / 2) * 2 * n1);
   A(w->cm_digits, fused ? 0 : B * std::max(1L, J / 2) * 2 * L * n1);
@@ -1065,16 +1078,22 @@ static void external_products(const DevRing& R, const Gadget& g, KeySel rgsw, co
 // other two stay within one, and the inverse ends in the layout the forward starts in:
 // 6 CTA barriers a CMux where 40 were. With the digit split and the conversions on doubles
 // and the dense first phase: 8191 CMuxes of a five-query batch 624 -> 410 us.
-template <int LOGN>
+//
+// TILED (the first level): cur holds fd_scan's tiled columns of nq queries, where a pair's
+// four residues of a slot are 32 consecutive bytes; the body's difference waits in shared
+// memory (n = 4096: is read again).
+template <int LOGN, bool TILED>
 __global__ void __launch_bounds__((1 << LOGN) / 8, LOGN >= 12 ? 1 : 2) k_cmux_fp(const u64* __restrict__ cur,
                                                                                 u64* __restrict__ nxt, KeySel ks,
-                                                                                const __grid_constant__ DevRing R,
+                                                                                long nq, const __grid_constant__ DevRing R,
                                                                                 const __grid_constant__ Gadget g) {
   constexpr int n = 1 << LOGN;
   // Transforms alternate between two exchange areas, so each needs one CTA barrier
   // (fp_forward, fp_inverse); at n = 4096 one area (32 KB) and a barrier before each.
   constexpr int NB = LOGN >= 12 ? 1 : 2;
+  constexpr bool KEEP = TILED && LOGN < 12;
   __shared__ double ssm[NB][n];
+  __shared__ double body[KEEP ? n : 1];
   int buf = 0;
   auto area = [&]() -> double* {
     if constexpr (NB == 1) {
@@ -1089,21 +1108,48 @@ __global__ void __launch_bounds__((1 << LOGN) / 8, LOGN >= 12 ? 1 : 2) k_cmux_fp
   const NttTable& T = R.t[0];
   const double q = T.qd, qinv = T.qinv;
   const u64* a = cur + (2 * o) * 2 * n;
+  const long tstep = 2 * FD_MT * nq;  // tiled: residues from a slot to the next
+  if (TILED) {
+    const long j = 2 * (o % ks.div), query = o / ks.div;  // ks.div CMuxes a query
+    a = cur + (((j / FD_MT) * n + 8 * tid) * nq + query) * 2 * FD_MT + 2 * (j % FD_MT);
+  }
   const u64* K = ks.base + ((o / ks.div) % ks.mod) * ks.stride;
   const int L = g.L;
   const bool dense = 4.0 * g.dB * q < 281474976710656.0;  // |digit| <= B / 2: fp_digit_phase's sums below 2^48
-  double am[8], ab[8];
+  double am[8], ab[8];  // in[2o] and the products
 #pragma unroll
-  for (int v = 0; v < 8; ++v) am[v] = ab[v] = 0.0;
+  for (int v = 0; v < 8; ++v) ab[v] = 0.0;
 #pragma unroll 1
   for (int p = 0; p < 2; ++p) {  // 0: mask digits (neg_s_m rows), 1: body digits (m rows)
     double val[8];
-    {
+    if (TILED && KEEP && p) {
+#pragma unroll
+      for (int v = 0; v < 8; ++v) val[v] = body[v * (n / 8) + tid];
+    } else if (TILED) {
+#pragma unroll
+      for (int v = 0; v < 8; ++v) {
+        u64 x[4];  // in[2o] mask, body, in[2o+1] mask, body of slot 8 tid + v
+        asm volatile("ld.global.v4.u64 {%0, %1, %2, %3}, [%4];"
+                     : "=l"(x[0]), "=l"(x[1]), "=l"(x[2]), "=l"(x[3])
+                     : "l"(a + v * tstep));
+        val[v] = __dadd_rn(fp_from_u64(x[2 + (KEEP ? 0 : p)]), -fp_from_u64(x[KEEP ? 0 : p]));
+        if (p == 0) am[v] = fp_from_u64(x[0]);
+        if (KEEP || p) ab[v] = __dadd_rn(ab[v], fp_from_u64(x[1]));
+        if (KEEP) body[v * (n / 8) + tid] = __dadd_rn(fp_from_u64(x[3]), -fp_from_u64(x[1]));
+      }
+    } else {
       u64 x[8], y[8];
       ld8(a + 2 * n + p * n + 8 * tid, x);
       ld8(a + p * n + 8 * tid, y);
 #pragma unroll
-      for (int v = 0; v < 8; ++v) val[v] = __dadd_rn(fp_from_u64(x[v]), -fp_from_u64(y[v]));
+      for (int v = 0; v < 8; ++v) {
+        const double yd = fp_from_u64(y[v]);
+        val[v] = __dadd_rn(fp_from_u64(x[v]), -yd);
+        if (p == 0)
+          am[v] = yd;
+        else
+          ab[v] = __dadd_rn(ab[v], yd);
+      }
     }
     fp_inverse<LOGN>(val, tid, T, area());
 #pragma unroll
@@ -1125,13 +1171,11 @@ __global__ void __launch_bounds__((1 << LOGN) / 8, LOGN >= 12 ? 1 : 2) k_cmux_fp
     }
   }
   u64 x[8];
-  ld8(a + 8 * tid, x);
 #pragma unroll
-  for (int v = 0; v < 8; ++v) x[v] = fp_to_u64(fp_canonical(__dadd_rn(fp_from_u64(x[v]), am[v]), q, qinv));
+  for (int v = 0; v < 8; ++v) x[v] = fp_to_u64(fp_canonical(am[v], q, qinv));
   st8(nxt + o * 2 * n + 8 * tid, x);
-  ld8(a + n + 8 * tid, x);
 #pragma unroll
-  for (int v = 0; v < 8; ++v) x[v] = fp_to_u64(fp_canonical(__dadd_rn(fp_from_u64(x[v]), ab[v]), q, qinv));
+  for (int v = 0; v < 8; ++v) x[v] = fp_to_u64(fp_canonical(ab[v], q, qinv));
   st8(nxt + o * 2 * n + n + 8 * tid, x);
 }
 
@@ -1217,11 +1261,12 @@ static bool cmux_fused_ok(const DevRing& R, const Gadget& g) {
          (R.n == 4096 || R.n == 2048 || R.n == 1024 || R.n == 512);
 }
 
+// tiled_nq > 0: cur holds the tiled columns of that many queries (cmux_takes_tiles).
 static void cmux_fused(const DevRing& R, const Gadget& g, const u64* cur, u64* nxt, KeySel ks, long count,
-                       cudaStream_t st) {
+                       long tiled_nq, cudaStream_t st) {
   // Levels of at most 64 CMuxes leave most SMs idle: split each CMux over a
   // four-CTA cluster to cut its latency.
-  if (count <= 64 && g.L == 2 && R.n <= 2048) {
+  if (count <= CMUX_CLUSTER_MAX && g.L == 2 && R.n <= 2048 && !tiled_nq) {
     switch (R.n) {
       case 2048: k_cmux_cluster_fp<11><<<(unsigned)(4 * count), 256, 0, st>>>(cur, nxt, ks, R, g); break;
       case 1024: k_cmux_cluster_fp<10><<<(unsigned)(4 * count), 128, 0, st>>>(cur, nxt, ks, R, g); break;
@@ -1230,12 +1275,19 @@ static void cmux_fused(const DevRing& R, const Gadget& g, const u64* cur, u64* n
     VIA_LAUNCHED();
     return;
   }
+#define VIA_CMUX_CASE(LG)                                                                                        \
+  if (tiled_nq)                                                                                                 \
+    k_cmux_fp<LG, true><<<(unsigned)count, (1 << LG) / 8, 0, st>>>(cur, nxt, ks, tiled_nq, R, g);               \
+  else                                                                                                          \
+    k_cmux_fp<LG, false><<<(unsigned)count, (1 << LG) / 8, 0, st>>>(cur, nxt, ks, 0, R, g);                     \
+  break;
   switch (R.n) {
-    case 4096: k_cmux_fp<12><<<(unsigned)count, 512, 0, st>>>(cur, nxt, ks, R, g); break;
-    case 2048: k_cmux_fp<11><<<(unsigned)count, 256, 0, st>>>(cur, nxt, ks, R, g); break;
-    case 1024: k_cmux_fp<10><<<(unsigned)count, 128, 0, st>>>(cur, nxt, ks, R, g); break;
-    default: k_cmux_fp<9><<<(unsigned)count, 64, 0, st>>>(cur, nxt, ks, R, g); break;
+    case 4096: VIA_CMUX_CASE(12)
+    case 2048: VIA_CMUX_CASE(11)
+    case 1024: VIA_CMUX_CASE(10)
+    default: VIA_CMUX_CASE(9)
   }
+#undef VIA_CMUX_CASE
   VIA_LAUNCHED();
 }
 
@@ -1419,7 +1471,8 @@ void answer_device_stages(Server& s, Workspace& w, const u64* d_query, int nq, u
   // ---- Step 4: FirstDim (answer.rs:204-205), one pass over the database for
   // the whole batch; the columns stay in the eval domain.
   to_eval(s.r2, w.sel.p, n1, B * 2 * I, st);
-  first_dim_queries(s, w.sel.p, w.fd_out.p, nq, reinterpret_cast<uint8_t*>(w.sel_bytes.p), st);
+  const bool tiled = stop_stage != 5 && cmux_takes_tiles(s, B);
+  first_dim_queries(s, w.sel.p, w.fd_out.p, nq, reinterpret_cast<uint8_t*>(w.sel_bytes.p), st, tiled);
   if (stop_stage == 5) {
     copy_out(w.fd_out.p, (size_t)J * 2 * n1);
     from_eval(s.r2, dump, n1, 2 * J, st);
@@ -1436,7 +1489,7 @@ void answer_device_stages(Server& s, Workspace& w, const u64* d_query, int nq, u
     KeySel bit{rgsw_b2 + i * rgsw2, half, B, nb * rgsw2};
     u64* nxt = cur == w.fd_out.p ? w.cm_b.p : w.fd_out.p;  // ping-pong between fd_out and cm_b
     if (cmux_fused_ok(s.r2, w.g_cmux)) {
-      cmux_fused(s.r2, w.g_cmux, cur, nxt, bit, B * half, st);
+      cmux_fused(s.r2, w.g_cmux, cur, nxt, bit, B * half, tiled && i == 0 ? B : 0, st);
       cur = nxt;
       continue;
     }

@@ -549,7 +549,7 @@ std::string tune_key(const Server& s, int nq) {
   std::string dev = prop.name;
   for (char& c : dev)
     if (c == ' ' || c == '\t') c = '_';
-  return "fd_tc/2 " + dev + " n=" + std::to_string(s.fd.n) + " I=" + std::to_string(s.fd.I) +
+  return "fd_tc/3 " + dev + " n=" + std::to_string(s.fd.n) + " I=" + std::to_string(s.fd.I) +
          " J=" + std::to_string(s.fd.J) + " q=" + std::to_string(s.fd.m.q) + " nq=" + std::to_string(nq);
 }
 
@@ -604,7 +604,7 @@ void autotune_scan(Server& s, Workspace& w, const std::vector<int>& sizes, const
     const std::string key = tune_key(s, nq);
     const CachedTile* hit = nullptr;
     for (const auto& e : cache)
-      if (e.first == key && fd_tile_valid(s.fd, nq, e.second.tile)) hit = &e.second;
+      if (e.first == key && fd_tile_valid(s.fd, nq, e.second.tile, cmux_takes_tiles(s, nq))) hit = &e.second;
     CachedTile best;
     uint32_t measured = 0;
     if (hit) {
@@ -628,6 +628,7 @@ void autotune_scan(Server& s, Workspace& w, const std::vector<int>& sizes, const
       measured = (uint32_t)r.size();
       append_tune_cache(cache_path, key, best);
     }
+    best.tile.tiled_only = cmux_takes_tiles(s, nq) ? 1 : 0;
     fd_set_tile(s.fd, nq, best.tile);
     if (out) out->push_back(via_scan_tuning{(uint32_t)nq, to_abi(best.tile), best.ms, best.default_ms, measured, 0});
   }
@@ -700,7 +701,7 @@ uint64_t via_scan_tile_candidates(via_server* s, uint32_t batch, via_scan_tile* 
   if (!s || !s->tensor_fd() || batch == 0 || batch > 4096) return 0;
   std::vector<FdTile> c;
   try {
-    c = fd_tile_candidates(s->fd, (int)batch);
+    c = fd_tile_candidates(s->fd, (int)batch, cmux_takes_tiles(*s, batch));
   } catch (...) {
     return 0;
   }

@@ -144,7 +144,9 @@ int workspace_batch(Server& s);
 void workspace_destroy(Server& s);
 uint8_t* workspace_sel_bytes(Server& s);
 // FirstDim of nq queries: sel_eval [nq][I][2][n1] -> out_eval [nq][J][2][n1] (eval at q2).
-void first_dim_queries(Server& s, const u64* sel_eval, u64* out_eval, int nq, uint8_t* scratch, cudaStream_t st);
+void first_dim_queries(Server& s, const u64* sel_eval, u64* out_eval, int nq, uint8_t* scratch, cudaStream_t st,
+                       bool tiled = false);  // tiled: fd_scan's tiled columns (tensor-core scans only)
+bool cmux_takes_tiles(Server& s, long nq);  // answers of nq queries scan into tiled columns
 std::vector<FdTuneResult> workspace_measure_tiles(Server& s, Workspace& w, int nq, int reps);
 // The scan autotuner (server.cu): measures (or reads from the cache file) the
 // fastest tile for every batch size on workspace w, records it in s.fd and
