@@ -50,3 +50,27 @@ def test_tiles(oracle, count):
     for k in {0, 1, count // 2, count - 2, count - 1}:
         m, b = cpu.answer(qs[k])
         assert np.array_equal(masks[k], m) and np.array_equal(bodies[k], b), k
+
+
+@pytest.mark.parametrize("base,depth", [(32, 15), (21, 18), (300, 9)])
+def test_other_gadgets(oracle, base, depth):
+    """Gadgets the GEMM steps do not serve (depth, B^6 above 2^26, digits beyond a byte) keep the
+    transform path for every step."""
+    import dataclasses
+
+    prm = dataclasses.replace(paper_preset(2, 2), ck_base=base, l_ck=depth)
+    c, gpu, cpu = _setup(oracle, prm, b"gemm-other")
+    q = c.query(3, b"other")
+    assert np.array_equal(gpu.debug_stage(q, 2), cpu.debug_stage(q, 2))
+
+
+def test_query_count_edges(oracle):
+    """Two LWEs a thread in the late steps' multiply-accumulate: an odd number of LWEs."""
+    prm = paper_preset(2, 2)
+    c, gpu, cpu = _setup(oracle, prm, b"gemm-odd")
+    # 41 queries x 2 LWEs (DMux group) and x 6 (the rest): both groups past the rule's line.
+    qs = np.stack([c.query(k % prm.capacity, b"o-%03d" % k) for k in range(41)])
+    masks, bodies = gpu.answer_many(qs)
+    for k in (0, 20, 40):
+        m, b = cpu.answer(qs[k])
+        assert np.array_equal(masks[k], m) and np.array_equal(bodies[k], b), k

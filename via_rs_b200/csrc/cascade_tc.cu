@@ -31,6 +31,12 @@ struct CtParams {
   int mtiles, out_kp, out_half;
 };
 
+// Item -> its first unit, and its units. Units 0 .. units - 1 are mask units.
+__host__ __device__ __forceinline__ int ct_item(const CtStep& S, int item, int& len) {
+  len = item < S.units ? 1 : S.chain;
+  return item < S.units ? item : S.units + (item - S.units) * S.chain;
+}
+
 // First output mask of a unit. Mask units of n >= 8 run over the coefficient blocks of
 // one output mask, body units over the output masks of one coefficient block.
 __host__ __device__ __forceinline__ int ct_first_mask(const CtStep& S, int unit) {
@@ -38,54 +44,6 @@ __host__ __device__ __forceinline__ int ct_first_mask(const CtStep& S, int unit)
   if (S.n < 8) return mu * S.G;
   return unit < S.units ? mu / (2 * S.n / CT_ROWS) : mu % S.half;
 }
-
-// The fixed-point fractions f[piece] (32 bits, rounded up by less than 3 ulp) of
-// the three base-T pieces of round(c S / Q) + o (S - 1) / (B - 1) mod S, most
-// significant piece first, for c / Q = y0 / q0 + y1 / q1 mod 1, |y_l| <= 0.5625 q_l.
-__device__ __forceinline__ void ct_pieces(double y0, double y1, const CtDigits& D, u32 (&f)[3]) {
-  int p[3];
-#pragma unroll
-  for (int i = 0; i < 3; ++i) {
-    // T y = qt q + r exactly, |r| <= 0.5625 q (fp_mulmod with its quotient kept);
-    // the quotient's low word is read off the rounding sum.
-    const double h0 = __dmul_rn(D.T, y0), h1 = __dmul_rn(D.T, y1);
-    const double l0 = __fma_rn(D.T, y0, -h0), l1 = __fma_rn(D.T, y1, -h1);
-    const double u0 = __fma_rn(h0, D.qinv[0], FP_ROUND), u1 = __fma_rn(h1, D.qinv[1], FP_ROUND);
-    p[i] = __double2loint(u0) + __double2loint(u1);
-    y0 = __dadd_rn(__fma_rn(-__dadd_rn(u0, -FP_ROUND), D.q[0], h0), l0);
-    y1 = __dadd_rn(__fma_rn(-__dadd_rn(u1, -FP_ROUND), D.q[1], h1), l1);
-  }
-  // Rounding: the remainder y0 / q0 + y1 / q1 to the nearest integer (no ties: Q is odd).
-  const double s = __fma_rn(y0, D.qinv[0], __dmul_rn(y1, D.qinv[1]));
-  const double us = __dadd_rn(s, FP_ROUND);
-  int rnd = __double2loint(us);
-  if (fabs(__dadd_rn(s, -__dadd_rn(us, -FP_ROUND))) > 0.5 - 1e-12) {  // too near to tell in doubles
-    const i128 num = (i128)(i64)y0 * (i128)D.qi[1] + (i128)(i64)y1 * (i128)D.qi[0];
-    const i128 Q = (i128)D.qi[0] * D.qi[1];
-    rnd = 2 * num > Q ? 1 : (2 * num < -Q ? -1 : 0);
-  }
-  // Pieces lie in (-1.2 T, 1.2 T); with off (below 3 T, at least 2 T) they are
-  // nonnegative and below 4.3 T < 2^29, where umulhi(x, M) >> sh = floor(x / T).
-  u32 carry = 2;
-#pragma unroll
-  for (int i = 2; i >= 0; --i) {
-    const u32 x = (u32)p[i] + (i == 2 ? (u32)rnd : 0u) + D.off + carry - 2;
-    carry = __umulhi(x, D.M) >> D.sh;
-    const u32 u = x - carry * D.Ti;
-    const u64 m = (u64)u * D.M;
-    f[i] = (u32)(m >> D.sh) + 1;
-  }
-}
-
-// The next base-B digit of a fraction, most significant first.
-__device__ __forceinline__ u32 ct_digit(u32& f, u32 base) {
-  const u64 m = (u64)f * base;
-  f = (u32)m;
-  return (u32)(m >> 32);
-}
-
-// Signed bytes of four unsigned digits w below 256: w - o.
-__device__ __forceinline__ u32 ct_signed(u32 w, u32 o) { return (w + (128 - o) * 0x01010101u) ^ 0x80808080u; }
 
 // First step's digits from the query: K position j kp + which L + s of LWE w holds
 // digit s of mask which * half + j. Thread = (8-LWE group, j, LWE of the group).
@@ -177,9 +135,9 @@ __global__ void __launch_bounds__(CT_THREADS, 1) k_ct_step(const __grid_constant
       u32 ph = 0, armed = 0, armed_par = 0;
       bool ok = true;
       for (int it = blockIdx.x; ok && it < items; it += gridDim.x) {
-        const int item = it / P.mtiles, mt = it % P.mtiles;
-        const int len = item < S.units ? 1 : S.chain;
-        const int unit0 = item < S.units ? item : S.units + (item - S.units) * S.chain;
+        const int mt = it % P.mtiles;
+        int len;
+        const int unit0 = ct_item(S, it / P.mtiles, len);
         const long left = P.nlwe - (long)mt * CT_M;
         const u32 ng = (u32)((min(left, (long)CT_M) + 7) / 8);
         const u32 abytes = CT_KC / 16 * ng * 128;
@@ -231,7 +189,9 @@ __global__ void __launch_bounds__(CT_THREADS, 1) k_ct_step(const __grid_constant
         }
         tc_fence_after();
         const u32 dacc = tmem + (u32)(a * CT_N);
-        const int nk = (it / P.mtiles < S.units ? 1 : S.chain) * S.chunks;
+        int nk;
+        ct_item(S, it / P.mtiles, nk);
+        nk *= S.chunks;
         for (int kc = 0; kc < nk; ++kc) {
           if (!mbar_wait(full + s, ph, abort_flag)) {
             ok = false;
@@ -271,7 +231,9 @@ __global__ void __launch_bounds__(CT_THREADS, 1) k_ct_step(const __grid_constant
     u32 aph = 0;
     bool ok = true;
     for (int it = blockIdx.x; ok && it < items; it += gridDim.x) {
-      const int item = it / P.mtiles, mt = it % P.mtiles;
+      const int mt = it % P.mtiles;
+      int len;
+      const int unit = ct_item(S, it / P.mtiles, len);
       const long w = (long)mt * CT_M + m;
       if (!__all_sync(0xffffffffu, mbar_wait(acc_full + a, aph, abort_flag))) {
         ok = false;
@@ -305,7 +267,7 @@ __global__ void __launch_bounds__(CT_THREADS, 1) k_ct_step(const __grid_constant
 #pragma unroll
       for (int l = 0; l < 2; ++l) {
         const double q = P.D.q[l], qinv = P.D.qinv[l];
-        const double* cc = P.c + ((size_t)item * 2 + l) * CT_ROWS + part * 4;
+        const double* cc = P.c + ((size_t)(it / P.mtiles) * 2 + l) * CT_ROWS + part * 4;
 #pragma unroll
         for (int r = 0; r < 4; ++r) {
           const u64 lo = (u64)v[l][0][r] + ((u64)v[l][1][r] << 8) + ((u64)v[l][2][r] << 16);
@@ -315,8 +277,8 @@ __global__ void __launch_bounds__(CT_THREADS, 1) k_ct_step(const __grid_constant
         }
       }
       const int r0 = part * 4;
-      if (item >= S.units) {  // body sums, canonical, added over the items of the same coefficients
-        const int yy = S.n >= 8 ? (item - S.units) * S.chain / S.half * CT_ROWS + r0 : r0 % n_out;
+      if (unit >= S.units) {  // body sums, canonical, added over the items of the same coefficients
+        const int yy = S.n >= 8 ? (unit - S.units) / S.half * CT_ROWS + r0 : r0 % n_out;
         unsigned long long* o = reinterpret_cast<unsigned long long*>(P.body) + (size_t)yy * 2 * P.nlwe + w;
 #pragma unroll
         for (int l = 0; l < 2; ++l) {
@@ -335,8 +297,8 @@ __global__ void __launch_bounds__(CT_THREADS, 1) k_ct_step(const __grid_constant
       }
       // Rows part * 4 .. + 3 of the unit: output mask jj, coefficients yy .. (n >= 2),
       // or masks jj, jj + 1 of two coefficients each (n = 1).
-      const int jj = S.n >= 8 ? item / upj : item * S.G + r0 / n_out;
-      const int yy = S.n >= 8 ? (item % upj) * CT_ROWS + r0 : r0 % n_out;
+      const int jj = S.n >= 8 ? unit / upj : unit * S.G + r0 / n_out;
+      const int yy = S.n >= 8 ? (unit % upj) * CT_ROWS + r0 : r0 % n_out;
       u32 f[4][3];
 #pragma unroll
       for (int r = 0; r < 4; ++r) ct_pieces(y[0][r], y[1][r], P.D, f[r]);
@@ -452,8 +414,8 @@ __global__ void k_ct_consts(const uint8_t* __restrict__ planes, CtStep st, DevRi
   const int lane = threadIdx.x & 31;
   if (gid >= (long)st.items() * 32) return;
   const int r = (int)(gid & 15), l = (int)((gid >> 4) & 1), item = (int)(gid >> 5);
-  const int unit0 = item < st.units ? item : st.units + (item - st.units) * st.chain;
-  const int len = item < st.units ? 1 : st.chain;
+  int len;
+  const int unit0 = ct_item(st, item, len);
   u64 sum[5] = {0, 0, 0, 0, 0};
   for (int k16 = lane; k16 < len * st.chunks * (CT_KC / 16); k16 += 32) {
     const uint8_t* base = planes + ((size_t)unit0 * st.chunks + k16 / (CT_KC / 16)) * CT_STAGE_B +
@@ -478,7 +440,9 @@ __global__ void k_ct_consts(const uint8_t* __restrict__ planes, CtStep st, DevRi
   }
 }
 
-CtDigits make_digits(const via_params& p, const DevRing& R) {
+}  // namespace
+
+CtDigits ct_digits(u64 base, const DevRing& R) {
   CtDigits D{};
   for (int l = 0; l < 2; ++l) {
     const u64 q = R.m[l].q;
@@ -489,32 +453,33 @@ CtDigits make_digits(const via_params& p, const DevRing& R) {
     D.yscale[l] = (double)h_inv(R.m[1 - l].q % q, q);
   }
   u64 T = 1;
-  for (int i = 0; i < CT_LP; ++i) T *= p.ck_base;
+  for (int i = 0; i < CT_LP; ++i) T *= base;
   D.T = (double)T;
   D.Ti = (u32)T;
-  D.base = (u32)p.ck_base;
-  D.o = (u32)(p.ck_base - 1 - p.ck_base / 2);
+  D.base = (u32)base;
+  D.o = (u32)(base - 1 - base / 2);
   int sh = 0;
   while (((u64)1 << (sh + 1)) < T) ++sh;  // 2^sh < T <= 2^(sh + 1)
   D.sh = sh;
   D.M = (u32)((((u128)1 << (32 + sh)) + T - 1) / T);
-  D.off = (u32)(D.o * ((T - 1) / (p.ck_base - 1)) + 2 * T);
+  D.off = (u32)(D.o * ((T - 1) / (base - 1)) + 2 * T);
   return D;
 }
 
-}  // namespace
-
-// Two-prime NTT rings of degree 256 .. 4096, primes of 26 to 40 bits (five bytes; a quotient of
-// T y / q fits the low word), gadgets of 18 digits with B^6 < 2^26 (a piece's arithmetic
-// fits 32 bits).
-bool ct_supported(const via_params& p, const DevRing& R) {
-  if (!R.ntt || R.nl != 2 || p.n1 < 256 || p.l_ck != CT_L || p.ck_base < 3) return false;
+// Two-prime NTT rings, primes of 26 to 40 bits (five bytes; a quotient of T y / q fits the low
+// word), gadgets of 18 digits with B^6 < 2^26 (a piece's arithmetic fits 32 bits).
+bool ct_digits_ok(u64 base, u32 L, const DevRing& R) {
+  if (!R.ntt || R.nl != 2 || L != CT_L || base < 3 || base > 255) return false;
   u64 T = 1;
-  for (int i = 0; i < CT_LP; ++i) T *= p.ck_base;
-  if (p.ck_base > 255 || T >= (1ull << 26)) return false;
+  for (int i = 0; i < CT_LP; ++i) T *= base;
+  if (T >= (1ull << 26)) return false;
   for (int l = 0; l < 2; ++l)
     if (R.m[l].q >= (1ull << 40) || R.m[l].q < (1ull << 26)) return false;
   return true;
+}
+
+bool ct_supported(const via_params& p, const DevRing& R) {
+  return p.n1 >= 256 && ct_digits_ok(p.ck_base, p.l_ck, R);
 }
 
 int ct_steps(const via_params&) { return 7; }  // input degrees 1 .. 64
@@ -528,32 +493,34 @@ void ct_prepare(Server& s) {
   if (!ct_supported(p, s.r1) || !s.cascade_eval.p || !s.fd_err.p) return;
   const int K = ct_steps(p), n1 = (int)p.n1;
   size_t bytes = 0, consts = 0;
-  std::vector<CtStep> steps;
   for (int k = 0; k < K; ++k) {
-    CtStep st = ct_step(n1, 1 << k);
-    st.b_off = bytes;
-    st.c_off = consts;
+    const CtStep st = ct_step(n1, 1 << k);
     bytes += (size_t)2 * st.units * st.chunks * CT_STAGE_B;
-    consts += (size_t)st.items() * 2 * CT_ROWS;
-    steps.push_back(st);
+    consts += (size_t)2 * st.units * 2 * CT_ROWS;  // room for items of one unit
   }
   ct_prepare_device();
   s.ct_planes.alloc(bytes / 8);
-  s.ct_consts.alloc(consts);
-  const CtDigits D = make_digits(p, s.r1);
+  s.ct_consts.alloc(2 * consts);  // for few and for many tiles
+  const CtDigits D = ct_digits(p.ck_base, s.r1);
   const u64 step_len = (u64)2 * n1 * CT_L * 2 * 2;
   const u64 inv0 = (u64)D.yscale[0], inv1 = (u64)D.yscale[1];
+  uint8_t* planes = reinterpret_cast<uint8_t*>(s.ct_planes.p);
+  double* cc = reinterpret_cast<double*>(s.ct_consts.p);
   for (int k = 0; k < K; ++k) {
-    const CtStep& st = steps[k];
-    uint8_t* planes = reinterpret_cast<uint8_t*>(s.ct_planes.p) + st.b_off;
+    const CtStep st = ct_step(n1, 1 << k);
     const long threads = (long)2 * st.units * st.chunks * (CT_KC / 16) * 32;
     k_ct_planes<<<(unsigned)((threads + 255) / 256), 256, 0, s.stream>>>(s.cascade_eval.p + k * step_len, st, s.r1, inv0,
                                                                         inv1, planes);
     VIA_LAUNCHED();
-    const long warps = (long)st.items() * 32;
-    k_ct_consts<<<(unsigned)((warps * 32 + 255) / 256), 256, 0, s.stream>>>(
-        planes, st, s.r1, D.o, reinterpret_cast<double*>(s.ct_consts.p) + st.c_off);
-    VIA_LAUNCHED();
+    for (int many = 0; many < 2; ++many) {
+      const CtStep c = ct_step(n1, 1 << k, many ? CT_MANY : 1);
+      const long warps = (long)c.items() * 32;
+      k_ct_consts<<<(unsigned)((warps * 32 + 255) / 256), 256, 0, s.stream>>>(planes, c, s.r1, D.o,
+                                                                             cc + many * consts);
+      VIA_LAUNCHED();
+    }
+    planes += (size_t)2 * st.units * st.chunks * CT_STAGE_B;
+    cc += (size_t)2 * st.units * 2 * CT_ROWS;
   }
   s.ct_steps = K;
 }
@@ -562,16 +529,16 @@ void ct_run(Server& s, const u64* d_query, long nlwe, uint8_t* da, uint8_t* db, 
             cudaStream_t st) {
   const via_params& p = s.prm;
   const int n1 = (int)p.n1;
-  const CtDigits D = make_digits(p, s.r1);
+  const CtDigits D = ct_digits(p.ck_base, s.r1);
   const int mtiles = (int)((nlwe + CT_M - 1) / CT_M);
-  CtStep cur = ct_step(n1, 1);
+  CtStep cur = ct_step(n1, 1, mtiles);
   const long threads = (nlwe + 7) / 8 * 8 * cur.half;
   k_ct_digits<<<(unsigned)((threads + 255) / 256), 256, 0, st>>>(d_query, nlwe, (long)lwe_len(p), n1, cur, D,
                                                                 (size_t)CT_M * cur.half * cur.kp, da);
   VIA_LAUNCHED();
-  size_t b_off = 0, c_off = 0;
+  size_t b_off = 0, c_off = mtiles >= CT_MANY ? s.ct_consts.n / 2 : 0;
   for (int k = 0; k < s.ct_steps; ++k) {
-    const CtStep nxt = ct_step(n1, 2 << k);
+    const CtStep nxt = ct_step(n1, 2 << k, mtiles);
     const bool last = k + 1 == s.ct_steps;
     CtParams P{};
     P.st = cur;
@@ -593,7 +560,7 @@ void ct_run(Server& s, const u64* d_query, long nlwe, uint8_t* da, uint8_t* db, 
     k_ct_step<<<std::min(items, s.fd.grid), CT_THREADS, CT_SMEM, st>>>(P);
     VIA_LAUNCHED();
     b_off += (size_t)2 * cur.units * cur.chunks * CT_STAGE_B;
-    c_off += (size_t)cur.items() * 2 * CT_ROWS;
+    c_off += (size_t)2 * cur.units * 2 * CT_ROWS;
     std::swap(da, db);
     cur = nxt;
   }

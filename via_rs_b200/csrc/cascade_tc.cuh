@@ -19,8 +19,7 @@
 #pragma once
 #include <vector>
 
-#include "gadget.cuh"
-#include "ntt_fp.cuh"
+#include "gadget_fp.cuh"
 #include "server.cuh"
 
 namespace via {
@@ -40,12 +39,12 @@ struct CtStep {
   int chunks;     // pipeline stages per unit
   int units;      // mask units; as many body units follow
   int chain;      // body units summed in one accumulator: body items are units / chain
-  size_t b_off;   // byte offset of its units in the key planes
-  size_t c_off;   // its column constants: [item][2][16] doubles
   __host__ __device__ int items() const { return units + units / chain; }
 };
 
-inline CtStep ct_step(int n1, int n) {
+constexpr int CT_MANY = 3;  // LWE tiles from which body chains are long
+
+inline CtStep ct_step(int n1, int n, int mtiles = 1) {
   CtStep s{};
   s.n = n;
   s.half = n1 / n / 2;
@@ -53,10 +52,14 @@ inline CtStep ct_step(int n1, int n) {
   s.G = n < 8 ? 8 / n : 1;
   s.chunks = (s.G * s.kp + CT_KC - 1) / CT_KC;
   s.units = n1 / CT_ROWS;
-  // Body sums run over every output mask, so units of the same coefficients chain in
-  // one accumulator: fewer epilogues and atomics, and with 128 mask units one item per SM
-  // for a single tile. Longer chains of the larger steps would outlast a mask item.
-  s.chain = n >= 128 ? 1 : (128 / n < 8 ? 128 / n : 8);
+  // Body sums run over every output mask, so units of the same coefficients chain in one
+  // accumulator: fewer epilogues and atomics (seven steps of 2688 LWEs 1700 us without
+  // chains, 1300 us with). With one or two tiles of LWEs, 128 mask units fill the GPU once
+  // and a chain must not outlast a mask unit, which shorter chains of larger steps
+  // keep to (18 LWEs, input degrees 16, 32, 64: 18.8, 23.5 and 28.3 us with the long
+  // chains, 16.3, 18 and 25.6 with these).
+  const int most = (mtiles >= CT_MANY ? 128 : n < 32 ? 64 : 32) / n;
+  s.chain = most < 1 ? 1 : (most < 8 ? most : 8);
   return s;
 }
 
@@ -70,6 +73,54 @@ struct CtDigits {
   u32 off;             // o (T - 1) / (B - 1) + 2 T
 };
 
+// The fixed-point fractions f[piece] (32 bits, rounded up by less than 3 ulp) of
+// the three base-T pieces of round(c S / Q) + o (S - 1) / (B - 1) mod S, most
+// significant piece first, for c / Q = y0 / q0 + y1 / q1 mod 1, |y_l| <= 0.5625 q_l.
+__device__ __forceinline__ void ct_pieces(double y0, double y1, const CtDigits& D, u32 (&f)[3]) {
+  int p[3];
+#pragma unroll
+  for (int i = 0; i < 3; ++i) {
+    // T y = qt q + r exactly, |r| <= 0.5625 q (fp_mulmod with its quotient kept);
+    // the quotient's low word is read off the rounding sum.
+    const double h0 = __dmul_rn(D.T, y0), h1 = __dmul_rn(D.T, y1);
+    const double l0 = __fma_rn(D.T, y0, -h0), l1 = __fma_rn(D.T, y1, -h1);
+    const double u0 = __fma_rn(h0, D.qinv[0], FP_ROUND), u1 = __fma_rn(h1, D.qinv[1], FP_ROUND);
+    p[i] = __double2loint(u0) + __double2loint(u1);
+    y0 = __dadd_rn(__fma_rn(-__dadd_rn(u0, -FP_ROUND), D.q[0], h0), l0);
+    y1 = __dadd_rn(__fma_rn(-__dadd_rn(u1, -FP_ROUND), D.q[1], h1), l1);
+  }
+  // Rounding: the remainder y0 / q0 + y1 / q1 to the nearest integer (no ties: Q is odd).
+  const double s = __fma_rn(y0, D.qinv[0], __dmul_rn(y1, D.qinv[1]));
+  const double us = __dadd_rn(s, FP_ROUND);
+  int rnd = __double2loint(us);
+  if (fabs(__dadd_rn(s, -__dadd_rn(us, -FP_ROUND))) > 0.5 - 1e-12) {  // too near to tell in doubles (2^-38)
+    const i128 num = (i128)(i64)y0 * (i128)D.qi[1] + (i128)(i64)y1 * (i128)D.qi[0];
+    const i128 Q = (i128)D.qi[0] * D.qi[1];
+    rnd = 2 * num > Q ? 1 : (2 * num < -Q ? -1 : 0);
+  }
+  // Pieces lie in (-1.2 T, 1.2 T); with off (below 3 T, at least 2 T) they are
+  // nonnegative and below 4.3 T < 2^29, where umulhi(x, M) >> sh = floor(x / T).
+  u32 carry = 2;
+#pragma unroll
+  for (int i = 2; i >= 0; --i) {
+    const u32 x = (u32)p[i] + (i == 2 ? (u32)rnd : 0u) + D.off + carry - 2;
+    carry = __umulhi(x, D.M) >> D.sh;
+    const u32 u = x - carry * D.Ti;
+    const u64 m = (u64)u * D.M;
+    f[i] = (u32)(m >> D.sh) + 1;
+  }
+}
+
+// The next base-B digit of a fraction, most significant first.
+__device__ __forceinline__ u32 ct_digit(u32& f, u32 base) {
+  const u64 m = (u64)f * base;
+  f = (u32)m;
+  return (u32)(m >> 32);
+}
+
+// Signed bytes of four unsigned digits w below 256: w - o.
+__device__ __forceinline__ u32 ct_signed(u32 w, u32 o) { return (w + (128 - o) * 0x01010101u) ^ 0x80808080u; }
+
 // Bytes per LWE of the digit buffers: the largest step's K bytes, and the slack a
 // stage of the last unit may read past it.
 inline size_t ct_digit_bytes(int n1) {
@@ -82,6 +133,10 @@ inline size_t ct_digit_bytes(int n1) {
   return b + CT_KC;
 }
 
+// Whether the digit split above serves this gadget, and its constants.
+bool ct_digits_ok(u64 base, u32 L, const DevRing& R);
+CtDigits ct_digits(u64 base, const DevRing& R);
+// Whether the GEMM steps serve this server's cascade.
 bool ct_supported(const via_params& p, const DevRing& R);
 // Number of leading steps run as GEMMs.
 int ct_steps(const via_params& p);

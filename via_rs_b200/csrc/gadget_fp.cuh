@@ -16,6 +16,14 @@ __device__ __forceinline__ double fp_scaled(double r, double S, double qinv) {
   return __dadd_rn(__fma_rn(__dmul_rn(r, S), qinv, FP_ROUND), -FP_ROUND);
 }
 
+// round((r0 q1 + r1 q0) / Q) for remainders whose quotient lies within 1e-12 of a tie, where
+// doubles cannot tell (probability 2^-38; out of line to keep the callers' code small).
+static __device__ __noinline__ int fp_round_exact(double r0, double r1, u64 q0, u64 q1) {
+  const i128 num = (i128)(i64)r0 * (i128)q1 + (i128)(i64)r1 * (i128)q0;
+  const i128 Q = (i128)q0 * q1;
+  return 2 * num > Q ? 1 : (2 * num < -Q ? -1 : 0);
+}
+
 // Two limbs: c / Q = y0 / q0 + y1 / q1 mod 1 with y_l = c_l (Q / q_l)^-1 mod q_l, and
 // S y_l = p_l q_l + r_l exactly. v = p0 + p1 + round(r0 / q0 + r1 / q1).
 __device__ __forceinline__ double fp_scaled2(double c0, double c1, const Gadget& g, const DevRing& R) {
@@ -28,11 +36,7 @@ __device__ __forceinline__ double fp_scaled2(double c0, double c1, const Gadget&
   const double r0 = __dadd_rn(__fma_rn(-p0, q0, h0), l0), r1 = __dadd_rn(__fma_rn(-p1, q1, h1), l1);
   const double s = __fma_rn(r0, i0, __dmul_rn(r1, i1));
   double rnd = __dadd_rn(__dadd_rn(s, FP_ROUND), -FP_ROUND);
-  if (fabs(__dadd_rn(s, -rnd)) > 0.5 - 1e-12) {  // too near a tie to tell in doubles
-    const i128 num = (i128)(i64)r0 * (i128)R.m[1].q + (i128)(i64)r1 * (i128)R.m[0].q;
-    const i128 Q = (i128)R.m[0].q * R.m[1].q;
-    rnd = 2 * num > Q ? 1.0 : (2 * num < -Q ? -1.0 : 0.0);
-  }
+  if (fabs(__dadd_rn(s, -rnd)) > 0.5 - 1e-12) rnd = (double)fp_round_exact(r0, r1, R.m[0].q, R.m[1].q);
   return __dadd_rn(__dadd_rn(p0, p1), rnd);
 }
 

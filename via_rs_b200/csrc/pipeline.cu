@@ -87,6 +87,39 @@ __global__ void k_decompose_i8(const u64* __restrict__ in, int n_in, long npolys
   });
 }
 
+// The same for the gadgets of ct_digits_ok, by exact steps on doubles (cascade_tc.cuh).
+// Thread = four consecutive coefficients, four digits a store. About 64 FP64 and 100 integer
+// operations a coefficient, where the 128-bit divisions of k_decompose_i8 take about 500: the
+// four late splits of 2688 LWEs 1034 -> 217 us.
+__global__ void __launch_bounds__(128) k_ct_decompose(const u64* __restrict__ in, int n_in, long npolys, CtDigits D,
+                                                      int8_t* __restrict__ out) {
+  const long gid = (long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (gid * 4 >= npolys * n_in) return;
+  const long p = gid * 4 / n_in;
+  const int i = (int)(gid * 4 % n_in);
+  const u64* src = in + p * 2 * n_in + i;
+  u32 f[4][3];
+  {
+    const ulonglong2 a0 = *reinterpret_cast<const ulonglong2*>(src), a1 = *reinterpret_cast<const ulonglong2*>(src + 2);
+    const ulonglong2 b0 = *reinterpret_cast<const ulonglong2*>(src + n_in),
+                     b1 = *reinterpret_cast<const ulonglong2*>(src + n_in + 2);
+    const u64 a[4] = {a0.x, a0.y, a1.x, a1.y}, b[4] = {b0.x, b0.y, b1.x, b1.y};
+#pragma unroll
+    for (int r = 0; r < 4; ++r)
+      ct_pieces(fp_mulmod(fp_from_u64(a[r]), D.yscale[0], D.q[0], D.qinv[0]),
+                fp_mulmod(fp_from_u64(b[r]), D.yscale[1], D.q[1], D.qinv[1]), D, f[r]);
+  }
+  int8_t* o = out + p * (long)CT_L * n_in + i;
+#pragma unroll
+  for (int x = 0; x < 3; ++x)
+#pragma unroll
+    for (int k = 0; k < CT_LP; ++k, o += n_in) {
+      const u32 d = ct_digit(f[0][x], D.base) | ct_digit(f[1][x], D.base) << 8 | ct_digit(f[2][x], D.base) << 16 |
+                    ct_digit(f[3][x], D.base) << 24;
+      *reinterpret_cast<u32*>(o) = ct_signed(d, D.o);
+    }
+}
+
 // Which eval-form key samples output o multiplies: K_o = base + ((o / div) % mod) * stride.
 // stride = 0 means "consecutive keys" (T*2*nl*n residues apart, T = samples per key).
 struct KeySel {
@@ -121,6 +154,68 @@ __global__ void k_mac_ntt(const u64* __restrict__ D, KeySel ks, u64* __restrict_
   const DevMod& m = R.m[l];
   out[(2 * o) * per + rem] = reduce128(am.hi, am.lo, m);
   out[(2 * o + 1) * per + rem] = reduce128(ab.hi, ab.lo, m);
+}
+
+// NS consecutive doubles or words of a thread: one 8- or 16-byte access.
+template <int NS, class V, class T>
+__device__ __forceinline__ void ld_slots(const T* p, T (&x)[NS]) {
+  if constexpr (NS == 2) {
+    const V v = __ldg(reinterpret_cast<const V*>(p));
+    x[0] = v.x;
+    x[1] = v.y;
+  } else {
+    x[0] = __ldg(p);
+  }
+}
+template <int NS>
+__device__ __forceinline__ void st_slots(u64* p, const u64 (&x)[NS]) {
+  if constexpr (NS == 2)
+    *reinterpret_cast<ulonglong2*>(p) = make_ulonglong2(x[0], x[1]);
+  else
+    *p = x[0];
+}
+
+// k_mac_ntt in double precision, for primes below 2^44 (ntt_fp.cuh): digits below 2 q, key
+// residues below q, every product within 0.5625 q. NS slots a thread: two (16-byte accesses)
+// once that leaves two blocks a SM. Bound by the digit and key bytes where each output has
+// its own key: 4099 external products at q1 490 us in 128-bit integers, 303 us here
+// (6.2 TB/s).
+template <int NS>
+__global__ void __launch_bounds__(256) k_mac_fp(const u64* __restrict__ D, KeySel ks, u64* __restrict__ out, int T,
+                                                int n, int nl, long nout, const __grid_constant__ DevRing R) {
+  const long gid = ((long)blockIdx.x * blockDim.x + threadIdx.x) * NS;
+  const long per = (long)nl * n;
+  if (gid >= nout * per) return;
+  const long o = gid / per;
+  const int rem = (int)(gid % per);
+  const int l = rem / n;
+  const double q = R.t[l].qd, qinv = R.t[l].qinv;
+  const u64* Ko = ks.base + ((o / ks.div) % ks.mod) * (ks.stride ? ks.stride : (long)T * 2 * per) + rem;
+  const u64* Do = D + o * (long)T * per + rem;
+  double m[NS], b[NS];
+#pragma unroll
+  for (int i = 0; i < NS; ++i) m[i] = b[i] = 0.0;
+#pragma unroll(NS == 1 ? 9 : 3)
+  for (int s = 0; s < T; ++s) {
+    u64 d[NS], km[NS], kb[NS];
+    ld_slots<NS, ulonglong2>(Do + s * per, d);
+    ld_slots<NS, ulonglong2>(Ko + (2 * s) * per, km);
+    ld_slots<NS, ulonglong2>(Ko + (2 * s + 1) * per, kb);
+#pragma unroll
+    for (int i = 0; i < NS; ++i) {
+      const double x = fp_from_u64(d[i]);
+      m[i] = __dadd_rn(m[i], fp_mulmod(x, fp_from_u64(km[i]), q, qinv));
+      b[i] = __dadd_rn(b[i], fp_mulmod(x, fp_from_u64(kb[i]), q, qinv));
+    }
+  }
+  u64 om[NS], ob[NS];
+#pragma unroll
+  for (int i = 0; i < NS; ++i) {
+    om[i] = fp_to_u64(fp_canonical(m[i], q, qinv));
+    ob[i] = fp_to_u64(fp_canonical(b[i], q, qinv));
+  }
+  st_slots(out + (2 * o) * per + rem, om);
+  st_slots(out + (2 * o + 1) * per + rem, ob);
 }
 
 // Schoolbook (non-NTT ring) variant: negacyclic products, exact.
@@ -228,15 +323,24 @@ __global__ void k_dmux_combine(u64* out, const u64* in, const u64* ext, long cou
 // of 64 queries took 728 us together with eight barriers a transform and 64-bit
 // integer digit splits, 307 us with one barrier and splits on doubles.
 template <int LOGN>
-__global__ void __launch_bounds__((1 << LOGN) / 8, 2) k_dmux_fp(u64* __restrict__ out, const u64* __restrict__ in,
+__global__ void __launch_bounds__((1 << LOGN) / 8, LOGN >= 12 ? 1 : 2) k_dmux_fp(u64* __restrict__ out, const u64* __restrict__ in,
                                                                   KeySel ks, const __grid_constant__ DevRing R,
                                                                   const __grid_constant__ Gadget g) {
   constexpr int n = 1 << LOGN;
   constexpr int L = 2;
   constexpr int nl = 2;
   using L0 = NttPhase<LOGN, false, 0>;
-  __shared__ double ssm[2][n];  // alternate between transforms: one CTA barrier each
+  constexpr int NB = LOGN >= 12 ? 1 : 2;  // exchange areas, as in k_cmux_fp
+  __shared__ double ssm[NB][n];
   int buf = 0;
+  auto area = [&]() -> double* {
+    if constexpr (NB == 1) {
+      __syncthreads();
+      return ssm[0];
+    } else {
+      return ssm[buf ^= 1];
+    }
+  };
   const int tid = threadIdx.x;
   const long o = blockIdx.x;
   const int l = blockIdx.y;
@@ -260,8 +364,7 @@ __global__ void __launch_bounds__((1 << LOGN) / 8, 2) k_dmux_fp(u64* __restrict_
       double e[8];
 #pragma unroll
       for (int v = 0; v < 8; ++v) e[v] = fp_next_digit(val[v], g);
-      fp_forward<LOGN>(e, tid, T, ssm[buf]);
-      buf ^= 1;
+      fp_forward<LOGN>(e, tid, T, area());
       const int smp = h * L + L - 1 - k;
       u64 key[8];
       ld8_nc(K + ((long)(2 * smp) * nl + l) * n + 8 * tid, key);
@@ -279,8 +382,7 @@ __global__ void __launch_bounds__((1 << LOGN) / 8, 2) k_dmux_fp(u64* __restrict_
   for (int part = 0; part < 2; ++part) {  // ext mask, ext body
 #pragma unroll
     for (int v = 0; v < 8; ++v) am[v] = fp_reduce(am[v], q, qinv);
-    fp_inverse<LOGN>(am, tid, T, ssm[buf]);
-    buf ^= 1;
+    fp_inverse<LOGN>(am, tid, T, area());
 #pragma unroll
     for (int v = 0; v < 8; ++v) {
       const long at = (long)(part * nl + l) * n + L0::index(v, tid);
@@ -357,7 +459,7 @@ static bool R_fp_small(const DevRing& R) {
 }
 
 static bool dmux_fp_ok(const DevRing& R, const Gadget& g) {
-  return R.ntt && R.nl == 2 && g.L == 2 && g.fp && ntt_fp_ok(R.t[0], R.t[1]) && R.n == 2048;
+  return R.ntt && R.nl == 2 && g.L == 2 && g.fp && ntt_fp_ok(R.t[0], R.t[1]) && (R.n == 2048 || R.n == 4096);
 }
 
 // Modulus switch (prim/switching/kernels/mod_switch.rs:59-61):
@@ -504,56 +606,104 @@ __global__ void __launch_bounds__(256) k_cascade_mac(const u64* __restrict__ D, 
 // key as exact doubles (below q). Every product is reduced to within 0.5625 q,
 // so a mask's 2 L products stay below 1.125 L q; the body partial is brought
 // back within q/2 after each output mask's 2 L products. Outputs as k_cascade_mac.
-// Two CTAs per SM leave room for nine digits' loads in flight per thread.
 // I8 (the first step, n_in = 1): the digits are read as the signed bytes of
 // k_decompose_i8, [lwe][idx][L], whose transform at degree 1 is the digit itself.
-template <bool I8>
+//
+// A thread takes NS output slots (two: those of one input slot, which share its digits, with
+// 16-byte key loads) for NL LWEs (which share the keys). TP threads along the slots x JJ
+// output masks = 256. FP64-issue and load bound: with NS = NL = 2, 4 + 2 NL loads feed 8 NL
+// products of 7 operations, where one slot and LWE a thread loaded 6 words for 4; a late
+// step of 2688 LWEs 885 -> 644 us.
+template <bool I8, int NL, int NS>
 __global__ void __launch_bounds__(256, 2) k_cascade_mac_fp(const double* __restrict__ D, const int8_t* __restrict__ D8,
                                                         const double* __restrict__ keys, int R, int n_in, int L,
-                                                        int TT, int JB, DevRing Rg, u64* __restrict__ mask_out,
-                                                        u64* __restrict__ bsk, long bsk_stride) {
-  __shared__ u64 part[256];
+                                                        int TP, int JB, long nlwe, const __grid_constant__ DevRing Rg,
+                                                        u64* __restrict__ mask_out, u64* __restrict__ bsk,
+                                                        long bsk_stride) {
+  __shared__ u64 part[NL][NS][256];
   const int nl = Rg.nl, n_out = 2 * n_in, half = R / 2;
-  const int JJ = 256 / TT;
+  const int JJ = 256 / TP;
   const int jb = blockIdx.x % JB;
-  const int tl = threadIdx.x % TT, jl = threadIdx.x / TT;
-  const int t = (blockIdx.x / JB) * TT + tl;
+  const int tl = threadIdx.x % TP, jl = threadIdx.x / TP;
+  const int t = ((blockIdx.x / JB) * TP + tl) * NS;  // first output slot
+  const int u = t >> 1;                              // its input slot
   const int l = blockIdx.y;
-  const long lwe = blockIdx.z;
   const DevMod& m = Rg.m[l];
   const double q = Rg.t[l].qd, qinv = Rg.t[l].qinv;
   const long dper = (long)nl * n_in, kper = (long)nl * n_out;
-  const double* Dw = D + lwe * R * L * dper + (long)l * n_in + (t >> 1);
+  long lwe[NL];  // past the end: the last LWE again, not stored
+#pragma unroll
+  for (int x = 0; x < NL; ++x) lwe[x] = min((long)blockIdx.z * NL + x, nlwe - 1);
   const double* Kl = keys + (long)l * n_out + t;
-  double ab = 0.0;
+  double ab[NL][NS];
+#pragma unroll
+  for (int x = 0; x < NL; ++x)
+#pragma unroll
+    for (int h = 0; h < NS; ++h) ab[x][h] = 0.0;
   for (int j = jl + jb * JJ; j < half; j += JJ * JB) {
-    double am = 0.0;
-    const double* d0 = Dw + (long)j * L * dper;
-    const double* d1 = Dw + (long)(j + half) * L * dper;
-    const double* k0 = Kl + (long)j * L * 2 * kper;
-    const double* k1 = Kl + (long)(j + half) * L * 2 * kper;
-    const int8_t* e0 = D8 + (lwe * R + j) * L;
-    const int8_t* e1 = D8 + (lwe * R + j + half) * L;
-#pragma unroll 9
-    for (int s = 0; s < L; ++s) {
-      const double a = I8 ? (double)e0[s] : d0[s * dper], b = I8 ? (double)e1[s] : d1[s * dper];
-      am = __dadd_rn(am, __dadd_rn(fp_mulmod(a, k0[(2 * s) * kper], q, qinv), fp_mulmod(b, k1[(2 * s) * kper], q, qinv)));
-      ab = __dadd_rn(ab, __dadd_rn(fp_mulmod(a, k0[(2 * s + 1) * kper], q, qinv),
-                                   fp_mulmod(b, k1[(2 * s + 1) * kper], q, qinv)));
+    double am[NL][NS];
+#pragma unroll
+    for (int x = 0; x < NL; ++x)
+#pragma unroll
+      for (int h = 0; h < NS; ++h) am[x][h] = 0.0;
+#pragma unroll 1
+    for (int i = 0; i < 2; ++i) {  // input masks j, j + half
+      const int idx = j + i * half;
+      const double* k = Kl + (long)idx * L * 2 * kper;
+      const double* d[NL];
+      const int8_t* e[NL];
+#pragma unroll
+      for (int x = 0; x < NL; ++x) {
+        d[x] = D + ((lwe[x] * R + idx) * L) * dper + (long)l * n_in + u;
+        e[x] = D8 + (lwe[x] * R + idx) * L;
+      }
+#pragma unroll(NS * NL == 1 ? 9 : 6)
+      for (int s = 0; s < L; ++s) {
+        double km[NS], kb[NS];
+        ld_slots<NS, double2>(k + (2 * s) * kper, km);
+        ld_slots<NS, double2>(k + (2 * s + 1) * kper, kb);
+#pragma unroll
+        for (int x = 0; x < NL; ++x) {
+          const double a = I8 ? (double)e[x][s] : d[x][s * dper];
+#pragma unroll
+          for (int h = 0; h < NS; ++h) {
+            am[x][h] = __dadd_rn(am[x][h], fp_mulmod(a, km[h], q, qinv));
+            ab[x][h] = __dadd_rn(ab[x][h], fp_mulmod(a, kb[h], q, qinv));
+          }
+        }
+      }
     }
-    mask_out[((lwe * half + j) * nl + l) * n_out + t] = negmod(__double2ull_rn(fp_canonical(am, q, qinv)), m.q);
-    ab = __fma_rn(-__dadd_rn(__fma_rn(ab, qinv, FP_ROUND), -FP_ROUND), q, ab);  // back within q/2
+#pragma unroll
+    for (int x = 0; x < NL; ++x) {
+      u64 out[NS];
+#pragma unroll
+      for (int h = 0; h < NS; ++h) {
+        out[h] = negmod(fp_to_u64(fp_canonical(am[x][h], q, qinv)), m.q);
+        ab[x][h] = fp_reduce(ab[x][h], q, qinv);
+      }
+      if ((long)blockIdx.z * NL + x < nlwe) st_slots(mask_out + ((lwe[x] * half + j) * nl + l) * n_out + t, out);
+    }
   }
-  part[threadIdx.x] = __double2ull_rn(fp_canonical(ab, q, qinv));
+#pragma unroll
+  for (int x = 0; x < NL; ++x)
+#pragma unroll
+    for (int h = 0; h < NS; ++h) part[x][h][threadIdx.x] = fp_to_u64(fp_canonical(ab[x][h], q, qinv));
   __syncthreads();
   if (jl == 0) {
-    u64 acc = part[tl];
-    for (int x = 1; x < JJ; ++x) acc = addmod(acc, part[x * TT + tl], m.q);
-    if (JB == 1)
-      bsk[(lwe * nl + l) * bsk_stride + t] = acc;
-    else
-      atomicAdd(reinterpret_cast<unsigned long long*>(bsk + (lwe * nl + l) * bsk_stride + t),
-                (unsigned long long)acc);
+#pragma unroll
+    for (int x = 0; x < NL; ++x) {
+      if ((long)blockIdx.z * NL + x >= nlwe) continue;
+#pragma unroll
+      for (int h = 0; h < NS; ++h) {
+        u64 acc = part[x][h][tl];
+        for (int y = 1; y < JJ; ++y) acc = addmod(acc, part[x][h][y * TP + tl], m.q);
+        u64* o = bsk + (lwe[x] * nl + l) * bsk_stride + t + h;
+        if (JB == 1)
+          *o = acc;
+        else
+          atomicAdd(reinterpret_cast<unsigned long long*>(o), (unsigned long long)acc);
+      }
+    }
   }
 }
 
@@ -761,6 +911,8 @@ static bool cmux_fused_ok(const DevRing& R, const Gadget& g);
 
 // Levels of at most this many CMuxes run on four-CTA clusters (cmux_fused).
 constexpr long CMUX_CLUSTER_MAX = 64;
+// DMux levels of at most this many products run on a cluster per product and limb.
+constexpr long EXT_CLUSTER_MAX = 16;
 
 // Whether the scan of nq queries writes tiled columns, which the CMux tree's first level
 // gathers: answers with the fused CMux and a first level of single-CTA CMuxes.
@@ -887,7 +1039,16 @@ static void from_eval(const DevRing& R, u64* data, int n, long segments, cudaStr
 // domain) against keys: out eval [nout][2][nl][n].
 static void mac(const DevRing& R, const u64* D, KeySel ks, u64* out, int T, int n, long nout, cudaStream_t st) {
   long items = nout * R.nl * n;
-  if (R.ntt)
+  // Two slots a thread where the buffers allow it (a primitive's caller may pass any 8-byte
+  // address) and the grid stays wide: the 16 LWEs of one query's DMux bits took 8.2 us with one
+  // slot a thread, 9.6 us with two.
+  const bool wide = items / 512 >= 2 * 148 && (((uintptr_t)out | (uintptr_t)D | (uintptr_t)ks.base) & 15) == 0;
+  const bool fp = R.ntt && ntt_fp_ok(R.t[0], R.t[R.nl - 1]) && T <= 128;
+  if (fp && wide)
+    k_mac_fp<2><<<blocks(items / 2), 256, 0, st>>>(D, ks, out, T, n, R.nl, nout, R);
+  else if (fp)
+    k_mac_fp<1><<<blocks(items), 256, 0, st>>>(D, ks, out, T, n, R.nl, nout, R);
+  else if (R.ntt)
     k_mac_ntt<<<blocks(items), 256, 0, st>>>(D, ks, out, T, n, R.nl, nout, R);
   else
     k_mac_schoolbook<<<blocks(items), 256, 0, st>>>(D, ks, out, T, n, R.nl, nout, R);
@@ -897,6 +1058,16 @@ static void mac(const DevRing& R, const u64* D, KeySel ks, u64* out, int T, int 
 static void decompose(const DevRing& R, const Gadget& g, const u64* in, int n_in, int stride, long npolys, u64* out,
                       cudaStream_t st) {
   k_decompose<<<blocks(npolys * n_in, 128), 128, 0, st>>>(in, n_in, stride, npolys, R, g, out);
+  VIA_LAUNCHED();
+}
+
+// Signed byte digits (bases up to 255); `in` is a 16-byte aligned buffer of canonical residues.
+static void decompose_i8(const DevRing& R, const Gadget& g, const u64* in, int n_in, long npolys, int8_t* out,
+                         cudaStream_t st) {
+  if (n_in >= 4 && ct_digits_ok(g.base, (u32)g.L, R))
+    k_ct_decompose<<<blocks(npolys * n_in / 4, 128), 128, 0, st>>>(in, n_in, npolys, ct_digits(g.base, R), out);
+  else
+    k_decompose_i8<<<blocks(npolys * n_in, 128), 128, 0, st>>>(in, n_in, npolys, R, g, out);
   VIA_LAUNCHED();
 }
 
@@ -968,8 +1139,7 @@ static void query_decomp_range(Server& s, Workspace& w, const u64* d_query, long
       const bool fp_mac = dig8 && s.cascade_eval_d.p;
       if (dig8 && (n_in > 1 || fp_mac)) {
         if (k != k0 || k0 == 0) {  // the last GEMM step left its successor's digits in dig8
-          k_decompose_i8<<<blocks(polys * n_in, 128), 128, 0, st>>>(mi, n_in, polys, R, w.g_ck, dig8);
-          VIA_LAUNCHED();
+          decompose_i8(R, w.g_ck, mi, n_in, polys, dig8, st);
         }
         if (n_in == 1)
           ;  // degree 1: the MAC reads the digits themselves
@@ -981,21 +1151,34 @@ static void query_decomp_range(Server& s, Workspace& w, const u64* d_query, long
         decompose(R, w.g_ck, mi, n_in, 1, polys, digits, st);
         if (n_in > 1) digits_to_eval(R, digits, n_in, polys * L * nl, st);
       }
-      int jj = std::min(rank_in / 2, 8), tt = std::min(n_out, 256 / jj);
+      // fp: two output slots a thread from three blocks a SM on (with one: 60 LWEs 26 us a
+      // step against 21, 18 LWEs 8.3 against 10.2), two LWEs as well from sixteen on.
+      const long full = (long)n1 * nl * nlwe / 256;  // blocks with one slot and LWE a thread
+      const int NS = fp_mac && n_in > 1 && full >= 3 * 148 ? 2 : 1, NL = NS == 2 && full >= 16 * 148 ? 2 : 1;
+      const int jj = std::min(rank_in / 2, 8), tt = std::min(n_out / NS, 256 / jj);
+      const long slots = n_out / NS / tt;
       // Split the output masks over JB blocks while the grid is below ~4 blocks
       // per SM and every block keeps at least one mask per thread row.
-      const long base = (long)(n_out / tt) * nl * nlwe;
-      const int iters = (rank_in / 2 + 256 / tt - 1) / (256 / tt);
+      const long lwes = (nlwe + NL - 1) / NL, base = slots * nl * lwes;
+      const int rows = 256 / tt, iters = (rank_in / 2 + rows - 1) / rows;
       int JB = 1;
       while (JB * 2 <= iters && base * JB * 2 <= CASCADE_SPLIT_BLOCKS) JB *= 2;
-      dim3 grid((unsigned)(n_out / tt * JB), (unsigned)nl, (unsigned)nlwe);
+      dim3 grid((unsigned)(slots * JB), (unsigned)nl, (unsigned)lwes);
       u64* bsk_k = bsk + (n_out - 2);  // this step's region
       const double* kd = reinterpret_cast<const double*>(s.cascade_eval_d.p) + k * step_len;
+      const double* dd = reinterpret_cast<const double*>(digits);
       if (fp_mac && n_in == 1)
-        k_cascade_mac_fp<true><<<grid, 256, 0, st>>>(nullptr, dig8, kd, rank_in, n_in, L, tt, JB, R, mo, bsk_k, 2L * n1);
+        k_cascade_mac_fp<true, 1, 1><<<grid, 256, 0, st>>>(nullptr, dig8, kd, rank_in, n_in, L, tt, JB, nlwe, R, mo, bsk_k,
+                                                        2L * n1);
+      else if (NL == 2)
+        k_cascade_mac_fp<false, 2, 2><<<grid, 256, 0, st>>>(dd, dig8, kd, rank_in, n_in, L, tt, JB, nlwe, R, mo, bsk_k,
+                                                         2L * n1);
+      else if (NS == 2)
+        k_cascade_mac_fp<false, 1, 2><<<grid, 256, 0, st>>>(dd, dig8, kd, rank_in, n_in, L, tt, JB, nlwe, R, mo, bsk_k,
+                                                            2L * n1);
       else if (fp_mac)
-        k_cascade_mac_fp<false><<<grid, 256, 0, st>>>(reinterpret_cast<const double*>(digits), dig8, kd, rank_in, n_in,
-                                                      L, tt, JB, R, mo, bsk_k, 2L * n1);
+        k_cascade_mac_fp<false, 1, 1><<<grid, 256, 0, st>>>(dd, dig8, kd, rank_in, n_in, L, tt, JB, nlwe, R, mo, bsk_k,
+                                                         2L * n1);
       else
         k_cascade_mac<<<grid, 256, 0, st>>>(digits, s.cascade_eval.p + k * step_len, rank_in, n_in, L, tt, JB, R, mo,
                                             bsk_k, 2L * n1);
@@ -1031,8 +1214,7 @@ static void query_decomp_range(Server& s, Workspace& w, const u64* d_query, long
   u64* gp = w.g_gp.p + lwe0 * 2 * lwe_n;
   u64* gdig = w.g_digits.p + lwe0 * L * lwe_n;
   if (dig8) {
-    k_decompose_i8<<<blocks(nlwe * n1, 128), 128, 0, st>>>(mi, n1, nlwe, R, w.g_ck, dig8);
-    VIA_LAUNCHED();
+    decompose_i8(R, w.g_ck, mi, n1, nlwe, dig8, st);
     ntt_forward_i8_lazy(dig8, gdig, n1, nl, nlwe * L * nl, R.t[0], R.t[1], st);
     mac(R, gdig, keys_shared(s.conv_eval.p), gp, L, n1, nlwe, st);
   } else {
@@ -1254,6 +1436,119 @@ __global__ void __cluster_dims__(4, 1, 1) __launch_bounds__((1 << LOGN) / 8, 2)
   cluster.sync();
 }
 
+// One external product per four-CTA cluster and limb (rgsw.rs:108-121), coefficient form in
+// and out, in double precision: levels and steps with too few products to fill the GPU,
+// where one product's latency sets the time. CTA r takes input half p = r & 1 and digit
+// k = r >> 1: one digit split, one forward transform, and its products with the sample's
+// mask and body (sample p L + L - 1 - k, L = 2) in shared memory. After a cluster barrier
+// ranks 0 and 1 sum the four partial masks / bodies over distributed shared memory and
+// transform them back.
+//   EXT_DMUX: out[2o] = in[o] - ext, out[2o+1] = ext            (a DMux level; mux.rs:129-137)
+//   EXT_CROT: d = rot - in, rot = -X^shift in; out = in + bit (x) d, in place (a CRot step;
+//             rotate.rs:128-150)
+// in [ct][2][nl][n], RGSWs [2L][2][nl][n] eval. Latency-bound: a digit split, two transforms and
+// two cluster barriers, where decompose, transform, multiply-accumulate and inverse kernels
+// took about 24 us a DMux level and 32 us a CRot step (live, ring of 2048), 16 and 12 us here.
+enum { EXT_DMUX = 0, EXT_CROT = 1 };
+template <int LOGN, int MODE>
+__global__ void __cluster_dims__(4, 1, 1) __launch_bounds__((1 << LOGN) / 8)
+    k_ext_cluster_fp(const u64* in, u64* out, KeySel ks, int shift, const __grid_constant__ DevRing R,
+                     const __grid_constant__ Gadget g) {
+  namespace cg = cooperative_groups;
+  constexpr int n = 1 << LOGN;
+  using L0 = NttPhase<LOGN, false, 0>;
+  extern __shared__ __align__(16) double ext_sm[];
+  double* pmask = ext_sm;      // the forward's exchanges, then the mask partial
+  double* pbody = ext_sm + n;  // the body partial
+  cg::cluster_group cluster = cg::this_cluster();
+  const int r = (int)cluster.block_rank();
+  const int p = r & 1, k = r >> 1;
+  const int tid = threadIdx.x, nl = R.nl, l = blockIdx.y;
+  const long o = blockIdx.x / 4;
+  const NttTable& T = R.t[l];
+  const double q = T.qd, qinv = T.qinv;
+  const u64* ct = in + o * 2 * nl * n;
+  const u64* K = ks.base + ((o / ks.div) % ks.mod) * ks.stride;
+  double e[8];
+#pragma unroll
+  for (int v = 0; v < 8; ++v) {
+    const int x = L0::index(v, tid);
+    const u64* c = ct + (long)p * nl * n + x;
+    double val;
+    if (MODE == EXT_DMUX) {
+      val = nl == 2 ? fp_scaled2(fp_from_u64(c[0]), fp_from_u64(c[n]), g, R)
+                    : fp_scaled(fp_reduce(fp_from_u64(c[0]), q, qinv), g.dS, qinv);
+    } else {
+      // rot[x] = -in[x - shift], or in[x - shift + n] where the index wraps.
+      const int src = x - shift;
+      const double s = fp_from_u64(c[src < 0 ? src + n - x : -shift]);
+      val = fp_scaled(fp_reduce(__dadd_rn(src < 0 ? s : -s, -fp_from_u64(c[0])), q, qinv), g.dS, qinv);
+    }
+    e[v] = fp_next_digit(val, g);
+    if (k) e[v] = fp_next_digit(val, g);
+  }
+  fp_forward<LOGN>(e, tid, T, pmask);
+  const int smp = p * 2 + 1 - k;
+  u64 km[8], kb[8];
+  ld8_nc(K + ((long)(2 * smp) * nl + l) * n + 8 * tid, km);
+  ld8_nc(K + ((long)(2 * smp + 1) * nl + l) * n + 8 * tid, kb);
+  __syncwarp();  // the warp's exchanges; its part of pmask is read by no other warp
+#pragma unroll
+  for (int v = 0; v < 8; ++v) {
+    pmask[8 * tid + v] = fp_mulmod(e[v], fp_from_u64(km[v]), q, qinv);
+    pbody[8 * tid + v] = fp_mulmod(e[v], fp_from_u64(kb[v]), q, qinv);
+  }
+  cluster.sync();
+  if (r < 2) {
+    double* mine = r ? pbody : pmask;
+#pragma unroll
+    for (int v = 0; v < 8; ++v) e[v] = mine[8 * tid + v];
+#pragma unroll
+    for (int y = 1; y < 4; ++y) {
+      const double* peer = cluster.map_shared_rank(mine, (r + y) & 3);
+#pragma unroll
+      for (int v = 0; v < 8; ++v) e[v] = __dadd_rn(e[v], peer[8 * tid + v]);
+    }
+#pragma unroll
+    for (int v = 0; v < 8; ++v) e[v] = fp_reduce(e[v], q, qinv);
+  }
+  cluster.sync();  // every CTA's partials have been read
+  if (r >= 2) return;
+  fp_inverse<LOGN>(e, tid, T, pmask);
+  const u64 qi = R.m[l].q;
+#pragma unroll
+  for (int v = 0; v < 8; ++v) {
+    const long at = (long)(r * nl + l) * n + L0::index(v, tid);
+    const u64 ext = fp_to_u64(fp_canonical(fp_mulmod(e[v], T.ninv_d[LOGN], q, qinv), q, qinv));
+    if (MODE == EXT_DMUX) {
+      out[(2 * o) * 2 * nl * n + at] = submod(ct[at], ext, qi);
+      out[(2 * o + 1) * 2 * nl * n + at] = ext;
+    } else {
+      out[o * 2 * nl * n + at] = addmod(ct[at], ext, qi);
+    }
+  }
+}
+
+// Rings and gadgets k_ext_cluster_fp serves. Raises its shared-memory limit (n = 4096: 64 KB) on the
+// current device.
+static bool ext_cluster_ok(const DevRing& R, const Gadget& g) {
+  return R.ntt && g.L == 2 && g.fp && ntt_fp_ok(R.t[0], R.t[R.nl - 1]) && (R.n == 2048 || R.n == 4096);
+}
+
+template <int MODE>
+static void ext_cluster(const DevRing& R, const Gadget& g, const u64* in, u64* out, KeySel ks, int shift, long count,
+                        cudaStream_t st) {
+  const dim3 grid((unsigned)(4 * count), (unsigned)R.nl);
+  const int smem = 2 * R.n * 8;
+  if (R.n == 4096) {
+    VIA_CUDA(cudaFuncSetAttribute(k_ext_cluster_fp<12, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    k_ext_cluster_fp<12, MODE><<<grid, 512, smem, st>>>(in, out, ks, shift, R, g);
+  } else {
+    k_ext_cluster_fp<11, MODE><<<grid, 256, smem, st>>>(in, out, ks, shift, R, g);
+  }
+  VIA_LAUNCHED();
+}
+
 // CMux level o < count: fused kernel when the ring has one NTT limb of a
 // supported degree and a small gadget, else diff -> external product -> add.
 static bool cmux_fused_ok(const DevRing& R, const Gadget& g) {
@@ -1442,11 +1737,18 @@ void answer_device_stages(Server& s, Workspace& w, const u64* d_query, int nq, u
     for (int i = 0; i < nd; ++i) {
       const long active = 1L << i;  // per query
       KeySel bit{w.rgsw_q1.p + i * rgsw1, active, B, nd * rgsw1};
-      // The fused level kernel is latency-bound at about 70 us for up to a wave of
-      // products (148 SMs x 2 CTAs, two per product); smaller levels keep the
-      // separate, wider kernels (about 40 us a level).
-      if (dmux_fp_ok(s.r1, w.g_dmux) && B * active >= 256) {
-        k_dmux_fp<11><<<dim3((unsigned)(B * active), 2), 256, 0, st>>>(out, in, bit, s.r1, w.g_dmux);
+      // One cluster per product and limb up to EXT_CLUSTER_MAX products, one CTA above.
+      if (B * active <= EXT_CLUSTER_MAX && ext_cluster_ok(s.r1, w.g_dmux)) {
+        ext_cluster<EXT_DMUX>(s.r1, w.g_dmux, in, out, bit, 0, B * active, st);
+        std::swap(in, out);
+        continue;
+      }
+      if (dmux_fp_ok(s.r1, w.g_dmux)) {
+        const dim3 grid((unsigned)(B * active), 2);
+        if (n1 == 4096)
+          k_dmux_fp<12><<<grid, 512, 0, st>>>(out, in, bit, s.r1, w.g_dmux);
+        else
+          k_dmux_fp<11><<<grid, 256, 0, st>>>(out, in, bit, s.r1, w.g_dmux);
         VIA_LAUNCHED();
         std::swap(in, out);
         continue;
@@ -1511,9 +1813,13 @@ void answer_device_stages(Server& s, Workspace& w, const u64* d_query, int nq, u
 
   // ---- Step 6: CRot, SlotExtract (rotate.rs:128-150).
   for (int i = 0; i < nr; ++i) {
+    KeySel bit{rgsw_b2 + (nc + i) * rgsw2, 1, B, nb * rgsw2};
+    if (ext_cluster_ok(s.r2, w.g_cmux) && w.g_cmux.small) {
+      ext_cluster<EXT_CROT>(s.r2, w.g_cmux, w.cr_ct.p, w.cr_ct.p, bit, n1 - (1 << i), B, st);
+      continue;
+    }
     k_crot_diff_batch<<<blocks(B * 2 * n1), 256, 0, st>>>(w.cr_ct.p, n1, n1 - (1 << i), B, s.r2.m[0], w.cr_diff.p);
     VIA_LAUNCHED();
-    KeySel bit{rgsw_b2 + (nc + i) * rgsw2, 1, B, nb * rgsw2};
     if (R_fp_small(s.r2)) {
       external_products(s.r2, w.g_cmux, bit, w.cr_diff.p, B, w.cr_digits.p, w.cr_ext.p, false, st);
       intt_epi<INTT_ADD>(s.r2, w.cr_ext.p, w.cr_ct.p, w.cr_ct.p, B, st);
@@ -1867,7 +2173,16 @@ void prim_key_switches(const DevRing& R, const Gadget& g, const u64* key, const 
   to_eval(R, key_eval, n, (long)g.L * 2 * R.nl, st);
   k_rotate_split<<<blocks(count * 2 * per), 256, 0, st>>>(cts, shifts, count, n, R.nl, R, masks, bodies);
   VIA_LAUNCHED();
-  gadget_product(R, g, masks, n, 1, 1, count, keys_shared(key_eval), prod, digits, st);
+  if (n >= 4 && ct_digits_ok(g.base, (u32)g.L, R)) {
+    // Digits as bytes (in the product's memory, which the products then overwrite).
+    int8_t* dig8 = reinterpret_cast<int8_t*>(prod);
+    static_assert(CT_L <= 2 * 2 * 8, "18 bytes of digits fit the product's 32 bytes a coefficient");
+    decompose_i8(R, g, masks, n, count, dig8, st);
+    ntt_forward_i8_lazy(dig8, digits, n, R.nl, count * g.L * R.nl, R.t[0], R.t[1], st);
+    mac(R, digits, keys_shared(key_eval), prod, g.L, n, count, st);
+  } else {
+    gadget_product(R, g, masks, n, 1, 1, count, keys_shared(key_eval), prod, digits, st);
+  }
   from_eval(R, prod, n, count * 2 * R.nl, st);
   k_key_switch_finish<<<blocks(count * per), 256, 0, st>>>(prod, bodies, count, n, R.nl, R, out);
   VIA_LAUNCHED();
