@@ -235,6 +235,18 @@ __global__ void __launch_bounds__(CT_THREADS, 1) k_ct_step(const __grid_constant
       int len;
       const int unit = ct_item(S, it / P.mtiles, len);
       const long w = (long)mt * CT_M + m;
+      double cr[2][4];  // the column constants, on their way while the accumulator fills
+      {
+        const double* cc = P.c + (size_t)(it / P.mtiles) * 2 * CT_ROWS + part * 4;
+#pragma unroll
+        for (int l = 0; l < 2; ++l)
+#pragma unroll
+          for (int r = 0; r < 4; r += 2) {
+            const double2 x = __ldg(reinterpret_cast<const double2*>(cc + l * CT_ROWS + r));
+            cr[l][r] = x.x;
+            cr[l][r + 1] = x.y;
+          }
+      }
       if (!__all_sync(0xffffffffu, mbar_wait(acc_full + a, aph, abort_flag))) {
         ok = false;
         break;
@@ -267,12 +279,11 @@ __global__ void __launch_bounds__(CT_THREADS, 1) k_ct_step(const __grid_constant
 #pragma unroll
       for (int l = 0; l < 2; ++l) {
         const double q = P.D.q[l], qinv = P.D.qinv[l];
-        const double* cc = P.c + ((size_t)(it / P.mtiles) * 2 + l) * CT_ROWS + part * 4;
 #pragma unroll
         for (int r = 0; r < 4; ++r) {
           const u64 lo = (u64)v[l][0][r] + ((u64)v[l][1][r] << 8) + ((u64)v[l][2][r] << 16);
           const u64 hi = (u64)v[l][3][r] + ((u64)v[l][4][r] << 8);
-          const double x = __dadd_rn(__dadd_rn(fp_from_u64(lo), fp_mulmod(fp_from_u64(hi), P.D.c24[l], q, qinv)), -__ldg(cc + r));
+          const double x = __dadd_rn(__dadd_rn(fp_from_u64(lo), fp_mulmod(fp_from_u64(hi), P.D.c24[l], q, qinv)), -cr[l][r]);
           y[l][r] = __fma_rn(-__dadd_rn(__fma_rn(x, qinv, FP_ROUND), -FP_ROUND), q, x);
         }
       }

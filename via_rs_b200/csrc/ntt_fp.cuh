@@ -107,7 +107,9 @@ struct FpPhase {
     }
   }
 
-  __device__ __forceinline__ static void forward(double (&e)[8], int tid, const NttTable& T) {
+  // W polynomials at once: one load of each twiddle, W independent butterflies of it.
+  template <int W>
+  __device__ __forceinline__ static void forward(double (&e)[W][8], int tid, const NttTable& T) {
     const double q = T.qd, qinv = T.qinv;
 #pragma unroll
     for (int sub = 0; sub < NSUB; ++sub) {
@@ -120,17 +122,21 @@ struct FpPhase {
 #pragma unroll
         for (int k = 0; k < (1 << R); ++k) {
           if (k & hk) continue;
-          double& a = e[sub * (1 << R) + k];
-          double& c = e[sub * (1 << R) + k + hk];
-          const double t = fp_mulmod(c, w[k >> (R - lvl)], q, qinv), av = a;
-          a = __dadd_rn(av, t);
-          c = __dadd_rn(av, -t);
+#pragma unroll
+          for (int x = 0; x < W; ++x) {
+            double& a = e[x][sub * (1 << R) + k];
+            double& c = e[x][sub * (1 << R) + k + hk];
+            const double t = fp_mulmod(c, w[k >> (R - lvl)], q, qinv), av = a;
+            a = __dadd_rn(av, t);
+            c = __dadd_rn(av, -t);
+          }
         }
       }
     }
   }
 
-  __device__ __forceinline__ static void inverse(double (&e)[8], int tid, const NttTable& T) {
+  template <int W>
+  __device__ __forceinline__ static void inverse(double (&e)[W][8], int tid, const NttTable& T) {
     const double q = T.qd, qinv = T.qinv;
 #pragma unroll
     for (int sub = 0; sub < NSUB; ++sub) {
@@ -143,11 +149,14 @@ struct FpPhase {
 #pragma unroll
         for (int k = 0; k < (1 << R); ++k) {
           if (k & hk) continue;
-          double& a = e[sub * (1 << R) + k];
-          double& c = e[sub * (1 << R) + k + hk];
-          const double av = a, cv = c;
-          a = __dadd_rn(av, cv);
-          c = fp_mulmod(__dadd_rn(av, -cv), w[k >> (R - lvl)], q, qinv);
+#pragma unroll
+          for (int x = 0; x < W; ++x) {
+            double& a = e[x][sub * (1 << R) + k];
+            double& c = e[x][sub * (1 << R) + k + hk];
+            const double av = a, cv = c;
+            a = __dadd_rn(av, cv);
+            c = fp_mulmod(__dadd_rn(av, -cv), w[k >> (R - lvl)], q, qinv);
+          }
         }
       }
     }
@@ -182,70 +191,107 @@ __device__ __forceinline__ void fp_sync() {
     __syncthreads();
 }
 
-// Forward transform of a segment held in the phase-0 layout (tid + k n / 8); leaves it as
+// Forward transform of W segments held in the phase-0 layout (tid + k n / 8); leaves each as
 // eight consecutive elements a thread, signed residues below |input| + 0.5625 LOGN q.
-// Phases before P have run. `ssm`: the exchange area (addressed through swz from `sbase`).
-// On entry no other warp may still read it.
-template <int LOGN, int P = 0>
-__device__ __forceinline__ void fp_forward(double (&e)[8], int tid, const NttTable& T, double* ssm, int sbase = 0) {
-  constexpr int NPH = (LOGN + 2) / 3;
+// Phases before P have run. `ssm`: W exchange areas of n elements each (addressed through
+// swz from `sbase`; W = 1 where several segments share a CTA). On entry no other warp may
+// still read them. A transform is a chain of about 90 dependent FP64 operations and a few
+// exchanges, 4 to 5 us however many run beside it: two at once (W = 2) take little longer
+// than one.
+template <int LOGN, int P = 0, int W = 1>
+__device__ __forceinline__ void fp_forward_w(double (&e)[W][8], int tid, const NttTable& T, double* ssm, int sbase = 0) {
+  constexpr int NPH = (LOGN + 2) / 3, n = 1 << LOGN;
   if constexpr (P > 0) {
     using Pv = FpPhase<LOGN, P - 1>;
     using Ph = FpPhase<LOGN, P>;
     if constexpr (P > 1) fp_sync<Pv::SPAN>();  // the previous exchange's reads
 #pragma unroll
-    for (int v = 0; v < 8; ++v) ssm[swz(sbase + Pv::Ix::index(v, tid))] = e[v];
+    for (int x = 0; x < W; ++x)
+#pragma unroll
+      for (int v = 0; v < 8; ++v) ssm[x * n + swz(sbase + Pv::Ix::index(v, tid))] = e[x][v];
     fp_sync<Pv::SPAN>();
 #pragma unroll
-    for (int v = 0; v < 8; ++v) e[v] = ssm[swz(sbase + Ph::Ix::index(v, tid))];
+    for (int x = 0; x < W; ++x)
+#pragma unroll
+      for (int v = 0; v < 8; ++v) e[x][v] = ssm[x * n + swz(sbase + Ph::Ix::index(v, tid))];
   }
-  FpPhase<LOGN, P>::forward(e, tid, T);
-  if constexpr (P + 1 < NPH) fp_forward<LOGN, P + 1>(e, tid, T, ssm, sbase);
-}
-
-// The phases after the first.
-template <int LOGN>
-__device__ __forceinline__ void fp_forward_rest(double (&e)[8], int tid, const NttTable& T, double* ssm, int sbase) {
-  fp_forward<LOGN, 1>(e, tid, T, ssm, sbase);
+  FpPhase<LOGN, P>::template forward<W>(e, tid, T);
+  if constexpr (P + 1 < NPH) fp_forward_w<LOGN, P + 1, W>(e, tid, T, ssm, sbase);
 }
 
 // The same from digits, with the dense first phase where the caller finds its sums below
 // 2^48 (uniform in the CTA).
-template <int LOGN>
-__device__ __forceinline__ void fp_forward_digits(double (&e)[8], int tid, const NttTable& T, double* ssm, int sbase,
-                                                  bool dense) {
-  if (dense)
-    fp_digit_phase(e, T);
-  else
-    FpPhase<LOGN, 0>::forward(e, tid, T);
-  if constexpr (LOGN > 3) fp_forward_rest<LOGN>(e, tid, T, ssm, sbase);
+template <int LOGN, int W>
+__device__ __forceinline__ void fp_forward_digits_w(double (&e)[W][8], int tid, const NttTable& T, double* ssm, int sbase,
+                                                    bool dense) {
+  if (dense) {
+#pragma unroll
+    for (int x = 0; x < W; ++x) fp_digit_phase(e[x], T);
+  } else {
+    FpPhase<LOGN, 0>::template forward<W>(e, tid, T);
+  }
+  if constexpr (LOGN > 3) fp_forward_w<LOGN, 1, W>(e, tid, T, ssm, sbase);
 }
 
-// Inverse transform, without the n^-1 scaling, of a segment held as eight consecutive
+// Inverse transforms, without the n^-1 scaling, of W segments held as eight consecutive
 // elements a thread, inputs below 4 q in magnitude; leaves signed values in the phase-0
 // layout: below 2^12 q for q <= 2^35 (inputs below q), else below 2^6 q, 2^48 in any case.
 // Primes above 2^35 return to q / 2 after the second phase (six stages at most between
 // reductions: 2 * 4 q * 2^5 < 2^48 for q < 2^40), above 2^40 after every phase. On
-// entry no other warp may still read the exchange area.
-template <int LOGN, int P = (LOGN + 2) / 3 - 1>
-__device__ __forceinline__ void fp_inverse(double (&e)[8], int tid, const NttTable& T, double* ssm, int sbase = 0) {
-  constexpr int LAST = (LOGN + 2) / 3 - 1;
-  FpPhase<LOGN, P>::inverse(e, tid, T);
+// entry no other warp may still read the exchange areas.
+template <int LOGN, int P, int W>
+__device__ __forceinline__ void fp_inverse_w(double (&e)[W][8], int tid, const NttTable& T, double* ssm, int sbase = 0) {
+  constexpr int LAST = (LOGN + 2) / 3 - 1, n = 1 << LOGN;
+  FpPhase<LOGN, P>::template inverse<W>(e, tid, T);
   if constexpr (P > 0) {
     using Ph = FpPhase<LOGN, P>;
     using Nx = FpPhase<LOGN, P - 1>;
     if (T.qd > 34359738368.0 && (P == LAST - 1 || T.qd > 1099511627776.0)) {
 #pragma unroll
-      for (int v = 0; v < 8; ++v) e[v] = fp_reduce(e[v], T.qd, T.qinv);
+      for (int x = 0; x < W; ++x)
+#pragma unroll
+        for (int v = 0; v < 8; ++v) e[x][v] = fp_reduce(e[x][v], T.qd, T.qinv);
     }
     if constexpr (P < LAST) fp_sync<Ph::SPAN>();  // the previous exchange's reads
 #pragma unroll
-    for (int v = 0; v < 8; ++v) ssm[swz(sbase + Ph::Ix::index(v, tid))] = e[v];
+    for (int x = 0; x < W; ++x)
+#pragma unroll
+      for (int v = 0; v < 8; ++v) ssm[x * n + swz(sbase + Ph::Ix::index(v, tid))] = e[x][v];
     fp_sync<Nx::SPAN>();
 #pragma unroll
-    for (int v = 0; v < 8; ++v) e[v] = ssm[swz(sbase + Nx::Ix::index(v, tid))];
-    fp_inverse<LOGN, P - 1>(e, tid, T, ssm, sbase);
+    for (int x = 0; x < W; ++x)
+#pragma unroll
+      for (int v = 0; v < 8; ++v) e[x][v] = ssm[x * n + swz(sbase + Nx::Ix::index(v, tid))];
+    fp_inverse_w<LOGN, P - 1, W>(e, tid, T, ssm, sbase);
   }
+}
+
+// One segment.
+template <int LOGN>
+__device__ __forceinline__ void fp_forward(double (&e)[8], int tid, const NttTable& T, double* ssm, int sbase = 0) {
+  fp_forward_w<LOGN, 0, 1>(reinterpret_cast<double(&)[1][8]>(e), tid, T, ssm, sbase);
+}
+template <int LOGN>
+__device__ __forceinline__ void fp_forward_digits(double (&e)[8], int tid, const NttTable& T, double* ssm, int sbase,
+                                                  bool dense) {
+  fp_forward_digits_w<LOGN, 1>(reinterpret_cast<double(&)[1][8]>(e), tid, T, ssm, sbase, dense);
+}
+template <int LOGN>
+__device__ __forceinline__ void fp_inverse(double (&e)[8], int tid, const NttTable& T, double* ssm, int sbase = 0) {
+  fp_inverse_w<LOGN, (LOGN + 2) / 3 - 1, 1>(reinterpret_cast<double(&)[1][8]>(e), tid, T, ssm, sbase);
+}
+// Two at once; `ssm` holds 2 n elements.
+template <int LOGN>
+__device__ __forceinline__ void fp_forward2(double (&e)[2][8], int tid, const NttTable& T, double* ssm) {
+  fp_forward_w<LOGN, 0, 2>(e, tid, T, ssm);
+}
+template <int LOGN>
+__device__ __forceinline__ void fp_forward_digits2(double (&e)[2][8], int tid, const NttTable& T, double* ssm, bool dense) {
+  fp_forward_digits_w<LOGN, 2>(e, tid, T, ssm, 0, dense);
+}
+template <int LOGN>
+__device__ __forceinline__ void fp_inverse2(double (&e)[2][8], int tid, const NttTable& T, double* ssm) {
+  fp_inverse_w<LOGN, (LOGN + 2) / 3 - 1, 2>(e, tid, T, ssm);
 }
 
 }  // namespace via

@@ -330,17 +330,7 @@ __global__ void __launch_bounds__((1 << LOGN) / 8, LOGN >= 12 ? 1 : 2) k_dmux_fp
   constexpr int L = 2;
   constexpr int nl = 2;
   using L0 = NttPhase<LOGN, false, 0>;
-  constexpr int NB = LOGN >= 12 ? 1 : 2;  // exchange areas, as in k_cmux_fp
-  __shared__ double ssm[NB][n];
-  int buf = 0;
-  auto area = [&]() -> double* {
-    if constexpr (NB == 1) {
-      __syncthreads();
-      return ssm[0];
-    } else {
-      return ssm[buf ^= 1];
-    }
-  };
+  extern __shared__ __align__(16) double pair_sm[];  // the exchange areas of two transforms
   const int tid = threadIdx.x;
   const long o = blockIdx.x;
   const int l = blockIdx.y;
@@ -348,50 +338,51 @@ __global__ void __launch_bounds__((1 << LOGN) / 8, LOGN >= 12 ? 1 : 2) k_dmux_fp
   const double q = T.qd, qinv = T.qinv;
   const u64* ct = in + o * 2 * nl * n;
   const u64* K = ks.base + ((o / ks.div) % ks.mod) * ks.stride;
-  double am[8], ab[8];
+  double a[2][8];  // mask and body sums
 #pragma unroll
-  for (int v = 0; v < 8; ++v) am[v] = ab[v] = 0.0;
+  for (int v = 0; v < 8; ++v) a[0][v] = a[1][v] = 0.0;
 #pragma unroll 1
   for (int h = 0; h < 2; ++h) {  // 0: mask digits (neg_s_m rows), 1: body digits (m rows)
-    double val[8];
+    double e[2][8];
 #pragma unroll
     for (int v = 0; v < 8; ++v) {
       const u64* c = ct + (long)h * nl * n + L0::index(v, tid);
-      val[v] = fp_scaled2(fp_from_u64(c[0]), fp_from_u64(c[n]), g, R);
+      double val = fp_scaled2(fp_from_u64(c[0]), fp_from_u64(c[n]), g, R);
+      e[0][v] = fp_next_digit(val, g);
+      e[1][v] = fp_next_digit(val, g);
     }
-#pragma unroll 1
-    for (int k = 0; k < L; ++k) {
-      double e[8];
+    __syncthreads();  // the previous transforms' reads
+    fp_forward2<LOGN>(e, tid, T, pair_sm);
 #pragma unroll
-      for (int v = 0; v < 8; ++v) e[v] = fp_next_digit(val[v], g);
-      fp_forward<LOGN>(e, tid, T, area());
-      const int smp = h * L + L - 1 - k;
-      u64 key[8];
-      ld8_nc(K + ((long)(2 * smp) * nl + l) * n + 8 * tid, key);
+    for (int k = 0; k < L; ++k)
 #pragma unroll
-      for (int v = 0; v < 8; ++v) am[v] = __dadd_rn(am[v], fp_mulmod(e[v], fp_from_u64(key[v]), q, qinv));
-      ld8_nc(K + ((long)(2 * smp + 1) * nl + l) * n + 8 * tid, key);
+      for (int part = 0; part < 2; ++part) {
+        u64 key[8];
+        ld8_nc(K + ((long)(2 * (h * L + L - 1 - k) + part) * nl + l) * n + 8 * tid, key);
 #pragma unroll
-      for (int v = 0; v < 8; ++v) ab[v] = __dadd_rn(ab[v], fp_mulmod(e[v], fp_from_u64(key[v]), q, qinv));
-    }
+        for (int v = 0; v < 8; ++v)
+          a[part][v] = __dadd_rn(a[part][v], fp_mulmod(e[k][v], fp_from_u64(key[v]), q, qinv));
+      }
   }
   const u64 qi = R.m[l].q;
   u64* o0 = out + (2 * o) * 2 * nl * n;
   u64* o1 = o0 + 2 * nl * n;
-#pragma unroll 1
-  for (int part = 0; part < 2; ++part) {  // ext mask, ext body
 #pragma unroll
-    for (int v = 0; v < 8; ++v) am[v] = fp_reduce(am[v], q, qinv);
-    fp_inverse<LOGN>(am, tid, T, area());
+  for (int v = 0; v < 8; ++v) {
+    a[0][v] = fp_reduce(a[0][v], q, qinv);
+    a[1][v] = fp_reduce(a[1][v], q, qinv);
+  }
+  __syncthreads();
+  fp_inverse2<LOGN>(a, tid, T, pair_sm);
+#pragma unroll
+  for (int part = 0; part < 2; ++part)
 #pragma unroll
     for (int v = 0; v < 8; ++v) {
       const long at = (long)(part * nl + l) * n + L0::index(v, tid);
-      const u64 ext = fp_to_u64(fp_canonical(fp_mulmod(am[v], T.ninv_d[LOGN], q, qinv), q, qinv));
+      const u64 ext = fp_to_u64(fp_canonical(fp_mulmod(a[part][v], T.ninv_d[LOGN], q, qinv), q, qinv));
       o0[at] = submod(ct[at], ext, qi);
       o1[at] = ext;
-      am[v] = ab[v];
     }
-  }
 }
 
 // Inverse transforms of RLWEs ext ([count][2][nl][n], eval form, canonical) in
@@ -1061,6 +1052,9 @@ static void decompose(const DevRing& R, const Gadget& g, const u64* in, int n_in
   VIA_LAUNCHED();
 }
 
+static bool shared_key_fp(const DevRing& R, const int8_t* dig8, const u64* key, const u64* bodies, int L, long count,
+                          u64* out, cudaStream_t st);
+
 // Signed byte digits (bases up to 255); `in` is a 16-byte aligned buffer of canonical residues.
 static void decompose_i8(const DevRing& R, const Gadget& g, const u64* in, int n_in, long npolys, int8_t* out,
                          cudaStream_t st) {
@@ -1215,12 +1209,15 @@ static void query_decomp_range(Server& s, Workspace& w, const u64* d_query, long
   u64* gdig = w.g_digits.p + lwe0 * L * lwe_n;
   if (dig8) {
     decompose_i8(R, w.g_ck, mi, n1, nlwe, dig8, st);
-    ntt_forward_i8_lazy(dig8, gdig, n1, nl, nlwe * L * nl, R.t[0], R.t[1], st);
-    mac(R, gdig, keys_shared(s.conv_eval.p), gp, L, n1, nlwe, st);
+    if (!shared_key_fp(R, dig8, s.conv_eval.p, nullptr, L, nlwe, gp, st)) {
+      ntt_forward_i8_lazy(dig8, gdig, n1, nl, nlwe * L * nl, R.t[0], R.t[1], st);
+      mac(R, gdig, keys_shared(s.conv_eval.p), gp, L, n1, nlwe, st);
+      from_eval(R, gp, n1, nlwe * 2 * nl, st);
+    }
   } else {
     gadget_product(R, w.g_ck, mi, n1, 1, 1, nlwe, keys_shared(s.conv_eval.p), gp, gdig, st);
+    from_eval(R, gp, n1, nlwe * 2 * nl, st);
   }
-  from_eval(R, gp, n1, nlwe * 2 * nl, st);
   k_assemble_rgsw<<<blocks(nlwe * 2 * nl * n1), 256, 0, st>>>(rlwe, gp, (int)p.l_query, nbits, n1, nl, R,
                                                                w.rgsw_q1.p + bit0 * rgsw1);
   VIA_LAUNCHED();
@@ -1255,110 +1252,117 @@ static void external_products(const DevRing& R, const Gadget& g, KeySel rgsw, co
 // within 0.5625 q, so the 2L products and the input residue sum to less than
 // (1 + 1.125 L) q before the final reduction.
 //
-// FP64-issue bound (about 3000 operations a thread, 2 CTAs of 8 warps an SM). At n = 2048
-// the first exchange of a forward transform and the last of an inverse cross warps, the
-// other two stay within one, and the inverse ends in the layout the forward starts in:
-// 6 CTA barriers a CMux where 40 were. With the digit split and the conversions on doubles
-// and the dense first phase: 8191 CMuxes of a five-query batch 624 -> 410 us.
+// FP64-issue bound (about 2800 operations a thread, 2 CTAs of 8 warps an SM; 60% of the pipe).
+// At n = 2048 the first exchange of a forward transform and the last of an inverse cross
+// warps, the other two stay within one, and the inverse ends in the layout the forward
+// starts in; transforms run two at a time (mask and body, then a half's two digits). 65536
+// CMuxes 6.58 ms with single transforms, two barriers on every exchange and integer digit
+// splits, 4.31 ms with one transform at a time, 4.08 ms; 128 CMuxes (one a SM) 25, 20, 16 us.
 //
 // TILED (the first level): cur holds fd_scan's tiled columns of nq queries, where a pair's
-// four residues of a slot are 32 consecutive bytes; the body's difference waits in shared
-// memory (n = 4096: is read again).
+// four residues of a slot are 32 consecutive bytes; in[2o] waits in shared memory.
 template <int LOGN, bool TILED>
 __global__ void __launch_bounds__((1 << LOGN) / 8, LOGN >= 12 ? 1 : 2) k_cmux_fp(const u64* __restrict__ cur,
                                                                                 u64* __restrict__ nxt, KeySel ks,
                                                                                 long nq, const __grid_constant__ DevRing R,
                                                                                 const __grid_constant__ Gadget g) {
   constexpr int n = 1 << LOGN;
-  // Transforms alternate between two exchange areas, so each needs one CTA barrier
-  // (fp_forward, fp_inverse); at n = 4096 one area (32 KB) and a barrier before each.
-  constexpr int NB = LOGN >= 12 ? 1 : 2;
-  constexpr bool KEEP = TILED && LOGN < 12;
-  __shared__ double ssm[NB][n];
-  __shared__ double body[KEEP ? n : 1];
-  int buf = 0;
-  auto area = [&]() -> double* {
-    if constexpr (NB == 1) {
-      __syncthreads();
-      return ssm[0];
-    } else {
-      return ssm[buf ^= 1];
-    }
-  };
+  extern __shared__ __align__(16) double pair_sm[];  // two transforms' exchange areas, then (TILED) in[2o]
+  double* keep = pair_sm + 2 * n;
   const int tid = threadIdx.x;
   const long o = blockIdx.x;
   const NttTable& T = R.t[0];
   const double q = T.qd, qinv = T.qinv;
-  const u64* a = cur + (2 * o) * 2 * n;
+  const u64* in = cur + (2 * o) * 2 * n;
   const long tstep = 2 * FD_MT * nq;  // tiled: residues from a slot to the next
   if (TILED) {
     const long j = 2 * (o % ks.div), query = o / ks.div;  // ks.div CMuxes a query
-    a = cur + (((j / FD_MT) * n + 8 * tid) * nq + query) * 2 * FD_MT + 2 * (j % FD_MT);
+    in = cur + (((j / FD_MT) * n + 8 * tid) * nq + query) * 2 * FD_MT + 2 * (j % FD_MT);
   }
   const u64* K = ks.base + ((o / ks.div) % ks.mod) * ks.stride;
   const int L = g.L;
   const bool dense = 4.0 * g.dB * q < 281474976710656.0;  // |digit| <= B / 2: fp_digit_phase's sums below 2^48
-  double am[8], ab[8];  // in[2o] and the products
+  double val[2][8];  // mask and body: difference, then scaled coefficients
+  if (TILED) {
 #pragma unroll
-  for (int v = 0; v < 8; ++v) ab[v] = 0.0;
-#pragma unroll 1
-  for (int p = 0; p < 2; ++p) {  // 0: mask digits (neg_s_m rows), 1: body digits (m rows)
-    double val[8];
-    if (TILED && KEEP && p) {
-#pragma unroll
-      for (int v = 0; v < 8; ++v) val[v] = body[v * (n / 8) + tid];
-    } else if (TILED) {
-#pragma unroll
-      for (int v = 0; v < 8; ++v) {
-        u64 x[4];  // in[2o] mask, body, in[2o+1] mask, body of slot 8 tid + v
-        asm volatile("ld.global.v4.u64 {%0, %1, %2, %3}, [%4];"
-                     : "=l"(x[0]), "=l"(x[1]), "=l"(x[2]), "=l"(x[3])
-                     : "l"(a + v * tstep));
-        val[v] = __dadd_rn(fp_from_u64(x[2 + (KEEP ? 0 : p)]), -fp_from_u64(x[KEEP ? 0 : p]));
-        if (p == 0) am[v] = fp_from_u64(x[0]);
-        if (KEEP || p) ab[v] = __dadd_rn(ab[v], fp_from_u64(x[1]));
-        if (KEEP) body[v * (n / 8) + tid] = __dadd_rn(fp_from_u64(x[3]), -fp_from_u64(x[1]));
-      }
-    } else {
-      u64 x[8], y[8];
-      ld8(a + 2 * n + p * n + 8 * tid, x);
-      ld8(a + p * n + 8 * tid, y);
-#pragma unroll
-      for (int v = 0; v < 8; ++v) {
-        const double yd = fp_from_u64(y[v]);
-        val[v] = __dadd_rn(fp_from_u64(x[v]), -yd);
-        if (p == 0)
-          am[v] = yd;
-        else
-          ab[v] = __dadd_rn(ab[v], yd);
-      }
+    for (int v = 0; v < 8; ++v) {
+      u64 x[4];  // in[2o] mask, body, in[2o+1] mask, body of slot 8 tid + v
+      asm volatile("ld.global.v4.u64 {%0, %1, %2, %3}, [%4];"
+                   : "=l"(x[0]), "=l"(x[1]), "=l"(x[2]), "=l"(x[3])
+                   : "l"(in + v * tstep));
+      const double m = fp_from_u64(x[0]), b = fp_from_u64(x[1]);
+      val[0][v] = __dadd_rn(fp_from_u64(x[2]), -m);
+      val[1][v] = __dadd_rn(fp_from_u64(x[3]), -b);
+      keep[v * (n / 8) + tid] = m;
+      keep[n + v * (n / 8) + tid] = b;
     }
-    fp_inverse<LOGN>(val, tid, T, area());
+  } else {
 #pragma unroll
-    for (int v = 0; v < 8; ++v) val[v] = fp_scaled(fp_mulmod(val[v], T.ninv_d[LOGN], q, qinv), g.dS, qinv);
-#pragma unroll 1
-    for (int k = 0; k < L; ++k) {
-      double e[8];
+    for (int p = 0; p < 2; ++p) {
+      u64 x[8], y[8];
+      ld8(in + 2 * n + p * n + 8 * tid, x);
+      ld8(in + p * n + 8 * tid, y);
 #pragma unroll
-      for (int v = 0; v < 8; ++v) e[v] = fp_next_digit(val[v], g);
-      fp_forward_digits<LOGN>(e, tid, T, area(), 0, dense);
-      const u64* Km = K + (long)(2 * (p * L + L - 1 - k)) * n + 8 * tid;
-      u64 key[8];
-      ld8_nc(Km, key);
-#pragma unroll
-      for (int v = 0; v < 8; ++v) am[v] = __dadd_rn(am[v], fp_mulmod(e[v], fp_from_u64(key[v]), q, qinv));
-      ld8_nc(Km + n, key);
-#pragma unroll
-      for (int v = 0; v < 8; ++v) ab[v] = __dadd_rn(ab[v], fp_mulmod(e[v], fp_from_u64(key[v]), q, qinv));
+      for (int v = 0; v < 8; ++v) val[p][v] = __dadd_rn(fp_from_u64(x[v]), -fp_from_u64(y[v]));
     }
   }
-  u64 x[8];
+  fp_inverse2<LOGN>(val, tid, T, pair_sm);
 #pragma unroll
-  for (int v = 0; v < 8; ++v) x[v] = fp_to_u64(fp_canonical(am[v], q, qinv));
-  st8(nxt + o * 2 * n + 8 * tid, x);
+  for (int p = 0; p < 2; ++p)
 #pragma unroll
-  for (int v = 0; v < 8; ++v) x[v] = fp_to_u64(fp_canonical(ab[v], q, qinv));
-  st8(nxt + o * 2 * n + n + 8 * tid, x);
+    for (int v = 0; v < 8; ++v)
+      val[p][v] = fp_scaled(fp_mulmod(val[p][v], T.ninv_d[LOGN], q, qinv), g.dS, qinv);
+  double a[2][8];  // mask and body sums
+#pragma unroll
+  for (int v = 0; v < 8; ++v) a[0][v] = a[1][v] = 0.0;
+#pragma unroll 1
+  for (int p = 0; p < 2; ++p) {  // 0: mask digits (neg_s_m rows), 1: body digits (m rows)
+#pragma unroll 1
+    for (int k = 0; k < L; k += 2) {
+      double e[2][8];
+#pragma unroll
+      for (int v = 0; v < 8; ++v) {
+        e[0][v] = fp_next_digit(val[0][v], g);
+        e[1][v] = fp_next_digit(val[0][v], g);
+      }
+      __syncthreads();  // the previous transforms' reads
+      fp_forward_digits2<LOGN>(e, tid, T, pair_sm, dense);
+#pragma unroll
+      for (int i = 0; i < 2; ++i) {
+        if (k + i >= L) break;  // an odd depth's last digit comes alone
+#pragma unroll
+        for (int part = 0; part < 2; ++part) {
+          u64 key[8];
+          ld8_nc(K + (long)(2 * (p * L + L - 1 - k - i) + part) * n + 8 * tid, key);
+#pragma unroll
+          for (int v = 0; v < 8; ++v)
+            a[part][v] = __dadd_rn(a[part][v], fp_mulmod(e[i][v], fp_from_u64(key[v]), q, qinv));
+        }
+      }
+    }
+#pragma unroll
+    for (int v = 0; v < 8; ++v) val[0][v] = val[1][v];
+  }
+#pragma unroll
+  for (int part = 0; part < 2; ++part) {
+    u64 x[8];
+    if (!TILED) ld8(in + part * n + 8 * tid, x);
+#pragma unroll
+    for (int v = 0; v < 8; ++v) {
+      const double y = TILED ? keep[part * n + v * (n / 8) + tid] : fp_from_u64(x[v]);
+      x[v] = fp_to_u64(fp_canonical(__dadd_rn(y, a[part][v]), q, qinv));
+    }
+    st8(nxt + o * 2 * n + part * n + 8 * tid, x);
+  }
+}
+
+// The dynamic shared memory (`doubles` of it) of a kernel above, its limit raised where needed.
+template <class K>
+static size_t pair_smem(K kernel, size_t doubles) {
+  const size_t bytes = doubles * 8;
+  if (bytes > 48 * 1024)
+    VIA_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
+  return bytes;
 }
 
 // The CMux of k_cmux_fp split over a cluster of four CTAs, for tree levels
@@ -1529,6 +1533,214 @@ __global__ void __cluster_dims__(4, 1, 1) __launch_bounds__((1 << LOGN) / 8)
   }
 }
 
+// ---------------------------------------------------------------------------
+// Fused gadget products on the transform's registers, double precision (ntt_fp.cuh).
+// ---------------------------------------------------------------------------
+constexpr long SHARED_KEY_MIN = 512;  // CTAs from which k_shared_key_fp runs
+
+// key (x) digits of one polynomial per CTA and limb, the key shared by all: signed digit
+// bytes dig8 [c][L][n] -> forward transforms -> products with the eval-form samples
+// [L][2][nl][n] -> inverse transforms of the two sums -> out [c][2][nl][n], coefficient
+// form. Digits and products never reach memory; the key streams from L2.
+//
+// ROTATED (a key switch of rotated ciphertexts, keyswitch.rs:99-102): out =
+// (-prod.mask, body - prod.body) with `bodies` [c][nl][n].
+//
+// FP64-issue bound: L + 2 transforms, two at a time, a CTA. 2048 key switches at q1 (L = 18)
+// 1049 us in separate kernels (digit transforms, multiply-accumulate, inverse, sum), 781 us.
+template <int LOGN, bool ROTATED>
+__global__ void __launch_bounds__((1 << LOGN) / 8, LOGN >= 12 ? 1 : LOGN == 11 ? 2 : 1)
+    k_shared_key_fp(const int8_t* __restrict__ dig8, const u64* __restrict__ key, const u64* __restrict__ bodies, int L,
+                    u64* __restrict__ out, const __grid_constant__ DevRing R) {
+  constexpr int n = 1 << LOGN;
+  using L0 = NttPhase<LOGN, false, 0>;
+  extern __shared__ __align__(16) double pair_sm[];
+  const int tid = threadIdx.x, nl = R.nl, l = blockIdx.y;
+  const long c = blockIdx.x;
+  const NttTable& T = R.t[l];
+  const double q = T.qd, qinv = T.qinv;
+  const int8_t* d = dig8 + c * (long)L * n;
+  const long per = (long)nl * n;
+  const u64* K = key + (long)l * n + 8 * tid;
+  const bool dense = q <= FP_DIGIT_Q;
+  double a[2][8];  // mask and body sums
+#pragma unroll
+  for (int v = 0; v < 8; ++v) a[0][v] = a[1][v] = 0.0;
+#pragma unroll 1
+  for (int s = 0; s < L; s += 2) {
+    const bool two = s + 1 < L;
+    double e[2][8];
+#pragma unroll
+    for (int v = 0; v < 8; ++v) {
+      e[0][v] = (double)d[(long)s * n + L0::index(v, tid)];
+      e[1][v] = two ? (double)d[(long)(s + 1) * n + L0::index(v, tid)] : 0.0;
+    }
+    __syncthreads();  // the previous transforms' reads
+    fp_forward_digits2<LOGN>(e, tid, T, pair_sm, dense);
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      if (i && !two) break;
+#pragma unroll
+      for (int part = 0; part < 2; ++part) {
+        u64 k[8];
+        ld8_nc(K + (2 * (s + i) + part) * per, k);
+#pragma unroll
+        for (int v = 0; v < 8; ++v)
+          a[part][v] = __dadd_rn(a[part][v], fp_mulmod(e[i][v], fp_from_u64(k[v]), q, qinv));
+      }
+    }
+  }
+#pragma unroll
+  for (int v = 0; v < 8; ++v) {
+    a[0][v] = fp_reduce(a[0][v], q, qinv);
+    a[1][v] = fp_reduce(a[1][v], q, qinv);
+  }
+  __syncthreads();
+  fp_inverse2<LOGN>(a, tid, T, pair_sm);
+  const u64 qi = R.m[l].q;
+#pragma unroll
+  for (int part = 0; part < 2; ++part)
+#pragma unroll
+    for (int v = 0; v < 8; ++v) {
+      const int x = L0::index(v, tid);
+      u64 w = fp_to_u64(fp_canonical(fp_mulmod(a[part][v], T.ninv_d[LOGN], q, qinv), q, qinv));
+      if (ROTATED) w = part ? submod(bodies[c * per + (long)l * n + x], w, qi) : negmod(w, qi);
+      out[(2 * c + part) * per + (long)l * n + x] = w;
+    }
+}
+
+// External products with RGSWs of their own (rgsw.rs:108-121): per CTA (pair, limb) the gadget
+// digits, the samples' forward transforms, products and inverse transforms. rgsw
+// [c][2L][2][nl][n] and cts, out [c][2][nl][n], all in coefficient form at any 8-byte
+// address. Each RGSW polynomial is read once and nothing else of its size is written.
+// FP64-issue bound (6 L + 2 transforms, two at a time): 4099 pairs at q1, L = 2: 1.93 ms in
+// separate kernels after a copy of the RGSWs, 1.80 ms.
+template <int LOGN>
+__global__ void __launch_bounds__((1 << LOGN) / 8, LOGN >= 12 ? 1 : LOGN == 11 ? 2 : 1)
+    k_external_fp(const u64* __restrict__ rgsw, const u64* __restrict__ cts, u64* __restrict__ out,
+                  const __grid_constant__ DevRing R, const __grid_constant__ Gadget g) {
+  constexpr int n = 1 << LOGN;
+  using L0 = NttPhase<LOGN, false, 0>;
+  extern __shared__ __align__(16) double pair_sm[];  // two exchange areas, then the scaled coefficients
+  double* keep = pair_sm + 2 * n;
+  const int tid = threadIdx.x, nl = R.nl, l = blockIdx.y, L = g.L;
+  const long c = blockIdx.x, per = (long)nl * n;
+  const NttTable& T = R.t[l];
+  const double q = T.qd, qinv = T.qinv;
+  const u64* ct = cts + c * 2 * per;
+  const u64* K = rgsw + c * 2 * L * 2 * per + (long)l * n;
+#pragma unroll
+  for (int h = 0; h < 2; ++h)
+#pragma unroll
+    for (int v = 0; v < 8; ++v) {
+      const u64* x = ct + h * per + L0::index(v, tid);
+      keep[h * n + v * (n / 8) + tid] = nl == 2 ? fp_scaled2(fp_from_u64(x[0]), fp_from_u64(x[n]), g, R)
+                                                : fp_scaled(fp_reduce(fp_from_u64(x[0]), q, qinv), g.dS, qinv);
+    }
+  double a[2][8];  // mask and body sums
+#pragma unroll
+  for (int v = 0; v < 8; ++v) a[0][v] = a[1][v] = 0.0;
+#pragma unroll 1
+  for (int k = 0; k < L; ++k) {
+    double e[2][8];  // digit k of the mask and of the body
+#pragma unroll
+    for (int h = 0; h < 2; ++h)
+#pragma unroll
+      for (int v = 0; v < 8; ++v) {
+        double val = keep[h * n + v * (n / 8) + tid];
+        e[h][v] = fp_next_digit(val, g);
+        keep[h * n + v * (n / 8) + tid] = val;
+      }
+    __syncthreads();  // the previous transforms' reads
+    fp_forward2<LOGN>(e, tid, T, pair_sm);
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const long smp = h * L + L - 1 - k;
+      double f[2][8];  // the sample's mask and body
+#pragma unroll
+      for (int part = 0; part < 2; ++part)
+#pragma unroll
+        for (int v = 0; v < 8; ++v) {
+          u64 x = K[(2 * smp + part) * per + L0::index(v, tid)];
+          if (x >= (1ull << 47)) x %= T.q;  // as the transforms take any word
+          f[part][v] = fp_from_u64(x);
+        }
+      __syncthreads();
+      fp_forward2<LOGN>(f, tid, T, pair_sm);
+#pragma unroll
+      for (int v = 0; v < 8; ++v) {
+        const double x = fp_reduce(e[h][v], q, qinv);  // the product's factor below q
+        a[0][v] = __dadd_rn(a[0][v], fp_mulmod(f[0][v], x, q, qinv));
+        a[1][v] = __dadd_rn(a[1][v], fp_mulmod(f[1][v], x, q, qinv));
+      }
+    }
+  }
+#pragma unroll
+  for (int v = 0; v < 8; ++v) {
+    a[0][v] = fp_reduce(a[0][v], q, qinv);
+    a[1][v] = fp_reduce(a[1][v], q, qinv);
+  }
+  __syncthreads();
+  fp_inverse2<LOGN>(a, tid, T, pair_sm);
+#pragma unroll
+  for (int part = 0; part < 2; ++part)
+#pragma unroll
+    for (int v = 0; v < 8; ++v)
+      out[(2 * c + part) * per + (long)l * n + L0::index(v, tid)] =
+          fp_to_u64(fp_canonical(fp_mulmod(a[part][v], T.ninv_d[LOGN], q, qinv), q, qinv));
+}
+
+// Runs k_shared_key_fp (a key switch of rotated ciphertexts where `bodies` is given); false
+// (nothing launched) for other rings, a key at an odd address, and products too few to fill
+// the GPU, whose transforms in a row take longer than separate kernels side by side
+// (240 CTAs 95 us, against 73 us).
+static bool shared_key_fp(const DevRing& R, const int8_t* dig8, const u64* key, const u64* bodies, int L, long count,
+                          u64* out, cudaStream_t st) {
+  if (!R.ntt || !ntt_fp_ok(R.t[0], R.t[R.nl - 1]) || ((uintptr_t)key & 31) || count * R.nl < SHARED_KEY_MIN) return false;
+  const dim3 grid((unsigned)count, (unsigned)R.nl);
+#define VIA_SK_CASE(LG)                                                                                          \
+  case 1 << LG:                                                                                                  \
+    if (bodies)                                                                                                  \
+      k_shared_key_fp<LG, true><<<grid, (1 << LG) / 8, pair_smem(k_shared_key_fp<LG, true>, 2 << LG), st>>>(     \
+          dig8, key, bodies, L, out, R);                                                                         \
+    else                                                                                                         \
+      k_shared_key_fp<LG, false><<<grid, (1 << LG) / 8, pair_smem(k_shared_key_fp<LG, false>, 2 << LG), st>>>(   \
+          dig8, key, bodies, L, out, R);                                                                         \
+    break;
+  switch (R.n) {
+    VIA_SK_CASE(8)
+    VIA_SK_CASE(9)
+    VIA_SK_CASE(10)
+    VIA_SK_CASE(11)
+    VIA_SK_CASE(12)
+    default: return false;
+  }
+#undef VIA_SK_CASE
+  VIA_LAUNCHED();
+  return true;
+}
+
+// Runs k_external_fp; false (nothing launched) for rings and gadgets it does not serve, and for
+// outputs that overlap an input: its CTAs write one limb while others may still read.
+static bool external_fp(const DevRing& R, const Gadget& g, const u64* rgsw, const u64* cts, long count, u64* out,
+                        cudaStream_t st) {
+  if (!R.ntt || !g.fp || !ntt_fp_ok(R.t[0], R.t[R.nl - 1]) || 2 * g.L > 256) return false;
+  const size_t per = (size_t)R.nl * R.n, len = (size_t)count * 2 * per;
+  const auto apart = [&](const u64* p, size_t words) { return out + len <= p || p + words <= out; };
+  if (!apart(cts, len) || !apart(rgsw, len * 2 * g.L)) return false;
+  const dim3 grid((unsigned)count, (unsigned)R.nl);
+  switch (R.n) {
+    case 4096: k_external_fp<12><<<grid, 512, pair_smem(k_external_fp<12>, 4 << 12), st>>>(rgsw, cts, out, R, g); break;
+    case 2048: k_external_fp<11><<<grid, 256, pair_smem(k_external_fp<11>, 4 << 11), st>>>(rgsw, cts, out, R, g); break;
+    case 1024: k_external_fp<10><<<grid, 128, pair_smem(k_external_fp<10>, 4 << 10), st>>>(rgsw, cts, out, R, g); break;
+    case 512: k_external_fp<9><<<grid, 64, pair_smem(k_external_fp<9>, 4 << 9), st>>>(rgsw, cts, out, R, g); break;
+    case 256: k_external_fp<8><<<grid, 32, pair_smem(k_external_fp<8>, 4 << 8), st>>>(rgsw, cts, out, R, g); break;
+    default: return false;
+  }
+  VIA_LAUNCHED();
+  return true;
+}
+
 // Rings and gadgets k_ext_cluster_fp serves. Raises its shared-memory limit (n = 4096: 64 KB) on the
 // current device.
 static bool ext_cluster_ok(const DevRing& R, const Gadget& g) {
@@ -1572,9 +1784,11 @@ static void cmux_fused(const DevRing& R, const Gadget& g, const u64* cur, u64* n
   }
 #define VIA_CMUX_CASE(LG)                                                                                        \
   if (tiled_nq)                                                                                                 \
-    k_cmux_fp<LG, true><<<(unsigned)count, (1 << LG) / 8, 0, st>>>(cur, nxt, ks, tiled_nq, R, g);               \
+    k_cmux_fp<LG, true><<<(unsigned)count, (1 << LG) / 8, pair_smem(k_cmux_fp<LG, true>, 4 << LG), st>>>(       \
+        cur, nxt, ks, tiled_nq, R, g);                                                                          \
   else                                                                                                          \
-    k_cmux_fp<LG, false><<<(unsigned)count, (1 << LG) / 8, 0, st>>>(cur, nxt, ks, 0, R, g);                     \
+    k_cmux_fp<LG, false><<<(unsigned)count, (1 << LG) / 8, pair_smem(k_cmux_fp<LG, false>, 2 << LG), st>>>(     \
+        cur, nxt, ks, 0, R, g);                                                                                 \
   break;
   switch (R.n) {
     case 4096: VIA_CMUX_CASE(12)
@@ -1746,9 +1960,9 @@ void answer_device_stages(Server& s, Workspace& w, const u64* d_query, int nq, u
       if (dmux_fp_ok(s.r1, w.g_dmux)) {
         const dim3 grid((unsigned)(B * active), 2);
         if (n1 == 4096)
-          k_dmux_fp<12><<<grid, 512, 0, st>>>(out, in, bit, s.r1, w.g_dmux);
+          k_dmux_fp<12><<<grid, 512, pair_smem(k_dmux_fp<12>, 2 * n1), st>>>(out, in, bit, s.r1, w.g_dmux);
         else
-          k_dmux_fp<11><<<grid, 256, 0, st>>>(out, in, bit, s.r1, w.g_dmux);
+          k_dmux_fp<11><<<grid, 256, pair_smem(k_dmux_fp<11>, 2 * n1), st>>>(out, in, bit, s.r1, w.g_dmux);
         VIA_LAUNCHED();
         std::swap(in, out);
         continue;
@@ -2121,6 +2335,7 @@ void answer_batch_device(Server& s, const u64* d_queries, u64* d_mask, u64* d_bo
 void prim_external_products(const DevRing& R, const Gadget& g, const u64* rgsw, const u64* cts, long count, u64* out,
                             u64* rgsw_eval, u64* digits, cudaStream_t st) {
   const long per = (long)R.nl * R.n;
+  if (external_fp(R, g, rgsw, cts, count, out, st)) return;
   VIA_CUDA(cudaMemcpyAsync(rgsw_eval, rgsw, (size_t)count * 2 * g.L * 2 * per * 8, cudaMemcpyDeviceToDevice, st));
   to_eval(R, rgsw_eval, R.n, count * 2 * g.L * 2 * R.nl, st);
   external_products(R, g, KeySel{rgsw_eval, 1, count, 0}, cts, count, digits, out, true, st);
@@ -2178,6 +2393,7 @@ void prim_key_switches(const DevRing& R, const Gadget& g, const u64* key, const 
     int8_t* dig8 = reinterpret_cast<int8_t*>(prod);
     static_assert(CT_L <= 2 * 2 * 8, "18 bytes of digits fit the product's 32 bytes a coefficient");
     decompose_i8(R, g, masks, n, count, dig8, st);
+    if (shared_key_fp(R, dig8, key_eval, bodies, g.L, count, out, st)) return;
     ntt_forward_i8_lazy(dig8, digits, n, R.nl, count * g.L * R.nl, R.t[0], R.t[1], st);
     mac(R, digits, keys_shared(key_eval), prod, g.L, n, count, st);
   } else {
