@@ -192,6 +192,14 @@ __global__ void k_u64_to_f64(const u64* __restrict__ in, double* __restrict__ ou
   if (gid < count) out[gid] = __ull2double_rn(in[gid]);
 }
 
+// The handle's stream, of the highest priority: its kernels go before those of the workspaces'
+// side streams.
+static void make_stream(Server& s) {
+  int least = 0, greatest = 0;
+  VIA_CUDA(cudaDeviceGetStreamPriorityRange(&least, &greatest));
+  VIA_CUDA(cudaStreamCreateWithPriority(&s.stream, cudaStreamNonBlocking, greatest));
+}
+
 static void transform_keys(Server& s) {
   const via_params& p = s.prm;
   // Cascade: step k (output degree 2^k) has 2*n1*L_CK*2*nl residues.
@@ -240,7 +248,7 @@ static void setup(Server& s, const via_params& p, const via_public_keys* keys, c
     throw ApiError(VIA_ERR_DIM_MISMATCH, "setup: more records than DB capacity (would silently drop)");
   if (n_records && !records) throw ApiError(VIA_ERR_INVALID_ARGUMENT, "records is null");
   VIA_CUDA(cudaGetDevice(&s.device));
-  VIA_CUDA(cudaStreamCreateWithFlags(&s.stream, cudaStreamNonBlocking));
+  make_stream(s);
   s.r1 = make_ring(s, p.n1, p.q1_0, p.q1_1);
   s.r2 = make_ring(s, p.n1, p.q2, 0);
   s.r3n1 = make_ring(s, p.n1, p.q3, 0);
@@ -327,7 +335,7 @@ static void setup_view(Server& s, const Server& base, uint32_t n_rec, const via_
   s.prm = p;
   VIA_CUDA(cudaGetDevice(&s.device));
   if (s.device != base.device) throw ApiError(VIA_ERR_INVALID_ARGUMENT, "a view must be made on its database's device");
-  VIA_CUDA(cudaStreamCreateWithFlags(&s.stream, cudaStreamNonBlocking));
+  make_stream(s);
   s.r1 = make_ring(s, p.n1, p.q1_0, p.q1_1);
   s.r2 = make_ring(s, p.n1, p.q2, 0);
   s.r3n1 = make_ring(s, p.n1, p.q3, 0);
