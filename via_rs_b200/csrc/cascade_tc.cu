@@ -89,9 +89,12 @@ __global__ void __launch_bounds__(256) k_ct_digits(const u64* __restrict__ q, lo
 // into a ring of shared-memory stages, warp 1 issues the MMAs into one of three TMEM
 // accumulator sets, sixteen epilogue warps fold the previous one.
 //
-// Bounds: at n <= 16 the epilogue (128 x 16 coefficients, 64 FP64 and about 100 integer
-// instructions each) is longer than the MMAs (18 n of 80 cycles each, 36 n K bytes); from
-// n = 64 on the MMAs and the key planes' L2 traffic (160 bytes a K byte) are.
+// Bounds: up to n = 32 the epilogue (128 x 16 coefficients, 64 FP64 and about 200 integer
+// instructions each, 10000 cycles a mask unit) is longer than the MMAs (36 n K bytes, 166
+// cycles for 32 of them: kind::i8 runs at 4000 multiply-adds a cycle and SM here); from
+// n = 64 on the MMAs are. One query (18 LWEs): 11 to 15 us a step up to n = 16, of which
+// 5 us are launch and first loads and 5 us one epilogue. 2688 LWEs: 116 us (n = 8) to 360 us
+// (n = 64) a step, against 2400 us in four kernels on transforms.
 __global__ void __launch_bounds__(CT_THREADS, 1) k_ct_step(const __grid_constant__ CtParams P) {
   extern __shared__ __align__(1024) uint8_t smem[];
   u64* full = reinterpret_cast<u64*>(smem + CT_STAGES * CT_STAGE);
@@ -493,8 +496,6 @@ bool ct_supported(const via_params& p, const DevRing& R) {
   return p.n1 >= 256 && ct_digits_ok(p.ck_base, p.l_ck, R);
 }
 
-int ct_steps(const via_params&) { return 7; }  // input degrees 1 .. 64
-
 void ct_prepare_device() {
   VIA_CUDA(cudaFuncSetAttribute(k_ct_step, cudaFuncAttributeMaxDynamicSharedMemorySize, CT_SMEM));
 }
@@ -548,9 +549,10 @@ void ct_run(Server& s, const u64* d_query, long nlwe, uint8_t* da, uint8_t* db, 
                                                                 (size_t)CT_M * cur.half * cur.kp, da);
   VIA_LAUNCHED();
   size_t b_off = 0, c_off = mtiles >= CT_MANY ? s.ct_consts.n / 2 : 0;
-  for (int k = 0; k < s.ct_steps; ++k) {
+  const int steps = ct_steps_for(s.ct_steps, nlwe);
+  for (int k = 0; k < steps; ++k) {
     const CtStep nxt = ct_step(n1, 2 << k, mtiles);
-    const bool last = k + 1 == s.ct_steps;
+    const bool last = k + 1 == steps;
     CtParams P{};
     P.st = cur;
     P.D = D;

@@ -138,8 +138,13 @@ bool ct_digits_ok(u64 base, u32 L, const DevRing& R);
 CtDigits ct_digits(u64 base, const DevRing& R);
 // Whether the GEMM steps serve this server's cascade.
 bool ct_supported(const via_params& p, const DevRing& R);
-// Number of leading steps run as GEMMs.
-int ct_steps(const via_params& p);
+// Leading steps prepared as GEMMs: input degrees 1 .. 128 (the last cascade step stays on
+// transforms). Their key planes take 406 MB at n1 = 2048.
+inline int ct_steps(const via_params& p) { return ilog2(p.n1) - 1 < 8 ? ilog2(p.n1) - 1 : 8; }
+// Steps run as GEMMs for nlwe LWEs, of `prepared`: input degree 128 from two tiles on, where
+// its 189 MB of planes serve enough of them (2688 LWEs: 513 us against 1370 us in the four
+// transform kernels, 180 LWEs 59 against 95; one query's 42 against 26).
+inline int ct_steps_for(int prepared, long nlwe) { return prepared > 7 && nlwe <= CT_M ? 7 : prepared; }
 // Builds the key planes and column constants from the coefficient-form cascade key.
 void ct_prepare(Server& s);
 // Raises the kernel's shared-memory limit on the current device.
