@@ -69,7 +69,7 @@ __device__ __forceinline__ i64 error_value(int err_kind, i64 err_bound, u64 x) {
 }
 
 // One CTA per query: LWE by LWE, the mask by a parallel scan of its candidates
-// (walk_mask, all limbs' draws nb bytes) and then the error's draws by thread 0,
+// (walk_mask, all limbs' draws nb bytes) and then the error's draws,
 // with the outputs of k_client_walk. Flag 2 where the scan could not decide.
 // Latency-bound, an LWE after another: the warp walk of k_client_walk took
 // 8184 us for 24 queries of 40 LWEs (paper preset).
@@ -79,7 +79,6 @@ __global__ void __launch_bounds__(WALK_THREADS) k_client_walk_scan(const u64* __
                                                                    u64* __restrict__ out, i64* __restrict__ errs,
                                                                    int* __restrict__ flag) {
   __shared__ WalkShared sh;
-  __shared__ u64 s_pos;
   const size_t q = blockIdx.x;
   const u64* words = blocks + q * nblk * RATE_LANES;
   const u64 avail = (u64)nblk * SHAKE_RATE;
@@ -91,25 +90,20 @@ __global__ void __launch_bounds__(WALK_THREADS) k_client_walk_scan(const u64* __
       return;
     }
     pos += (u64)used * W.nb;
-    if (threadIdx.x == 0) {
-      int attempt = 0;
-      u64 x = 0;
-      bool ok = false;
-      for (; attempt < 64 && !ok && pos + D.nbytes[2] <= avail; ++attempt) {
-        x = 0;
-        for (int b = 0; b < D.nbytes[2]; ++b, ++pos)
-          x |= (u64)((words[pos >> 3] >> (8 * (pos & 7))) & 0xFF) << (8 * b);
-        x &= D.mask[2];
-        ok = x < D.bound[2];
-      }
-      if (!ok) atomicMax(flag, 2);  // the stream's end or 64 rejections: the general walk decides
-      errs[q * n_lwe + j] = error_value(err_kind, err_bound, x);
-      s_pos = ok ? pos : ~(u64)0;
+    u64 x = 0;  // every thread draws the error itself, from the same bytes
+    bool ok = false;
+    for (int attempt = 0; attempt < 64 && !ok && pos + D.nbytes[2] <= avail; ++attempt) {
+      x = 0;
+      for (int b = 0; b < D.nbytes[2]; ++b, ++pos)
+        x |= (u64)((words[pos >> 3] >> (8 * (pos & 7))) & 0xFF) << (8 * b);
+      x &= D.mask[2];
+      ok = x < D.bound[2];
     }
-    __syncthreads();
-    pos = s_pos;
-    __syncthreads();
-    if (pos == ~(u64)0) return;
+    if (threadIdx.x == 0) errs[q * n_lwe + j] = error_value(err_kind, err_bound, x);
+    if (!ok) {  // the stream's end or 64 rejections: the general walk decides
+      if (threadIdx.x == 0) atomicMax(flag, 2);
+      return;
+    }
   }
 }
 

@@ -181,7 +181,7 @@ __device__ __forceinline__ void st_slots(u64* p, const u64 (&x)[NS]) {
 // its own key: 4099 external products at q1 490 us in 128-bit integers, 303 us here
 // (6.2 TB/s).
 template <int NS>
-__global__ void __launch_bounds__(256) k_mac_fp(const u64* __restrict__ D, KeySel ks, u64* __restrict__ out, int T,
+__global__ void __launch_bounds__(256, NS == 1 ? 2 : 4) k_mac_fp(const u64* __restrict__ D, KeySel ks, u64* __restrict__ out, int T,
                                                 int n, int nl, long nout, const __grid_constant__ DevRing R) {
   const long gid = ((long)blockIdx.x * blockDim.x + threadIdx.x) * NS;
   const long per = (long)nl * n;
@@ -471,6 +471,30 @@ __global__ void k_mod_switch(const u64* __restrict__ in, DevRing S, u64* __restr
     r = div_exact(num, Qs, dQs);
   u64 rr = (u64)r;
   out[p * n + i] = rr >= dst.q ? rr - dst.q : rr;
+}
+
+// The same from a two-prime ring in double precision: round(c q_dst / Q) is fp_scaled2's value
+// with q_dst for S, an integer within 1.2 q_dst of zero. Two coefficients a
+// thread. Bound by its 24 bytes a coefficient: the 67 million coefficients of 64 queries'
+// rows 830 us with 128-bit divisions, MOD_SWITCH_FIGURES
+__global__ void __launch_bounds__(256) k_mod_switch_fp(const u64* __restrict__ in, const __grid_constant__ DevRing S,
+                                                       const __grid_constant__ Gadget g, u64* __restrict__ out,
+                                                       double q, long ncoef, int n) {
+  const long gid = ((long)blockIdx.x * blockDim.x + threadIdx.x) * 2;
+  if (gid >= ncoef) return;
+  const long p = gid / n;
+  const int i = (int)(gid - p * n);
+  const ulonglong2 a = *reinterpret_cast<const ulonglong2*>(in + (p * 2) * n + i);
+  const ulonglong2 b = *reinterpret_cast<const ulonglong2*>(in + (p * 2 + 1) * n + i);
+  double v[2] = {fp_scaled2(fp_from_u64(a.x), fp_from_u64(b.x), g, S),
+                 fp_scaled2(fp_from_u64(a.y), fp_from_u64(b.y), g, S)};
+#pragma unroll
+  for (int k = 0; k < 2; ++k) {
+    if (v[k] < 0.0) v[k] = __dadd_rn(v[k], q);
+    if (v[k] < 0.0) v[k] = __dadd_rn(v[k], q);
+    if (v[k] >= q) v[k] = __dadd_rn(v[k], -q);
+  }
+  *reinterpret_cast<ulonglong2*>(out + gid) = make_ulonglong2(fp_to_u64(v[0]), fp_to_u64(v[1]));
 }
 
 // ---------------------------------------------------------------------------
@@ -1085,6 +1109,16 @@ static double to_double(u128 x) { return (double)(u64)(x >> 64) * 18446744073709
 
 static void mod_switch(const DevRing& S, const u64* in, const DevRing& D, u64* out, long npolys, int n, cudaStream_t st) {
   long nco = npolys * n;
+  // Odd primes below 2^44, a target below 2^40 and rounding ties that cannot happen.
+  if (S.ntt && S.nl == 2 && ntt_fp_ok(S.t[0], S.t[1]) && D.m[0].q < (1ull << 40) && n % 2 == 0) {
+    Gadget g{};
+    g.dS = (double)D.m[0].q;
+    g.ys[0] = (double)h_inv(S.m[1].q % S.m[0].q, S.m[0].q);
+    g.ys[1] = (double)h_inv(S.m[0].q % S.m[1].q, S.m[1].q);
+    k_mod_switch_fp<<<blocks(nco / 2), 256, 0, st>>>(in, S, g, out, (double)D.m[0].q, nco, n);
+    VIA_LAUNCHED();
+    return;
+  }
   k_mod_switch<<<blocks(nco), 256, 0, st>>>(in, S, out, D.m[0], nco, n, to_double(S.Q()));
   VIA_LAUNCHED();
 }

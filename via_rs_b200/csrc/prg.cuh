@@ -71,7 +71,9 @@ __host__ __device__ inline const KeccakConsts& keccak_consts() {
 __host__ __device__ __forceinline__ u64 rotl64(u64 v, int s) { return s == 0 ? v : (v << s) | (v >> (64 - s)); }
 
 __host__ __device__ inline void keccak_f1600(u64 (&A)[25]) {
+  constexpr KeccakConsts R = make_keccak_consts();  // rotation amounts fold into the instructions
   const KeccakConsts& K = keccak_consts();
+#pragma unroll 1
   for (int r = 0; r < 24; ++r) {
     u64 C[5], D[5], B[25];
 #pragma unroll
@@ -83,7 +85,7 @@ __host__ __device__ inline void keccak_f1600(u64 (&A)[25]) {
 #pragma unroll
     for (int x = 0; x < 5; ++x)
 #pragma unroll
-      for (int y = 0; y < 5; ++y) B[y + 5 * ((2 * x + 3 * y) % 5)] = rotl64(A[x + 5 * y], K.rot[x + 5 * y]);
+      for (int y = 0; y < 5; ++y) B[y + 5 * ((2 * x + 3 * y) % 5)] = rotl64(A[x + 5 * y], R.rot[x + 5 * y]);
 #pragma unroll
     for (int x = 0; x < 5; ++x)
 #pragma unroll
@@ -98,17 +100,19 @@ __host__ __device__ inline void prg_block(const uint8_t* seed, int seed_len, u64
   u64 A[25];
 #pragma unroll
   for (int i = 0; i < 25; ++i) A[i] = 0;
-  uint8_t msg[SHAKE_RATE];
-  for (int i = 0; i < SHAKE_RATE; ++i) msg[i] = 0;
-  for (int i = 0; i < seed_len; ++i) msg[i] = seed[i];
-  for (int i = 0; i < 8; ++i) msg[seed_len + i] = (uint8_t)(counter >> (8 * i));
-  msg[seed_len + 8] ^= 0x1F;        // SHAKE domain bits and the first pad bit
-  msg[SHAKE_RATE - 1] ^= 0x80;      // last pad bit
-  for (int l = 0; l < RATE_LANES; ++l) {
+  // seed || counter || 0x1F as little-endian words (at most 73 bytes), then the last pad bit.
+#pragma unroll
+  for (int l = 0; l < 10; ++l) {
     u64 v = 0;
-    for (int b = 0; b < 8; ++b) v |= (u64)msg[8 * l + b] << (8 * b);
-    A[l] ^= v;
+#pragma unroll
+    for (int b = 0; b < 8; ++b) {
+      const int i = 8 * l + b, c = i - seed_len;
+      const u64 byte = i < seed_len ? seed[i] : c < 8 ? (counter >> (8 * c)) & 0xFF : c == 8 ? 0x1F : 0;
+      v |= byte << (8 * b);
+    }
+    A[l] = v;
   }
+  A[RATE_LANES - 1] ^= (u64)0x80 << 56;
   keccak_f1600(A);
 #pragma unroll
   for (int l = 0; l < RATE_LANES; ++l) out[l] = A[l];
@@ -187,6 +191,9 @@ __device__ inline long walk_mask(const u64* __restrict__ words, u64 avail, u64 p
   for (long c0 = 0; base < total; c0 += (long)WALK_THREADS * WALK_V) {
     const u64 at = pos + (u64)(c0 + (long)tid * WALK_V) * W.nb;
     const bool have = at + (u64)WALK_V * W.nb <= avail;
+    // The next chunk or, after the last, what the caller draws next.
+    if (lane % 2 == 0 && at + (u64)WALK_THREADS * WALK_V * W.nb < avail)
+      asm volatile("prefetch.global.L1 [%0];" ::"l"(words + ((at + (u64)WALK_THREADS * WALK_V * W.nb) >> 3)));
     u64 w[9];
     const int sh8 = 8 * (int)(at & 7);
 #pragma unroll
@@ -228,6 +235,19 @@ __device__ inline long walk_mask(const u64* __restrict__ words, u64 avail, u64 p
         acc |= (u32)((v[i] & W.mask[1]) < W.q[1]) << (8 + i);
       }
     }
+    // No candidate of the chunk rejected, by either limb (the paper preset's primes lie within
+    // 2^-12 of a power of two): candidate and draw index coincide.
+    const int s0 = W.nl == 2 ? base & 1 : 0;
+    if (__syncthreads_and((acc & (W.nl == 2 ? 0xFFFF : 0xFF)) == (W.nl == 2 ? 0xFFFF : 0xFF))) {
+#pragma unroll
+      for (int i = 0; i < WALK_V; ++i) {
+        const int d = base + tid * WALK_V + i, l = W.nl == 2 ? (s0 + i) & 1 : 0;
+        if (d < total) out[(size_t)l * n1 + (W.nl == 2 ? d >> 1 : d)] = v[i] & W.mask[l];
+      }
+      if (base + WALK_THREADS * WALK_V >= total) return c0 + (total - base);
+      base += WALK_THREADS * WALK_V;
+      continue;
+    }
     const u32 own = (u32)walk_count(acc, W.nl, 0) | ((u32)walk_count(acc, W.nl, 1) << 16);
     u32 incl = own;
 #pragma unroll
@@ -240,12 +260,15 @@ __device__ inline long walk_mask(const u64* __restrict__ words, u64 avail, u64 p
     __syncthreads();  // the previous chunk's readers are done with sh
     if (lane == 31) sh.warp_cnt[warp] = incl;
     __syncthreads();
-    u32 before = 0, all = 0;
-    for (int k = 0; k < WALK_THREADS / 32; ++k) {
-      if (k == warp) before = all;
-      all = walk_compose(all, sh.warp_cnt[k]);
+    // Every warp scans the warps' counts itself.
+    u32 wi = lane < WALK_THREADS / 32 ? sh.warp_cnt[lane] : 0;
+#pragma unroll
+    for (int d = 1; d < WALK_THREADS / 32; d <<= 1) {
+      const u32 o = __shfl_up_sync(0xffffffffu, wi, d);
+      if (lane >= d) wi = walk_compose(o, wi);
     }
-    const int s0 = W.nl == 2 ? base & 1 : 0;
+    const u32 all = __shfl_sync(0xffffffffu, wi, WALK_THREADS / 32 - 1);
+    const u32 before = warp ? __shfl_sync(0xffffffffu, wi, warp - 1) : 0;
     const auto from = [](u32 f, int s) { return (int)(s ? f >> 16 : f & 0xFFFF); };
     int d = base + from(walk_compose(before, excl), s0);
     const int d0 = d;
