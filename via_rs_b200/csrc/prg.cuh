@@ -137,7 +137,9 @@ __host__ __device__ inline void prg_block(const uint8_t* seed, int seed_len, u64
 // than `avail` bytes: the caller then takes the sequential path, which decides
 // it exactly.
 // ---------------------------------------------------------------------------
-constexpr int WALK_THREADS = 512;
+// 4608 candidates a chunk: a mask of 4096 draws and its few rejections in one (512 threads need
+// a second chunk for nearly every mask: 24 queries of 40 masks 261 us, 195 with 576).
+constexpr int WALK_THREADS = 576;
 constexpr int WALK_V = 8;
 constexpr long WALK_UNDECIDED = -1;
 
@@ -158,6 +160,7 @@ struct WalkShared {
   u32 warp_cnt[WALK_THREADS / 32];  // accepted from parity 0 | from parity 1 << 16
   long end;                         // candidates consumed once the last draw is accepted
   int undecided, total;
+  u64 draw[WALK_THREADS * WALK_V];  // a chunk's draws, on their way to coalesced stores
 };
 
 // Accepted candidates of `acc` (bit i: limb 0; bit 8 + i: limb 1) from parity s.
@@ -235,14 +238,24 @@ __device__ inline long walk_mask(const u64* __restrict__ words, u64 avail, u64 p
         acc |= (u32)((v[i] & W.mask[1]) < W.q[1]) << (8 + i);
       }
     }
-    // No candidate of the chunk rejected, by either limb (the paper preset's primes lie within
-    // 2^-12 of a power of two): candidate and draw index coincide.
+    // No rejected draw in the chunk (six masks of ten with the paper preset's primes, 2^-20 and
+    // 2^-12 short of a power of two): candidate and draw index coincide.
     const int s0 = W.nl == 2 ? base & 1 : 0;
-    if (__syncthreads_and((acc & (W.nl == 2 ? 0xFFFF : 0xFF)) == (W.nl == 2 ? 0xFFFF : 0xFF))) {
+    u32 need = 0;  // the thread's candidates that are draws then
+#pragma unroll
+    for (int i = 0; i < WALK_V; ++i)
+      if (base + tid * WALK_V + i < total) need |= 1u << (i + (W.nl == 2 ? 8 * ((s0 + i) & 1) : 0));
+    if (__syncthreads_and((acc & need) == need)) {
+      // Through shared memory, so that a warp's stores are consecutive (a thread's own eight
+      // draws would be 32 bytes apart from its neighbour's).
+      const auto slot = [](int x) { return x ^ ((x >> 4) & 15); };
+#pragma unroll
+      for (int i = 0; i < WALK_V; ++i) sh.draw[slot(tid * WALK_V + i)] = v[i] & W.mask[W.nl == 2 ? (s0 + i) & 1 : 0];
+      __syncthreads();
 #pragma unroll
       for (int i = 0; i < WALK_V; ++i) {
-        const int d = base + tid * WALK_V + i, l = W.nl == 2 ? (s0 + i) & 1 : 0;
-        if (d < total) out[(size_t)l * n1 + (W.nl == 2 ? d >> 1 : d)] = v[i] & W.mask[l];
+        const int x = i * WALK_THREADS + tid, d = base + x, l = W.nl == 2 ? d & 1 : 0;
+        if (d < total) out[(size_t)l * n1 + (W.nl == 2 ? d >> 1 : d)] = sh.draw[slot(x)];
       }
       if (base + WALK_THREADS * WALK_V >= total) return c0 + (total - base);
       base += WALK_THREADS * WALK_V;

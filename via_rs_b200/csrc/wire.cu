@@ -46,10 +46,9 @@ struct Sampler {
 
 // The mask and the body of one compressed packet per CTA: LWE lwe[pkt] of `query`
 // ([nl][n1] limb-major, then nl body residues). err: 2 where walk_mask could not
-// decide. Latency-bound: a chunk of 4096 candidates is one pass of the paper
-// preset's mask, four of the secure preset's. Against one thread walking each
-// stream (k_prg_masks): 3412 us before, see WALK figures below, for 42 packets
-// of the paper preset.
+// decide. Latency-bound: a chunk of 4608 candidates is one pass of the paper
+// preset's mask, several of the secure preset's. Against one thread walking each
+// stream (k_prg_masks): 40 packets of the paper preset 3412 us there, 6.5 here.
 __global__ void __launch_bounds__(WALK_THREADS) k_prg_masks_scan(const u64* __restrict__ blocks,
                                                                  const u64* __restrict__ bodies,
                                                                  const int* __restrict__ lwe, int nblk, int n1,
