@@ -476,7 +476,7 @@ __global__ void k_mod_switch(const u64* __restrict__ in, DevRing S, u64* __restr
 // The same from a two-prime ring in double precision: round(c q_dst / Q) is fp_scaled2's value
 // with q_dst for S, an integer within 1.2 q_dst of zero. Two coefficients a
 // thread. Bound by its 24 bytes a coefficient: the 67 million coefficients of 64 queries'
-// rows 830 us with 128-bit divisions, MOD_SWITCH_FIGURES
+// rows 830 us with 128-bit divisions, 251 here
 __global__ void __launch_bounds__(256) k_mod_switch_fp(const u64* __restrict__ in, const __grid_constant__ DevRing S,
                                                        const __grid_constant__ Gadget g, u64* __restrict__ out,
                                                        double q, long ncoef, int n) {
@@ -777,6 +777,60 @@ __global__ void k_pack_rlwe(const u64* masks, const u64* body, const u64* __rest
     b = submod(b, reduce64(gemm[(long)(((2 << k) - 2 + (i >> (K - 1 - k))) * 2 + l) * stride + w], m), m.q);
   }
   out[(2 * w + 1) * per + rem] = b;
+}
+
+// The cascade's RLWEs [lwe][2][nl][n1] in one kernel for double-precision rings (both primes
+// below 2^40): per CTA (LWE, limb) the eval-form body of k_cascade_body_final, its inverse
+// transform, the GEMM steps' sums of k_pack_rlwe, and the mask. Arguments as theirs; the GEMM
+// steps' sums are loaded by one thread a coefficient that has any, all loads at once, while the
+// transform has its own to wait for (one after the other in the epilogue 338 us of the 360 below
+// stayed). 2688 LWEs of degree 2048 in 2 launches 360 us as three kernels (eval body, transform,
+// assembly), 155 here, which is memory: 64 KB in and 64 KB out an LWE at 2.3 TB/s; 60 LWEs 27 us
+// before, 16 here; 8 LWEs 15 and 9.5.
+template <int LOGN>
+__global__ void __launch_bounds__((1 << LOGN) / 8)
+    k_cascade_rlwe_fp(const u64* __restrict__ masks, const u64* __restrict__ b0, long b0_stride,
+                      const u64* __restrict__ bsk, const u64* __restrict__ gemm, long stride, int k0,
+                      u64* __restrict__ out, const __grid_constant__ DevRing R) {
+  constexpr int n = 1 << LOGN, K = LOGN;
+  using L0 = NttPhase<LOGN, false, 0>;
+  __shared__ double ssm[n];
+  __shared__ u64 gsum[1 << 8];  // the GEMM steps' sums at the coefficients x << (K - k0)
+  const int tid = threadIdx.x, nl = R.nl, l = blockIdx.y;
+  const long w = blockIdx.x, per = (long)nl * n;
+  const NttTable& T = R.t[l];
+  const double q = T.qd, qinv = T.qinv;
+  const DevMod& m = R.m[l];
+  if (tid < (1 << k0)) {  // at most 8 sums below 2^49 each, all loads at once
+    u64 s = 0;
+#pragma unroll
+    for (int k = 0; k < 8; ++k)
+      if (k < k0 && (tid & ((1 << (k0 - 1 - k)) - 1)) == 0)
+        s += gemm[(long)(((2 << k) - 2 + (tid >> (k0 - 1 - k))) * 2 + l) * stride + w];
+    gsum[tid] = reduce64(s, m);
+  }
+  const u64* sk = bsk + (w * nl + l) * 2 * n;
+  const double b = fp_from_u64(b0[w * b0_stride + l]);
+  double e[8];
+#pragma unroll
+  for (int v = 0; v < 8; ++v) e[v] = 0.0;
+#pragma unroll 4
+  for (int k = k0; k < K; ++k) {  // sums of at most 2^4 canonical terms each, below 2^44
+    const u64* s = sk + (2 << k) - 2;
+#pragma unroll
+    for (int v = 0; v < 8; ++v) e[v] = __dadd_rn(e[v], fp_from_u64(s[(8 * tid + v) >> (K - 1 - k)]));
+  }
+#pragma unroll
+  for (int v = 0; v < 8; ++v) e[v] = fp_reduce(__dadd_rn(b, -e[v]), q, qinv);
+  fp_inverse<LOGN>(e, tid, T, ssm);  // its CTA barrier also publishes gsum
+#pragma unroll
+  for (int v = 0; v < 8; ++v) {
+    const int x = L0::index(v, tid);
+    u64 c = fp_to_u64(fp_canonical(fp_mulmod(e[v], T.ninv_d[LOGN], q, qinv), q, qinv));
+    if (k0 && (x & ((1 << (K - k0)) - 1)) == 0) c = submod(c, gsum[x >> (K - k0)], m.q);
+    out[(2 * w + 1) * per + (long)l * n + x] = c;
+    out[(2 * w) * per + (long)l * n + x] = masks[w * per + (long)l * n + x];
+  }
 }
 
 // rlwe_to_rgsw assembly (prim/gates/convert.rs:162-178): for bit b, level i:
@@ -1233,16 +1287,29 @@ static void query_decomp_range(Server& s, Workspace& w, const u64* d_query, long
     std::swap(mi, mo);
     std::swap(bi, bo);
   }
-  if (R.ntt) {  // the cascade's body, from the LWE bodies in bi and every step's sums
-    k_cascade_body_final<<<blocks(nlwe * nl * n1), 256, 0, st>>>(k0 ? query + (long)nl * n1 : bi,
-                                                                 k0 ? (long)lwe_len(p) : nl, bsk, k0, k, nl, nlwe, R, bo);
+  // The cascade's body, from the LWE bodies and every step's sums.
+  const u64* lwe_body = k0 ? query + (long)nl * n1 : bi;
+  const long body_stride = k0 ? (long)lwe_len(p) : nl;
+  const bool small_primes = R.ntt && R.m[0].q < (1ull << 40) && R.m[1].q < (1ull << 40) && k0 <= 8;
+  if (small_primes && (n1 == 2048 || n1 == 4096)) {
+    const dim3 grid((unsigned)nlwe, (unsigned)nl);
+    const u64* gemm = w.c_gemm_body.p + lwe0;
+    if (n1 == 2048)
+      k_cascade_rlwe_fp<11><<<grid, 256, 0, st>>>(mi, lwe_body, body_stride, bsk, gemm, nlwe_all, k0, rlwe, R);
+    else
+      k_cascade_rlwe_fp<12><<<grid, 512, 0, st>>>(mi, lwe_body, body_stride, bsk, gemm, nlwe_all, k0, rlwe, R);
     VIA_LAUNCHED();
-    from_eval(R, bo, n1, nlwe * nl, st);
-    std::swap(bi, bo);
+  } else {
+    if (R.ntt) {
+      k_cascade_body_final<<<blocks(nlwe * nl * n1), 256, 0, st>>>(lwe_body, body_stride, bsk, k0, k, nl, nlwe, R, bo);
+      VIA_LAUNCHED();
+      from_eval(R, bo, n1, nlwe * nl, st);
+      std::swap(bi, bo);
+    }
+    k_pack_rlwe<<<blocks(nlwe * nl * n1), 256, 0, st>>>(mi, bi, w.c_gemm_body.p + lwe0, nlwe_all, k0, k, nlwe, n1, nl, R,
+                                                        rlwe);
+    VIA_LAUNCHED();
   }
-  k_pack_rlwe<<<blocks(nlwe * nl * n1), 256, 0, st>>>(mi, bi, w.c_gemm_body.p + lwe0, nlwe_all, k0, k, nlwe, n1, nl, R,
-                                                      rlwe);
-  VIA_LAUNCHED();
   // RLWE -> RGSW with the conversion key (prim/gates/convert.rs:162-178); the
   // final rank-1 masks are already contiguous [lwe][nl][n1] in `mi`.
   u64* gp = w.g_gp.p + lwe0 * 2 * lwe_n;
