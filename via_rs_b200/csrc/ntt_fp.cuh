@@ -56,7 +56,8 @@ __device__ __forceinline__ double fp_reduce(double x, double q, double qinv) {
   return __fma_rn(-__dadd_rn(__fma_rn(x, qinv, FP_ROUND), -FP_ROUND), q, x);
 }
 
-// Eight consecutive words of a thread, as two 32-byte accesses.
+// Eight consecutive words of a thread, as two 32-byte accesses. Keys (ld8_nc) stay in L1
+// before anything else.
 __device__ __forceinline__ void ld8(const u64* p, u64 (&x)[8]) {
 #pragma unroll
   for (int h = 0; h < 2; ++h)
@@ -64,10 +65,18 @@ __device__ __forceinline__ void ld8(const u64* p, u64 (&x)[8]) {
                  : "=l"(x[4 * h]), "=l"(x[4 * h + 1]), "=l"(x[4 * h + 2]), "=l"(x[4 * h + 3])
                  : "l"(p + 4 * h));
 }
+// Read (or written) once: not worth a line of L1 where keys want it.
+__device__ __forceinline__ void ld8_stream(const u64* p, u64 (&x)[8]) {
+#pragma unroll
+  for (int h = 0; h < 2; ++h)
+    asm volatile("ld.global.L1::no_allocate.v4.u64 {%0, %1, %2, %3}, [%4];"
+                 : "=l"(x[4 * h]), "=l"(x[4 * h + 1]), "=l"(x[4 * h + 2]), "=l"(x[4 * h + 3])
+                 : "l"(p + 4 * h));
+}
 __device__ __forceinline__ void ld8_nc(const u64* p, u64 (&x)[8]) {
 #pragma unroll
   for (int h = 0; h < 2; ++h)
-    asm("ld.global.nc.v4.u64 {%0, %1, %2, %3}, [%4];"
+    asm("ld.global.nc.L1::evict_last.v4.u64 {%0, %1, %2, %3}, [%4];"
         : "=l"(x[4 * h]), "=l"(x[4 * h + 1]), "=l"(x[4 * h + 2]), "=l"(x[4 * h + 3])
         : "l"(p + 4 * h));
 }
@@ -75,6 +84,14 @@ __device__ __forceinline__ void st8(u64* p, const u64 (&x)[8]) {
 #pragma unroll
   for (int h = 0; h < 2; ++h)
     asm volatile("st.global.v4.u64 [%0], {%1, %2, %3, %4};" ::"l"(p + 4 * h), "l"(x[4 * h]), "l"(x[4 * h + 1]),
+                 "l"(x[4 * h + 2]), "l"(x[4 * h + 3])
+                 : "memory");
+}
+
+__device__ __forceinline__ void st8_stream(u64* p, const u64 (&x)[8]) {
+#pragma unroll
+  for (int h = 0; h < 2; ++h)
+    asm volatile("st.global.L1::no_allocate.v4.u64 [%0], {%1, %2, %3, %4};" ::"l"(p + 4 * h), "l"(x[4 * h]), "l"(x[4 * h + 1]),
                  "l"(x[4 * h + 2]), "l"(x[4 * h + 3])
                  : "memory");
 }
@@ -182,6 +199,8 @@ __device__ __forceinline__ void fp_digit_phase(double (&e)[8], const NttTable& T
     e[2 * i + 1] = __dadd_rn(ev[i], -o);
   }
 }
+
+__device__ __forceinline__ void fp_prefetch(const u64* p) { asm volatile("prefetch.global.L1 [%0];" ::"l"(p)); }
 
 template <int SPAN>
 __device__ __forceinline__ void fp_sync() {

@@ -1359,12 +1359,15 @@ static void external_products(const DevRing& R, const Gadget& g, KeySel rgsw, co
 // within 0.5625 q, so the 2L products and the input residue sum to less than
 // (1 + 1.125 L) q before the final reduction.
 //
-// FP64-issue bound (about 2800 operations a thread, 2 CTAs of 8 warps an SM; 60% of the pipe).
+// FP64-issue bound (about 2800 operations a thread, 2 CTAs of 8 warps an SM; 63% of the pipe).
 // At n = 2048 the first exchange of a forward transform and the last of an inverse cross
 // warps, the other two stay within one, and the inverse ends in the layout the forward
 // starts in; transforms run two at a time (mask and body, then a half's two digits). 65536
 // CMuxes 6.58 ms with single transforms, two barriers on every exchange and integer digit
-// splits, 4.31 ms with one transform at a time, 4.08 ms; 128 CMuxes (one a SM) 25, 20, 16 us.
+// splits, 4.31 ms with one transform at a time, 4.08 ms with keys and inputs competing for L1,
+// 3.89 ms with the inputs (read once) kept out of it, the keys (128 KB a selector, shared by
+// neighbouring CTAs) held there and fetched into it while the digits are transformed; the
+// tiled level of 131072 9.05 and 8.28 ms; 128 CMuxes (one a SM) 25, 20, 16.4 and 14.0 us.
 //
 // TILED (the first level): cur holds fd_scan's tiled columns of nq queries, where a pair's
 // four residues of a slot are 32 consecutive bytes; in[2o] waits in shared memory.
@@ -1394,7 +1397,7 @@ __global__ void __launch_bounds__((1 << LOGN) / 8, LOGN >= 12 ? 1 : 2) k_cmux_fp
 #pragma unroll
     for (int v = 0; v < 8; ++v) {
       u64 x[4];  // in[2o] mask, body, in[2o+1] mask, body of slot 8 tid + v
-      asm volatile("ld.global.v4.u64 {%0, %1, %2, %3}, [%4];"
+      asm volatile("ld.global.L1::no_allocate.v4.u64 {%0, %1, %2, %3}, [%4];"
                    : "=l"(x[0]), "=l"(x[1]), "=l"(x[2]), "=l"(x[3])
                    : "l"(in + v * tstep));
       const double m = fp_from_u64(x[0]), b = fp_from_u64(x[1]);
@@ -1407,8 +1410,8 @@ __global__ void __launch_bounds__((1 << LOGN) / 8, LOGN >= 12 ? 1 : 2) k_cmux_fp
 #pragma unroll
     for (int p = 0; p < 2; ++p) {
       u64 x[8], y[8];
-      ld8(in + 2 * n + p * n + 8 * tid, x);
-      ld8(in + p * n + 8 * tid, y);
+      ld8_stream(in + 2 * n + p * n + 8 * tid, x);
+      ld8_stream(in + p * n + 8 * tid, y);
 #pragma unroll
       for (int v = 0; v < 8; ++v) val[p][v] = __dadd_rn(fp_from_u64(x[v]), -fp_from_u64(y[v]));
     }
@@ -1432,6 +1435,12 @@ __global__ void __launch_bounds__((1 << LOGN) / 8, LOGN >= 12 ? 1 : 2) k_cmux_fp
         e[0][v] = fp_next_digit(val[0][v], g);
         e[1][v] = fp_next_digit(val[0][v], g);
       }
+#pragma unroll
+      for (int i = 0; i < 2; ++i)  // the products' keys
+#pragma unroll
+        for (int part = 0; part < 2; ++part)
+          if (k + i < L)
+            fp_prefetch(K + (long)(2 * (p * L + L - 1 - k - i) + part) * n + 8 * tid);
       __syncthreads();  // the previous transforms' reads
       fp_forward_digits2<LOGN>(e, tid, T, pair_sm, dense);
 #pragma unroll
@@ -1453,13 +1462,13 @@ __global__ void __launch_bounds__((1 << LOGN) / 8, LOGN >= 12 ? 1 : 2) k_cmux_fp
 #pragma unroll
   for (int part = 0; part < 2; ++part) {
     u64 x[8];
-    if (!TILED) ld8(in + part * n + 8 * tid, x);
+    if (!TILED) ld8_stream(in + part * n + 8 * tid, x);
 #pragma unroll
     for (int v = 0; v < 8; ++v) {
       const double y = TILED ? keep[part * n + v * (n / 8) + tid] : fp_from_u64(x[v]);
       x[v] = fp_to_u64(fp_canonical(__dadd_rn(y, a[part][v]), q, qinv));
     }
-    st8(nxt + o * 2 * n + part * n + 8 * tid, x);
+    st8_stream(nxt + o * 2 * n + part * n + 8 * tid, x);
   }
 }
 
