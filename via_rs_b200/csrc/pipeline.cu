@@ -1216,7 +1216,37 @@ static void query_decomp_range(Server& s, Workspace& w, const u64* d_query, long
     k_lwe_to_mlwe<<<blocks(nlwe * nl * (n1 + 1)), 256, 0, st>>>(query, n1, nl, nlwe, mi, bi);
     VIA_LAUNCHED();
   }
-  if (R.ntt) VIA_CUDA(cudaMemsetAsync(bsk, 0, (size_t)nlwe * 2 * lwe_n * 8, st));
+  // Eval rings: how a step of input degree n_in spreads over the grid.
+  const bool fp_mac = dig8 && s.cascade_eval_d.p;
+  struct Split {
+    int NS, NL, tt, JB;
+    long slots, lwes;
+  };
+  const auto split = [&](int n_in) {
+    const int n_out = 2 * n_in, rank_in = n1 / n_in;
+    // fp: two output slots a thread from three blocks a SM on (with one: 60 LWEs 26 us a
+    // step against 21, 18 LWEs 8.3 against 10.2), two LWEs as well from sixteen on.
+    const long full = (long)n1 * nl * nlwe / 256;  // blocks with one slot and LWE a thread
+    Split d;
+    d.NS = fp_mac && n_in > 1 && full >= 3 * 148 ? 2 : 1;
+    d.NL = d.NS == 2 && full >= 16 * 148 ? 2 : 1;
+    const int jj = std::min(rank_in / 2, 8);
+    d.tt = std::min(n_out / d.NS, 256 / jj);
+    d.slots = n_out / d.NS / d.tt;
+    // Split the output masks over JB blocks while the grid is below ~4 blocks
+    // per SM and every block keeps at least one mask per thread row.
+    d.lwes = (nlwe + d.NL - 1) / d.NL;
+    const long base = d.slots * nl * d.lwes;
+    const int rows = 256 / d.tt, iters = (rank_in / 2 + rows - 1) / rows;
+    d.JB = 1;
+    while (d.JB * 2 <= iters && base * d.JB * 2 <= CASCADE_SPLIT_BLOCKS) d.JB *= 2;
+    return d;
+  };
+  // Blocks that share a step's body sums add to them; a step of one block a sum stores it (the
+  // 134 MB of 2048 LWEs 315 us to clear).
+  bool shared_sums = false;
+  for (int n_in = 1 << k0; R.ntt && n_in < n1; n_in <<= 1) shared_sums |= split(n_in).JB > 1;
+  if (shared_sums) VIA_CUDA(cudaMemsetAsync(bsk, 0, (size_t)nlwe * 2 * lwe_n * 8, st));
   const u64 step_len = (u64)2 * n1 * L * 2 * nl;
   int k = k0;
   for (int n_in = 1 << k0; n_in < n1; n_in <<= 1, ++k) {
@@ -1224,7 +1254,6 @@ static void query_decomp_range(Server& s, Workspace& w, const u64* d_query, long
     const long polys = nlwe * rank_in;
     if (R.ntt) {
       // Digits at the input degree; see k_cascade_mac for the repeated slots.
-      const bool fp_mac = dig8 && s.cascade_eval_d.p;
       if (dig8 && (n_in > 1 || fp_mac)) {
         if (k != k0 || k0 == 0) {  // the last GEMM step left its successor's digits in dig8
           decompose_i8(R, w.g_ck, mi, n_in, polys, dig8, st);
@@ -1239,29 +1268,19 @@ static void query_decomp_range(Server& s, Workspace& w, const u64* d_query, long
         decompose(R, w.g_ck, mi, n_in, 1, polys, digits, st);
         if (n_in > 1) digits_to_eval(R, digits, n_in, polys * L * nl, st);
       }
-      // fp: two output slots a thread from three blocks a SM on (with one: 60 LWEs 26 us a
-      // step against 21, 18 LWEs 8.3 against 10.2), two LWEs as well from sixteen on.
-      const long full = (long)n1 * nl * nlwe / 256;  // blocks with one slot and LWE a thread
-      const int NS = fp_mac && n_in > 1 && full >= 3 * 148 ? 2 : 1, NL = NS == 2 && full >= 16 * 148 ? 2 : 1;
-      const int jj = std::min(rank_in / 2, 8), tt = std::min(n_out / NS, 256 / jj);
-      const long slots = n_out / NS / tt;
-      // Split the output masks over JB blocks while the grid is below ~4 blocks
-      // per SM and every block keeps at least one mask per thread row.
-      const long lwes = (nlwe + NL - 1) / NL, base = slots * nl * lwes;
-      const int rows = 256 / tt, iters = (rank_in / 2 + rows - 1) / rows;
-      int JB = 1;
-      while (JB * 2 <= iters && base * JB * 2 <= CASCADE_SPLIT_BLOCKS) JB *= 2;
-      dim3 grid((unsigned)(slots * JB), (unsigned)nl, (unsigned)lwes);
+      const Split d = split(n_in);
+      const int tt = d.tt, JB = d.JB;
+      dim3 grid((unsigned)(d.slots * JB), (unsigned)nl, (unsigned)d.lwes);
       u64* bsk_k = bsk + (n_out - 2);  // this step's region
       const double* kd = reinterpret_cast<const double*>(s.cascade_eval_d.p) + k * step_len;
       const double* dd = reinterpret_cast<const double*>(digits);
       if (fp_mac && n_in == 1)
         k_cascade_mac_fp<true, 1, 1><<<grid, 256, 0, st>>>(nullptr, dig8, kd, rank_in, n_in, L, tt, JB, nlwe, R, mo, bsk_k,
                                                         2L * n1);
-      else if (NL == 2)
+      else if (d.NL == 2)
         k_cascade_mac_fp<false, 2, 2><<<grid, 256, 0, st>>>(dd, dig8, kd, rank_in, n_in, L, tt, JB, nlwe, R, mo, bsk_k,
                                                          2L * n1);
-      else if (NS == 2)
+      else if (d.NS == 2)
         k_cascade_mac_fp<false, 1, 2><<<grid, 256, 0, st>>>(dd, dig8, kd, rank_in, n_in, L, tt, JB, nlwe, R, mo, bsk_k,
                                                             2L * n1);
       else if (fp_mac)
