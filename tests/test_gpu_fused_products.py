@@ -1,11 +1,13 @@
 """The fused gadget products (shared key, and RGSWs of their own) against the oracle over the ring
-degrees they are instantiated for and the ones just outside, with the counts at the line between
-six CTAs a polynomial and one; outputs in place of an input take the general path."""
+degrees they are instantiated for and the ones just outside, with the counts at the line to
+separate kernels (512 CTAs); outputs in place of an input take the general path. DMux trees
+whose levels lie on both sides of the line between a cluster a product and one CTA."""
 import numpy as np
 import pytest
 
 from via_rs_b200 import prims
-from via_rs_b200.params import PAPER_Q1, PAPER_Q2, SECURE_Q1
+from via_rs_b200.params import PAPER_Q1, PAPER_Q2, SECURE_Q1, paper_preset, secure_preset
+from via_rs_b200.server import PublicKeys, Server
 
 pytestmark = pytest.mark.gpu
 
@@ -39,8 +41,8 @@ def test_external_products(oracle, q, n, base, L, in_place):
 
 
 @pytest.mark.parametrize("q,n,count", [(PAPER_Q1, 128, 3), (PAPER_Q1, 256, 3), (PAPER_Q1, 512, 3), (PAPER_Q1, 1024, 3),
-                                       (PAPER_Q1, 2048, 37), (PAPER_Q1, 2048, 38), (SECURE_Q1, 4096, 2),
-                                       (SECURE_Q1, 4096, 38)])
+                                       (PAPER_Q1, 2048, 255), (PAPER_Q1, 2048, 256), (SECURE_Q1, 4096, 2),
+                                       (SECURE_Q1, 4096, 256)])
 def test_key_switches(oracle, q, n, count):
     import torch
 
@@ -56,3 +58,14 @@ def test_key_switches(oracle, q, n, count):
                          out.data_ptr())
     want = oracle.key_switch(q, n, base, L, key.reshape(-1), ct.reshape(-1), shifts)
     assert np.array_equal(out.cpu().numpy().view(np.uint64).reshape(-1), want)
+
+
+@pytest.mark.parametrize("preset,rows", [("paper", 128), ("secure", 64)])
+def test_dmux_levels(oracle, preset, rows):
+    prm = {"paper": paper_preset, "secure": secure_preset}[preset](rows, 2)
+    c = oracle.Client(prm, b"dmux-levels")
+    recs = np.random.default_rng(7).integers(0, 16, size=(prm.capacity, prm.n_rec), dtype=np.uint64)
+    gpu = Server.setup(prm, PublicKeys(c.cascade_key, c.conv_key, c.rsk), recs)
+    cpu = oracle.Server(prm, c.cascade_key, c.conv_key, c.rsk, recs)
+    q = c.query(prm.capacity - 1, b"q")
+    assert np.array_equal(gpu.debug_stage(q, 3), cpu.debug_stage(q, 3))

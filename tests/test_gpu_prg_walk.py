@@ -16,8 +16,8 @@ from via_rs_b200.wire import from_wire, prg_packet
 pytestmark = pytest.mark.gpu
 
 PRESETS = {
-    "paper": lambda: paper_preset(1, 4),  # 4096 candidates: one chunk
-    "secure": lambda: secure_preset(1, 2),  # acceptance 0.63: four chunks
+    "paper": lambda: paper_preset(1, 4),  # 4096 draws: one chunk
+    "secure": lambda: secure_preset(1, 2),  # acceptance 0.63: several chunks
     "toy": lambda: toy_preset(1, 2),  # one limb, acceptance 0.5, 64 draws
     "n8": lambda: n8_preset(1, 2),  # 8 draws
 }

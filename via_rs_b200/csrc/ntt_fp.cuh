@@ -200,6 +200,13 @@ __device__ __forceinline__ void fp_digit_phase(double (&e)[8], const NttTable& T
   }
 }
 
+// Both twiddle tables of degree 2^LOGN into L1, a line a thread of 2^LOGN / 8: kernels of one
+// or two transforms would otherwise wait for L2 in every phase.
+template <int LOGN>
+__device__ __forceinline__ void fp_prefetch_twiddles(int tid, const NttTable& T) {
+  const double* t = tid < (1 << LOGN) / 16 ? T.psi_d + 16 * tid : T.ipsi_d + 16 * (tid - (1 << LOGN) / 16);
+  asm volatile("prefetch.global.L1 [%0];" ::"l"(t));
+}
 __device__ __forceinline__ void fp_prefetch(const u64* p) { asm volatile("prefetch.global.L1 [%0];" ::"l"(p)); }
 
 template <int SPAN>

@@ -801,6 +801,7 @@ __global__ void __launch_bounds__((1 << LOGN) / 8)
   const NttTable& T = R.t[l];
   const double q = T.qd, qinv = T.qinv;
   const DevMod& m = R.m[l];
+  fp_prefetch_twiddles<LOGN>(tid, T);
   if (tid < (1 << k0)) {  // at most 8 sums below 2^49 each, all loads at once
     u64 s = 0;
 #pragma unroll
@@ -980,8 +981,10 @@ static bool cmux_fused_ok(const DevRing& R, const Gadget& g);
 
 // Levels of at most this many CMuxes run on four-CTA clusters (cmux_fused).
 constexpr long CMUX_CLUSTER_MAX = 64;
-// DMux levels of at most this many products run on a cluster per product and limb.
-constexpr long EXT_CLUSTER_MAX = 16;
+// DMux levels of at most this many coefficients (products x degree) run on a cluster per product
+// and limb: 32 products of degree 2048 16.1 us against 20.1 us for one CTA each, 32 of degree
+// 4096, whose CTAs fill an SM, 33.0 against 30.2.
+constexpr long EXT_CLUSTER_MAX = 65536;
 
 // Whether the scan of nq queries writes tiled columns, which the CMux tree's first level
 // gathers: answers with the fused CMux and a first level of single-CTA CMuxes.
@@ -1505,22 +1508,26 @@ static size_t pair_smem(K kernel, size_t doubles) {
 // time. CTA r of the cluster takes input half p = r & 1 (mask or body),
 // inverse-transforms its difference, and forward-transforms its digit k = r >> 1;
 // its products with the sample's mask and body (sample p L + L - 1 - k) are
-// reduced mod q into its shared memory. After a cluster barrier, ranks 0 and 1
-// add in[2o] and the four partial masks / bodies, read over distributed shared
-// memory; a second barrier keeps every CTA's shared memory alive until those
-// reads are done. Two transforms per CTA instead of six for one CTA. L = 2 and
-// n <= 2048 (48 KB of static shared memory).
+// reduced mod q into its shared memory. After a cluster barrier, each rank
+// adds in[2o] and the four partials of its half of the mask or body, read over
+// distributed shared memory; a second barrier keeps every CTA's shared memory
+// alive until those reads are done. Two transforms per CTA instead of six for
+// one CTA. L = 2.
 // In double precision with the bounds of k_cmux_fp: each CTA's products are
-// signed residues within 0.5625 q, kept as doubles in shared memory; ranks 0
-// and 1 add the four partials to in[2o] and reduce once.
+// signed residues within 0.5625 q, kept as doubles in shared memory.
+// Latency-bound: an L2 wait for keys and twiddles in every phase until they are fetched into
+// L1 with the inputs, and the final sums from conflict-free partials by all four ranks (two
+// ranks, eight dependent rounds each, before): a CMux of degree 2048 8.5 us, 7.0 here, 64 of
+// them 13.6 and 10.7; of degree 4096 23.4 us as one CTA, 11.5 here, 64 22.9 both ways.
 template <int LOGN>
-__global__ void __cluster_dims__(4, 1, 1) __launch_bounds__((1 << LOGN) / 8, 2)
+__global__ void __cluster_dims__(4, 1, 1) __launch_bounds__((1 << LOGN) / 8, LOGN >= 12 ? 1 : 2)
     k_cmux_cluster_fp(const u64* __restrict__ cur, u64* __restrict__ nxt, KeySel ks, const __grid_constant__ DevRing R,
                       const __grid_constant__ Gadget g) {
   namespace cg = cooperative_groups;
   constexpr int n = 1 << LOGN;
-  __shared__ double ssm[n];    // the inverse's exchanges, then the mask partial
-  __shared__ double pbody[n];  // the forward's exchanges, then the body partial
+  extern __shared__ __align__(16) double cmux_sm[];
+  double* ssm = cmux_sm;        // the inverse's exchanges, then the mask partial
+  double* pbody = cmux_sm + n;  // the forward's exchanges, then the body partial
   cg::cluster_group cluster = cg::this_cluster();
   const int r = (int)cluster.block_rank();
   const int p = r & 1, k = r >> 1;
@@ -1529,13 +1536,17 @@ __global__ void __cluster_dims__(4, 1, 1) __launch_bounds__((1 << LOGN) / 8, 2)
   const NttTable& T = R.t[0];
   const double q = T.qd, qinv = T.qinv;
   const u64* a = cur + (2 * o) * 2 * n;
-  const u64* K = ks.base + ((o / ks.div) % ks.mod) * ks.stride;
+  const int smp = p * 2 + 1 - k;  // sample L - 1 - k of half p (L = 2)
+  const u64* K = ks.base + ((o / ks.div) % ks.mod) * ks.stride + (long)(2 * smp) * n + 8 * tid;
   const bool dense = 4.0 * g.dB * q < 281474976710656.0;
   double e[8];
   {
     u64 x[8], y[8];
     ld8(a + 2 * n + p * n + 8 * tid, x);
     ld8(a + p * n + 8 * tid, y);
+    fp_prefetch_twiddles<LOGN>(tid, T);
+    fp_prefetch(K);
+    fp_prefetch(K + n);
 #pragma unroll
     for (int v = 0; v < 8; ++v) e[v] = __dadd_rn(fp_from_u64(x[v]), -fp_from_u64(y[v]));
   }
@@ -1547,31 +1558,33 @@ __global__ void __cluster_dims__(4, 1, 1) __launch_bounds__((1 << LOGN) / 8, 2)
     if (k) e[v] = fp_next_digit(val, g);
   }
   fp_forward_digits<LOGN>(e, tid, T, pbody, 0, dense);
-  const int smp = p * 2 + 1 - k;  // sample L - 1 - k of half p (L = 2)
   u64 km[8], kb[8];
-  ld8_nc(K + (long)(2 * smp) * n + 8 * tid, km);
-  ld8_nc(K + (long)(2 * smp + 1) * n + 8 * tid, kb);
-  // The warp's lanes are done with their part of pbody; every thread left ssm before the
-  // forward transform's CTA barrier.
-  __syncwarp();
+  ld8_nc(K, km);
+  ld8_nc(K + n, kb);
+  __syncthreads();  // the exchanges; the partials' layout (slot 8 tid + v at v n / 8 + tid) crosses warps
 #pragma unroll
   for (int v = 0; v < 8; ++v) {
-    ssm[8 * tid + v] = fp_mulmod(e[v], fp_from_u64(km[v]), q, qinv);
-    pbody[8 * tid + v] = fp_mulmod(e[v], fp_from_u64(kb[v]), q, qinv);
+    ssm[v * (n / 8) + tid] = fp_mulmod(e[v], fp_from_u64(km[v]), q, qinv);
+    pbody[v * (n / 8) + tid] = fp_mulmod(e[v], fp_from_u64(kb[v]), q, qinv);
   }
   cluster.sync();
-  if (r < 2) {  // rank 0: the output mask, rank 1: the output body
-    double* parts[4];
+  // Ranks 0 and 2 the output mask, 1 and 3 the body; four of a thread's eight slots each.
+  const long at = p * n + 8 * tid + 4 * k;
+  u64 x[4];
+  asm volatile("ld.global.v4.u64 {%0, %1, %2, %3}, [%4];" : "=l"(x[0]), "=l"(x[1]), "=l"(x[2]), "=l"(x[3]) : "l"(a + at));
 #pragma unroll
-    for (int rr = 0; rr < 4; ++rr) parts[rr] = cluster.map_shared_rank(r == 0 ? ssm : pbody, rr);
-    u64* out = nxt + o * 2 * n + (long)r * n;
-    for (int x = tid; x < n; x += blockDim.x) {
-      double acc = __ull2double_rn(a[(long)r * n + x]);
+  for (int v = 0; v < 4; ++v) e[v] = fp_from_u64(x[v]);
 #pragma unroll
-      for (int rr = 0; rr < 4; ++rr) acc = __dadd_rn(acc, parts[rr][x]);
-      out[x] = __double2ull_rn(fp_canonical(acc, q, qinv));
-    }
+  for (int y = 0; y < 4; ++y) {
+    const double* part = cluster.map_shared_rank(p ? pbody : ssm, (r + y) & 3) + 4 * k * (n / 8) + tid;
+#pragma unroll
+    for (int v = 0; v < 4; ++v) e[v] = __dadd_rn(e[v], part[v * (n / 8)]);
   }
+#pragma unroll
+  for (int v = 0; v < 4; ++v) x[v] = fp_to_u64(fp_canonical(e[v], q, qinv));
+  asm volatile("st.global.v4.u64 [%0], {%1, %2, %3, %4};" ::"l"(nxt + o * 2 * n + at), "l"(x[0]), "l"(x[1]), "l"(x[2]),
+               "l"(x[3])
+               : "memory");
   cluster.sync();
 }
 
@@ -1587,7 +1600,9 @@ __global__ void __cluster_dims__(4, 1, 1) __launch_bounds__((1 << LOGN) / 8, 2)
 //             rotate.rs:128-150)
 // in [ct][2][nl][n], RGSWs [2L][2][nl][n] eval. Latency-bound: a digit split, two transforms and
 // two cluster barriers, where decompose, transform, multiply-accumulate and inverse kernels
-// took about 24 us a DMux level and 32 us a CRot step (live, ring of 2048), 16 and 12 us here.
+// took about 24 us a DMux level and 32 us a CRot step (live, ring of 2048), 16 and 12 us in
+// this kernel while keys and twiddles came from L2 and the partials' layout had bank
+// conflicts, 12.5 and 9 us since (degree 4096: 26 and 18 us a DMux level).
 enum { EXT_DMUX = 0, EXT_CROT = 1 };
 template <int LOGN, int MODE>
 __global__ void __cluster_dims__(4, 1, 1) __launch_bounds__((1 << LOGN) / 8)
@@ -1607,7 +1622,11 @@ __global__ void __cluster_dims__(4, 1, 1) __launch_bounds__((1 << LOGN) / 8)
   const NttTable& T = R.t[l];
   const double q = T.qd, qinv = T.qinv;
   const u64* ct = in + o * 2 * nl * n;
-  const u64* K = ks.base + ((o / ks.div) % ks.mod) * ks.stride;
+  const int smp = p * 2 + 1 - k;
+  const u64* K = ks.base + ((o / ks.div) % ks.mod) * ks.stride + ((long)(2 * smp) * nl + l) * n + 8 * tid;
+  fp_prefetch_twiddles<LOGN>(tid, T);
+  fp_prefetch(K);
+  fp_prefetch(K + (long)nl * n);
   double e[8];
 #pragma unroll
   for (int v = 0; v < 8; ++v) {
@@ -1627,26 +1646,25 @@ __global__ void __cluster_dims__(4, 1, 1) __launch_bounds__((1 << LOGN) / 8)
     if (k) e[v] = fp_next_digit(val, g);
   }
   fp_forward<LOGN>(e, tid, T, pmask);
-  const int smp = p * 2 + 1 - k;
   u64 km[8], kb[8];
-  ld8_nc(K + ((long)(2 * smp) * nl + l) * n + 8 * tid, km);
-  ld8_nc(K + ((long)(2 * smp + 1) * nl + l) * n + 8 * tid, kb);
-  __syncwarp();  // the warp's exchanges; its part of pmask is read by no other warp
+  ld8_nc(K, km);
+  ld8_nc(K + (long)nl * n, kb);
+  __syncthreads();  // the exchanges; the partials' layout (slot 8 tid + v at v n / 8 + tid) crosses warps
 #pragma unroll
   for (int v = 0; v < 8; ++v) {
-    pmask[8 * tid + v] = fp_mulmod(e[v], fp_from_u64(km[v]), q, qinv);
-    pbody[8 * tid + v] = fp_mulmod(e[v], fp_from_u64(kb[v]), q, qinv);
+    pmask[v * (n / 8) + tid] = fp_mulmod(e[v], fp_from_u64(km[v]), q, qinv);
+    pbody[v * (n / 8) + tid] = fp_mulmod(e[v], fp_from_u64(kb[v]), q, qinv);
   }
   cluster.sync();
   if (r < 2) {
     double* mine = r ? pbody : pmask;
 #pragma unroll
-    for (int v = 0; v < 8; ++v) e[v] = mine[8 * tid + v];
+    for (int v = 0; v < 8; ++v) e[v] = mine[v * (n / 8) + tid];
 #pragma unroll
     for (int y = 1; y < 4; ++y) {
       const double* peer = cluster.map_shared_rank(mine, (r + y) & 3);
 #pragma unroll
-      for (int v = 0; v < 8; ++v) e[v] = __dadd_rn(e[v], peer[8 * tid + v]);
+      for (int v = 0; v < 8; ++v) e[v] = __dadd_rn(e[v], peer[v * (n / 8) + tid]);
     }
 #pragma unroll
     for (int v = 0; v < 8; ++v) e[v] = fp_reduce(e[v], q, qinv);
@@ -1907,13 +1925,19 @@ static bool cmux_fused_ok(const DevRing& R, const Gadget& g) {
 static void cmux_fused(const DevRing& R, const Gadget& g, const u64* cur, u64* nxt, KeySel ks, long count,
                        long tiled_nq, cudaStream_t st) {
   // Levels of at most 64 CMuxes leave most SMs idle: split each CMux over a
-  // four-CTA cluster to cut its latency.
-  if (count <= CMUX_CLUSTER_MAX && g.L == 2 && R.n <= 2048 && !tiled_nq) {
+  // four-CTA cluster to cut its latency (both sides measured at k_cmux_cluster_fp).
+  if (count <= CMUX_CLUSTER_MAX && g.L == 2 && !tiled_nq) {
+#define VIA_CMUX_CASE(LG)                                                                                       \
+  k_cmux_cluster_fp<LG><<<(unsigned)(4 * count), (1 << LG) / 8, pair_smem(k_cmux_cluster_fp<LG>, 2 << LG), st>>>( \
+      cur, nxt, ks, R, g);                                                                                      \
+  break;
     switch (R.n) {
-      case 2048: k_cmux_cluster_fp<11><<<(unsigned)(4 * count), 256, 0, st>>>(cur, nxt, ks, R, g); break;
-      case 1024: k_cmux_cluster_fp<10><<<(unsigned)(4 * count), 128, 0, st>>>(cur, nxt, ks, R, g); break;
-      default: k_cmux_cluster_fp<9><<<(unsigned)(4 * count), 64, 0, st>>>(cur, nxt, ks, R, g); break;
+      case 4096: VIA_CMUX_CASE(12)
+      case 2048: VIA_CMUX_CASE(11)
+      case 1024: VIA_CMUX_CASE(10)
+      default: VIA_CMUX_CASE(9)
     }
+#undef VIA_CMUX_CASE
     VIA_LAUNCHED();
     return;
   }
@@ -2086,8 +2110,8 @@ void answer_device_stages(Server& s, Workspace& w, const u64* d_query, int nq, u
     for (int i = 0; i < nd; ++i) {
       const long active = 1L << i;  // per query
       KeySel bit{w.rgsw_q1.p + i * rgsw1, active, B, nd * rgsw1};
-      // One cluster per product and limb up to EXT_CLUSTER_MAX products, one CTA above.
-      if (B * active <= EXT_CLUSTER_MAX && ext_cluster_ok(s.r1, w.g_dmux)) {
+      // One cluster per product and limb for few products (EXT_CLUSTER_MAX), one CTA above.
+      if (B * active * n1 <= EXT_CLUSTER_MAX && ext_cluster_ok(s.r1, w.g_dmux)) {
         ext_cluster<EXT_DMUX>(s.r1, w.g_dmux, in, out, bit, 0, B * active, st);
         std::swap(in, out);
         continue;
