@@ -129,13 +129,10 @@ __host__ __device__ __forceinline__ u128 mul128x64(u128 a, u64 b) {
 struct Gadget {
   u64 base;
   int L;
-  int c;          // digits taken from the low chunk (B^c < 2^62); L - c from the high
   u128 S;         // B^L
-  u64 Bc;         // B^c
-  double dBc, dS_over_Q, dQ;
+  double dS_over_Q, dQ;
   u128 Q, halfQ;
   u64 half_base;
-  u64 magic;      // floor(2^64 / B) for the 64-bit digit divisions
   bool small;     // Q * (S + 1) < 2^53: one limb, and the scaling is exact in doubles
   // Exact integer scaling round(|c| S / Q):
   //  mode 0: one modulus Q < 2^64 with Q * S < 2^127: num = |c| S + floor(Q/2)
@@ -148,7 +145,6 @@ struct Gadget {
   int mode;
   Div64 dq, dq1;  // mode 0: Q; mode 1: q0 and q1
   u64 q0, q1;     // mode 1 limbs
-  Div64 dbc;      // B^c, for the two-chunk split when S >= 2^64
   // Digit extraction in 32-bit pieces of c32 digits (B^c32 < 2^32).
   int c32;
   Div64 dc32;     // B^c32
@@ -165,30 +161,22 @@ inline Gadget make_gadget(u64 base, int L, u128 Q, u64 q0 = 0, u64 q1 = 0) {
   g.L = L;
   u128 S = 1;
   int c = 0;
-  u128 Bc = 1;
   for (int i = 0; i < L; ++i) {
     if ((long double)S * base >= 1.7e38L) throw CudaError(100, "gadget: B^L exceeds 2^127");
     S *= base;
-    if (S < ((u128)1 << 62)) {
-      c = i + 1;
-      Bc = S;
-    }
+    if (S < ((u128)1 << 62)) c = i + 1;
   }
-  // The high chunk holds L - c digits plus a carry; it must fit 62 bits.
+  // Served: the low c digits below 2^62, and the others too.
   u128 hi = 1;
   for (int i = c; i < L; ++i) hi *= base;
   if (hi >= ((u128)1 << 62)) throw CudaError(100, "gadget: B^L too large for two chunks");
-  g.c = c;
   g.S = S;
-  g.Bc = (u64)Bc;
-  g.dBc = (double)(u64)Bc;
   g.Q = Q;
   g.halfQ = Q / 2;
   g.dQ = (double)(u64)(Q >> 64) * 18446744073709551616.0 + (double)(u64)Q;
   double dS = (double)(u64)(S >> 64) * 18446744073709551616.0 + (double)(u64)S;
   g.dS_over_Q = dS / g.dQ;
   g.half_base = base / 2;
-  g.magic = (u64)(((u128)1 << 64) / base);
   g.small = Q < ((u128)1 << 53) && S < ((u128)1 << 53) && Q * (S + 1) < ((u128)1 << 53);
   // Exact integer scaling mode (see the struct). (long double) products only
   // decide the mode; the arithmetic itself is exact.
@@ -207,7 +195,6 @@ inline Gadget make_gadget(u64 base, int L, u128 Q, u64 q0 = 0, u64 q1 = 0) {
   } else {
     g.mode = 2;
   }
-  if (c < L) g.dbc = make_div64((u64)Bc);
   int c32 = 0;
   u64 b32 = 1;
   while (c32 < L && (u128)b32 * base < ((u128)1 << 32)) {
@@ -231,34 +218,6 @@ inline Gadget make_gadget(u64 base, int L, u128 Q, u64 q0 = 0, u64 q1 = 0) {
 // The gadget of a ring: Q and (for a two-prime RNS ring) its limbs.
 inline Gadget make_gadget(u64 base, int L, const DevRing& R) {
   return R.nl == 2 ? make_gadget(base, L, R.Q(), R.m[0].q, R.m[1].q) : make_gadget(base, L, R.Q());
-}
-
-// u / B and u % B for u < 2^63 via a reciprocal and a fix-up.
-__host__ __device__ __forceinline__ u64 divB(u64 u, const Gadget& g, u64& rem) {
-  u64 q = mulhi(u, g.magic);
-  u64 r = u - q * g.base;
-  for (int it = 0; it < 4 && r >= g.base; ++it) {
-    r -= g.base;
-    ++q;
-  }
-  rem = r;
-  return q;
-}
-
-// Extract `cnt` balanced digits of u (LSB first) into d[]; returns the carry-out.
-__host__ __device__ __forceinline__ u64 digits64(u64 u, int cnt, const Gadget& g, i64* d) {
-  for (int k = 0; k < cnt; ++k) {
-    u64 r;
-    u64 q = divB(u, g, r);
-    if (r > g.half_base) {
-      d[k] = (i64)r - (i64)g.base;
-      u = q + 1;
-    } else {
-      d[k] = (i64)r;
-      u = q;
-    }
-  }
-  return u;
 }
 
 // floor(n / d) for a 64-bit n.
@@ -338,45 +297,6 @@ __host__ __device__ __forceinline__ u128 gadget_scaled(u64 a0, u64 a1, const Dev
   return gadget_scaled_fp(v, g);
 }
 
-// Splits the scaled value into the two 64-bit chunks the digit loop consumes:
-// lo < B^c holds digits 0..c-1, hi holds digits c..L-1 (plus lo's carry).
-__host__ __device__ __forceinline__ void gadget_chunks(u128 u, const Gadget& g, u64& lo, u64& hi) {
-  if (g.c >= g.L) {
-    lo = (u64)u;
-    hi = 0;
-  } else {
-    u64 rem;
-    hi = (u64)div128by64(u, g.dbc, rem);
-    lo = rem;
-  }
-}
-
-// Next balanced digit (k-th, LSB first) from the running chunk value `cur`;
-// at k == c the high chunk takes over with the low chunk's carry.
-__host__ __device__ __forceinline__ i64 gadget_next_digit(u64& cur, u64 hi, int k, const Gadget& g) {
-  if (k == g.c) cur = hi + cur;
-  u64 r;
-  u64 q = divB(cur, g, r);
-  if (r > g.half_base) {
-    cur = q + 1;
-    return (i64)r - (i64)g.base;
-  }
-  cur = q;
-  return (i64)r;
-}
-
-// Next balanced digit of a single-chunk (small) gadget.
-__host__ __device__ __forceinline__ i64 gadget_next_digit_small(u64& cur, const Gadget& g) {
-  u64 r;
-  u64 q = divB(cur, g, r);
-  if (r > g.half_base) {
-    cur = q + 1;
-    return (i64)r - (i64)g.base;
-  }
-  cur = q;
-  return (i64)r;
-}
-
 __host__ __device__ __forceinline__ u32 mulhi32(u32 a, u32 b) {
 #ifdef __CUDA_ARCH__
   return __umulhi(a, b);
@@ -425,27 +345,6 @@ __host__ __device__ __forceinline__ void for_each_digit(u128 v, const Gadget& g,
     }
     carry = x;
   }
-}
-
-// The next balanced digit of a running 32-bit value x < 2^32 (LSB first).
-__host__ __device__ __forceinline__ i64 gadget_next_digit32(u32& x, const Gadget& g) {
-  const u32 B = (u32)g.base;
-  u32 q = mulhi32(x, g.bmagic);
-  u64 r = (u64)x - (u64)q * B;
-  if (r >= B) {
-    r -= B;
-    ++q;
-  }
-  if (r >= B) {
-    r -= B;
-    ++q;
-  }
-  if (r > g.half_base) {
-    x = q + 1;
-    return (i64)r - (i64)B;
-  }
-  x = q;
-  return (i64)r;
 }
 
 // Digits of one coefficient given its residues (nl limbs). Writes L signed

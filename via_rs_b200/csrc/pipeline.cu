@@ -859,63 +859,6 @@ __global__ void k_assemble_rgsw(const u64* rlwe, const u64* gp, int L, long bits
   *dst_m = rlwe[(2 * w + mb) * per + r2];
 }
 
-// CRot (rotate.rs:128-150, SlotExtract): rot = -(X^(n - 2^i) * ct); diff = rot - ct.
-__global__ void k_crot_diff(const u64* ct, int n, int k, DevMod m, u64* diff) {
-  int gid = blockIdx.x * blockDim.x + threadIdx.x;
-  if (gid >= 2 * n) return;
-  int p = gid / n, i = gid % n;
-  // (X^k * a)[i] = a[i-k] (negated on wrap); rot = -(that).
-  int src = i - k;
-  bool wrap = src < 0;
-  if (wrap) src += n;
-  u64 v = ct[p * n + src];
-  u64 xk = wrap ? negmod(v, m.q) : v;
-  u64 rot = negmod(xk, m.q);
-  diff[p * n + i] = submod(rot, ct[p * n + i], m.q);
-}
-
-// Ring switch inputs (prim/switching/ring_switch.rs:358-385): for j < d,
-// mask_proj_j[t] = (X^j * mask)[d t]; body_proj_0[t] = body[d t].
-__global__ void k_ring_switch_proj(const u64* ct, int n1, int n2, DevMod m, u64* mask_proj, u64* body_proj) {
-  int d = n1 / n2;
-  int gid = blockIdx.x * blockDim.x + threadIdx.x;
-  if (gid >= (d + 1) * n2) return;
-  int j = gid / n2, t = gid % n2;
-  if (j == d) {
-    body_proj[t] = ct[n1 + d * t];
-    return;
-  }
-  int src = d * t - j;
-  bool wrap = src < 0;
-  if (wrap) src += n1;
-  u64 v = ct[src];
-  mask_proj[j * n2 + t] = wrap ? negmod(v, m.q) : v;
-}
-
-// acc over j of gp_j (eval or coeff, summed as residues): out = -(sum mask), body_proj - sum body.
-__global__ void k_ring_switch_sum(const u64* gp, int d, int n2, DevMod m, u64* acc) {
-  int gid = blockIdx.x * blockDim.x + threadIdx.x;
-  if (gid >= 2 * n2) return;
-  int mb = gid / n2, t = gid % n2;
-  u64 s = 0;
-  for (int j = 0; j < d; ++j) s = addmod(s, gp[(2 * j + mb) * n2 + t], m.q);
-  acc[mb * n2 + t] = s;
-}
-
-__global__ void k_ring_switch_finish(const u64* acc, const u64* body_proj, int n2, DevMod m3, DevMod m4, double dq3,
-                                     u64* out_mask, u64* out_body) {
-  int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= n2) return;
-  u64 q3 = m3.q;
-  u64 mask = negmod(acc[t], q3);
-  u64 body = submod(body_proj[t], acc[n2 + t], q3);
-  out_mask[t] = mask;  // mask: q3 -> q3 is the identity rescale
-  // body: q3 -> q4 (mod_switch_asym, prim/switching/mod_switch.rs:124-154).
-  u128 num = (u128)body * m4.q + q3 / 2;
-  u64 r = (u64)div_exact(num, (u128)q3, dq3);
-  out_body[t] = r >= m4.q ? r - m4.q : r;
-}
-
 // ---------------------------------------------------------------------------
 // Host-side orchestration.
 // ---------------------------------------------------------------------------
@@ -1959,7 +1902,8 @@ static void cmux_fused(const DevRing& R, const Gadget& g, const u64* cur, u64* n
   VIA_LAUNCHED();
 }
 
-// CRot diff for nq RLWEs: rot = -(X^k * ct), diff = rot - ct.
+// CRot diff for nq RLWEs (rotate.rs:128-150): rot = -(X^k * ct), diff = rot - ct, with
+// (X^k * a)[i] = a[i-k], negated on wrap.
 __global__ void k_crot_diff_batch(const u64* ct, int n, int k, long nq, DevMod m, u64* diff) {
   long gid = (long)blockIdx.x * blockDim.x + threadIdx.x;
   if (gid >= nq * 2 * n) return;
@@ -1973,6 +1917,8 @@ __global__ void k_crot_diff_batch(const u64* ct, int n, int k, long nq, DevMod m
   diff[p * n + i] = submod(negmod(xk, m.q), ct[p * n + i], m.q);
 }
 
+// Ring switch inputs (prim/switching/ring_switch.rs:358-385): for j < d,
+// mask_proj_j[t] = (X^j * mask)[d t]; body_proj_0[t] = body[d t].
 __global__ void k_ring_switch_proj_batch(const u64* ct, int n1, int n2, long nq, DevMod m, u64* mask_proj,
                                          u64* body_proj) {
   const int d = n1 / n2;
@@ -1993,6 +1939,7 @@ __global__ void k_ring_switch_proj_batch(const u64* ct, int n1, int n2, long nq,
   mask_proj[(q * d + j) * n2 + t] = wrap ? negmod(v, m.q) : v;
 }
 
+// The sums over j of gp_j (eval or coefficient form).
 __global__ void k_ring_switch_sum_batch(const u64* gp, int d, int n2, long nq, DevMod m, u64* acc) {
   long gid = (long)blockIdx.x * blockDim.x + threadIdx.x;
   if (gid >= nq * 2 * n2) return;
