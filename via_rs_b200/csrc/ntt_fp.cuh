@@ -43,6 +43,9 @@ __device__ __forceinline__ double fp_canonical(double x, double q, double qinv) 
   return r;
 }
 
+// A product's residue (|r| <= 0.5625 q) -> canonical residue.
+__device__ __forceinline__ double fp_wrap(double r, double q) { return r < 0 ? __dadd_rn(r, q) : r; }
+
 // Integers below 2^52 to and from doubles, exactly, without the conversion unit: the
 // double 2^52 + x has the bit pattern 0x4330000000000000 | x.
 __device__ __forceinline__ double fp_from_u64(u64 x) {

@@ -379,7 +379,7 @@ __global__ void __launch_bounds__((1 << LOGN) / 8, LOGN >= 12 ? 1 : 2) k_dmux_fp
 #pragma unroll
     for (int v = 0; v < 8; ++v) {
       const long at = (long)(part * nl + l) * n + L0::index(v, tid);
-      const u64 ext = fp_to_u64(fp_canonical(fp_mulmod(a[part][v], T.ninv_d[LOGN], q, qinv), q, qinv));
+      const u64 ext = fp_to_u64(fp_wrap(fp_mulmod(a[part][v], T.ninv_d[LOGN], q, qinv), q));
       o0[at] = submod(ct[at], ext, qi);
       o1[at] = ext;
     }
@@ -415,7 +415,7 @@ __global__ void __launch_bounds__((1 << LOGN) / 8) k_intt_fp_epi(const u64* __re
 #pragma unroll
   for (int v = 0; v < 8; ++v) {
     const int c = L0::index(v, tid);
-    const u64 val = fp_to_u64(fp_canonical(fp_mulmod(e[v], T.ninv_d[LOGN], q, qinv), q, qinv));
+    const u64 val = fp_to_u64(fp_wrap(fp_mulmod(e[v], T.ninv_d[LOGN], q, qinv), q));
     if constexpr (MODE == INTT_STORE) {
       out[seg * n + c] = val;
     } else if constexpr (MODE == INTT_DMUX) {
@@ -827,7 +827,7 @@ __global__ void __launch_bounds__((1 << LOGN) / 8)
 #pragma unroll
   for (int v = 0; v < 8; ++v) {
     const int x = L0::index(v, tid);
-    u64 c = fp_to_u64(fp_canonical(fp_mulmod(e[v], T.ninv_d[LOGN], q, qinv), q, qinv));
+    u64 c = fp_to_u64(fp_wrap(fp_mulmod(e[v], T.ninv_d[LOGN], q, qinv), q));
     if (k0 && (x & ((1 << (K - k0)) - 1)) == 0) c = submod(c, gsum[x >> (K - k0)], m.q);
     out[(2 * w + 1) * per + (long)l * n + x] = c;
     out[(2 * w) * per + (long)l * n + x] = masks[w * per + (long)l * n + x];
@@ -1619,7 +1619,7 @@ __global__ void __cluster_dims__(4, 1, 1) __launch_bounds__((1 << LOGN) / 8)
 #pragma unroll
   for (int v = 0; v < 8; ++v) {
     const long at = (long)(r * nl + l) * n + L0::index(v, tid);
-    const u64 ext = fp_to_u64(fp_canonical(fp_mulmod(e[v], T.ninv_d[LOGN], q, qinv), q, qinv));
+    const u64 ext = fp_to_u64(fp_wrap(fp_mulmod(e[v], T.ninv_d[LOGN], q, qinv), q));
     if (MODE == EXT_DMUX) {
       out[(2 * o) * 2 * nl * n + at] = submod(ct[at], ext, qi);
       out[(2 * o + 1) * 2 * nl * n + at] = ext;
@@ -1643,7 +1643,8 @@ constexpr long SHARED_KEY_MIN = 512;  // CTAs from which k_shared_key_fp runs
 // (-prod.mask, body - prod.body) with `bodies` [c][nl][n].
 //
 // FP64-issue bound: L + 2 transforms, two at a time, a CTA. 2048 key switches at q1 (L = 18)
-// 1049 us in separate kernels (digit transforms, multiply-accumulate, inverse, sum), 781 us.
+// 1049 us in separate kernels (digit transforms, multiply-accumulate, inverse, sum), 781 us, and
+// 760 with the keys fetched into L1 while the digits are transformed.
 template <int LOGN, bool ROTATED>
 __global__ void __launch_bounds__((1 << LOGN) / 8, LOGN >= 12 ? 1 : LOGN == 11 ? 2 : 1)
     k_shared_key_fp(const int8_t* __restrict__ dig8, const u64* __restrict__ key, const u64* __restrict__ bodies, int L,
@@ -1671,6 +1672,9 @@ __global__ void __launch_bounds__((1 << LOGN) / 8, LOGN >= 12 ? 1 : LOGN == 11 ?
       e[0][v] = (double)d[(long)s * n + L0::index(v, tid)];
       e[1][v] = two ? (double)d[(long)(s + 1) * n + L0::index(v, tid)] : 0.0;
     }
+#pragma unroll
+    for (int r = 0; r < 4; ++r)  // the products' keys
+      if (r < 2 || two) fp_prefetch(K + (2 * s + r) * per);
     __syncthreads();  // the previous transforms' reads
     fp_forward_digits2<LOGN>(e, tid, T, pair_sm, dense);
 #pragma unroll
@@ -1699,7 +1703,7 @@ __global__ void __launch_bounds__((1 << LOGN) / 8, LOGN >= 12 ? 1 : LOGN == 11 ?
 #pragma unroll
     for (int v = 0; v < 8; ++v) {
       const int x = L0::index(v, tid);
-      u64 w = fp_to_u64(fp_canonical(fp_mulmod(a[part][v], T.ninv_d[LOGN], q, qinv), q, qinv));
+      u64 w = fp_to_u64(fp_wrap(fp_mulmod(a[part][v], T.ninv_d[LOGN], q, qinv), q));
       if (ROTATED) w = part ? submod(bodies[c * per + (long)l * n + x], w, qi) : negmod(w, qi);
       out[(2 * c + part) * per + (long)l * n + x] = w;
     }
@@ -1710,7 +1714,8 @@ __global__ void __launch_bounds__((1 << LOGN) / 8, LOGN >= 12 ? 1 : LOGN == 11 ?
 // [c][2L][2][nl][n] and cts, out [c][2][nl][n], all in coefficient form at any 8-byte
 // address. Each RGSW polynomial is read once and nothing else of its size is written.
 // FP64-issue bound (6 L + 2 transforms, two at a time): 4099 pairs at q1, L = 2: 1.93 ms in
-// separate kernels after a copy of the RGSWs, 1.80 ms.
+// separate kernels after a copy of the RGSWs, 1.80 ms with each sample word loaded, then
+// checked, 1.21 ms with a polynomial's loads all in flight and the next one's lines fetched.
 template <int LOGN>
 __global__ void __launch_bounds__((1 << LOGN) / 8, LOGN >= 12 ? 1 : LOGN == 11 ? 2 : 1)
     k_external_fp(const u64* __restrict__ rgsw, const u64* __restrict__ cts, u64* __restrict__ out,
@@ -1725,6 +1730,13 @@ __global__ void __launch_bounds__((1 << LOGN) / 8, LOGN >= 12 ? 1 : LOGN == 11 ?
   const double q = T.qd, qinv = T.qinv;
   const u64* ct = cts + c * 2 * per;
   const u64* K = rgsw + c * 2 * L * 2 * per + (long)l * n;
+  // A sample's mask and body (2 n / 16 lines, one a thread) on their way while other polynomials
+  // are transformed.
+  const auto fetch = [&](int h, int k) {
+    const long smp = h * L + L - 1 - k;
+    fp_prefetch(K + (2 * smp + (tid >= n / 16)) * per + 16 * (tid % (n / 16)));
+  };
+  fetch(0, 0);
 #pragma unroll
   for (int h = 0; h < 2; ++h)
 #pragma unroll
@@ -1752,15 +1764,26 @@ __global__ void __launch_bounds__((1 << LOGN) / 8, LOGN >= 12 ? 1 : LOGN == 11 ?
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
       const long smp = h * L + L - 1 - k;
-      double f[2][8];  // the sample's mask and body
+      u64 x[2][8], any = 0;  // the sample's mask and body
 #pragma unroll
       for (int part = 0; part < 2; ++part)
 #pragma unroll
-        for (int v = 0; v < 8; ++v) {
-          u64 x = K[(2 * smp + part) * per + L0::index(v, tid)];
-          if (x >= (1ull << 47)) x %= T.q;  // as the transforms take any word
-          f[part][v] = fp_from_u64(x);
-        }
+        for (int v = 0; v < 8; ++v) any |= x[part][v] = K[(2 * smp + part) * per + L0::index(v, tid)];
+      if (any >= (1ull << 47)) {  // as the transforms take any word
+#pragma unroll
+        for (int part = 0; part < 2; ++part)
+#pragma unroll
+          for (int v = 0; v < 8; ++v) x[part][v] %= T.q;
+      }
+      double f[2][8];
+#pragma unroll
+      for (int part = 0; part < 2; ++part)
+#pragma unroll
+        for (int v = 0; v < 8; ++v) f[part][v] = fp_from_u64(x[part][v]);
+      if (h == 0)
+        fetch(1, k);
+      else if (k + 1 < L)
+        fetch(0, k + 1);
       __syncthreads();
       fp_forward2<LOGN>(f, tid, T, pair_sm);
 #pragma unroll
@@ -1783,7 +1806,7 @@ __global__ void __launch_bounds__((1 << LOGN) / 8, LOGN >= 12 ? 1 : LOGN == 11 ?
 #pragma unroll
     for (int v = 0; v < 8; ++v)
       out[(2 * c + part) * per + (long)l * n + L0::index(v, tid)] =
-          fp_to_u64(fp_canonical(fp_mulmod(a[part][v], T.ninv_d[LOGN], q, qinv), q, qinv));
+          fp_to_u64(fp_wrap(fp_mulmod(a[part][v], T.ninv_d[LOGN], q, qinv), q));
 }
 
 // Runs k_shared_key_fp (a key switch of rotated ciphertexts where `bodies` is given); false
