@@ -321,7 +321,9 @@ __global__ void k_dmux_combine(u64* out, const u64* in, const u64* ext, long cou
 // the two sums. Buffers: [ct][2][nl][n], RGSW [2L][2][nl][n] eval at q1; nl = 2
 // primes below 2^44. FP64-issue and latency bound: the levels of 256 to 1024 products
 // of 64 queries took 728 us together with eight barriers a transform and 64-bit
-// integer digit splits, 307 us with one barrier and splits on doubles.
+// integer digit splits, 307 us with one barrier and splits on doubles, 295 us with all of a
+// half's loads before its splits (each waited behind the previous split's rare branch; a level
+// of 8192 products 1621 and 1217 us).
 template <int LOGN>
 __global__ void __launch_bounds__((1 << LOGN) / 8, LOGN >= 12 ? 1 : 2) k_dmux_fp(u64* __restrict__ out, const u64* __restrict__ in,
                                                                   KeySel ks, const __grid_constant__ DevRing R,
@@ -344,10 +346,16 @@ __global__ void __launch_bounds__((1 << LOGN) / 8, LOGN >= 12 ? 1 : 2) k_dmux_fp
 #pragma unroll 1
   for (int h = 0; h < 2; ++h) {  // 0: mask digits (neg_s_m rows), 1: body digits (m rows)
     double e[2][8];
+    u64 x0[8], x1[8];  // all loads before the splits, whose rare branch they would wait behind
 #pragma unroll
     for (int v = 0; v < 8; ++v) {
       const u64* c = ct + (long)h * nl * n + L0::index(v, tid);
-      double val = fp_scaled2(fp_from_u64(c[0]), fp_from_u64(c[n]), g, R);
+      x0[v] = c[0];
+      x1[v] = c[n];
+    }
+#pragma unroll
+    for (int v = 0; v < 8; ++v) {
+      double val = fp_scaled2(fp_from_u64(x0[v]), fp_from_u64(x1[v]), g, R);
       e[0][v] = fp_next_digit(val, g);
       e[1][v] = fp_next_digit(val, g);
     }
@@ -925,8 +933,8 @@ static bool cmux_fused_ok(const DevRing& R, const Gadget& g);
 // Levels of at most this many CMuxes run on four-CTA clusters (cmux_fused).
 constexpr long CMUX_CLUSTER_MAX = 64;
 // DMux levels of at most this many coefficients (products x degree) run on a cluster per product
-// and limb: 32 products of degree 2048 16.1 us against 20.1 us for one CTA each, 32 of degree
-// 4096, whose CTAs fill an SM, 33.0 against 30.2.
+// and limb: 32 products of degree 2048 14.2 us against 15.8 us for one CTA each (k_dmux_fp); of
+// degree 4096, whose CTAs fill an SM, 33.0 against 27.3.
 constexpr long EXT_CLUSTER_MAX = 65536;
 
 // Whether the scan of nq queries writes tiled columns, which the CMux tree's first level
@@ -1545,7 +1553,8 @@ __global__ void __cluster_dims__(4, 1, 1) __launch_bounds__((1 << LOGN) / 8, LOG
 // two cluster barriers, where decompose, transform, multiply-accumulate and inverse kernels
 // took about 24 us a DMux level and 32 us a CRot step (live, ring of 2048), 16 and 12 us in
 // this kernel while keys and twiddles came from L2 and the partials' layout had bank
-// conflicts, 12.5 and 9 us since (degree 4096: 26 and 18 us a DMux level).
+// conflicts, 12.5 and 9 us without, 10.5 us a DMux level with its loads before the splits
+// (degree 4096: 26, 18 and 16.4 us).
 enum { EXT_DMUX = 0, EXT_CROT = 1 };
 template <int LOGN, int MODE>
 __global__ void __cluster_dims__(4, 1, 1) __launch_bounds__((1 << LOGN) / 8)
@@ -1570,20 +1579,30 @@ __global__ void __cluster_dims__(4, 1, 1) __launch_bounds__((1 << LOGN) / 8)
   fp_prefetch_twiddles<LOGN>(tid, T);
   fp_prefetch(K);
   fp_prefetch(K + (long)nl * n);
-  double e[8];
+  // All loads before the splits, whose rare branch they would wait behind: x0, x1 the limbs of a
+  // coefficient (DMUX), or it and the one `shift` places before (CROT).
+  u64 x0[8], x1[8];
 #pragma unroll
   for (int v = 0; v < 8; ++v) {
     const int x = L0::index(v, tid);
     const u64* c = ct + (long)p * nl * n + x;
+    x0[v] = c[0];
+    if (MODE == EXT_DMUX)
+      x1[v] = nl == 2 ? c[n] : 0;
+    else
+      x1[v] = c[x < shift ? n - shift : -shift];
+  }
+  double e[8];
+#pragma unroll
+  for (int v = 0; v < 8; ++v) {
     double val;
     if (MODE == EXT_DMUX) {
-      val = nl == 2 ? fp_scaled2(fp_from_u64(c[0]), fp_from_u64(c[n]), g, R)
-                    : fp_scaled(fp_reduce(fp_from_u64(c[0]), q, qinv), g.dS, qinv);
+      val = nl == 2 ? fp_scaled2(fp_from_u64(x0[v]), fp_from_u64(x1[v]), g, R)
+                    : fp_scaled(fp_reduce(fp_from_u64(x0[v]), q, qinv), g.dS, qinv);
     } else {
       // rot[x] = -in[x - shift], or in[x - shift + n] where the index wraps.
-      const int src = x - shift;
-      const double s = fp_from_u64(c[src < 0 ? src + n - x : -shift]);
-      val = fp_scaled(fp_reduce(__dadd_rn(src < 0 ? s : -s, -fp_from_u64(c[0])), q, qinv), g.dS, qinv);
+      const double s = fp_from_u64(x1[v]);
+      val = fp_scaled(fp_reduce(__dadd_rn(L0::index(v, tid) < shift ? s : -s, -fp_from_u64(x0[v])), q, qinv), g.dS, qinv);
     }
     e[v] = fp_next_digit(val, g);
     if (k) e[v] = fp_next_digit(val, g);
@@ -1715,7 +1734,8 @@ __global__ void __launch_bounds__((1 << LOGN) / 8, LOGN >= 12 ? 1 : LOGN == 11 ?
 // address. Each RGSW polynomial is read once and nothing else of its size is written.
 // FP64-issue bound (6 L + 2 transforms, two at a time): 4099 pairs at q1, L = 2: 1.93 ms in
 // separate kernels after a copy of the RGSWs, 1.80 ms with each sample word loaded, then
-// checked, 1.21 ms with a polynomial's loads all in flight and the next one's lines fetched.
+// checked, 1.21 ms with a polynomial's loads all in flight and the next one's lines fetched,
+// 1.09 ms with the ciphertext's loads before its splits as well.
 template <int LOGN>
 __global__ void __launch_bounds__((1 << LOGN) / 8, LOGN >= 12 ? 1 : LOGN == 11 ? 2 : 1)
     k_external_fp(const u64* __restrict__ rgsw, const u64* __restrict__ cts, u64* __restrict__ out,
@@ -1738,13 +1758,19 @@ __global__ void __launch_bounds__((1 << LOGN) / 8, LOGN >= 12 ? 1 : LOGN == 11 ?
   };
   fetch(0, 0);
 #pragma unroll
-  for (int h = 0; h < 2; ++h)
+  for (int h = 0; h < 2; ++h) {
+    u64 x0[8], x1[8];  // all loads before the splits, whose rare branch they would wait behind
 #pragma unroll
     for (int v = 0; v < 8; ++v) {
       const u64* x = ct + h * per + L0::index(v, tid);
-      keep[h * n + v * (n / 8) + tid] = nl == 2 ? fp_scaled2(fp_from_u64(x[0]), fp_from_u64(x[n]), g, R)
-                                                : fp_scaled(fp_reduce(fp_from_u64(x[0]), q, qinv), g.dS, qinv);
+      x0[v] = x[0];
+      x1[v] = nl == 2 ? x[n] : 0;
     }
+#pragma unroll
+    for (int v = 0; v < 8; ++v)
+      keep[h * n + v * (n / 8) + tid] = nl == 2 ? fp_scaled2(fp_from_u64(x0[v]), fp_from_u64(x1[v]), g, R)
+                                                : fp_scaled(fp_reduce(fp_from_u64(x0[v]), q, qinv), g.dS, qinv);
+  }
   double a[2][8];  // mask and body sums
 #pragma unroll
   for (int v = 0; v < 8; ++v) a[0][v] = a[1][v] = 0.0;
