@@ -321,7 +321,7 @@ __global__ void k_dmux_combine(u64* out, const u64* in, const u64* ext, long cou
 // the two sums. Buffers: [ct][2][nl][n], RGSW [2L][2][nl][n] eval at q1; nl = 2
 // primes below 2^44. FP64-issue and latency bound: the levels of 256 to 1024 products
 // of 64 queries took 728 us together with eight barriers a transform and 64-bit
-// integer digit splits, 307 us with one barrier and splits on doubles, 295 us with all of a
+// integer digit splits, 362 us with one barrier and splits on doubles, 295 us with all of a
 // half's loads before its splits (each waited behind the previous split's rare branch; a level
 // of 8192 products 1621 and 1217 us).
 template <int LOGN>
