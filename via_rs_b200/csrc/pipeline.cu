@@ -819,7 +819,7 @@ __global__ void __launch_bounds__((1 << LOGN) / 8)
     gsum[tid] = reduce64(s, m);
   }
   const u64* sk = bsk + (w * nl + l) * 2 * n;
-  const double b = fp_from_u64(b0[w * b0_stride + l]);
+  const double b = fp_from_u64(reduce64(b0[w * b0_stride + l], m));  // the caller's word: any 64 bits
   double e[8];
 #pragma unroll
   for (int v = 0; v < 8; ++v) e[v] = 0.0;
