@@ -1,10 +1,13 @@
 """Caller words that are not canonical residues are taken mod their prime: the results are
 compared with the oracle's on the reduced words, at values where double-precision integers
 (2^52, 2^53) and the transforms' bounds (2^47) end."""
+import dataclasses
+
 import numpy as np
 import pytest
 
-from via_rs_b200.params import paper_preset, secure_preset
+from via_rs_b200 import prims
+from via_rs_b200.params import PAPER_Q1, PAPER_Q2, SECURE_Q1, paper_preset, secure_preset
 from via_rs_b200.server import PublicKeys, Server
 
 pytestmark = pytest.mark.gpu
@@ -22,10 +25,33 @@ def _words(rng, q, shape):
     return np.where(pick == 2, rng.integers(0, 1 << 64, size=shape, dtype=np.uint64), w)
 
 
+def _raw(rng, primes, polys, n):
+    """Raw words [polys][nl][n] and the same words reduced."""
+    raw = np.stack([_words(rng, q, (polys, n)) for q in primes], axis=1)
+    return raw, raw % np.array(primes, dtype=np.uint64)[:, None]
+
+
+def _dev(torch, a):
+    return torch.from_numpy(np.ascontiguousarray(a).view(np.int64)).cuda()
+
+
+def _host(t):
+    return t.cpu().numpy().view(np.uint64).reshape(-1)
+
+
+PRESETS = {
+    "paper": lambda: paper_preset(2, 2),
+    "secure": lambda: secure_preset(2, 2),
+    # Key gadgets without GEMM steps: byte digits, 64-bit digits.
+    "bytes": lambda: dataclasses.replace(paper_preset(2, 2), ck_base=21, l_ck=18),
+    "words": lambda: dataclasses.replace(paper_preset(2, 2), ck_base=300, l_ck=9),
+}
+
+
 @pytest.mark.parametrize("part", ["body", "mask"])
-@pytest.mark.parametrize("preset", ["paper", "secure"])
+@pytest.mark.parametrize("preset", sorted(PRESETS))
 def test_query_words(oracle, preset, part):
-    prm = {"paper": paper_preset, "secure": secure_preset}[preset](2, 2)
+    prm = PRESETS[preset]()
     recs = np.zeros((prm.capacity, prm.n_rec), dtype=np.uint64)
     c = oracle.Client(prm, b"raw-query")
     gpu = Server.setup(prm, PublicKeys(c.cascade_key, c.conv_key, c.rsk), recs)
@@ -43,3 +69,20 @@ def test_query_words(oracle, preset, part):
     red = raw.copy()
     red[:, at] %= primes
     assert np.array_equal(gpu.debug_stage(raw.reshape(-1), 1), cpu.debug_stage(red.reshape(-1), 1))
+
+
+@pytest.mark.parametrize("primes,n,base,L", [(PAPER_Q1, 256, 55879, 2), (PAPER_Q1, 2048, 55879, 2),
+                                             ((PAPER_Q2,), 2048, 81, 2), (SECURE_Q1, 4096, 18073, 2)])
+@pytest.mark.parametrize("in_place", [False, True])
+def test_external_product_words(oracle, primes, n, base, L, in_place):
+    import torch
+
+    rng = np.random.default_rng(62)
+    count = 3
+    rgsw, rgsw_red = _raw(rng, primes, count * 4 * L, n)
+    ct, ct_red = _raw(rng, primes, count * 2, n)
+    d_rgsw, d_ct = _dev(torch, rgsw), _dev(torch, ct)
+    out = d_ct if in_place else torch.empty_like(d_ct)
+    prims.external_product_dev(prims.ring(n, primes), base, L, d_rgsw.data_ptr(), d_ct.data_ptr(), count, out.data_ptr())
+    want = oracle.external_product(primes, n, base, L, rgsw_red.reshape(-1), ct_red.reshape(-1))
+    assert np.array_equal(_host(out), want)

@@ -42,11 +42,13 @@ __global__ void k_decompose(const u64* __restrict__ in, int n_in, int stride, lo
   const int nl = R.nl;
   const u64* src = in + p * nl * n_in;
   u64 a0 = src[i], a1 = nl == 2 ? src[n_in + i] : 0;
+  if (a0 >= R.m[0].q) a0 = reduce64(a0, R.m[0]);  // a caller's word may be any 64 bits
+  if (a1 >= R.m[1].q) a1 = reduce64(a1, R.m[1]);
   const int n_out = n_in * stride;
   const long step = (long)nl * n_out;
   // Digit k goes to sample slot L - 1 - k.
   u64* o = out + p * (long)g.L * step + (long)(g.L - 1) * step + (long)i * stride;
-  if (g.fp && R.ntt && stride == 1 && a0 < R.m[0].q && a1 < R.m[1].q) {
+  if (g.fp && R.ntt && stride == 1) {
     double v = nl == 2 ? fp_scaled2(fp_from_u64(a0), fp_from_u64(a1), g, R)
                        : fp_scaled(fp_reduce(fp_from_u64(a0), (double)R.m[0].q, R.t[0].qinv), g.dS, R.t[0].qinv);
     for (int k = 0; k < g.L; ++k, o -= step) {
@@ -79,7 +81,9 @@ __global__ void k_decompose_i8(const u64* __restrict__ in, int n_in, long npolys
   const int i = (int)(gid % n_in);
   const int nl = R.nl;
   const u64* src = in + p * nl * n_in;
-  const u64 a0 = src[i], a1 = nl == 2 ? src[n_in + i] : 0;
+  u64 a0 = src[i], a1 = nl == 2 ? src[n_in + i] : 0;
+  if (a0 >= R.m[0].q) a0 = reduce64(a0, R.m[0]);  // a query's word may be any 64 bits
+  if (a1 >= R.m[1].q) a1 = reduce64(a1, R.m[1]);
   int8_t* o = out + p * (long)g.L * n_in + (long)(g.L - 1) * n_in + i;
   for_each_digit(gadget_scaled(a0, a1, R, g), g, [&](int, i64 d) {
     *o = (int8_t)d;
@@ -1759,12 +1763,19 @@ __global__ void __launch_bounds__((1 << LOGN) / 8, LOGN >= 12 ? 1 : LOGN == 11 ?
   fetch(0, 0);
 #pragma unroll
   for (int h = 0; h < 2; ++h) {
-    u64 x0[8], x1[8];  // all loads before the splits, whose rare branch they would wait behind
+    u64 x0[8], x1[8], any = 0;  // all loads before the splits, whose rare branch they would wait behind
 #pragma unroll
     for (int v = 0; v < 8; ++v) {
       const u64* x = ct + h * per + L0::index(v, tid);
-      x0[v] = x[0];
-      x1[v] = nl == 2 ? x[n] : 0;
+      any |= x0[v] = x[0];
+      any |= x1[v] = nl == 2 ? x[n] : 0;
+    }
+    if (any >= (1ull << 47)) {  // any 64-bit word, as of the samples below
+#pragma unroll
+      for (int v = 0; v < 8; ++v) {
+        x0[v] %= R.m[0].q;
+        x1[v] %= R.m[1].q;
+      }
     }
 #pragma unroll
     for (int v = 0; v < 8; ++v)
