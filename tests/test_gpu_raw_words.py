@@ -86,3 +86,21 @@ def test_external_product_words(oracle, primes, n, base, L, in_place):
     prims.external_product_dev(prims.ring(n, primes), base, L, d_rgsw.data_ptr(), d_ct.data_ptr(), count, out.data_ptr())
     want = oracle.external_product(primes, n, base, L, rgsw_red.reshape(-1), ct_red.reshape(-1))
     assert np.array_equal(_host(out), want)
+
+
+@pytest.mark.parametrize("n,count", [(16, 3), (256, 3), (2048, 2), (2048, 256)])
+def test_key_switch_mask_words(oracle, n, count):
+    import torch
+
+    rng = np.random.default_rng(63)
+    base = L = 18
+    key, key_red = _raw(rng, PAPER_Q1, L * 2, n)
+    ct, ct_red = _raw(rng, PAPER_Q1, count * 2, n)
+    ct[1::2] = ct_red[1::2]  # bodies: residues
+    shifts = rng.integers(0, 2 * n, size=count, dtype=np.uint64)
+    d = [_dev(torch, x) for x in (key, ct, shifts)]
+    out = torch.empty((count * 2, 2, n), dtype=torch.int64, device="cuda")
+    prims.key_switch_dev(prims.ring(n, PAPER_Q1), base, L, d[0].data_ptr(), d[1].data_ptr(), d[2].data_ptr(), count,
+                         out.data_ptr())
+    want = oracle.key_switch(PAPER_Q1, n, base, L, key_red.reshape(-1), ct_red.reshape(-1), shifts)
+    assert np.array_equal(_host(out), want)

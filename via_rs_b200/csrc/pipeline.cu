@@ -1097,7 +1097,8 @@ static void decompose(const DevRing& R, const Gadget& g, const u64* in, int n_in
 static bool shared_key_fp(const DevRing& R, const int8_t* dig8, const u64* key, const u64* bodies, int L, long count,
                           u64* out, cudaStream_t st);
 
-// Signed byte digits (bases up to 255); `in` is a 16-byte aligned buffer of canonical residues.
+// Signed byte digits (bases up to 255). `in` is a 16-byte aligned buffer, and of canonical residues
+// where n_in is 4 or more.
 static void decompose_i8(const DevRing& R, const Gadget& g, const u64* in, int n_in, long npolys, int8_t* out,
                          cudaStream_t st) {
   if (n_in >= 4 && ct_digits_ok(g.base, (u32)g.L, R))
@@ -2518,7 +2519,9 @@ __global__ void k_rotate_split(const u64* __restrict__ cts, const u64* __restric
   const int part = (int)((gid / per) % 2);
   const int l = (int)((gid % per) / n), i = (int)(gid % n);
   const u64 k = shifts[c] % (u64)(2 * n);
-  const u64 v = cts[gid];
+  u64 v = cts[gid];
+  // A mask is split into digits, by steps on doubles among others: any 64-bit word mod q here.
+  if (part == 0 && v >= R.m[l].q) v = reduce64(v, R.m[l]);
   const u64 pos = (u64)i + k;  // < 3n
   const int dst = (int)(pos % (u64)n);
   const bool neg = ((pos / (u64)n) & 1) != 0;
