@@ -7,7 +7,7 @@ import numpy as np
 import pytest
 
 from via_rs_b200 import prims
-from via_rs_b200.params import PAPER_Q1, PAPER_Q2, SECURE_Q1, paper_preset, secure_preset
+from via_rs_b200.params import PAPER_Q1, PAPER_Q2, PAPER_Q3, SECURE_Q1, paper_preset, secure_preset
 from via_rs_b200.server import PublicKeys, Server
 
 pytestmark = pytest.mark.gpu
@@ -104,3 +104,30 @@ def test_key_switch_mask_words(oracle, n, count):
                          out.data_ptr())
     want = oracle.key_switch(PAPER_Q1, n, base, L, key_red.reshape(-1), ct_red.reshape(-1), shifts)
     assert np.array_equal(_host(out), want)
+
+
+# A prime of each of the inverse's schedules: up to 2^35, up to 2^40, below 2^44.
+@pytest.mark.parametrize("primes,n", [((PAPER_Q2,), 2048), ((PAPER_Q3,), 512), (PAPER_Q1, 2048), (PAPER_Q1, 64),
+                                      (SECURE_Q1, 4096), ((17_592_186_028_033,), 4096)])
+@pytest.mark.parametrize("inverse", [False, True])
+def test_transform_words(oracle, primes, n, inverse):
+    import torch
+
+    rng = np.random.default_rng(64)
+    blocks = n.bit_length() - 1
+    count = 5 + blocks
+    raw, _ = _raw(rng, primes, count, n)
+    # Where an inverse grows most: 2^b equal words, then 2^b zeros, so that the words add up for b
+    # stages and the next one takes the difference.
+    for b in range(blocks):
+        raw[b] = np.where(np.arange(n) >> b & 1, 0, (1 << 47) - 1).astype(np.uint64)
+    red = raw % np.array(primes, dtype=np.uint64)[:, None]
+    ring, d = prims.ring(n, primes), _dev(torch, raw)
+    if not inverse:
+        prims.ntt_forward_dev(ring, d.data_ptr(), count)
+        assert np.array_equal(_host(d), oracle.ntt(primes, n, red).reshape(-1))
+    else:  # canonical coefficients whose transform is the reduced input
+        prims.ntt_inverse_dev(ring, d.data_ptr(), count)
+        got = d.cpu().numpy().view(np.uint64).reshape(red.shape)
+        assert (got < np.array(primes, dtype=np.uint64)[:, None]).all()
+        assert np.array_equal(oracle.ntt(primes, n, got).reshape(-1), red.reshape(-1))

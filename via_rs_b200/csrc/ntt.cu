@@ -231,8 +231,7 @@ __global__ void __launch_bounds__(ntt_cta<LOGN>()) k_ntt_reg_i8(const int8_t* __
 
 // ---------------------------------------------------------------------------
 // The register-resident transforms in double precision (ntt_fp.cuh), for primes
-// below 2^44: exact integer arithmetic on doubles. Inputs are residues below 2^47
-// (larger values are reduced first); outputs:
+// below 2^44: exact integer arithmetic on doubles. Inputs are any 64-bit words; outputs:
 //  * forward: canonical residues, or (LAZY) nonnegative residues below 2 q;
 //  * inverse: canonical residues;
 //  * of digits (k_ntt_fp_i8): the signed doubles themselves (DOUT), within
@@ -276,7 +275,10 @@ __global__ void __launch_bounds__(ntt_cta<LOGN>()) k_ntt_fp(u64* __restrict__ da
   u64 any = 0;
 #pragma unroll
   for (int v = 0; v < 8; ++v) any |= x[v];
-  if (any >= (1ull << 47)) {  // any 64-bit word is taken, on a path of its own: 16384 polynomials 669 -> 641 us
+  // Any 64-bit word is taken, on a path of its own (16384 polynomials 669 -> 641 us): a forward
+  // transform adds at most 7 q to a word, an inverse may double it in every stage (fp_inverse_w:
+  // below 2 q, here no wider than q).
+  if (INV ? __clzll(any) < __clzll(T.q) : any >= (1ull << 47)) {
 #pragma unroll
     for (int v = 0; v < 8; ++v) x[v] %= T.q;
   }

@@ -1,5 +1,5 @@
 // The register-resident negacyclic transform of ntt.cuh in double precision,
-// for single primes q < 2^36. Residues are integer-valued doubles in a signed
+// for primes q < 2^44. Residues are integer-valued doubles in a signed
 // range, and every product is exact:
 //
 //   fp_mulmod(a, b): ph = fl(a b), pl = a b - ph (one FMA: the error-free
@@ -17,9 +17,9 @@
 //
 // Bounds: forward butterflies (a, c) -> (a + t, a - t), t = fp_mulmod(c, w), grow by at
 // most 0.5625 q per stage; inverse butterflies (a, c) -> (a + c, fp_mulmod(a - c, w)) at
-// most double per stage, so inputs below q of a prime below 2^36 stay below 2^12 q < 2^48
-// after twelve stages. Larger primes bring the values back within q / 2 on the way
-// (fp_inverse). The inverse ends with an fp_mulmod by n^-1.
+// most double per stage, so inputs below 2 q of a prime up to 2^35 stay below 2^48 through
+// twelve stages. Larger primes bring the values back within q / 2 on the way
+// (fp_inverse_w). The inverse ends with an fp_mulmod by n^-1.
 #pragma once
 #include "ntt.cuh"
 
@@ -263,11 +263,11 @@ __device__ __forceinline__ void fp_forward_digits_w(double (&e)[W][8], int tid, 
 }
 
 // Inverse transforms, without the n^-1 scaling, of W segments held as eight consecutive
-// elements a thread, inputs below 4 q in magnitude; leaves signed values in the phase-0
-// layout: below 2^12 q for q <= 2^35 (inputs below q), else below 2^6 q, 2^48 in any case.
-// Primes above 2^35 return to q / 2 after the second phase (six stages at most between
-// reductions: 2 * 4 q * 2^5 < 2^48 for q < 2^40), above 2^40 after every phase. On
-// entry no other warp may still read the exchange areas.
+// elements a thread, inputs below 2 q in magnitude; leaves signed values in the phase-0
+// layout, at most 2^48: every stage may double them, so 2 q * 2^12 for q <= 2^35. Primes above
+// 2^35 return to q / 2 after the second phase (six stages at most before it: 2 q * 2^6 <= 2^47
+// for q < 2^40), above 2^40 after every phase (2 q * 2^3 < 2^48 for q < 2^44). On entry no other
+// warp may still read the exchange areas.
 template <int LOGN, int P, int W>
 __device__ __forceinline__ void fp_inverse_w(double (&e)[W][8], int tid, const NttTable& T, double* ssm, int sbase = 0) {
   constexpr int LAST = (LOGN + 2) / 3 - 1, n = 1 << LOGN;
