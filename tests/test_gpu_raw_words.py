@@ -7,6 +7,7 @@ import numpy as np
 import pytest
 
 from via_rs_b200 import prims
+from via_rs_b200.client import Client
 from via_rs_b200.params import PAPER_Q1, PAPER_Q2, PAPER_Q3, SECURE_Q1, paper_preset, secure_preset
 from via_rs_b200.server import PublicKeys, Server
 
@@ -131,3 +132,23 @@ def test_transform_words(oracle, primes, n, inverse):
         got = d.cpu().numpy().view(np.uint64).reshape(red.shape)
         assert (got < np.array(primes, dtype=np.uint64)[:, None]).all()
         assert np.array_equal(oracle.ntt(primes, n, got).reshape(-1), red.reshape(-1))
+
+
+@pytest.mark.parametrize("below", [1 << 64, 1 << 33, 1 << 32])
+def test_client_key_words(oracle, below):
+    """Recovery with a key of words up to `below`, and the same residues."""
+    prm = paper_preset(2, 2)
+    oc = oracle.Client(prm, b"raw-key")
+    sk1, sk2 = oc.secret_keys()
+    rng = np.random.default_rng(65)
+    lifts = rng.integers(0, below // prm.q3 - 1, size=prm.n2, dtype=np.uint64)
+    raw = sk2 + lifts * np.uint64(prm.q3)
+    assert np.array_equal(raw % np.uint64(prm.q3), sk2)
+    assert below < 1 << 64 or int(np.bitwise_or.reduce(raw)) == below - 1  # an or that leaves no word above it
+    client = Client(prm, sk1, raw)
+    masks = rng.integers(0, prm.q3, size=(3, prm.n2), dtype=np.uint64)
+    masks[0] = prm.q3 - 1
+    bodies = rng.integers(0, prm.q4, size=(3, prm.n2), dtype=np.uint64)
+    got = client.recover_many(masks, bodies)
+    for k in range(3):
+        assert np.array_equal(got[k], oc.recover(masks[k], bodies[k]))

@@ -316,7 +316,7 @@ struct Client {
   cudaStream_t stream = nullptr;
   DevBuf sk1, sk2;
   KeptScratch scratch;
-  u64 sk2_top = 0;  // the or of sk2's words, plus one
+  u64 sk2_bits = 0;  // the or of sk2's words
   int err_kind = 0;
   i64 err_bound = 1;
   ~Client() {
@@ -451,8 +451,7 @@ via_status via_client_create(const via_params* params, const uint64_t* sk1, cons
     const int nl = params->q1_1 ? 2 : 1;
     c->sk1.alloc((size_t)nl * params->n1);
     c->sk2.alloc(params->n2);
-    for (u32 i = 0; i < params->n2; ++i) c->sk2_top |= sk2[i];
-    c->sk2_top += 1;
+    for (u32 i = 0; i < params->n2; ++i) c->sk2_bits |= sk2[i];
     VIA_CUDA(cudaMemcpy(c->sk1.p, sk1, c->sk1.n * 8, cudaMemcpyHostToDevice));
     VIA_CUDA(cudaMemcpy(c->sk2.p, sk2, c->sk2.n * 8, cudaMemcpyHostToDevice));
     *out = c.release();
@@ -495,12 +494,12 @@ via_status via_client_recover(via_client* c, const uint64_t* masks, const uint64
     VIA_CUDA(cudaMemcpyAsync(dm, masks, len * 8, cudaMemcpyHostToDevice, c->stream));
     VIA_CUDA(cudaMemcpyAsync(db, bodies, len * 8, cudaMemcpyHostToDevice, c->stream));
     const int threads = (int)std::min<u64>(p.n2, 1024);
-    // The caller's residues are held to 32 bits here, not to q3: any value that
-    // does not fit takes the 128-bit sums.
-    u64 top = p.q3;
-    for (size_t i = 0; i < len; ++i) top |= masks[i];
-    const bool narrow = (top >> 32) == 0 && c->sk2_top <= ((u64)1 << 32) &&
-                        (u128)top * c->sk2_top * p.n2 < ((u128)1 << 64);
+    // The caller's words (masks and key) are held to 32 bits here, not to q3: any value that
+    // does not fit takes the 128-bit sums. An or is at least each of its words.
+    u64 bits = p.q3;
+    for (size_t i = 0; i < len; ++i) bits |= masks[i];
+    const bool narrow = (bits >> 32) == 0 && (c->sk2_bits >> 32) == 0 &&
+                        (u128)bits * c->sk2_bits * p.n2 < ((u128)1 << 64);
     if (narrow)
       k_client_recover<true><<<(unsigned)count, threads, 2 * p.n2 * 4, c->stream>>>(
           dm, db, c->sk2.p, (int)p.n2, make_devmod(p.q3), p.q4, p.p, dout);
