@@ -70,15 +70,22 @@ void DevBuf::free() {
   n = 0;
 }
 
-// Raises VIA_ERR_TIMEOUT once the FirstDim scan has reported that one of its
-// bounded waits ran out (the word stays set for the handle's lifetime).
-static void check_device_flags(Server& s, cudaStream_t st) {
-  if (!s.fd_err.p) return;
+std::string device_flags(Server& s, cudaStream_t st) {
+  if (!s.fd_err.p) return "";
   int flag = 0;
   VIA_CUDA(cudaMemcpyAsync(&flag, s.fd_err.p, sizeof(int), cudaMemcpyDeviceToHost, st));
   VIA_CUDA(cudaStreamSynchronize(st));
-  if (flag)
-    throw ApiError(VIA_ERR_TIMEOUT, "a bounded device wait ran out in the scan or the cascade (flag " + std::to_string(flag) + ")");
+  return flag ? device_flag_text(flag) : "";
+}
+std::string device_flag_text(int flag) {
+  return "a bounded device wait ran out in the scan or the cascade (flag " + std::to_string(flag) + ")";
+}
+
+// Raises VIA_ERR_TIMEOUT once the scan or the cascade has reported that one of its bounded
+// waits ran out.
+static void check_device_flags(Server& s, cudaStream_t st) {
+  const std::string e = device_flags(s, st);
+  if (!e.empty()) throw ApiError(VIA_ERR_TIMEOUT, e);
 }
 
 int ilog2(u64 v) { return v <= 1 ? 0 : 63 - __builtin_clzll(v); }

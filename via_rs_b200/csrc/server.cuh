@@ -86,7 +86,7 @@ struct Server {
   std::shared_ptr<DevBuf> db;
   std::shared_ptr<DevBuf> planes;
   FdPlan fd;
-  DevBuf fd_err;  // one device word the scan sets when a bounded wait runs out
+  DevBuf fd_err;  // one device word the scan and the cascade's GEMM steps set when a bounded wait runs out
   // Eval-form keys (crates/via-server/src/prepared_keys.rs:69-79).
   DevBuf cascade_eval;  // include/via_gpu.h cascade layout, each segment transformed
   DevBuf cascade_eval_d;  // the same residues as exact doubles (q1 primes below 2^44), for the double-precision MAC
@@ -113,6 +113,10 @@ struct Server {
 
 // Shared helpers.
 void set_last_error(const std::string& m);  // the message via_last_error() returns
+// Waits for st, then what the handle's error word says: empty, or that bounded waits ran out (the
+// word stays set until the test hook is turned off). Synchronous answers end with it.
+std::string device_flags(Server& s, cudaStream_t st);
+std::string device_flag_text(int flag);
 void validate_params(const via_params& p);
 u64 lwe_len(const via_params& p);
 u64 query_lwes(const via_params& p);

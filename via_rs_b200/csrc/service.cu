@@ -157,7 +157,7 @@ void Service::finish(Lane& L, cudaError_t e) {
     if (e != cudaSuccess || timeout) {
       r->state = 3;
       r->status = timeout ? VIA_ERR_TIMEOUT : VIA_ERR_CUDA;
-      r->error = timeout ? "FirstDim scan: a bounded device wait ran out" : cudaGetErrorString(e);
+      r->error = timeout ? device_flag_text(*L.h_err) : cudaGetErrorString(e);
       ++failed;
       continue;
     }

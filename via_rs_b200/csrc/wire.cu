@@ -283,7 +283,8 @@ via_status via_server_answer_wire(via_server* s, const uint8_t* wire, uint64_t l
     answer_graph(*s, 1, s->stream);
     VIA_CUDA(cudaMemcpyAsync(out_mask, workspace_answer_mask(*s), p.n2 * 8, cudaMemcpyDeviceToHost, s->stream));
     VIA_CUDA(cudaMemcpyAsync(out_body, workspace_answer_body(*s), p.n2 * 8, cudaMemcpyDeviceToHost, s->stream));
-    VIA_CUDA(cudaStreamSynchronize(s->stream));
+    const std::string e = device_flags(*s, s->stream);
+    if (!e.empty()) throw ApiErr(VIA_ERR_TIMEOUT, e);
   });
 }
 
