@@ -39,3 +39,22 @@ def test_wire_answer_reports_the_wait(oracle):
     gpu.set_scan_fault(0)
     got = answer_wire(gpu, wire)
     assert np.array_equal(got[0], want[0]) and np.array_equal(got[1], want[1])
+
+
+@pytest.mark.parametrize("queries", [1, 17])  # 8 and 136 LWEs: part of one tile, two tiles
+def test_cascade_wait_runs_out_and_handle_recovers(oracle, queries):
+    prm = paper_preset(2, 2, 512)
+    c, gpu, cpu = _setup(oracle, prm)
+    qs = np.stack([c.query(k % prm.capacity, b"w-%02d" % k) for k in range(queries)])
+    gpu.set_scan_fault(2000)
+    with pytest.raises(DeviceError) as e:
+        gpu.debug_stage(qs[0], 1)  # the cascade alone
+    flag = int(str(e.value).split("flag ")[1].rstrip(")"))
+    assert e.value.code == VIA_ERR_TIMEOUT and flag & 64 and not flag & 15, flag
+    _times_out(lambda: gpu.answer_many(qs))
+    gpu.set_scan_fault(0)
+    assert np.array_equal(gpu.debug_stage(qs[0], 1), cpu.debug_stage(qs[0], 1))
+    masks, bodies = gpu.answer_many(qs)
+    for k in (0, queries - 1):
+        m, b = cpu.answer(qs[k])
+        assert np.array_equal(masks[k], m) and np.array_equal(bodies[k], b), k

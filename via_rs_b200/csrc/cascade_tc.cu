@@ -29,6 +29,7 @@ struct CtParams {
   long nlwe;
   size_t a_tile, out_tile;  // bytes per 128-LWE tile
   int mtiles, out_kp, out_half;
+  unsigned fault_ns;  // test hook: > 0 makes the epilogue's first wait run out after this long
 };
 
 // Item -> its first unit, and its units. Units 0 .. units - 1 are mask units.
@@ -102,7 +103,8 @@ __global__ void __launch_bounds__(CT_THREADS, 1) k_ct_step(const __grid_constant
   u64* acc_full = empty + CT_STAGES;
   u64* acc_empty = acc_full + CT_ACC;
   u64* drain = acc_empty + CT_ACC;
-  u32* tmem_slot = reinterpret_cast<u32*>(drain + 1);
+  u64* never = drain + 1;  // the test hook's barrier: initialised, never arrived on
+  u32* tmem_slot = reinterpret_cast<u32*>(never + 1);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (threadIdx.x == 0) {
@@ -115,6 +117,7 @@ __global__ void __launch_bounds__(CT_THREADS, 1) k_ct_step(const __grid_constant
       mbar_init(acc_empty + a, CT_EPI * 32);
     }
     mbar_init(drain, 1);
+    mbar_init(never, 1);
     *abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
@@ -232,7 +235,7 @@ __global__ void __launch_bounds__(CT_THREADS, 1) k_ct_step(const __grid_constant
     const int n_out = 2 * S.n;
     int a = 0;
     u32 aph = 0;
-    bool ok = true;
+    bool ok = P.fault_ns == 0 || mbar_wait_never(never, P.fault_ns);
     for (int it = blockIdx.x; ok && it < items; it += gridDim.x) {
       const int mt = it % P.mtiles;
       int len;
@@ -567,6 +570,7 @@ void ct_run(Server& s, const u64* d_query, long nlwe, uint8_t* da, uint8_t* db, 
     P.a_tile = (size_t)CT_M * cur.half * cur.kp;
     P.out_tile = (size_t)CT_M * nxt.half * nxt.kp;
     P.mtiles = mtiles;
+    P.fault_ns = s.fd.fault_wait_ns;
     P.out_kp = nxt.kp;
     P.out_half = nxt.half;
     const int items = cur.items() * mtiles;

@@ -49,17 +49,6 @@ struct KParams {
   double qd, qinv, c24, c48;  // q2, its rounded inverse, 2^24 and 2^48 mod q2, as doubles
 };
 
-// The test hook's wait: polls a barrier that no thread or copy ever completes
-// until `limit_ns` has passed (or WAIT_SPINS polls), then reports failure.
-__device__ bool mbar_wait_never(u64* bar, unsigned limit_ns) {
-  const unsigned long long t0 = global_ns();
-  for (unsigned it = 0; it < WAIT_SPINS; ++it) {
-    if (mbar_try_wait(bar, 0)) return true;
-    if ((it & 31) == 0 && global_ns() - t0 > limit_ns) return false;
-  }
-  return false;
-}
-
 // Work unit u -> (slot t, c-tile ct) in the tile's order.
 __device__ __forceinline__ void unit_coords(const KParams& P, int u, int& t, int& ct) {
   if (P.order) {

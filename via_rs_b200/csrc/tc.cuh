@@ -53,6 +53,17 @@ static __device__ bool mbar_wait(u64* bar, u32 parity, volatile int* abort_flag,
   return false;
 }
 
+// The test hook's wait: polls a barrier that no thread or copy ever completes
+// until `limit_ns` has passed (or WAIT_SPINS polls), then reports failure.
+static __device__ bool mbar_wait_never(u64* bar, unsigned limit_ns) {
+  const unsigned long long t0 = global_ns();
+  for (unsigned it = 0; it < WAIT_SPINS; ++it) {
+    if (mbar_try_wait(bar, 0)) return true;
+    if ((it & 31) == 0 && global_ns() - t0 > limit_ns) return false;
+  }
+  return false;
+}
+
 __device__ __forceinline__ void bulk_g2s(void* dst, const void* src, u32 bytes, u64* bar) {
   asm volatile(
       "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(smem_addr(dst)),

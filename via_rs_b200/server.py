@@ -230,7 +230,7 @@ class Server:
         check(_lib.lib().via_server_set_scan_tile(self._h, batch, t))
 
     def set_scan_fault(self, wait_us: int) -> None:
-        """Test hook (via_server_set_scan_fault): scans make a bounded wait run out
+        """Test hook (via_server_set_scan_fault): scans and the cascade's GEMM steps make a bounded wait run out
         after wait_us microseconds and report VIA_ERR_TIMEOUT; 0 turns it off."""
         check(_lib.lib().via_server_set_scan_fault(self._h, wait_us))
 
