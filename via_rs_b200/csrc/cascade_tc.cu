@@ -507,25 +507,33 @@ void ct_prepare(Server& s) {
   const via_params& p = s.prm;
   if (!ct_supported(p, s.r1) || !s.cascade_eval.p || !s.fd_err.p) return;
   const int K = ct_steps(p), n1 = (int)p.n1;
-  size_t bytes = 0, consts = 0;
-  for (int k = 0; k < K; ++k) {
-    const CtStep st = ct_step(n1, 1 << k);
-    bytes += (size_t)2 * st.units * st.chunks * CT_STAGE_B;
-    consts += (size_t)2 * st.units * 2 * CT_ROWS;  // room for items of one unit
-  }
   ct_prepare_device();
-  s.ct_planes.alloc(bytes / 8);
-  s.ct_consts.alloc(2 * consts);  // for few and for many tiles
   const CtDigits D = ct_digits(p.ck_base, s.r1);
   const u64 step_len = (u64)2 * n1 * CT_L * 2 * 2;
   const u64 inv0 = (u64)D.yscale[0], inv1 = (u64)D.yscale[1];
-  uint8_t* planes = reinterpret_cast<uint8_t*>(s.ct_planes.p);
-  double* cc = reinterpret_cast<double*>(s.ct_consts.p);
+  const auto plane_bytes = [](const CtStep& st) { return (size_t)2 * st.units * st.chunks * CT_STAGE_B; };
+  const auto plane_blocks = [](const CtStep& st) {
+    return (unsigned)(((long)2 * st.units * st.chunks * (CT_KC / 16) * 32 + 255) / 256);
+  };
+  size_t bytes = 0, consts = 0;
   for (int k = 0; k < K; ++k) {
     const CtStep st = ct_step(n1, 1 << k);
-    const long threads = (long)2 * st.units * st.chunks * (CT_KC / 16) * 32;
-    k_ct_planes<<<(unsigned)((threads + 255) / 256), 256, 0, s.stream>>>(s.cascade_eval.p + k * step_len, st, s.r1, inv0,
-                                                                        inv1, planes);
+    bytes += plane_bytes(st);
+    consts += (size_t)2 * st.units * 2 * CT_ROWS;  // room for items of one unit
+  }
+  auto keys = std::make_shared<CtKeys>();
+  try {
+    keys->planes.alloc(bytes / 8);
+    keys->consts.alloc(2 * consts);  // for few and for many tiles
+  } catch (const CudaError& e) {
+    if (e.status != 101) throw;
+    return;  // no room: the transforms need no planes
+  }
+  uint8_t* planes = reinterpret_cast<uint8_t*>(keys->planes.p);
+  double* cc = reinterpret_cast<double*>(keys->consts.p);
+  for (int k = 0; k < K; ++k) {
+    const CtStep st = ct_step(n1, 1 << k);
+    k_ct_planes<<<plane_blocks(st), 256, 0, s.stream>>>(s.cascade_eval.p + k * step_len, st, s.r1, inv0, inv1, planes);
     VIA_LAUNCHED();
     for (int many = 0; many < 2; ++many) {
       const CtStep c = ct_step(n1, 1 << k, many ? CT_MANY : 1);
@@ -534,13 +542,14 @@ void ct_prepare(Server& s) {
                                                                              cc + many * consts);
       VIA_LAUNCHED();
     }
-    planes += (size_t)2 * st.units * st.chunks * CT_STAGE_B;
+    planes += plane_bytes(st);
     cc += (size_t)2 * st.units * 2 * CT_ROWS;
   }
-  s.ct_steps = K;
+  keys->steps = K;
+  std::atomic_store(&s.ct, std::shared_ptr<const CtKeys>(std::move(keys)));
 }
 
-void ct_run(Server& s, const u64* d_query, long nlwe, uint8_t* da, uint8_t* db, int8_t* dig8, u64* body,
+void ct_run(Server& s, const CtKeys& keys, const u64* d_query, long nlwe, uint8_t* da, uint8_t* db, int8_t* dig8, u64* body,
             cudaStream_t st) {
   const via_params& p = s.prm;
   const int n1 = (int)p.n1;
@@ -551,8 +560,8 @@ void ct_run(Server& s, const u64* d_query, long nlwe, uint8_t* da, uint8_t* db, 
   k_ct_digits<<<(unsigned)((threads + 255) / 256), 256, 0, st>>>(d_query, nlwe, (long)lwe_len(p), n1, cur, D,
                                                                 (size_t)CT_M * cur.half * cur.kp, da);
   VIA_LAUNCHED();
-  size_t b_off = 0, c_off = mtiles >= CT_MANY ? s.ct_consts.n / 2 : 0;
-  const int steps = ct_steps_for(s.ct_steps, nlwe);
+  size_t b_off = 0, c_off = mtiles >= CT_MANY ? keys.consts.n / 2 : 0;
+  const int steps = ct_steps_for(keys.steps, nlwe);
   for (int k = 0; k < steps; ++k) {
     const CtStep nxt = ct_step(n1, 2 << k, mtiles);
     const bool last = k + 1 == steps;
@@ -560,8 +569,8 @@ void ct_run(Server& s, const u64* d_query, long nlwe, uint8_t* da, uint8_t* db, 
     P.st = cur;
     P.D = D;
     P.a = da;
-    P.b = reinterpret_cast<const uint8_t*>(s.ct_planes.p) + b_off;
-    P.c = reinterpret_cast<const double*>(s.ct_consts.p) + c_off;
+    P.b = reinterpret_cast<const uint8_t*>(keys.planes.p) + b_off;
+    P.c = reinterpret_cast<const double*>(keys.consts.p) + c_off;
     P.out = last ? nullptr : db;
     P.dig8 = dig8;
     P.body = body + ((2L << k) - 2) * 2 * nlwe;

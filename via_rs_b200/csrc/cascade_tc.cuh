@@ -145,17 +145,18 @@ inline int ct_steps(const via_params& p) { return ilog2(p.n1) - 1 < 8 ? ilog2(p.
 // its 189 MB of planes serve enough of them (2688 LWEs: 513 us against 1370 us in the four
 // transform kernels, 180 LWEs 59 against 95; one query's 42 against 26).
 inline int ct_steps_for(int prepared, long nlwe) { return prepared > 7 && nlwe <= CT_M ? 7 : prepared; }
-// Builds the key planes and column constants from the coefficient-form cascade key.
+// Builds s.ct from the coefficient-form cascade key; leaves it null where the steps do not serve
+// the server or its memory does not hold them.
 void ct_prepare(Server& s);
 // Raises the kernel's shared-memory limit on the current device.
 void ct_prepare_device();
-// Runs the leading ct.steps steps for nlwe LWEs of d_query ([lwe][nl (n1 + 1)]): leaves the
+// Runs the leading steps for nlwe LWEs of d_query ([lwe][nl (n1 + 1)]): leaves the
 // next step's signed digits in dig8 ([lwe][rank][L][degree]) and adds every step's body
 // sums (coefficient form) to body[((2 n - 2 + y) * 2 + limb) * nlwe + lwe] (n the step's
 // input degree, y < 2 n; ct_body_words(steps) words per LWE, zeroed by the caller), so that
 // the lanes of a warp, which are LWEs, add to consecutive words. da and db are
 // digit buffers of ct_digit_bytes(n1) bytes per LWE, LWEs rounded up to 8.
-void ct_run(Server& s, const u64* d_query, long nlwe, uint8_t* da, uint8_t* db, int8_t* dig8, u64* body,
+void ct_run(Server& s, const CtKeys& keys, const u64* d_query, long nlwe, uint8_t* da, uint8_t* db, int8_t* dig8, u64* body,
             cudaStream_t st);
 inline size_t ct_body_words(int steps) { return (((size_t)2 << steps) - 2) * 2; }
 

@@ -881,7 +881,8 @@ struct Workspace {
   int bmax = 1;              // queries the buffers are sized for
   // Cascade.
   DevBuf c_masks_a, c_masks_b, c_body_a, c_body_b, c_digits, c_P, c_bsum, c_rlwe;
-  DevBuf c_gemm_body;  // body sums of the GEMM steps (cascade_tc.cuh)
+  std::shared_ptr<const CtKeys> ct;  // the GEMM steps' keys (cascade_tc.cuh), null: none
+  DevBuf c_gemm_body;                // their body sums
   DevBuf c_dig8;   // 8-bit cascade / conversion-key digits [lwe][n1 * L_CK] bytes (base <= 255)
   // RLWE -> RGSW.
   // RGSWs grouped by use: the DMux bits of every query ([q][nd]), then the
@@ -979,11 +980,12 @@ static size_t workspace_build(Server& s, int bmax, Workspace* w, bool count_only
   // NTT rings transform the cascade digits at the input degree (half of the
   // embedded degree); the other rings use the embedded digits and the P buffer.
   // The GEMM steps' two digit buffers lie in the same memory.
-  const long tc_words = s.ct_steps ? 2 * (long)(ct_digit_bytes((int)n1) / 8) * ((nlwe + 7) / 8 * 8) : 0;
+  w->ct = std::atomic_load(&s.ct);
+  const long tc_words = w->ct ? 2 * (long)(ct_digit_bytes((int)n1) / 8) * ((nlwe + 7) / 8 * 8) : 0;
   A(w->c_digits, std::max(nlwe * (s.r1.ntt ? 1 : 2) * n1 * Lck * nl, tc_words));
   A(w->c_P, s.r1.ntt ? 0 : nlwe * 2 * n1 * 2 * nl);
   A(w->c_bsum, 2 * nlwe * n1 * nl);
-  A(w->c_gemm_body, s.ct_steps ? (long)ct_body_words(s.ct_steps) * nlwe : 0);
+  A(w->c_gemm_body, w->ct ? (long)ct_body_words(w->ct->steps) * nlwe : 0);
   A(w->c_dig8, p.ck_base <= 255 && s.r1.ntt ? (nlwe * n1 * Lck + 7) / 8 : 0);
   A(w->c_rlwe, nlwe * 2 * n1 * nl);
   A(w->g_digits, nlwe * Lck * nl * n1);
@@ -1031,7 +1033,21 @@ static size_t workspace_build(Server& s, int bmax, Workspace* w, bool count_only
 
 std::unique_ptr<Workspace, WorkspaceDeleter> workspace_make(Server& s, int bmax) {
   std::unique_ptr<Workspace, WorkspaceDeleter> w(new Workspace());
-  workspace_build(s, bmax, w.get(), false);
+  bool built = true;
+  try {
+    workspace_build(s, bmax, w.get(), false);
+  } catch (const CudaError& e) {
+    if (e.status != 101) throw;
+    w.reset(new Workspace());
+    const size_t need = workspace_bytes(s, bmax) + ((size_t)96 << 20);  // about 48 allocations in pieces of 2 MiB
+    size_t avail = 0, total = 0;
+    VIA_CUDA(cudaMemGetInfo(&avail, &total));
+    const std::shared_ptr<const CtKeys> ct = std::atomic_load(&s.ct);
+    if (!ct || ct.use_count() > 2 || avail + ct->planes.n * 8 < need) throw;  // 2: the handle's and this one
+    std::atomic_store(&s.ct, std::shared_ptr<const CtKeys>());
+    built = false;
+  }
+  if (!built) workspace_build(s, bmax, w.get(), false);
   // The answer's own kernels go before the side stream's, which have until the CMux tree: five
   // queries at 64 x 1024 reached the scan after 950 us when both groups' cascades shared the
   // SMs evenly, and after 787 us this way (1390 -> 1340 us an answer). A graph's kernels keep the priority of the stream they were
@@ -1148,8 +1164,8 @@ static void cascade_gemm(Server& s, Workspace& w, const u64* d_query, long nlwe,
   u64* body = w.c_gemm_body.p;
   uint8_t* da = reinterpret_cast<uint8_t*>(w.c_digits.p);
   uint8_t* db = da + ct_digit_bytes((int)n1) * ((nlwe + 7) / 8 * 8);
-  VIA_CUDA(cudaMemsetAsync(body, 0, ct_body_words(ct_steps_for(s.ct_steps, nlwe)) * nlwe * 8, st));
-  ct_run(s, d_query, nlwe, da, db, reinterpret_cast<int8_t*>(w.c_dig8.p), body, st);
+  VIA_CUDA(cudaMemsetAsync(body, 0, ct_body_words(ct_steps_for(w.ct->steps, nlwe)) * nlwe * 8, st));
+  ct_run(s, *w.ct, d_query, nlwe, da, db, reinterpret_cast<int8_t*>(w.c_dig8.p), body, st);
 }
 
 static void query_decomp_range(Server& s, Workspace& w, const u64* d_query, long nlwe_all, long lwe0, long nlwe,
@@ -1169,7 +1185,7 @@ static void query_decomp_range(Server& s, Workspace& w, const u64* d_query, long
   u64* rlwe = w.c_rlwe.p + lwe0 * 2 * lwe_n;
   // Bases up to 255: digits as bytes, lifted and transformed by the 8-bit NTT.
   int8_t* dig8 = w.c_dig8.p ? reinterpret_cast<int8_t*>(w.c_dig8.p) + lwe0 * (long)n1 * L : nullptr;
-  const int k0 = ct_steps_for(s.ct_steps, nlwe_all);  // steps already run as GEMMs
+  const int k0 = w.ct ? ct_steps_for(w.ct->steps, nlwe_all) : 0;  // steps already run as GEMMs
   const u64* query = d_query + lwe0 * (long)lwe_len(p);
   if (!k0) {
     k_lwe_to_mlwe<<<blocks(nlwe * nl * (n1 + 1)), 256, 0, st>>>(query, n1, nl, nlwe, mi, bi);
@@ -2080,7 +2096,7 @@ void answer_device_stages(Server& s, Workspace& w, const u64* d_query, int nq, u
   }
   u64* const rgsw_b1 = w.rgsw_q1.p + B * nd * rgsw1;  // the CMux / CRot bits' group
   u64* const rgsw_b2 = w.rgsw_q2.p + B * nd * rgsw2;
-  if (s.ct_steps) cascade_gemm(s, w, qsrc, nlwe_all, st);
+  if (w.ct) cascade_gemm(s, w, qsrc, nlwe_all, st);
   // Answers that run to the end expand the CMux / CRot bits (the rest of their cascades,
   // RGSWs and q1 -> q2 switch) on the side stream while the DMux tree and the
   // database scan run on `st`; `st` waits for them before the CMux tree. The

@@ -67,6 +67,12 @@ class ScratchLease {
   DevBuf own_;
 };
 
+// The cascade's leading steps as GEMMs (cascade_tc.cuh): their key planes and column constants.
+struct CtKeys {
+  DevBuf planes, consts;
+  int steps = 0;
+};
+
 struct Workspace;  // per-query scratch (pipeline.cu)
 struct WorkspaceDeleter {
   void operator()(Workspace* w) const;
@@ -90,10 +96,9 @@ struct Server {
   // Eval-form keys (crates/via-server/src/prepared_keys.rs:69-79).
   DevBuf cascade_eval;  // include/via_gpu.h cascade layout, each segment transformed
   DevBuf cascade_eval_d;  // the same residues as exact doubles (q1 primes below 2^44), for the double-precision MAC
-  // The cascade's leading steps as GEMMs (cascade_tc.cuh): their key planes and column
-  // constants; ct_steps of them (0: none).
-  DevBuf ct_planes, ct_consts;
-  int ct_steps = 0;
+  // The cascade's leading steps as GEMMs, or null: every step on transforms. Workspaces keep
+  // the ones they were made with. Read and replaced with std::atomic_load / atomic_store: a service makes its workspaces without `mu`.
+  std::shared_ptr<const CtKeys> ct;
   DevBuf conv_eval;     // L_CK samples at (q1, n1)
   DevBuf rsk_eval;      // d RLevs at (q3, n2)
   // VIA-B repack keys (n_rec < n2): the cascade steps of output degree 2 n_rec .. n1,
@@ -136,6 +141,8 @@ constexpr int VIA_B_CHUNK = 64;
 void derive_repack_keys(Server& s);
 void answer_batch_device(Server& s, const u64* d_queries, u64* d_mask, u64* d_body, cudaStream_t st);
 void workspace_create(Server& s, int bmax);
+// Where the memory lacks and the handle's GEMM key planes (nobody else's) would make up for it, they
+// go and the handle's cascades run on transforms from then on.
 std::unique_ptr<Workspace, WorkspaceDeleter> workspace_make(Server& s, int bmax);
 size_t workspace_bytes(Server& s, int bmax);  // device bytes of a workspace for bmax queries
 u64* ws_query(Workspace& w);
