@@ -1,5 +1,5 @@
 """The key planes of the cascade's GEMM steps take 409 MB a key set at degree 2048: a handle that
-lacks the memory does without them."""
+lacks the memory does without them, and views of one key share them."""
 import numpy as np
 import pytest
 
@@ -68,3 +68,31 @@ def test_reserve_without_room_beside_the_planes(oracle):
     del filler
     _free(torch)
     assert np.array_equal(got[0], want[0]) and np.array_equal(got[1], want[1])
+
+
+def test_views_share_planes_of_one_key(oracle):
+    import torch
+
+    prm = paper_preset(2, 4)
+    pv = prm.with_dims(prm.num_rows, prm.num_cols, 256)
+    c, recs, keys = _setup(oracle, prm)
+    cv, _, vkeys = _setup(oracle, pv)
+    co, _, okeys = _setup(oracle, prm, b"other")
+    base = Server.setup(prm, keys, recs)
+    cells = recs.reshape(prm.n1 // prm.n_rec, -1, prm.n_rec).transpose(1, 2, 0).reshape(-1, prm.n1)
+    d = prm.n1 // pv.n_rec
+    vrecs = np.concatenate([cells[:, k::d] for k in range(d)])
+    free = [_free(torch)]
+    view = base.view(256, vkeys)
+    free.append(_free(torch))
+    other = base.view(prm.n2, okeys)
+    free.append(_free(torch))
+    assert np.array_equal(c.cascade_key, cv.cascade_key) and not np.array_equal(c.cascade_key, co.cascade_key)
+    assert free[0] - free[1] < PLANES < free[1] - free[2]
+    base.close()  # what it lent stays
+    idx = [1, prm.capacity - 1]
+    m, b = view.answer_batch(cv.batch_query(idx, b"v"))
+    for t, rec in enumerate(cv.recover_batch(m, b)):
+        assert np.array_equal(rec, vrecs[idx[t]])
+    q = co.query(7, b"o")
+    assert np.array_equal(co.recover(*other.answer(q)), recs[7])

@@ -380,9 +380,10 @@ __global__ void __launch_bounds__(CT_THREADS, 1) k_ct_step(const __grid_constant
 
 // Key planes of one step: thread = (unit, 16 K bytes, limb, row), five 16-byte core-matrix
 // rows each. key: the step's coefficient-form samples [R][L][2][2][n_out]. Mask entries
-// are -K (Q / q_l)^-1 mod q_l, body entries K.
+// are -K (Q / q_l)^-1 mod q_l, body entries K. CHECK: sets *differs where `planes` holds others.
+template <bool CHECK>
 __global__ void k_ct_planes(const u64* __restrict__ key, CtStep st, DevRing R, u64 inv0, u64 inv1,
-                            uint8_t* __restrict__ planes) {
+                            uint8_t* __restrict__ planes, int* differs) {
   const long gid = (long)blockIdx.x * blockDim.x + threadIdx.x;
   const int k16s = st.chunks * (CT_KC / 16);
   if (gid >= (long)2 * st.units * k16s * 32) return;
@@ -419,8 +420,13 @@ __global__ void k_ct_planes(const u64* __restrict__ key, CtStep st, DevRing R, u
 #pragma unroll
   for (int k = 0; k < 5; ++k) {
     const int row = (l * 5 + k) * CT_ROWS + r;
-    *reinterpret_cast<uint4*>(base + (row / 8) * 128 + (row % 8) * 16) =
-        make_uint4(word[k][0], word[k][1], word[k][2], word[k][3]);
+    uint4* at = reinterpret_cast<uint4*>(base + (row / 8) * 128 + (row % 8) * 16);
+    if (CHECK) {
+      const uint4 v = *at;
+      if (v.x != word[k][0] || v.y != word[k][1] || v.z != word[k][2] || v.w != word[k][3]) *differs = 1;
+    } else {
+      *at = make_uint4(word[k][0], word[k][1], word[k][2], word[k][3]);
+    }
   }
 }
 
@@ -503,7 +509,7 @@ void ct_prepare_device() {
   VIA_CUDA(cudaFuncSetAttribute(k_ct_step, cudaFuncAttributeMaxDynamicSharedMemorySize, CT_SMEM));
 }
 
-void ct_prepare(Server& s) {
+void ct_prepare(Server& s, const Server* base) {
   const via_params& p = s.prm;
   if (!ct_supported(p, s.r1) || !s.cascade_eval.p || !s.fd_err.p) return;
   const int K = ct_steps(p), n1 = (int)p.n1;
@@ -515,6 +521,26 @@ void ct_prepare(Server& s) {
   const auto plane_blocks = [](const CtStep& st) {
     return (unsigned)(((long)2 * st.units * st.chunks * (CT_KC / 16) * 32 + 255) / 256);
   };
+  const std::shared_ptr<const CtKeys> lent = base ? std::atomic_load(&base->ct) : nullptr;
+  if (lent) {
+    DevBuf differs(1);
+    VIA_CUDA(cudaMemsetAsync(differs.p, 0, 8, s.stream));
+    uint8_t* planes = reinterpret_cast<uint8_t*>(lent->planes.p);
+    for (int k = 0; k < K; ++k) {
+      const CtStep st = ct_step(n1, 1 << k);
+      k_ct_planes<true><<<plane_blocks(st), 256, 0, s.stream>>>(s.cascade_eval.p + k * step_len, st, s.r1, inv0, inv1,
+                                                                planes, reinterpret_cast<int*>(differs.p));
+      VIA_LAUNCHED();
+      planes += plane_bytes(st);
+    }
+    int other = 0;
+    VIA_CUDA(cudaMemcpyAsync(&other, differs.p, sizeof(int), cudaMemcpyDeviceToHost, s.stream));
+    VIA_CUDA(cudaStreamSynchronize(s.stream));
+    if (!other) {
+      std::atomic_store(&s.ct, lent);
+      return;
+    }
+  }
   size_t bytes = 0, consts = 0;
   for (int k = 0; k < K; ++k) {
     const CtStep st = ct_step(n1, 1 << k);
@@ -533,7 +559,8 @@ void ct_prepare(Server& s) {
   double* cc = reinterpret_cast<double*>(keys->consts.p);
   for (int k = 0; k < K; ++k) {
     const CtStep st = ct_step(n1, 1 << k);
-    k_ct_planes<<<plane_blocks(st), 256, 0, s.stream>>>(s.cascade_eval.p + k * step_len, st, s.r1, inv0, inv1, planes);
+    k_ct_planes<false><<<plane_blocks(st), 256, 0, s.stream>>>(s.cascade_eval.p + k * step_len, st, s.r1, inv0, inv1,
+                                                               planes, nullptr);
     VIA_LAUNCHED();
     for (int many = 0; many < 2; ++many) {
       const CtStep c = ct_step(n1, 1 << k, many ? CT_MANY : 1);

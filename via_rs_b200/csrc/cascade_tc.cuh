@@ -146,8 +146,8 @@ inline int ct_steps(const via_params& p) { return ilog2(p.n1) - 1 < 8 ? ilog2(p.
 // transform kernels, 180 LWEs 59 against 95; one query's 42 against 26).
 inline int ct_steps_for(int prepared, long nlwe) { return prepared > 7 && nlwe <= CT_M ? 7 : prepared; }
 // Builds s.ct from the coefficient-form cascade key; leaves it null where the steps do not serve
-// the server or its memory does not hold them.
-void ct_prepare(Server& s);
+// the server or its memory does not hold them. `base` (a view's) lends its own where they are equal.
+void ct_prepare(Server& s, const Server* base);
 // Raises the kernel's shared-memory limit on the current device.
 void ct_prepare_device();
 // Runs the leading steps for nlwe LWEs of d_query ([lwe][nl (n1 + 1)]): leaves the

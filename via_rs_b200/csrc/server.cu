@@ -228,7 +228,7 @@ static void transform_keys(Server& s) {
     ntt_forward(s.rsk_eval.p, p.n2, 1, (long)(p.n1 / p.n2) * p.l_rsk * 2, s.r3.t[0], s.r3.t[1], s.stream);
 }
 
-static void load_keys(Server& s, const via_public_keys* keys, bool planes) {
+static void load_keys(Server& s, const via_public_keys* keys, const Server* base, bool planes) {
   if (!keys) return;
   const via_params& p = s.prm;
   if (!keys->cascade_key || !keys->conv_key || !keys->rsk) throw ApiError(VIA_ERR_INVALID_ARGUMENT, "null key buffer");
@@ -239,15 +239,15 @@ static void load_keys(Server& s, const via_public_keys* keys, bool planes) {
   VIA_CUDA(cudaMemcpyAsync(s.conv_eval.p, keys->conv_key, s.conv_eval.n * 8, cudaMemcpyHostToDevice, s.stream));
   VIA_CUDA(cudaMemcpyAsync(s.rsk_eval.p, keys->rsk, s.rsk_eval.n * 8, cudaMemcpyHostToDevice, s.stream));
   derive_repack_keys(s);  // VIA-B: from the coefficient-form cascade key, before it is transformed
-  if (planes) ct_prepare(s);  // the GEMM steps' key planes, likewise
+  if (planes) ct_prepare(s, base);  // the GEMM steps' key planes, likewise
   transform_keys(s);
 }
 
 // The keys, and the workspace for one query. Where that does not fit the memory beside GEMM key
 // planes of the handle's own, it is done without them.
-static void load(Server& s, const via_public_keys* keys) {
+static void load(Server& s, const via_public_keys* keys, const Server* base) {
   try {
-    load_keys(s, keys, true);
+    load_keys(s, keys, base, true);
     workspace_create(s, 1);
     return;
   } catch (const CudaError& e) {
@@ -255,7 +255,7 @@ static void load(Server& s, const via_public_keys* keys) {
   }
   VIA_CUDA(cudaStreamSynchronize(s.stream));
   s.ct.reset();
-  load_keys(s, keys, false);
+  load_keys(s, keys, base, false);
   workspace_create(s, 1);
 }
 
@@ -341,7 +341,7 @@ static void setup(Server& s, const via_params& p, const via_public_keys* keys, c
   VIA_CUDA(cudaStreamSynchronize(s.stream));
   cells.free();
 
-  load(s, keys);
+  load(s, keys, nullptr);
   VIA_CUDA(cudaStreamSynchronize(s.stream));
 }
 
@@ -371,7 +371,7 @@ static void setup_view(Server& s, const Server& base, uint32_t n_rec, const via_
     VIA_CUDA(cudaMemsetAsync(s.fd_err.p, 0, 8, s.stream));
     s.fd.err = reinterpret_cast<int*>(s.fd_err.p);
   }
-  load(s, keys);
+  load(s, keys, &base);
   VIA_CUDA(cudaStreamSynchronize(s.stream));
 }
 

@@ -97,7 +97,8 @@ struct Server {
   DevBuf cascade_eval;  // include/via_gpu.h cascade layout, each segment transformed
   DevBuf cascade_eval_d;  // the same residues as exact doubles (q1 primes below 2^44), for the double-precision MAC
   // The cascade's leading steps as GEMMs, or null: every step on transforms. Workspaces keep
-  // the ones they were made with. Read and replaced with std::atomic_load / atomic_store: a service makes its workspaces without `mu`.
+  // the ones they were made with; views of the same cascade key share their base's. Read and
+  // replaced with std::atomic_load / atomic_store: a service makes its workspaces without `mu`.
   std::shared_ptr<const CtKeys> ct;
   DevBuf conv_eval;     // L_CK samples at (q1, n1)
   DevBuf rsk_eval;      // d RLevs at (q3, n2)
