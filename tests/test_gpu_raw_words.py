@@ -46,6 +46,7 @@ PRESETS = {
     # Key gadgets without GEMM steps: byte digits, 64-bit digits.
     "bytes": lambda: dataclasses.replace(paper_preset(2, 2), ck_base=21, l_ck=18),
     "words": lambda: dataclasses.replace(paper_preset(2, 2), ck_base=300, l_ck=9),
+    "degree_512": lambda: dataclasses.replace(paper_preset(2, 2), n1=512),  # its body has kernels of its own
 }
 
 
@@ -72,14 +73,13 @@ def test_query_words(oracle, preset, part):
     assert np.array_equal(gpu.debug_stage(raw.reshape(-1), 1), cpu.debug_stage(red.reshape(-1), 1))
 
 
-@pytest.mark.parametrize("primes,n,base,L", [(PAPER_Q1, 256, 55879, 2), (PAPER_Q1, 2048, 55879, 2),
-                                             ((PAPER_Q2,), 2048, 81, 2), (SECURE_Q1, 4096, 18073, 2)])
+@pytest.mark.parametrize("primes,n,base,L,count", [(PAPER_Q1, 256, 55879, 2, 3), (PAPER_Q1, 2048, 55879, 2, 3),
+                                                   ((PAPER_Q2,), 2048, 81, 2, 3), (SECURE_Q1, 4096, 18073, 2, 32)])
 @pytest.mark.parametrize("in_place", [False, True])
-def test_external_product_words(oracle, primes, n, base, L, in_place):
+def test_external_product_words(oracle, primes, n, base, L, count, in_place):
     import torch
 
     rng = np.random.default_rng(62)
-    count = 3
     rgsw, rgsw_red = _raw(rng, primes, count * 4 * L, n)
     ct, ct_red = _raw(rng, primes, count * 2, n)
     d_rgsw, d_ct = _dev(torch, rgsw), _dev(torch, ct)

@@ -1893,11 +1893,23 @@ static bool shared_key_fp(const DevRing& R, const int8_t* dig8, const u64* key, 
   return true;
 }
 
-// Runs k_external_fp; false (nothing launched) for rings and gadgets it does not serve, and for
-// outputs that overlap an input: its CTAs write one limb while others may still read.
+// CTAs from which k_external_fp runs whatever its gadget's depth. With fewer, a CTA's 3 L + 2 pairs of
+// transforms in a row take longer than separate kernels side by side, except for shallow gadgets of
+// small rings (us a call, fused and separate kernels; q1, two CTAs a product):
+//   degree 2048: L = 2, 1 product 53, 55; L = 4, 1 64, 51, 16 65, 60, 32 66, 74; L = 11, 1 123, 54,
+//     16 125, 77, 32 126, 116, 48 130, 151
+//   degree 4096: L = 2, 1 73, 60, 16 73, 68, 24 73, 74, 32 74, 80; L = 8, 16 167, 100, 48 171, 217
+//   degree 1024: L = 4, 1 46, 49; L = 8, 1 62, 51, 32 70, 68;  degree 256: L = 4, 1 42, 50; L = 8, 1 54, 48
+// The many: 1024 products of degree 2048, L = 11, 1211 fused and about 3500 before there was this kernel.
+constexpr long EXTERNAL_MIN = 64;
+
+// Runs k_external_fp; false (nothing launched) for rings and gadgets it does not serve, for few products
+// of a deep gadget (EXTERNAL_MIN), and for outputs that overlap an input: its CTAs write one limb
+// while others may still read.
 static bool external_fp(const DevRing& R, const Gadget& g, const u64* rgsw, const u64* cts, long count, u64* out,
                         cudaStream_t st) {
-  if (!R.ntt || !g.fp || !ntt_fp_ok(R.t[0], R.t[R.nl - 1]) || 2 * g.L > 256) return false;
+  if (!R.ntt || !g.fp || !ntt_fp_ok(R.t[0], R.t[R.nl - 1])) return false;
+  if ((g.L > 4 || g.L * R.n > 4096) && count * R.nl < EXTERNAL_MIN) return false;
   const size_t per = (size_t)R.nl * R.n, len = (size_t)count * 2 * per;
   const auto apart = [&](const u64* p, size_t words) { return out + len <= p || p + words <= out; };
   if (!apart(cts, len) || !apart(rgsw, len * 2 * g.L)) return false;
