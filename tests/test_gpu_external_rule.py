@@ -24,3 +24,24 @@ def test_both_sides(oracle, primes, n, base, L, count):
     prims.external_product_dev(prims.ring(n, primes), base, L, d[0].data_ptr(), d[1].data_ptr(), count, out.data_ptr())
     want = oracle.external_product(primes, n, base, L, rgsw.reshape(-1), ct.reshape(-1))
     assert np.array_equal(out.cpu().numpy().view(np.uint64).reshape(-1), want)
+
+
+def test_fused_products_take_no_scratch():
+    """A batch of the fused kernel runs in the memory its buffers leave (the separate kernels would want
+    1.5 times the RGSWs again)."""
+    import torch
+
+    n, L, count = 2048, 2, 2048
+    rgsw = torch.randint(0, min(PAPER_Q1), (count * 4 * L, 2, n), dtype=torch.int64, device="cuda")
+    ct = torch.randint(0, min(PAPER_Q1), (count * 2, 2, n), dtype=torch.int64, device="cuda")
+    out = torch.empty_like(ct)
+    ring = prims.ring(n, PAPER_Q1)
+    prims.external_product_dev(ring, 55879, L, rgsw.data_ptr(), ct.data_ptr(), 1, out.data_ptr())
+    want = out[:2].clone()
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    filler = torch.empty(torch.cuda.mem_get_info()[0] - (200 << 20), dtype=torch.uint8, device="cuda")
+    prims.external_product_dev(ring, 55879, L, rgsw.data_ptr(), ct.data_ptr(), count, out.data_ptr())
+    del filler
+    torch.cuda.empty_cache()
+    assert torch.equal(out[:2], want)

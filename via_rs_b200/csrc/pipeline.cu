@@ -1911,8 +1911,8 @@ constexpr long EXTERNAL_MIN = 64;
 // Runs k_external_fp; false (nothing launched) for rings and gadgets it does not serve, for few products
 // of a deep gadget (EXTERNAL_MIN), and for outputs that overlap an input: its CTAs write one limb
 // while others may still read.
-static bool external_fp(const DevRing& R, const Gadget& g, const u64* rgsw, const u64* cts, long count, u64* out,
-                        cudaStream_t st) {
+bool external_fp(const DevRing& R, const Gadget& g, const u64* rgsw, const u64* cts, long count, u64* out,
+                 cudaStream_t st) {
   if (!R.ntt || !g.fp || !ntt_fp_ok(R.t[0], R.t[R.nl - 1])) return false;
   if ((g.L > 4 || g.L * R.n > 4096) && count * R.nl < EXTERNAL_MIN) return false;
   const size_t per = (size_t)R.nl * R.n, len = (size_t)count * 2 * per;
@@ -2531,11 +2531,10 @@ void answer_batch_device(Server& s, const u64* d_queries, u64* d_mask, u64* d_bo
 // reference re-transforms its samples per call too, rlev.rs:211-219), then the
 // mask and body digits meet the neg_s_m and m samples.
 //   rgsw [count][2L][2][nl][n], cts/out [count][2][nl][n].
-// Scratch: rgsw_eval (count * 2L * 2 * nl * n), digits (count * 2L * nl * n).
+// For what external_fp declines. Scratch: rgsw_eval (count * 2L * 2 * nl * n), digits (count * 2L * nl * n).
 void prim_external_products(const DevRing& R, const Gadget& g, const u64* rgsw, const u64* cts, long count, u64* out,
                             u64* rgsw_eval, u64* digits, cudaStream_t st) {
   const long per = (long)R.nl * R.n;
-  if (external_fp(R, g, rgsw, cts, count, out, st)) return;
   VIA_CUDA(cudaMemcpyAsync(rgsw_eval, rgsw, (size_t)count * 2 * g.L * 2 * per * 8, cudaMemcpyDeviceToDevice, st));
   to_eval(R, rgsw_eval, R.n, count * 2 * g.L * 2 * R.nl, st);
   external_products(R, g, KeySel{rgsw_eval, 1, count, 0}, cts, count, digits, out, true, st);

@@ -19,6 +19,8 @@
 
 namespace via {
 
+bool external_fp(const DevRing& R, const Gadget& g, const u64* rgsw, const u64* cts, long count, u64* out,
+                 cudaStream_t st);
 void prim_external_products(const DevRing& R, const Gadget& g, const u64* rgsw, const u64* cts, long count, u64* out,
                             u64* rgsw_eval, u64* digits, cudaStream_t st);
 void prim_key_switches(const DevRing& R, const Gadget& g, const u64* key, const u64* cts, const u64* shifts, long count,
@@ -149,11 +151,13 @@ via_status via_external_product_dev(const via_ring_desc* ring, uint64_t base, ui
     std::lock_guard<std::mutex> g(g_mu);
     const DevRing& R = prim_ring(ring);
     const Gadget gd = prim_gadget(R, base, levels);
-    const size_t per = (size_t)R.nl * R.n;
-    const size_t ev = count * 2 * levels * 2 * per, dg = count * 2 * levels * per;
-    u64* s = prim_scratch(ev + dg);
     cudaStream_t st = (cudaStream_t)stream;
-    prim_external_products(R, gd, rgsw, rlwe, (long)count, out, s, s + ev, st);
+    if (!external_fp(R, gd, rgsw, rlwe, (long)count, out, st)) {
+      const size_t per = (size_t)R.nl * R.n;
+      const size_t ev = count * 2 * levels * 2 * per, dg = count * 2 * levels * per;
+      u64* s = prim_scratch(ev + dg);
+      prim_external_products(R, gd, rgsw, rlwe, (long)count, out, s, s + ev, st);
+    }
     VIA_CUDA(cudaStreamSynchronize(st));  // the scratch is reused by the next call
   });
 }
