@@ -4,11 +4,12 @@ import numpy as np
 import pytest
 
 from via_rs_b200.params import paper_preset
-from via_rs_b200.server import PublicKeys, Server
+from via_rs_b200.server import DeviceError, PublicKeys, Server
 
 pytestmark = pytest.mark.gpu
 
-PLANES = 406 << 20  # bytes, degree 2048
+PLANES = 406_000_000  # bytes, degree 2048 (and 3 MB of constants)
+VIA_ERR_OUT_OF_MEMORY = 101
 
 
 def _setup(oracle, prm, seed=b"key-planes"):
@@ -67,6 +68,26 @@ def test_reserve_without_room_beside_the_planes(oracle):
     gpu.close()
     del filler
     _free(torch)
+    assert np.array_equal(got[0], want[0]) and np.array_equal(got[1], want[1])
+
+
+def test_reserve_that_does_not_fit(oracle):
+    """The handle goes on answering with the workspace it had."""
+    import torch
+
+    prm = paper_preset(2, 4)
+    c, recs, keys = _setup(oracle, prm)
+    q = c.query(5, b"q")
+    gpu = Server.setup(prm, keys, recs)
+    want = gpu.answer(q)
+    filler = torch.empty(_free(torch) - (2 << 30), dtype=torch.uint8, device="cuda")
+    with pytest.raises(DeviceError) as e:
+        gpu.reserve(4096)
+    got = gpu.answer(q)
+    gpu.close()
+    del filler
+    _free(torch)
+    assert e.value.code == VIA_ERR_OUT_OF_MEMORY
     assert np.array_equal(got[0], want[0]) and np.array_equal(got[1], want[1])
 
 

@@ -546,12 +546,19 @@ via_status via_debug_stage(via_server* s, const uint64_t* query, uint64_t n_lwe,
   });
 }
 
-// Grows the workspace (and drops cached graphs) when a batch exceeds it.
+// Grows the workspace (and drops cached graphs) when a batch exceeds it. A batch that does not fit
+// leaves the handle with a workspace of the old size.
 static void ensure_batch(via_server* s, u64 nq) {
-  if ((int)nq <= workspace_batch(*s)) return;
+  const int had = workspace_batch(*s);
+  if ((int)nq <= had) return;
   VIA_CUDA(cudaStreamSynchronize(s->stream));
   workspace_destroy(*s);
-  workspace_create(*s, (int)nq);
+  try {
+    workspace_create(*s, (int)nq);
+  } catch (...) {
+    workspace_create(*s, std::max(had, 1));
+    throw;
+  }
 }
 
 via_status via_server_reserve(via_server* s, uint64_t max_queries) {
