@@ -31,6 +31,12 @@
  *               CMux bits LSB-first, CRot bits LSB-first, L_QUERY levels each).
  *      answer : ModSwitchedCiphertext<n2> = mask (n2 residues mod q3) then
  *               body (n2 residues mod q4).
+ *  - A query's words, and those of the primitives' ciphertexts, may be any 64
+ *    bits: they are taken mod their prime (a key switch's body words pass as
+ *    they are).
+ *  - The kernels of an answer have a priority one step above CUDA's default, on
+ *    whatever stream the answer is enqueued, and go before those of the
+ *    process's default-priority streams. Steps above are the caller's to use.
  *  - Status codes are the reference's ViaError discriminants + 1
  *    (crates/via-protocol/src/error.rs:20-64), then device-side codes.
  */

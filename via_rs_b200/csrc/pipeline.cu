@@ -1050,12 +1050,11 @@ std::unique_ptr<Workspace, WorkspaceDeleter> workspace_make(Server& s, int bmax)
   if (!built) workspace_build(s, bmax, w.get(), false);
   // The answer's own kernels go before the side stream's, which have until the CMux tree: five
   // queries at 64 x 1024 reached the scan after 950 us when both groups' cascades shared the
-  // SMs evenly, and after 787 us this way (1390 -> 1340 us an answer). A graph's kernels keep the priority of the stream they were
-  // captured on.
-  int least = 0, greatest = 0;
-  VIA_CUDA(cudaDeviceGetStreamPriorityRange(&least, &greatest));
-  VIA_CUDA(cudaStreamCreateWithPriority(&w->capture, cudaStreamNonBlocking, greatest));
-  VIA_CUDA(cudaStreamCreateWithPriority(&w->side, cudaStreamNonBlocking, least));
+  // SMs evenly, and after 787 us this way (1390 -> 1340 us an answer). A graph's kernels keep the
+  // priority of the stream they were captured on, whatever stream it is launched on.
+  const StreamPriorities prio = stream_priorities();
+  VIA_CUDA(cudaStreamCreateWithPriority(&w->capture, cudaStreamNonBlocking, prio.answer));
+  VIA_CUDA(cudaStreamCreateWithPriority(&w->side, cudaStreamNonBlocking, prio.side));
   VIA_CUDA(cudaEventCreateWithFlags(&w->ev_fork, cudaEventDisableTiming));
   VIA_CUDA(cudaEventCreateWithFlags(&w->ev_join, cudaEventDisableTiming));
   return w;

@@ -199,12 +199,14 @@ __global__ void k_u64_to_f64(const u64* __restrict__ in, double* __restrict__ ou
   if (gid < count) out[gid] = __ull2double_rn(in[gid]);
 }
 
-// The handle's stream, of the highest priority: its kernels go before those of the workspaces'
-// side streams.
-static void make_stream(Server& s) {
+StreamPriorities stream_priorities() {
   int least = 0, greatest = 0;
   VIA_CUDA(cudaDeviceGetStreamPriorityRange(&least, &greatest));
-  VIA_CUDA(cudaStreamCreateWithPriority(&s.stream, cudaStreamNonBlocking, greatest));
+  return {std::max(least - 1, greatest), least};
+}
+
+static void make_stream(Server& s) {
+  VIA_CUDA(cudaStreamCreateWithPriority(&s.stream, cudaStreamNonBlocking, stream_priorities().answer));
 }
 
 static void transform_keys(Server& s) {

@@ -132,6 +132,13 @@ u64 rsk_len(const via_params& p);
 int ilog2(u64 v);
 u64 h_inv(u64 a, u64 m);  // a^-1 mod m, 0 if not invertible
 
+// An answer's own kernels go one step before those of its side stream, which have the default
+// priority (CUDA's least): the other steps are left to the caller's streams.
+struct StreamPriorities {
+  int answer, side;
+};
+StreamPriorities stream_priorities();
+
 // Pipeline entry points (pipeline.cu).
 constexpr int STOP_AFTER_CROT = -1;  // answer_device_stages: leave the CRot outputs in the workspace
 // VIA-B batch size T = n2 / n_rec (the record-fit boundary); 1 for VIA-C servers.
