@@ -27,3 +27,15 @@ def test_cascade_and_answers(oracle, n1, queries):
     for k in {0, queries - 1}:
         m, b = cpu.answer(qs[k])
         assert np.array_equal(masks[k], m) and np.array_equal(bodies[k], b), k
+
+
+@pytest.mark.parametrize("base", [482, 509])  # the last gadget the fused CMux takes at this prime's size, and one past it
+def test_cmux_gadgets_at_the_scaling_line(oracle, base):
+    prm = dataclasses.replace(paper_preset(2, 8), q2=34_347_294_721, b_cmux=base)
+    recs = np.random.default_rng(base).integers(0, 16, size=(prm.capacity, prm.n_rec), dtype=np.uint64)
+    c = oracle.Client(prm, b"line-%d" % base)
+    gpu = Server.setup(prm, PublicKeys(c.cascade_key, c.conv_key, c.rsk), recs)
+    cpu = oracle.Server(prm, c.cascade_key, c.conv_key, c.rsk, recs)
+    q = c.query(prm.capacity - 1, b"q")
+    got, want = gpu.answer(q), cpu.answer(q)
+    assert np.array_equal(got[0], want[0]) and np.array_equal(got[1], want[1])

@@ -133,7 +133,7 @@ struct Gadget {
   double dS_over_Q, dQ;
   u128 Q, halfQ;
   u64 half_base;
-  bool small;     // Q * (S + 1) < 2^53: one limb, and the scaling is exact in doubles
+  bool small;     // Q (S + 1) < 8/9 2^53: one limb, and the scaling is exact in doubles (gadget_fp.cuh)
   // Exact integer scaling round(|c| S / Q):
   //  mode 0: one modulus Q < 2^64 with Q * S < 2^127: num = |c| S + floor(Q/2)
   //          fits 128 bits, one 128-by-64 division by Q;
@@ -177,7 +177,7 @@ inline Gadget make_gadget(u64 base, int L, u128 Q, u64 q0 = 0, u64 q1 = 0) {
   double dS = (double)(u64)(S >> 64) * 18446744073709551616.0 + (double)(u64)S;
   g.dS_over_Q = dS / g.dQ;
   g.half_base = base / 2;
-  g.small = Q < ((u128)1 << 53) && S < ((u128)1 << 53) && Q * (S + 1) < ((u128)1 << 53);
+  g.small = Q < ((u128)1 << 53) && S < ((u128)1 << 53) && 9 * Q * (S + 1) < 8 * ((u128)1 << 53);
   // Exact integer scaling mode (see the struct). (long double) products only
   // decide the mode; the arithmetic itself is exact.
   const long double lS = (long double)(u64)(S >> 64) * 18446744073709551616.0L + (long double)(u64)S;
@@ -235,7 +235,7 @@ __host__ __device__ __forceinline__ u64 div64by64(u64 n, const Div64& D, u64& re
 // floor((|c| B^L + floor(Q/2)) / Q) with c's sign (gadget.rs:115-151,
 // wide.rs:145-153). The balanced digits (gadget.rs:168-190) depend only on
 // this value mod B^L.
-// A `small` gadget (one limb, Q (S + 1) < 2^53) has a 64-bit numerator and a
+// A `small` gadget (one limb, Q (S + 1) < 8/9 2^53) has a 64-bit numerator and a
 // result below S < 2^53, the single digit chunk.
 __host__ __device__ __forceinline__ u64 gadget_scaled_small(u64 a0, const Gadget& g) {
   const u64 Q = (u64)g.Q, hq = (u64)g.halfQ, S = (u64)g.S;

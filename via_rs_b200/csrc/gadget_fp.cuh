@@ -10,8 +10,9 @@
 
 namespace via {
 
-// One limb, Q (S + 1) < 2^53 (a small gadget): r S is exact and the product with the
-// rounded 1 / Q errs by less than half its distance from a tie. |r| <= 0.5625 Q.
+// One limb, Q S < 8/9 2^53 (a small gadget), |r| <= 9/16 Q: r S is exact, and its product with the
+// rounded 1 / Q, within 2^-53 of it in proportion, errs by less than 9/16 S 2^-53 < 1 / (2 Q), its
+// distance from a tie. (Not so up to 2^53: Q = 34347294721, S = 509^2, r = 0.537 Q misses.)
 __device__ __forceinline__ double fp_scaled(double r, double S, double qinv) {
   return __dadd_rn(__fma_rn(__dmul_rn(r, S), qinv, FP_ROUND), -FP_ROUND);
 }
