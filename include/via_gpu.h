@@ -229,9 +229,12 @@ via_status via_first_dim_scan_many_dev(via_server* s, const uint64_t* sel_eval, 
  * scans each, in two passes over the candidates) and keeps the candidate whose
  * faster pass is fastest; scans of other batch sizes use the entry
  * of the nearest tuned size above (else below) of the same kind (one query, or
- * a batch). With a cache_path, entries measured before for the same device,
- * ring degree, grid and modulus are read from that file instead of measured,
- * and new measurements are appended to it. Answer graphs captured before the
+ * a batch). Answers of many CMuxes have their scan write its columns in tiles
+ * for the CMux tree; such batch sizes are measured so, and the stand-alone scans
+ * above, which write plain columns, keep their default or a tile set for them.
+ * With a cache_path, entries measured before for the same device, ring degree,
+ * grid, modulus and layout are read from that file instead of measured, and new
+ * measurements are appended to it. Answer graphs captured before the
  * call are re-captured on next use. Servers on non-NTT rings have no tiles:
  * their entries report 0 candidates. `out` (may be NULL) receives one entry
  * per batch size. No counterpart in the reference, whose FirstDim is a

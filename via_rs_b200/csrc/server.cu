@@ -578,17 +578,18 @@ namespace via {
 // Scan autotuner: measures every candidate tile of the FirstDim scan for the
 // given batch sizes on this server's database and keeps the fastest. A cache
 // file (one line per measured configuration, keyed by device name, ring degree,
-// grid and modulus) lets later processes skip the measurement.
+// grid, modulus and output layout) lets later processes skip the measurement.
 namespace {
 
-std::string tune_key(const Server& s, int nq) {
+std::string tune_key(Server& s, int nq) {
   cudaDeviceProp prop{};
   VIA_CUDA(cudaGetDeviceProperties(&prop, s.device));
   std::string dev = prop.name;
   for (char& c : dev)
     if (c == ' ' || c == '\t') c = '_';
-  return "fd_tc/3 " + dev + " n=" + std::to_string(s.fd.n) + " I=" + std::to_string(s.fd.I) +
-         " J=" + std::to_string(s.fd.J) + " q=" + std::to_string(s.fd.m.q) + " nq=" + std::to_string(nq);
+  return "fd_tc/4 " + dev + " n=" + std::to_string(s.fd.n) + " I=" + std::to_string(s.fd.I) +
+         " J=" + std::to_string(s.fd.J) + " q=" + std::to_string(s.fd.m.q) + " nq=" + std::to_string(nq) +
+         (cmux_takes_tiles(s, nq) ? " out=tiled" : "");
 }
 
 struct CachedTile {
