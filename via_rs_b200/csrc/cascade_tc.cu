@@ -182,7 +182,7 @@ __global__ void __launch_bounds__(CT_THREADS, 1) k_ct_step(const __grid_constant
       int s = 0, a = 0;
       u32 ph = 0, aph = 0;
       bool ok = true;
-      const u32 idesc = idesc_i8(CT_N, false);
+      const u32 idesc = idesc_u8(CT_N);
       constexpr u32 lbo_b = CT_N / 8 * 128;
       for (int it = blockIdx.x; ok && it < items; it += gridDim.x) {
         const long left = P.nlwe - (long)(it % P.mtiles) * CT_M;
@@ -490,7 +490,8 @@ CtDigits ct_digits(u64 base, const DevRing& R) {
 }
 
 // Two-prime NTT rings, primes of 26 to 40 bits (five bytes; a quotient of T y / q fits the low
-// word), gadgets of 18 digits with B^6 < 2^26 (a piece's arithmetic fits 32 bits).
+// word), gadgets of 18 digits with B^6 < 2^26 (a piece's arithmetic fits 32 bits; B up to 20, and
+// the test on B alone keeps B^6 within 64 bits).
 bool ct_digits_ok(u64 base, u32 L, const DevRing& R) {
   if (!R.ntt || R.nl != 2 || L != CT_L || base < 3 || base > 255) return false;
   u64 T = 1;

@@ -172,7 +172,7 @@ __global__ void __launch_bounds__(fd_threads(EPI), 1) k_fd_tc(KParams P) {
       u32 ph = 0, aph = 0;
       bool ok = true;
       const u32 lbo_a = (FD_MT / 8) * 128, lbo_b = (u32)(P.Np / 8) * 128;
-      const u32 idesc = idesc_i8(P.Np, false);
+      const u32 idesc = idesc_u8(P.Np);
       const u32 zero_addr = smem_addr(zero_tile);
       for (int u = blockIdx.x; ok && u < units; u += gridDim.x) {
         for (int jt = 0; ok && jt < P.n_jt; ++jt) {

@@ -182,8 +182,8 @@ __device__ __forceinline__ void st_slots(u64* p, const u64 (&x)[NS]) {
 // k_mac_ntt in double precision, for primes below 2^44 (ntt_fp.cuh): digits below 2 q, key
 // residues below q, every product within 0.5625 q. NS slots a thread: two (16-byte accesses)
 // once that leaves two blocks a SM. Bound by the digit and key bytes where each output has
-// its own key: 4099 external products at q1 490 us in 128-bit integers, 303 us here
-// (6.2 TB/s).
+// its own key, as external products in place: 4099 of them at q1 490 us in 128-bit integers, 303 us
+// here (6.2 TB/s).
 template <int NS>
 __global__ void __launch_bounds__(256, NS == 1 ? 2 : 4) k_mac_fp(const u64* __restrict__ D, KeySel ks, u64* __restrict__ out, int T,
                                                 int n, int nl, long nout, const __grid_constant__ DevRing R) {
@@ -797,8 +797,8 @@ __global__ void k_pack_rlwe(const u64* masks, const u64* body, const u64* __rest
 // steps' sums are loaded by one thread a coefficient that has any, all loads at once, while the
 // transform has its own to wait for (one after the other in the epilogue 338 us of the 360 below
 // stayed). 2688 LWEs of degree 2048 in 2 launches 360 us as three kernels (eval body, transform,
-// assembly), 155 here, which is memory: 64 KB in and 64 KB out an LWE at 2.3 TB/s; 60 LWEs 27 us
-// before, 16 here; 8 LWEs 15 and 9.5.
+// assembly), 155 here: 64 KB in and 64 KB out an LWE at 2.3 TB/s, 35% of the copy bandwidth, as every
+// CTA is a chain of loads, one transform and stores; 60 LWEs 27 us before, 16 here; 8 LWEs 15 and 9.5.
 template <int LOGN>
 __global__ void __launch_bounds__((1 << LOGN) / 8)
     k_cascade_rlwe_fp(const u64* __restrict__ masks, const u64* __restrict__ b0, long b0_stride,
@@ -1073,9 +1073,9 @@ int workspace_batch(Server& s) { return s.ws ? s.ws->bmax : 0; }
 static void to_eval(const DevRing& R, u64* data, int n, long segments, cudaStream_t st) {
   if (R.ntt) ntt_forward(data, n, R.nl, segments, R.t[0], R.t[1], st);
 }
-// Eval form of gadget digits: the lazy forward transform (outputs below
-// (1 + 2 log2 n) q < 2^44 for q < 2^40, n <= 4096); their consumers add at most
-// a few dozen products with key residues below q into 128-bit sums.
+// Eval form of gadget digits: the lazy forward transform, whose outputs are below 2 q on doubles
+// (primes below 2^44, what k_mac_fp wants) and below (1 + 2 log2 n) q in integers; k_mac_ntt adds at
+// most a few dozen products with key residues below q into 128-bit sums.
 static void digits_to_eval(const DevRing& R, u64* data, int n, long segments, cudaStream_t st) {
   if (R.ntt) ntt_forward_lazy(data, n, R.nl, segments, R.t[0], R.t[1], st);
 }

@@ -82,11 +82,8 @@ __device__ __forceinline__ u64 smem_desc(u32 addr, u32 lbo, u32 sbo) {
          (1ull << 46);
 }
 
-// kind::i8 instruction descriptor: K-major A (unsigned, or signed with a_signed)
-// and unsigned B, S32 accumulator, M = 128.
-__device__ __forceinline__ u32 idesc_i8(int n, bool a_signed) {
-  return (2u << 4) | (a_signed ? 1u << 7 : 0u) | ((u32)(n >> 3) << 17) | ((u32)(128 >> 4) << 24);
-}
+// kind::i8 instruction descriptor: unsigned A and B, K-major, S32 accumulator, M = 128.
+__device__ __forceinline__ u32 idesc_u8(int n) { return (2u << 4) | ((u32)(n >> 3) << 17) | ((u32)(128 >> 4) << 24); }
 
 __device__ __forceinline__ void mma_i8(u32 d_tmem, u64 adesc, u64 bdesc, u32 idesc, u32 accumulate) {
   asm volatile(
