@@ -41,6 +41,20 @@ def test_wire_answer_reports_the_wait(oracle):
     assert np.array_equal(got[0], want[0]) and np.array_equal(got[1], want[1])
 
 
+def test_batched_scan_reports_the_wait(oracle):
+    import torch
+
+    prm = paper_preset(4, 8)
+    _, gpu, _ = _setup(oracle, prm)
+    sel = torch.zeros(2 * prm.num_rows * 2 * prm.n1, dtype=torch.int64, device="cuda")
+    out = torch.empty(2 * prm.num_cols * 2 * prm.n1, dtype=torch.int64, device="cuda")
+    gpu.set_scan_fault(2000)
+    _times_out(lambda: gpu.scan_many_dev(sel.data_ptr(), 2, out.data_ptr()))
+    gpu.set_scan_fault(0)
+    gpu.scan_many_dev(sel.data_ptr(), 2, out.data_ptr())
+    assert not out.any()
+
+
 @pytest.mark.parametrize("queries", [1, 17])  # 8 and 136 LWEs: part of one tile, two tiles
 def test_cascade_wait_runs_out_and_handle_recovers(oracle, queries):
     prm = paper_preset(2, 2, 512)

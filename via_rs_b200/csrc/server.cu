@@ -481,6 +481,7 @@ via_status via_first_dim_scan_many_dev(via_server* s, const uint64_t* sel_eval, 
     first_dim_queries(*s, sel_eval, out_eval, (int)n_queries, reinterpret_cast<uint8_t*>(scratch.p),
                       (cudaStream_t)stream);
     VIA_CUDA(cudaStreamSynchronize((cudaStream_t)stream));  // scratch is freed on return
+    check_device_flags(*s, (cudaStream_t)stream);
   });
 }
 
