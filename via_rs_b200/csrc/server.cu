@@ -71,10 +71,9 @@ void DevBuf::free() {
 }
 
 std::string device_flags(Server& s, cudaStream_t st) {
-  if (!s.fd_err.p) return "";
   int flag = 0;
-  VIA_CUDA(cudaMemcpyAsync(&flag, s.fd_err.p, sizeof(int), cudaMemcpyDeviceToHost, st));
-  VIA_CUDA(cudaStreamSynchronize(st));
+  if (s.fd_err.p) VIA_CUDA(cudaMemcpyAsync(&flag, s.fd_err.p, sizeof(int), cudaMemcpyDeviceToHost, st));
+  VIA_CUDA(cudaStreamSynchronize(st));  // servers without the word too: the caller's outputs are on their way
   return flag ? device_flag_text(flag) : "";
 }
 std::string device_flag_text(int flag) {
