@@ -139,7 +139,7 @@ CtDigits ct_digits(u64 base, const DevRing& R);
 // Whether the GEMM steps serve this server's cascade.
 bool ct_supported(const via_params& p, const DevRing& R);
 // Leading steps prepared as GEMMs: input degrees 1 .. 128 (the last cascade step stays on
-// transforms). Their key planes take 406 MB at n1 = 2048.
+// transforms). Their key planes take 409 MB at n1 = 2048, 818 MB at 4096.
 inline int ct_steps(const via_params& p) { return ilog2(p.n1) - 1 < 8 ? ilog2(p.n1) - 1 : 8; }
 // Steps run as GEMMs for nlwe LWEs, of `prepared`: input degree 128 from two tiles on, where
 // its 189 MB of planes serve enough of them (2688 LWEs: 513 us against 1370 us in the four
