@@ -8,7 +8,7 @@ import pytest
 
 from via_rs_b200 import prims
 from via_rs_b200.client import Client
-from via_rs_b200.params import PAPER_Q1, PAPER_Q2, PAPER_Q3, SECURE_Q1, paper_preset, secure_preset
+from via_rs_b200.params import PAPER_Q1, PAPER_Q2, PAPER_Q3, SECURE_Q1, paper_preset, secure_preset, toy_preset
 from via_rs_b200.server import PublicKeys, Server
 
 pytestmark = pytest.mark.gpu
@@ -46,6 +46,8 @@ PRESETS = {
     # Key gadgets without GEMM steps: byte digits, 64-bit digits.
     "bytes": lambda: dataclasses.replace(paper_preset(2, 2), ck_base=21, l_ck=18),
     "words": lambda: dataclasses.replace(paper_preset(2, 2), ck_base=300, l_ck=9),
+    "wide": lambda: dataclasses.replace(paper_preset(2, 2), q1=(35184371884033, 35184371703809)),  # integer transforms
+    "toy": lambda: toy_preset(2, 2),  # no transforms
     "degree_512": lambda: dataclasses.replace(paper_preset(2, 2), n1=512),  # its body has kernels of its own
 }
 

@@ -81,9 +81,7 @@ __global__ void k_decompose_i8(const u64* __restrict__ in, int n_in, long npolys
   const int i = (int)(gid % n_in);
   const int nl = R.nl;
   const u64* src = in + p * nl * n_in;
-  u64 a0 = src[i], a1 = nl == 2 ? src[n_in + i] : 0;
-  if (a0 >= R.m[0].q) a0 = reduce64(a0, R.m[0]);  // a query's word may be any 64 bits
-  if (a1 >= R.m[1].q) a1 = reduce64(a1, R.m[1]);
+  const u64 a0 = src[i], a1 = nl == 2 ? src[n_in + i] : 0;
   int8_t* o = out + p * (long)g.L * n_in + (long)(g.L - 1) * n_in + i;
   for_each_digit(gadget_scaled(a0, a1, R, g), g, [&](int, i64 d) {
     *o = (int8_t)d;
@@ -512,8 +510,9 @@ __global__ void __launch_bounds__(256) k_mod_switch_fp(const u64* __restrict__ i
 // ---------------------------------------------------------------------------
 // Cascade (prim/conversion/cascade.rs + conv.rs:122-148) helpers.
 // ---------------------------------------------------------------------------
-// LWE [lwe][nl*(n1+1)] -> rank-n1 MLWE of degree 1: masks [lwe][idx][nl], body [lwe][nl].
-__global__ void k_lwe_to_mlwe(const u64* __restrict__ q, int n1, int nl, long nlwe, u64* masks, u64* body) {
+// LWE [lwe][nl*(n1+1)] -> rank-n1 MLWE of degree 1: masks [lwe][idx][nl], body [lwe][nl], residues of
+// the query's words (any 64 bits).
+__global__ void k_lwe_to_mlwe(const u64* __restrict__ q, int n1, int nl, long nlwe, DevRing R, u64* masks, u64* body) {
   long gid = (long)blockIdx.x * blockDim.x + threadIdx.x;
   long per = (long)nl * (n1 + 1);
   if (gid >= nlwe * per) return;
@@ -521,10 +520,10 @@ __global__ void k_lwe_to_mlwe(const u64* __restrict__ q, int n1, int nl, long nl
   int r = (int)(gid % per);
   if (r < nl * n1) {
     int l = r / n1, idx = r % n1;
-    masks[(w * n1 + idx) * nl + l] = q[w * per + r];
+    masks[(w * n1 + idx) * nl + l] = reduce64(q[w * per + r], R.m[l]);
   } else {
     int l = r - nl * n1;
-    body[w * nl + l] = q[w * per + r];
+    body[w * nl + l] = reduce64(q[w * per + r], R.m[l]);
   }
 }
 
@@ -752,7 +751,7 @@ __global__ void k_cascade_body_final(const u64* __restrict__ b0, long b0_stride,
   const u64* sk = bsk + ll * 2 * n1;
   u64 acc = 0;
   for (int k = k0; k < K; ++k) acc = addmod(acc, reduce64(sk[(2 << k) - 2 + (t >> (K - 1 - k))], m), m.q);
-  body[gid] = submod(b0[ll / nl * b0_stride + l], acc, m.q);
+  body[gid] = submod(reduce64(b0[ll / nl * b0_stride + l], m), acc, m.q);  // the caller's word after GEMM steps
 }
 
 // body_out[lwe] = embed_at(body_in[lwe], N_out, 0) - bsum[lwe] (coefficient form).
@@ -1112,8 +1111,7 @@ static void decompose(const DevRing& R, const Gadget& g, const u64* in, int n_in
 static bool shared_key_fp(const DevRing& R, const int8_t* dig8, const u64* key, const u64* bodies, int L, long count,
                           u64* out, cudaStream_t st);
 
-// Signed byte digits (bases up to 255). `in` is a 16-byte aligned buffer, and of canonical residues
-// where n_in is 4 or more.
+// Signed byte digits (bases up to 255); `in` is a 16-byte aligned buffer of canonical residues.
 static void decompose_i8(const DevRing& R, const Gadget& g, const u64* in, int n_in, long npolys, int8_t* out,
                          cudaStream_t st) {
   if (n_in >= 4 && ct_digits_ok(g.base, (u32)g.L, R))
@@ -1187,7 +1185,7 @@ static void query_decomp_range(Server& s, Workspace& w, const u64* d_query, long
   const int k0 = w.ct ? ct_steps_for(w.ct->steps, nlwe_all) : 0;  // steps already run as GEMMs
   const u64* query = d_query + lwe0 * (long)lwe_len(p);
   if (!k0) {
-    k_lwe_to_mlwe<<<blocks(nlwe * nl * (n1 + 1)), 256, 0, st>>>(query, n1, nl, nlwe, mi, bi);
+    k_lwe_to_mlwe<<<blocks(nlwe * nl * (n1 + 1)), 256, 0, st>>>(query, n1, nl, nlwe, R, mi, bi);
     VIA_LAUNCHED();
   }
   // Eval rings: how a step of input degree n_in spreads over the grid.
